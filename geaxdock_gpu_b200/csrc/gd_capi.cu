@@ -177,6 +177,19 @@ cudaMemPool_t ctx_pool(int device) {
   return g_pool[device];
 }
 
+void dfree(gd_ctx *c, void *p) {
+  for (auto *v : {&c->pool_allocs, &c->allocs}) {
+    auto it = std::find(v->begin(), v->end(), p);
+    if (it == v->end()) continue;
+    if (v == &c->pool_allocs)
+      cudaFreeAsync(p, c->stream);
+    else
+      cudaFree(p);
+    v->erase(it);
+    return;
+  }
+}
+
 int check_complex(const gd_complex_desc &d, int idx) {
   if (d.n_lig < 1 || d.n_prt < 1 || d.n_tmp < 1)
     return fail(GD_ERR_INVALID, "complex %d: n_lig/n_prt/n_tmp must be >= 1", idx);
@@ -850,6 +863,9 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   c->n_groups = goff;
   if ((rc = upload(c, &c->d_cx, dcx)) || (rc = upload(c, &c->d_group_base, group_base)))
     return bail(rc);
+  if ((rc = build_pocket_lists(c, dcx))) return bail(rc);
+  CK(cudaMemcpyAsync(c->d_cx, dcx.data(), sizeof(GdDevComplex) * dcx.size(),
+                     cudaMemcpyHostToDevice, c->stream));
 
   /* ---- replica state ---- */
   const int R = c->n_rep;

@@ -6,6 +6,7 @@
  *                       records and state (the reference's Run and launcher, src/run.cu:33-288,
  *                       src/kernel_cuda_lancher_siglegpu.cu)
  *   gd_capi_layout.cu   the device layout of one complex
+ *   gd_pocket.cu        the pocket grid's point lists of the short-range terms
  *   gd_capi_tile.cu     the tile, its autotuning, chains, RNG streams and the wait bound
  *   gd_capi_stream.cu   records downloaded while the run proceeds (gd_records_stream)
  *   gd_capi_eval.cu     pose energies, placed coordinates and the energy trace
@@ -206,6 +207,9 @@ int dalloc(gd_ctx *c, T **p, size_t n) {
   return GD_OK;
 }
 
+/* frees a buffer of dalloc before the context ends (stream-ordered) */
+void dfree(gd_ctx *c, void *p);
+
 template <class T>
 int upload(gd_ctx *c, T **p, const std::vector<T> &v) {
   int rc = dalloc(c, p, v.size());
@@ -259,6 +263,9 @@ void da_drop_graphs(gd_ctx *c);
  * thr: the contact thresholds [ligand type][point type] */
 int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1],
                    const gd_complex_desc &d, int ci, GdDevComplex &g);
+
+/* ---- the pocket grid's point lists (gd_pocket.cu) ---- */
+int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx);
 
 /* ---- allocation-free pose evaluation (gd_capi_noalloc.cu) ---- */
 int noalloc_prepare(int device);

@@ -141,10 +141,15 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
   {
     bool pt_used[GD_MAXTP1] = {false};
     for (int i = 0; i < d.n_prt * P; ++i) pt_used[d.prt_t[i]] = true;
-    float r2 = std::max(81.0f, f.near2);
+    float rc2 = f.near2;
     for (int tl = 0; tl < GD_MAXTP2; ++tl)
       for (int tp = 0; tp < GD_MAXTP1; ++tp)
-        if (lt_used[tl] && pt_used[tp]) r2 = std::max(r2, thr[tl][tp]);
+        if (lt_used[tl] && pt_used[tp]) rc2 = std::max(rc2, thr[tl][tp]);
+    const float r2 = std::max(81.0f, rc2);
+    /* the pocket grid's lists, with the same margin for the kernel's FP32 cell of an atom */
+    g.pg_rc = sqrtf(rc2) + 0.05f;
+    g.pg_rh = 9.0f + 0.05f;
+    for (int a = 0; a < 3; ++a) g.pg_org[a] = g.pocket[a] - 0.5f * GD_PG_N * GD_PG_EDGE;
     double lo[3] = {1e30, 1e30, 1e30}, hi[3] = {-1e30, -1e30, -1e30};
     for (int i = 0; i < d.n_prt * P; ++i) {
       const double v[3] = {d.prt_x[i], d.prt_y[i], d.prt_z[i]};
@@ -175,8 +180,8 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
     g.sr_n[1] = (int)n[1];
     g.sr_n[2] = (int)n[2];
     g.sr_n[3] = ncell;
-    sr_a.assign((size_t)d.n_prt * P, make_float4(0, 0, 0, 0));
-    sr_b.assign((size_t)d.n_prt * P, make_float4(0, 0, 0, 0));
+    sr_a.assign((size_t)d.n_prt * (P + 1), make_float4(1e6f, 1e6f, 1e6f, 0.0f));
+    sr_b.assign((size_t)d.n_prt * (P + 1), make_float4(0, 0, 0, 0));
     sr_start.assign((size_t)d.n_prt * (ncell + 1), 0);
     std::vector<int> cid(P);
     for (int pc = 0; pc < d.n_prt; ++pc) {
@@ -196,11 +201,11 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
       for (int p = 0; p < P; ++p) {
         const int i = fill[cid[p]]++;
         const int kind = (d.prt_hflag[o + p] == 1 ? 1 : 0) | (d.prt_c[o + p] == 2 ? 2 : 0);
-        sr_a[(size_t)o + i] =
+        sr_a[(size_t)o + pc + i] =
             make_float4(d.prt_x[o + p], d.prt_y[o + p], d.prt_z[o + p],
                         bits_as_float(d.prt_t[o + p] | (kind & 1 ? 256 : 0) |
                                       (kind & 2 ? 512 : 0)));
-        sr_b[(size_t)o + i] = make_float4((kind & 1) ? d.prt_hpp[o + p] : 0.0f,
+        sr_b[(size_t)o + pc + i] = make_float4((kind & 1) ? d.prt_hpp[o + p] : 0.0f,
                                           bits_as_float((kind & 2) ? d.prt_seq3r[o + p] : -1),
                                           d.prt_ele[o + p] * inv_el1, 0.0f);
       }
@@ -241,19 +246,28 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
       ref_start[(size_t)pc * (L + 1) + L] = (int)ref_pts.size();
     }
   }
+  /* KDE points sorted by ligand type, in their given order within a type */
   std::vector<float4> kde(std::max(1, d.pnk));
-  for (int i = 0; i < d.pnk; ++i)
-    kde[i] = make_float4(d.kde_x[i], d.kde_y[i], d.kde_z[i], (float)d.kde_t[i]);
+  std::vector<int> kde_start(GD_MAXTP2 + 1, 0);
+  for (int i = 0; i < d.pnk; ++i) ++kde_start[d.kde_t[i] + 1];
+  for (int t = 0; t < GD_MAXTP2; ++t) kde_start[t + 1] += kde_start[t];
+  {
+    std::vector<int> fill(kde_start.begin(), kde_start.end() - 1);
+    for (int i = 0; i < d.pnk; ++i)
+      kde[fill[d.kde_t[i]]++] = make_float4(d.kde_x[i], d.kde_y[i], d.kde_z[i], 0.0f);
+  }
   const size_t nm = (size_t)d.pos * d.mcs_ld;
-  std::vector<float> mx(d.mcs_x, d.mcs_x + nm), my(d.mcs_y, d.mcs_y + nm),
-      mz(d.mcs_z, d.mcs_z + nm), mt(d.mcs_tcc, d.mcs_tcc + d.pos);
+  std::vector<float4> mcs(nm);
+  for (size_t i = 0; i < nm; ++i) mcs[i] = make_float4(d.mcs_x[i], d.mcs_y[i], d.mcs_z[i], 0.0f);
+  std::vector<float> mt(d.mcs_tcc, d.mcs_tcc + d.pos);
   std::vector<float> psp(d.psp, d.psp + (size_t)GD_MAXTP2 * d.psp_ld);
   std::vector<float> mb(d.n_tmp);
   for (int t = 0; t < d.n_tmp; ++t) mb[t] = d.temp[t].minus_beta;
 
   float4 *p_lig_pos; int2 *p_lig_meta; float *p_lig_center; float4 *p_pt_a, *p_pt_b;
   float4 *p_sr_a, *p_sr_b; int *p_sr_start;
-  int4 *p_seg; int *p_seg_count; unsigned short *p_far_cnt; float4 *p_kde; float *p_mx, *p_my, *p_mz, *p_mt, *p_psp, *p_mb;
+  int4 *p_seg; int *p_seg_count; unsigned short *p_far_cnt; float4 *p_kde, *p_mcs; int *p_kde_start;
+  float *p_mt, *p_psp, *p_mb;
   int *p_ref_start; float4 *p_ref_pts;
   if ((rc = upload(c, &p_lig_pos, lig_pos)) || (rc = upload(c, &p_lig_meta, lig_meta)) ||
       (rc = upload(c, &p_lig_center, lig_center)) || (rc = upload(c, &p_pt_a, pt_a)) ||
@@ -261,8 +275,8 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
       (rc = upload(c, &p_sr_b, sr_b)) || (rc = upload(c, &p_sr_start, sr_start)) ||
       (rc = upload(c, &p_seg, seg)) || (rc = upload(c, &p_far_cnt, far_cnt)) ||
       (rc = upload(c, &p_seg_count, seg_count)) || (rc = upload(c, &p_kde, kde)) ||
-      (rc = upload(c, &p_mx, mx)) || (rc = upload(c, &p_my, my)) ||
-      (rc = upload(c, &p_mz, mz)) || (rc = upload(c, &p_mt, mt)) ||
+      (rc = upload(c, &p_kde_start, kde_start)) || (rc = upload(c, &p_mcs, mcs)) ||
+      (rc = upload(c, &p_mt, mt)) ||
       (rc = upload(c, &p_psp, psp)) || (rc = upload(c, &p_mb, mb)) ||
       (rc = upload(c, &p_ref_start, ref_start)) || (rc = upload(c, &p_ref_pts, ref_pts)))
     return rc;
@@ -273,7 +287,7 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
   g.pt_a = p_pt_a; g.pt_b = p_pt_b; g.seg = p_seg; g.seg_count = p_seg_count;
   g.far_cnt = p_far_cnt;
   g.sr_a = p_sr_a; g.sr_b = p_sr_b; g.sr_start = p_sr_start;
-  g.kde = p_kde; g.mcs_x = p_mx; g.mcs_y = p_my; g.mcs_z = p_mz; g.mcs_tcc = p_mt;
+  g.kde = p_kde; g.kde_start = p_kde_start; g.mcs = p_mcs; g.mcs_tcc = p_mt;
   g.psp = p_psp; g.minus_beta = p_mb; g.ref_start = p_ref_start; g.ref_pts = p_ref_pts;
   return GD_OK;
 }

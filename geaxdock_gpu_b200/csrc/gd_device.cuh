@@ -36,6 +36,10 @@
 #define GD_CELL 4.0f           /* edge of the short-range cell grid (A) */
 /* shared-memory bytes of the contact-threshold table at the front of the kernel's buffer */
 #define GD_THR_BYTES (GD_MAXTP2 * GD_MAXTP1 * 4)
+/* the pocket grid: GD_PG_N^3 cells of GD_PG_EDGE A, a 40 A cube centred on the pocket centre */
+#define GD_PG_N 10
+#define GD_PG_CELLS (GD_PG_N * GD_PG_N * GD_PG_N)
+#define GD_PG_EDGE 4.0f
 #define GD_MAX_CELLS (1 << 22) /* cells per conformer grid; a larger box widens the cells */
 #define GD_MAX_CELLS_ALL (1 << 25) /* cells of all conformers of a complex together */
 #define GD_MAX_TPB 256         /* threads per CTA: 3 CTAs of 256 fit the register file */
@@ -84,16 +88,25 @@ struct GdDevComplex {
    *   pt_a = (-x0, -x1, -y0, -y1), pt_b = (-z0, -z1, ele0 / el1, ele1 / el1) */
   const float4 *pt_a;
   const float4 *pt_b;
-  /* the cell list, [n_prt*pnp] points and [n_prt*(sr_n[3] + 1)] cell starts (conformer-local
+  /* the cell list, [n_prt*(pnp + 1)] points (the last of a conformer a sentinel far away) and [n_prt*(sr_n[3] + 1)] cell starts (conformer-local
    * point indices): sr_a = (x, y, z, bits of type | 256 if hydrophobic | 512 if class 2),
    * sr_b = (hpp, PSP column bits, ele / el1, 0) */
   const float4 *sr_a;
   const float4 *sr_b;
   const int *sr_start;
+  /* the pocket grid's point lists (gd_pocket.cu): cell c's contact list is pg_idx[pg_base[pc] +
+   * pg_start[s] ..) with s = pc (2 GD_PG_CELLS + 1) + 2 c, up to entry s + 1, its kind list from
+   * there to entry s + 2 (whole quads of indices into sr_a / sr_b) */
+  const unsigned short *pg_idx;
+  const int *pg_start;
+  const long long *pg_base;   /* [n_prt] */
+  float pg_org[3];
+  float pg_rc, pg_rh;         /* the lists' radii around a cell's box: contacts, hydrophobic */
   const int4 *seg;            /* [n_prt*GD_MAX_SEG] */
   const int *seg_count;       /* [n_prt] */
-  const float4 *kde;          /* [pnk] x, y, z, type (exact small integer as float) */
-  const float *mcs_x, *mcs_y, *mcs_z; /* [pos*mcs_ld] */
+  const float4 *kde;          /* [pnk] x, y, z, 0: sorted by type, in their given order within one */
+  const int *kde_start;       /* [GD_MAXTP2 + 1] the first KDE point of each ligand type */
+  const float4 *mcs;          /* [pos*mcs_ld] x, y, z, 0 (x invalid: GD_MCS_INVALID_COORD) */
   const float *mcs_tcc;       /* [pos] */
   const float *psp;           /* [GD_MAXTP2*psp_ld] */
   const float *minus_beta;    /* [n_tmp] */

@@ -296,8 +296,8 @@ __device__ __forceinline__ void short_range(const GdDevComplex &cx, int pc,
   const int z1 = min(nz - 1, (int)floorf((az + R - oz) * ic));
   if (y0 > y1 || z0 > z1) return;
   const int *__restrict__ st = cx.sr_start + (size_t)pc * (cx.sr_n[3] + 1);
-  const float4 *__restrict__ PA = cx.sr_a + (size_t)pc * cx.pnp;
-  const float4 *__restrict__ PB = cx.sr_b + (size_t)pc * cx.pnp;
+  const float4 *__restrict__ PA = cx.sr_a + (size_t)pc * (cx.pnp + 1);
+  const float4 *__restrict__ PB = cx.sr_b + (size_t)pc * (cx.pnp + 1);
   /* point range of row (iy, iz) within the remaining radius; empty when out of reach */
   auto bounds = [&](int iy, int iz, int &b0, int &b1) {
     b0 = b1 = 0;
@@ -363,6 +363,89 @@ __device__ __forceinline__ void short_range(const GdDevComplex &cx, int pc,
   }
 }
 
+/* The same terms for an atom inside the pocket grid, from its cell's two point lists
+ * (gd_pocket.cu): the same points' terms added in the same order as short_range with parts = 1.
+ * With parts > 1 (the S lanes of a split atom) lane `part` takes every parts-th quad. Bound by the
+ * latency of a load per point: four points are in flight, and a point past the end of a list
+ * is the sentinel. A warp's pass went from 87-135 k cycles (the row walk) to 20-34 k: 6,820
+ * replicas of 40 atoms on 3,000 points, 11 steps, 11.75 -> 9.64 ms with the epilogue's changes. */
+__device__ __forceinline__ void short_range_lists(const GdDevComplex &cx, int pc, int cell,
+                                                  const float *__restrict__ thr,
+                                                  const float *__restrict__ psprow,
+                                                  const GdForceConst &f, float ax, float ay,
+                                                  float az, int part, int parts, ShortSums &s) {
+  s.hsum = 0.0;
+  s.psp = 0.0f;
+  s.ele = 0.0f;
+  s.ncon = 0;
+  const int *__restrict__ st = cx.pg_start + (size_t)pc * (2 * GD_PG_CELLS + 1) + 2 * cell;
+  const int s0 = __ldg(st), s1 = __ldg(st + 1), s2 = __ldg(st + 2);
+  const ushort4 *__restrict__ ix =
+      reinterpret_cast<const ushort4 *>(cx.pg_idx + __ldg(cx.pg_base + pc));
+  const float4 *__restrict__ PA = cx.sr_a + (size_t)pc * (cx.pnp + 1);
+  const float4 *__restrict__ PB = cx.sr_b + (size_t)pc * (cx.pnp + 1);
+  for (int i = (s0 >> 2) + part; i < (s1 >> 2); i += parts) {
+    const ushort4 id = __ldg(ix + i);
+    const int k[4] = {id.x, id.y, id.z, id.w};
+    float4 p[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) p[u] = __ldg(PA + k[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float d2 = dist2(ax, ay, az, p[u].x, p[u].y, p[u].z);
+      s.ncon += d2 <= thr[__float_as_int(p[u].w) & 255] ? 1 : 0;
+      if (d2 < f.near2) {
+        const float e = __ldg(&PB[k[u]].z);
+        const float ri = rsqrt_a(d2);
+        const float s1_ = __fmul_rn(f.el1, __fmul_rn(d2, ri));
+        const float gn = __fmaf_rn(__fmul_rn(s1_, s1_), __fmaf_rn(f.b1, s1_, f.a1), f.el0);
+        /* ep (el1 gn) - ep ri = ele_p gn - ele_p g_far */
+        s.ele += __fmaf_rn(e * f.el1, gn, -(e * ri));
+      }
+    }
+  }
+  for (int i = (s1 >> 2) + part; i < (s2 >> 2); i += parts) {
+    const ushort4 id = __ldg(ix + i);
+    const int k[4] = {id.x, id.y, id.z, id.w};
+    float4 p[4];
+    float2 b[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      p[u] = __ldg(PA + k[u]);
+      b[u] = __ldg(reinterpret_cast<const float2 *>(PB + k[u]));
+    }
+    float ps[4];
+    double h[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const float d2 = dist2(ax, ay, az, p[u].x, p[u].y, p[u].z);
+      const int meta = __float_as_int(p[u].w);
+      float t = __fmaf_rn(d2, HPC_C4, -HPC_C3);
+      t = __fmaf_rn(d2, t, HPC_C2);
+      t = __fmaf_rn(d2, t, -HPC_C1);
+      t = __fmul_rn(b[u].x, __fmaf_rn(d2, t, 1.0f));
+      h[u] = (meta & 256) && d2 <= 81.0f ? (double)t : 0.0;
+      ps[u] = (meta & 512) && d2 <= thr[meta & 255] ? __ldg(psprow + __float_as_int(b[u].y))
+                                                    : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      s.hsum += h[u];
+      s.psp += ps[u];
+    }
+  }
+}
+
+/* The pocket-grid cell of a position, -1 outside the grid (a NaN position is outside). */
+__device__ __forceinline__ int pocket_cell(const GdDevComplex &cx, float x, float y, float z) {
+  const float inv = 1.0f / GD_PG_EDGE;
+  const float fx = floorf((x - cx.pg_org[0]) * inv), fy = floorf((y - cx.pg_org[1]) * inv),
+              fz = floorf((z - cx.pg_org[2]) * inv);
+  const float n = (float)GD_PG_N;
+  if (!(fx >= 0.0f && fx < n && fy >= 0.0f && fy < n && fz >= 0.0f && fz < n)) return -1;
+  return ((int)fz * GD_PG_N + (int)fy) * GD_PG_N + (int)fx;
+}
+
 /* Per-replica state of the CTA's slots, in shared memory. */
 struct Slot {
   int rep, lig_conf, accept, n_acc;
@@ -385,6 +468,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 }
 
 #define NQ 10 /* vdw ele pmf psp hdb hsum->hpc kde rmsd ncon tp */
+#define MCS_U 4 /* restraint positions in flight in the epilogue */
 
 /* One segment range of the pair loop, dispatched on the segment's flags (bit 2: live
  * hydrogen-bond term). */
@@ -711,7 +795,12 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       for (int h = 0; h < PACK; ++h) {
         if (!ok[h]) continue;
         ShortSums sr;
-        short_range(cx, pc, thr_s + tl * GD_MAXTP1, psprow, f, ax[h], ay[h], az[h], sp, S, sr);
+        const int cell = pocket_cell(cx, ax[h], ay[h], az[h]);
+        if (cell >= 0)
+          short_range_lists(cx, pc, cell, thr_s + tl * GD_MAXTP1, psprow, f, ax[h], ay[h], az[h],
+                            sp, S, sr);
+        else
+          short_range(cx, pc, thr_s + tl * GD_MAXTP1, psprow, f, ax[h], ay[h], az[h], sp, S, sr);
         const int v = vl[h];
         part[1 * T + v] = (double)sr.ele;
         part[3 * T + v] = (double)sr.psp;
@@ -836,15 +925,17 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
         const double hpc2 = (part[5 * T + v] - (double)f.hpl0[tl]) / (double)f.hpl1[tl];
         part[5 * T + v] = 0.5 * hpc2 * hpc2 - (double)f.hpl2[tl];
         float ks = 0.0f;
-        int kn = 0;
-        for (int kk = 0; kk < cx.pnk; ++kk) {
+        /* the KDE points lie sorted by type, in their given order within a type: the atom sums
+         * its own type's points only. Latency-bound (a chain of additions per atom): four loads
+         * in flight. One conformer of 454 points walked whole took 96 k cycles a step. */
+        const int k0 = __ldg(cx.kde_start + tl), k1 = __ldg(cx.kde_start + tl + 1);
+#pragma unroll 4
+        for (int kk = k0; kk < k1; ++kk) {
           const float4 kd = __ldg(cx.kde + kk);
-          if ((int)kd.w == tl) {
-            const float dx = ax[h] - kd.x, dy = ay[h] - kd.y, dz = az[h] - kd.z;
-            ks += expf(f.kde2 * (dx * dx + dy * dy + dz * dz));
-            ++kn;
-          }
+          const float dx = ax[h] - kd.x, dy = ay[h] - kd.y, dz = az[h] - kd.z;
+          ks += expf(f.kde2 * (dx * dx + dy * dy + dz * dz));
         }
+        const int kn = k1 - k0;
         part[6 * T + v] = kn ? (double)ks / (double)kn : 0.0;
         const Slot &sl = slots[sl_of[h]];
         const float *lc = cx.lig_center + sl.lig_conf * 3;
@@ -867,36 +958,61 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       /* ---- per-replica epilogue: one warp per slot ---- */
       for (int js = warp; js < k; js += nwarps) {
         Slot &sl = slots[js];
-        /* slot totals are written back over the slot's first partial */
+        /* slot totals are written back over the slot's first partial; five quantities at a time,
+         * so that their shuffles overlap (one at a time the chain took 7-9 k cycles a step) */
         double *tot = part + js * SL;
 #pragma unroll 1
-        for (int qi = 0; qi < NQ; ++qi) {
-          double v = 0.0;
-          for (int i = lane; i < SL; i += 32) v += part[qi * T + js * SL + i];
-          v = warp_sum(v);
-          if (lane == 0) tot[qi * T] = v;
+        for (int q0 = 0; q0 < NQ; q0 += 5) {
+          double v[5];
+#pragma unroll
+          for (int u = 0; u < 5; ++u) v[u] = 0.0;
+          for (int i = lane; i < SL; i += 32)
+#pragma unroll
+            for (int u = 0; u < 5; ++u) v[u] += part[(q0 + u) * T + js * SL + i];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < 5; ++u) v[u] += __shfl_down_sync(0xffffffffu, v[u], o);
+          if (lane == 0)
+#pragma unroll
+            for (int u = 0; u < 5; ++u) tot[(q0 + u) * T] = v[u];
         }
-        /* MCS position restraints */
+        /* MCS position restraints, MCS_U positions at a time: their loads and shuffles overlap
+         * (one at a time, each waited for its own: 20-29 k cycles a step at 8-11 positions) */
         double elhm = 0.0;
-        for (int m = 0; m < cx.pos; ++m) {
-          double sm = 0.0;
-          int cnt = 0;
+        const int *meta_y = &cx.lig_meta[sl.lig_conf * L].y;
+#pragma unroll 1
+        for (int m0 = 0; m0 < cx.pos; m0 += MCS_U) {
+          double sm[MCS_U];
+          unsigned cnt = 0; /* the positions' atom counts (<= GD_MAXLIG), 8 bits each */
+#pragma unroll
+          for (int u = 0; u < MCS_U; ++u) sm[u] = 0.0;
           for (int i = lane; i < L; i += 32) {
-            const int idx = cx.lig_meta[sl.lig_conf * L + i].y;
-            const float mx = cx.mcs_x[(size_t)m * cx.mcs_ld + idx];
-            if (mx != GD_MCS_INVALID_COORD) {
-              const float4 at = atoms[js * SL + i];
-              const float dx = at.x - mx;
-              const float dy = at.y - cx.mcs_y[(size_t)m * cx.mcs_ld + idx];
-              const float dz = at.z - cx.mcs_z[(size_t)m * cx.mcs_ld + idx];
-              sm += (double)(dx * dx + dy * dy + dz * dz);
-              ++cnt;
+            const int idx = __ldg(meta_y + 2 * i);
+            const float4 at = atoms[js * SL + i];
+#pragma unroll
+            for (int u = 0; u < MCS_U; ++u) {
+              const int m = min(m0 + u, cx.pos - 1);
+              const float4 r = __ldg(cx.mcs + (size_t)m * cx.mcs_ld + idx);
+              if (r.x != GD_MCS_INVALID_COORD) {
+                const float dx = at.x - r.x, dy = at.y - r.y, dz = at.z - r.z;
+                sm[u] += (double)(dx * dx + dy * dy + dz * dz);
+                cnt += 1u << (8 * u);
+              }
             }
           }
-          sm = warp_sum(sm);
+          cnt = __reduce_add_sync(0xffffffffu, cnt);
 #pragma unroll
-          for (int o = 16; o > 0; o >>= 1) cnt += __shfl_down_sync(0xffffffffu, cnt, o);
-          if (lane == 0 && cnt) elhm += (double)cx.mcs_tcc[m] * sqrt(sm / (double)cnt);
+          for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int u = 0; u < MCS_U; ++u) sm[u] += __shfl_down_sync(0xffffffffu, sm[u], o);
+          if (lane == 0)
+#pragma unroll
+            for (int u = 0; u < MCS_U; ++u) {
+              const unsigned n = (cnt >> (8 * u)) & 255u;
+              if (m0 + u < cx.pos && n)
+                elhm += (double)cx.mcs_tcc[m0 + u] * sqrt(sm[u] / (double)n);
+            }
         }
         if (lane == 0) {
           const double Ld = (double)L;
