@@ -863,7 +863,8 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   c->n_groups = goff;
   if ((rc = upload(c, &c->d_cx, dcx)) || (rc = upload(c, &c->d_group_base, group_base)))
     return bail(rc);
-  if ((rc = build_pocket_lists(c, dcx))) return bail(rc);
+  if ((rc = build_pocket_lists(c, dcx)) || (rc = build_far_fields(c, ff, cxs, dcx)))
+    return bail(rc);
   CK(cudaMemcpyAsync(c->d_cx, dcx.data(), sizeof(GdDevComplex) * dcx.size(),
                      cudaMemcpyHostToDevice, c->stream));
 

@@ -7,6 +7,7 @@
  *                       src/kernel_cuda_lancher_siglegpu.cu)
  *   gd_capi_layout.cu   the device layout of one complex
  *   gd_pocket.cu        the pocket grid's point lists of the short-range terms
+ *   gd_farfield.cu      the far points of large proteins as fields over the pocket grid
  *   gd_capi_tile.cu     the tile, its autotuning, chains, RNG streams and the wait bound
  *   gd_capi_stream.cu   records downloaded while the run proceeds (gd_records_stream)
  *   gd_capi_eval.cu     pose energies, placed coordinates and the energy trace
@@ -266,6 +267,10 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
 
 /* ---- the pocket grid's point lists (gd_pocket.cu) ---- */
 int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx);
+
+/* ---- the far fields of large proteins (gd_farfield.cu) ---- */
+int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs,
+                     std::vector<GdDevComplex> &dcx);
 
 /* ---- allocation-free pose evaluation (gd_capi_noalloc.cu) ---- */
 int noalloc_prepare(int device);

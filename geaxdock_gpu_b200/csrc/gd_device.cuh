@@ -40,6 +40,14 @@
 #define GD_PG_N 10
 #define GD_PG_CELLS (GD_PG_N * GD_PG_N * GD_PG_N)
 #define GD_PG_EDGE 4.0f
+/* the far fields: cells of GD_FF_EDGE A, a cube of GD_FF_N^3 centred on the pocket centre, of
+ * which those reaching no further than half its edge from the centre are tabulated; Chebyshev
+ * series of total degree GD_FF_DEG, GD_FF_NC coefficients (padded to whole float4) */
+#define GD_FF_N 18
+#define GD_FF_CELLS (GD_FF_N * GD_FF_N * GD_FF_N)
+#define GD_FF_EDGE 2.0f
+#define GD_FF_DEG 4
+#define GD_FF_NC (((GD_FF_DEG + 1) * (GD_FF_DEG + 2) * (GD_FF_DEG + 3) / 6 + 3) / 4 * 4)
 #define GD_MAX_CELLS (1 << 22) /* cells per conformer grid; a larger box widens the cells */
 #define GD_MAX_CELLS_ALL (1 << 25) /* cells of all conformers of a complex together */
 #define GD_MAX_TPB 256         /* threads per CTA: 3 CTAs of 256 fit the register file */
@@ -119,7 +127,47 @@ struct GdDevComplex {
    * the atom, where every type pair's pmf exponent is below -25.5 in base 2. */
   const unsigned short *far_cnt;
   float far_r, far_inv_w;
+  /* the far fields (gd_farfield.cu; ff_tab null: none). Far-field cell c's table is number ff_id[c] (-1:
+   * not tabulated) of its conformer's ff_cells, ff_fields series of GD_FF_NC coefficients: ele,
+   * then vdw of ligand type t at 1 + ff_slot[t]. ff_pmf[(pc * GD_FAR_BINS + bin) * GD_MAXTP2 + t]:
+   * the far points' pmf sum. A cell's far points: in each segment those past the count of bin
+   * gd_ff_bin(cell) + ff_extra[point type]. */
+  const float *ff_tab;
+  const short *ff_id;
+  const double *ff_pmf;
+  int ff_fields, ff_cells;
+  float ff_r;                 /* r_f: a cell's far points are at least this far from its atoms */
+  unsigned char ff_slot[GD_MAXTP2], ff_extra[GD_MAXTP1 + 2];
 };
+
+#ifdef __CUDACC__
+/* The far-field cell of a position, -1 outside the cube (a NaN position is outside). */
+__device__ __forceinline__ int gd_ff_cell(const GdDevComplex &cx, float x, float y, float z) {
+  const float inv = 1.0f / GD_FF_EDGE, n = (float)GD_FF_N, o = 0.5f * GD_FF_N;
+  const float fx = floorf((x - cx.pocket[0]) * inv + o), fy = floorf((y - cx.pocket[1]) * inv + o),
+              fz = floorf((z - cx.pocket[2]) * inv + o);
+  if (!(fx >= 0.0f && fx < n && fy >= 0.0f && fy < n && fz >= 0.0f && fz < n)) return -1;
+  return ((int)fz * GD_FF_N + (int)fy) * GD_FF_N + (int)fx;
+}
+/* Radius bin of a far-field cell: every point past the bin's counts lies beyond the box's
+ * largest distance from the pocket centre plus ff_r. GD_FAR_BINS - 1 counts every point. */
+__device__ __forceinline__ int gd_ff_bin(const GdDevComplex &cx, int cell) {
+  const int ix = cell % GD_FF_N, iy = (cell / GD_FF_N) % GD_FF_N, iz = cell / (GD_FF_N * GD_FF_N);
+  const int mx = max(GD_FF_N / 2 - ix, ix + 1 - GD_FF_N / 2),
+            my = max(GD_FF_N / 2 - iy, iy + 1 - GD_FF_N / 2),
+            mz = max(GD_FF_N / 2 - iz, iz + 1 - GD_FF_N / 2);
+  const float rho = GD_FF_EDGE * sqrtf((float)(mx * mx + my * my + mz * mz)) + cx.ff_r;
+  return (int)fminf(rho * cx.far_inv_w, (float)(GD_FAR_BINS - 1));
+}
+/* First far slot of segment sg (range and type g) for a cell of that bin: an even slot, or the
+ * segment's end. */
+__device__ __forceinline__ int gd_ff_near(const GdDevComplex &cx, int pc, int sg, const int4 g,
+                                          int bin) {
+  const int b = min(bin + (int)cx.ff_extra[g.z], GD_FAR_BINS - 1);
+  const int n = cx.far_cnt[((size_t)pc * GD_MAX_SEG + sg) * GD_FAR_BINS + b];
+  return min(g.y, g.x + ((n + 1) & ~1));
+}
+#endif
 
 /* One CTA's unit of work: `count` consecutive replicas of one protein conformer. */
 struct GdTileDesc {

@@ -446,6 +446,71 @@ __device__ __forceinline__ int pocket_cell(const GdDevComplex &cx, float x, floa
   return ((int)fz * GD_PG_N + (int)fy) * GD_PG_N + (int)fx;
 }
 
+/* A float4 of the far-field tables: read once per atom and step, kept out of L1, which holds the
+ * point lists. */
+__device__ __forceinline__ float4 ldg_stream(const float4 *p) {
+  float4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "l"(p));
+  return v;
+}
+
+/* The far points' ele and vdw sums at (x, y, z) of a tabulated cell (gd_farfield.cu): two
+ * Chebyshev series of total degree 4 in the cell's coordinates, about 110 FMAs and 18 loads from
+ * L2, for what the pair loop spent on more than half of 3,000 points. */
+__device__ __forceinline__ void far_field(const GdDevComplex &cx, int pc, int cell, int id, int tl,
+                                          float x, float y, float z, float &ele, float &vdw) {
+  const float4 *te = reinterpret_cast<const float4 *>(
+      cx.ff_tab + ((size_t)pc * cx.ff_cells + id) * cx.ff_fields * GD_FF_NC);
+  const float4 *tv = te + (1 + cx.ff_slot[tl]) * (GD_FF_NC / 4);
+  const int ix = cell % GD_FF_N, iy = (cell / GD_FF_N) % GD_FF_N, iz = cell / (GD_FF_N * GD_FF_N);
+  const float s = 2.0f / GD_FF_EDGE;
+  const float u = (x - cx.pocket[0]) * s - (float)(2 * ix + 1 - GD_FF_N),
+              v = (y - cx.pocket[1]) * s - (float)(2 * iy + 1 - GD_FF_N),
+              w = (z - cx.pocket[2]) * s - (float)(2 * iz + 1 - GD_FF_N);
+  constexpr int N = GD_FF_DEG + 1;
+  static_assert(GD_FF_NC % 4 == 0, "whole float4 per series");
+  float tu[N], tw[N];
+  tu[0] = tw[0] = 1.0f;
+  tu[1] = u;
+  tw[1] = w;
+#pragma unroll
+  for (int i = 2; i < N; ++i) {
+    tu[i] = 2.0f * u * tu[i - 1] - tu[i - 2];
+    tw[i] = 2.0f * w * tw[i - 1] - tw[i - 2];
+  }
+  ele = vdw = 0.0f;
+  float4 ce, cv;
+  int n = 0;
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    float ek = 0.0f, vk = 0.0f, t0 = 1.0f, t1 = v;
+#pragma unroll
+    for (int j = 0; j < N - k; ++j) {
+      float ej = 0.0f, vj = 0.0f;
+#pragma unroll
+      for (int i = 0; i < N - k - j; ++i, ++n) {
+        if ((n & 3) == 0) {
+          ce = ldg_stream(te + (n >> 2));
+          cv = ldg_stream(tv + (n >> 2));
+        }
+        const float a = (n & 3) == 0 ? ce.x : (n & 3) == 1 ? ce.y : (n & 3) == 2 ? ce.z : ce.w;
+        const float b = (n & 3) == 0 ? cv.x : (n & 3) == 1 ? cv.y : (n & 3) == 2 ? cv.z : cv.w;
+        ej = __fmaf_rn(a, tu[i], ej);
+        vj = __fmaf_rn(b, tu[i], vj);
+      }
+      ek = __fmaf_rn(ej, t0, ek);
+      vk = __fmaf_rn(vj, t0, vk);
+      const float t2 = 2.0f * v * t1 - t0;
+      t0 = t1;
+      t1 = t2;
+    }
+    ele = __fmaf_rn(ek, tw[k], ele);
+    vdw = __fmaf_rn(vk, tw[k], vdw);
+  }
+}
+
 /* Per-replica state of the CTA's slots, in shared memory. */
 struct Slot {
   int rep, lig_conf, accept, n_acc;
@@ -791,8 +856,12 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       /* ---- short-range terms from the cell list (the S lanes of an atom take every S-th row
        * of its walk), before the pair loop: warps whose walk is short start the loop while
        * the others still walk ---- */
+      /* lbin: the radius bin past which each lane's points come from the far fields
+       * (GD_FAR_BINS - 1: every point runs in the loop) */
+      int lbin[PACK];
 #pragma unroll
       for (int h = 0; h < PACK; ++h) {
+        lbin[h] = GD_FAR_BINS - 1;
         if (!ok[h]) continue;
         ShortSums sr;
         const int cell = pocket_cell(cx, ax[h], ay[h], az[h]);
@@ -806,6 +875,21 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
         part[3 * T + v] = (double)sr.psp;
         part[5 * T + v] = sr.hsum;
         part[8 * T + v] = (double)sr.ncon;
+        const int fcell = cx.ff_tab != nullptr ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
+        if (fcell >= 0) {
+          const int id = __ldg(cx.ff_id + fcell);
+          const int bin = gd_ff_bin(cx, fcell);
+          if (id >= 0 && bin < GD_FAR_BINS - 1) {
+            lbin[h] = bin;
+            if (sp == 0) {
+              float fe, fv;
+              far_field(cx, pc, fcell, id, tl, ax[h], ay[h], az[h], fe, fv);
+              part[0 * T + v] = (double)fv;
+              part[1 * T + v] += (double)fe;
+              part[2 * T + v] = __ldg(cx.ff_pmf + ((size_t)pc * GD_FAR_BINS + bin) * GD_MAXTP2 + tl);
+            }
+          }
+        }
       }
 
       /* ---- far-point bin of the warp: a point further from the pocket centre than far_r +
@@ -823,7 +907,9 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       fbin = (int)__reduce_max_sync(0xffffffffu, (unsigned)fbin);
       const unsigned short *fcnt = cx.far_cnt + (size_t)pc * GD_MAX_SEG * GD_FAR_BINS + fbin;
 
-      /* ---- CalcEnergy_d pair loop over the protein ring ---- */
+      /* ---- CalcEnergy_d pair loop over the protein ring (sg0: the first segment that reaches
+       * past the chunks done) ---- */
+      int sg0 = 0;
       for (int ci = 0; ci < nch; ++ci) {
         const int q = resident ? ci : s * nch + ci;
         const int b = q & 1;
@@ -842,9 +928,21 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
           const float4 *PA = bpa + b * (D >> 1); /* local slot = slot - c0 */
           const float4 *PB = bpb + b * (D >> 1);
           const int c0 = ci * D, c1 = min(pnp_pad, c0 + D);
-          for (int sg = 0; sg < nseg; ++sg) {
+          for (int sg = sg0; sg < nseg; ++sg) {
             const int4 g = segs[sg];
-            const int i0 = max(g.x, c0) - c0, i1 = min(g.y, c1) - c0;
+            if (g.x >= c1) break;
+            if (g.y <= c1) sg0 = sg + 1;
+            const int i0 = max(g.x, c0) - c0;
+            /* each lane's end of the segment: where its far field takes over */
+            int il[PACK], i1 = 0;
+#pragma unroll
+            for (int h = 0; h < PACK; ++h) {
+              const int e = PACK > 1 && !ok[h] ? g.x
+                            : lbin[h] == GD_FAR_BINS - 1 ? g.y
+                                                         : gd_ff_near(cx, pc, sg, g, lbin[h]);
+              il[h] = min(e, c1) - c0;
+              i1 = max(i1, il[h]);
+            }
             if (i0 >= i1) continue;
             const float4 *pr = reinterpret_cast<const float4 *>(pprow + g.z);
             const float4 q0 = __ldg(pr), q1 = __ldg(pr + 1), q2 = __ldg(pr + 2);
@@ -869,10 +967,29 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
                 pair_range_split<false, UNROLL>(PA, PB, i0, im, i1, sp, S, ax[0], ay[0], az[0],
                                                 pq, f, acc[0]);
             } else {
-              if (i0 < im)
-                pair_dispatch<UNROLL, PACK, false>(g.w, PA, PB, i0, im, ax, ay, az, pq, f, acc);
-              if (im < i1)
-                pair_dispatch<UNROLL, PACK, true>(g.w, PA, PB, im, i1, ax, ay, az, pq, f, acc);
+              if constexpr (PACK == 1) {
+                if (i0 < im)
+                  pair_dispatch<UNROLL, 1, false>(g.w, PA, PB, i0, im, ax, ay, az, pq, f, acc);
+                if (im < i1)
+                  pair_dispatch<UNROLL, 1, true>(g.w, PA, PB, im, i1, ax, ay, az, pq, f, acc);
+              } else {
+                /* both lanes' points together, then the rest of the lane that has more */
+                const int ib = max(i0, min(il[0], il[1])), imb = min(im, ib);
+                if (i0 < imb)
+                  pair_dispatch<UNROLL, 2, false>(g.w, PA, PB, i0, imb, ax, ay, az, pq, f, acc);
+                if (imb < ib)
+                  pair_dispatch<UNROLL, 2, true>(g.w, PA, PB, imb, ib, ax, ay, az, pq, f, acc);
+#pragma unroll
+                for (int h = 0; h < PACK; ++h) {
+                  const int j0 = max(ib, im);
+                  if (ib < min(im, il[h]))
+                    pair_dispatch<UNROLL, 1, false>(g.w, PA, PB, ib, min(im, il[h]), ax + h, ay + h,
+                                                    az + h, pq, f, acc + h);
+                  if (j0 < il[h])
+                    pair_dispatch<UNROLL, 1, true>(g.w, PA, PB, j0, il[h], ax + h, ay + h, az + h,
+                                                   pq, f, acc + h);
+                }
+              }
             }
 #pragma unroll
             for (int h = 0; h < PACK; ++h) {
