@@ -286,13 +286,61 @@ void build_tiles(const gd_ctx *c, int r0, int r1, std::vector<GdTileDesc> &out) 
   });
 }
 
-size_t smem_bytes(const gd_ctx *c) {
-  int kmax = 1;
-  for (const auto &x : c->info) kmax = std::max(kmax, x.k);
-  const size_t slot = GD_SLOT_BYTES;
-  return 16 + GD_THR_BYTES + (size_t)2 * c->chunk * 16 + (size_t)c->threads * 16 +
-         (size_t)10 * c->threads * 8 +
-         (size_t)kmax * slot;
+size_t smem_bytes(const LaunchShape &s) {
+  return 16 + GD_THR_BYTES + (size_t)2 * s.chunk * 16 + (size_t)s.lanes * 16 +
+         (size_t)10 * s.lanes * 8 + (size_t)s.kmax * GD_SLOT_BYTES;
+}
+
+LaunchShape ctx_shape(const gd_ctx *c) {
+  LaunchShape s = {c->threads, c->chunk, c->fold, c->split, c->unroll, c->pack, 1};
+  for (const auto &x : c->info) s.kmax = std::max(s.kmax, x.k);
+  return s;
+}
+
+/* A launch with too few replicas to give every scheduler warps to switch between is bound by the
+ * latency of one warp's pass over the protein: it is split, the lanes of an atom in S warps that
+ * each run some of its segments. As many splits as keep every tile resident (16 warps an SM at the
+ * split variants' 128 registers): a second wave costs more than the split gives. 252 replicas of
+ * 34 atoms, 344 points, 101 steps: S = 1 / 2 / 3 / 4 / 5 6,100 / 3,700 / 2,710 / 2,540 / 3,780 us
+ * (two tiles an SM, of 16 warps from S = 5 on); 128 replicas of 28 atoms, 1,500 points: S = 1 / 2 /
+ * 4 / 8 / 16 10,600 / 4,770 / 3,030 / 2,020 / 1,910 us. */
+int auto_split(const gd_ctx *c, const std::vector<WorkList> &w, std::vector<int> *k) {
+  const int most = GD_MAX_TPB_SPLIT / 32;
+  int best = 0, best_wa = 1;
+  /* wa: warps of a tile per split; the fewest warps on the fullest SM, and of those the smallest
+   * tiles */
+  for (int wa = 1; wa <= most; ++wa) {
+    long long tiles = 0;
+    for (const WorkList &x : w) {
+      const int kk = std::min(std::min(wa * 32 / x.lna, GD_MAX_SLOTS), x.block);
+      if (kk < 1) {
+        tiles = -1;
+        break;
+      }
+      tiles += x.n_blocks * ((x.block + kk - 1) / kk);
+    }
+    if (tiles < 0) continue;
+    const long long warps = (tiles + c->num_sms - 1) / c->num_sms * wa;
+    if (warps <= most && (best == 0 || warps < best)) {
+      best = (int)warps;
+      best_wa = wa;
+    }
+  }
+  const int S = best ? most / best : 1;
+  if (S > 1) {
+    k->clear();
+    for (const WorkList &x : w)
+      k->push_back(std::min(std::min(best_wa * 32 / x.lna, GD_MAX_SLOTS), x.block));
+  }
+  return S;
+}
+
+LaunchShape split_shape(int split, int k_lna, int kmax, int pnp_pad) {
+  /* two buffers hold the protein; the sums fold where the default tile's do, so that the shape
+   * does not change the energies */
+  const int half = (pnp_pad + 1) / 2;
+  const int chunk = std::min(4096, std::max(1, (half + GD_CHUNK - 1) / GD_CHUNK) * GD_CHUNK);
+  return {split * ((k_lna + 31) / 32) * 32, chunk, GD_CHUNK, split, 4, 1, kmax};
 }
 
 int ensure_counters(gd_ctx *c, int n) {
@@ -344,26 +392,18 @@ McKernel mc_kernel(int unroll, int split, bool da, int pack) {
   return split > 1 ? mc_variant<true, false>(unroll) : mc_variant<false, false>(unroll);
 }
 
-/* replicas per thread of a launch: the context's packing for the plain modes without split */
-int launch_pack(const gd_ctx *c, int split, bool da) {
-  return (!da && (split ? split : c->split) <= 1) ? c->pack : 1;
+/* threads per CTA of a launch: the tile's lanes over the replicas per thread (two only for the
+ * plain modes without split) */
+int launch_threads(const LaunchShape &s) { return s.lanes / s.pack; }
+
+McKernel launch_kernel(const LaunchShape &s, bool da) {
+  return mc_kernel(s.unroll, s.split, da, s.pack);
 }
 
-/* threads per CTA of a launch: the tile's lanes over the replicas per thread */
-int launch_threads(const gd_ctx *c, int split, bool da) {
-  return c->threads / launch_pack(c, split, da);
-}
-
-McKernel launch_kernel(const gd_ctx *c, int split, bool da, int unroll) {
-  const int S = split ? split : c->split;
-  return mc_kernel(unroll ? unroll : c->unroll, S, da, launch_pack(c, split, da));
-}
-
-int grid_for(gd_ctx *c, int n_tiles, size_t smem, int split, bool da, int unroll) {
+int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da) {
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, launch_kernel(c, split, da, unroll),
-                                                    launch_threads(c, split, da),
-                                                    smem) != cudaSuccess ||
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, launch_kernel(s, da), launch_threads(s),
+                                                    smem_bytes(s)) != cudaSuccess ||
       nb < 1)
     nb = 1;
   return std::max(1, std::min(n_tiles, nb * c->num_sms));
@@ -375,6 +415,7 @@ GdMcArgs base_args(gd_ctx *c) {
   a.cx = c->d_cx;
   a.pp = c->d_pp;
   a.chunk = c->chunk;
+  a.fold = c->fold;
   a.split = c->split;
   a.move_kind = c->mc.move_kind;
   a.seed = c->mc.seed;
@@ -396,8 +437,9 @@ GdMcArgs base_args(gd_ctx *c) {
   return a;
 }
 
-int set_kernel_attrs(const gd_ctx *c, size_t smem, int split, bool da, int unroll) {
-  const McKernel k = launch_kernel(c, split, da, unroll);
+int set_kernel_attrs(const LaunchShape &s, bool da) {
+  const McKernel k = launch_kernel(s, da);
+  const size_t smem = smem_bytes(s);
   CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   /* shared memory for the CTAs an SM can hold and the rest as L1, which caches the cell
    * lists of the short-range pass: the carveout is the share of the SM's maximum shared
@@ -408,7 +450,7 @@ int set_kernel_attrs(const gd_ctx *c, size_t smem, int split, bool da, int unrol
   CK(cudaGetDevice(&dev));
   CK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
   CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-  const int threads = launch_threads(c, split, da);
+  const int threads = launch_threads(s);
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem));
   if (nb >= 1 && per_sm > 0) {
     /* the driver rounds the carveout up to one of the SM's shared-memory sizes; aim at the
@@ -433,17 +475,20 @@ int set_kernel_attrs(const gd_ctx *c, size_t smem, int split, bool da, int unrol
   return GD_OK;
 }
 
-int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter) {
+int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter,
+              const LaunchShape &s) {
   if (n_tiles <= 0) return GD_OK;
-  const size_t smem = smem_bytes(c);
-  int rc = set_kernel_attrs(c, smem);
+  int rc = set_kernel_attrs(s);
   if (rc) return rc;
+  a.chunk = s.chunk;
+  a.fold = s.fold;
+  a.split = s.split;
   a.tiles = d_tiles;
   a.n_tiles = n_tiles;
   a.tile_counter = counter;
   CK(cudaMemsetAsync(counter, 0, sizeof(int), c->stream));
-  const int grid = grid_for(c, n_tiles, smem);
-  launch_kernel(c)<<<grid, launch_threads(c), smem, c->stream>>>(a, c->fc);
+  const int grid = grid_for(c, n_tiles, s);
+  launch_kernel(s)<<<grid, launch_threads(s), smem_bytes(s), c->stream>>>(a, c->fc);
   CK(cudaGetLastError());
   return GD_OK;
 }
@@ -896,6 +941,31 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   c->threads = pick_threads(c->info);
   for (auto &x : c->info)
     x.k = std::max(1, std::min(c->threads / x.lna, std::min(GD_MAX_SLOTS, x.n_tmp * x.n_lig)));
+  {
+    int lna = 1, pad = 4, k_lna = 1, kmax = 1;
+    for (const auto &x : c->info) {
+      lna = std::max(lna, x.lna);
+      pad = std::max(pad, x.pnp_pad);
+    }
+    std::vector<WorkList> work;
+    std::vector<int> k;
+    for (const auto &x : c->info) work.push_back({x.n_prt, x.n_tmp * x.n_lig, x.lna});
+    const int S = auto_split(c, work, &k);
+    if (S > 1) {
+      for (int ci = 0; ci < n_complexes; ++ci) {
+        ComplexInfo &x = c->info[ci];
+        x.k = k[ci];
+        k_lna = std::max(k_lna, x.k * x.lna);
+        kmax = std::max(kmax, x.k);
+      }
+      const LaunchShape s = split_shape(S, k_lna, kmax, pad);
+      c->threads = s.lanes;
+      c->chunk = s.chunk;
+      c->fold = s.fold;
+      c->split = s.split;
+      c->unroll = s.unroll;
+    }
+  }
   build_tiles(c, 0, R - 1, c->full_tiles);
   c->tiles_cap = (int)c->full_tiles.size() + 16 * n_complexes;
   {
@@ -936,7 +1006,7 @@ int gd_mc_init(gd_ctx *c) {
   CK(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
   if ((rc = rs_flush(c))) return rc;
   if ((rc = rs_restart(c, 0, c->n_rep - 1))) return rc;
-  rc = launch_mc(c, a, c->d_tiles, n, c->d_counters);
+  rc = launch_mc(c, a, c->d_tiles, n, c->d_counters, ctx_shape(c));
   if (rc) return rc;
   c->initialized = true;
   c->exchange_calls = 0;
@@ -967,7 +1037,7 @@ int gd_mc_run(gd_ctx *c, int r0, int r1, int s1, int s2) {
   a.mode = 0;
   a.n_steps = c->mc.steps_per_exchange;
   a.step0 = s1 + s2;
-  if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters))) return rc;
+  if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters, ctx_shape(c)))) return rc;
   return rs_enqueue(c, c->mc.steps_per_exchange);
 }
 
@@ -1003,8 +1073,8 @@ int gd_mc_run_fused(gd_ctx *c, int s1, int n_steps, int exchange) {
   auto it = c->graphs.find(key);
   if (it == c->graphs.end()) {
     CK(cudaStreamSynchronize(c->stream));
-    const size_t smem = smem_bytes(c);
-    if ((rc = set_kernel_attrs(c, smem))) return rc;
+    const LaunchShape shape = ctx_shape(c);
+    if ((rc = set_kernel_attrs(shape))) return rc;
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(c->d_counters, 0, sizeof(int) * n_ctr, c->stream);
@@ -1012,7 +1082,7 @@ int gd_mc_run_fused(gd_ctx *c, int s1, int n_steps, int exchange) {
     for (int k = 0; k < nch; ++k) {
       const Chain &ch = c->chain[k];
       cudaStream_t st = chain_stream(c, k);
-      const int grid = grid_for(c, ch.t_cnt, smem);
+      const int grid = grid_for(c, ch.t_cnt, shape);
       for (int i = 0; i < chunks; ++i) {
         GdMcArgs a = base_args(c);
         a.mode = 0;
@@ -1032,7 +1102,7 @@ int gd_mc_run_fused(gd_ctx *c, int s1, int n_steps, int exchange) {
           a.x_spd = c->mc.steps_per_dump;
           a.x_spe = spe;
         }
-        launch_kernel(c)<<<grid, launch_threads(c), smem, st>>>(a, c->fc);
+        launch_kernel(shape)<<<grid, launch_threads(shape), smem_bytes(shape), st>>>(a, c->fc);
       }
     }
     chains_join(c, nch);

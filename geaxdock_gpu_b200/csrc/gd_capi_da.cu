@@ -137,6 +137,49 @@ int da_upload_epi(gd_ctx *c) {
   return GD_OK;
 }
 
+/* replicas of an lna-atom ligand that fill the warps of a split of a 256-thread CTA */
+int da_fill(int S, int lna, int lna_max) {
+  const int wa = std::max((lna_max + 31) / 32, GD_MAX_TPB / 32 / S);
+  return std::max(1, std::min(GD_MAX_SLOTS, wa * 32 / lna));
+}
+
+/* The exact stage's replicas per CTA for complex ci at split S: what fills the warps of a split,
+ * at most the tile's count where one was set. */
+int da_tile_k(const gd_ctx *c, int ci, int S) {
+  const ComplexInfo &x = c->info[ci];
+  if (S <= 1) return x.k;
+  int lna = 1;
+  for (const auto &y : c->info) lna = std::max(lna, y.lna);
+  return std::min(c->tile_auto ? x.n_tmp * x.n_lig : x.k, da_fill(S, x.lna, lna));
+}
+
+/* point pairs in flight of the exact stage at split S: with one lane per atom (most proposals
+ * surviving: collect steps, or a pass rate above 0.4, da_choose_split) the stage is
+ * throughput-bound beside the other chains' front kernels, and the 80-register variant with two
+ * point pairs in flight leaves them room on the SMs; split (few survivors) one tile's latency sets
+ * the step, and the tile's own unroll is kept (four pairs in flight shorten a tile). */
+LaunchShape da_shape(const gd_ctx *c, int S) {
+  LaunchShape s = ctx_shape(c);
+  s.pack = 1;
+  if (S <= 1) {
+    s.unroll = std::min(s.unroll, 2);
+    return s;
+  }
+  int k_lna = 1, pad = 4;
+  s.kmax = 1;
+  for (int ci = 0; ci < c->n_complex; ++ci) {
+    const int k = da_tile_k(c, ci, S);
+    k_lna = std::max(k_lna, k * c->info[ci].lna);
+    s.kmax = std::max(s.kmax, k);
+    pad = std::max(pad, c->info[ci].pnp_pad);
+  }
+  const LaunchShape q = split_shape(S, k_lna, s.kmax, pad);
+  if (c->tile_auto) return q;
+  s.lanes = q.lanes;
+  s.split = S;
+  return s;
+}
+
 /* groups and the exact kernel's static tile list for the current tile shapes and the exact
  * stage's split S: tile i of group g covers pose slots [b0 + i k, b0 + i k + cap), k the
  * replicas a CTA holds at split S, and carries (g << 8) | cap */
@@ -155,7 +198,7 @@ int da_build_groups(gd_ctx *c, int S) {
       q.pc = p;
       q.b0 = x.rep_offset + p * block;
       q.n = block;
-      q.k = std::max(1, std::min(x.k, c->threads / (S * x.lna)));
+      q.k = da_tile_k(c, ci, S);
       q.n_tiles = (block + q.k - 1) / q.k;
       q.tile_base = (int)tiles.size();
       q.pad = 0;
@@ -208,7 +251,7 @@ int da_build_groups(gd_ctx *c, int S) {
 /* largest split every complex of the batch fits into the context's CTA */
 int da_max_split(const gd_ctx *c) {
   int m = 16;
-  for (const auto &x : c->info) m = std::min(m, std::max(1, c->threads / x.lna));
+  for (const auto &x : c->info) m = std::min(m, GD_MAX_TPB_SPLIT / 32 / ((x.lna + 31) / 32));
   return m;
 }
 
@@ -226,15 +269,6 @@ int da_choose_split(const gd_ctx *c, bool collect) {
   const int S = p > 0.4 ? 1 : (p > 0.13 ? 2 : (p > 0.05 ? 3 : 4));
   return std::max(c->split, std::min(S, mx));
 }
-
-/* unroll of the exact stage at split S: with one lane per atom (most proposals surviving:
- * collect steps, or a pass rate above 0.4, da_choose_split) the stage is throughput-bound
- * beside the other chains' front kernels, and the 80-register variant with two point pairs in
- * flight leaves them room on the SMs; split over several lanes (few survivors) one tile's
- * latency sets the step, and the tile's own unroll is kept (four pairs in flight shorten a
- * tile). Config 1, DA / plain at pass 0.96 / 0.50 / 0.20 (splits 1 / 1 / 2): two pairs 1.08 /
- * 1.91 / 3.08, four pairs 1.04 / 1.94 / 3.38. */
-int da_unroll(const gd_ctx *c, int S) { return S > 1 ? c->unroll : std::min(c->unroll, 2); }
 
 gd::GdDaDev da_args(gd_ctx *c) {
   DaState *d = c->da;
@@ -285,7 +319,7 @@ gd::GdDaDev da_args(gd_ctx *c) {
 /* the exact stage of step j of one chain: gd_mc_kernel mode 3 over the chain's part of the
  * static tile list */
 void da_launch_exact(gd_ctx *c, const Chain &ch, int k, int n_steps, int j, bool collect,
-                     size_t smem, cudaStream_t st, int S, int U) {
+                     cudaStream_t st, const LaunchShape &shape) {
   DaState *d = c->da;
   const int ng = (int)d->groups.size();
   const int t0 = d->groups[ch.g0].tile_base;
@@ -308,16 +342,18 @@ void da_launch_exact(gd_ctx *c, const Chain &ch, int k, int n_steps, int j, bool
   a.da_g0 = ch.g0;
   a.da_g1 = ch.g1;
   a.da_collect = collect ? 1 : 0;
-  a.split = S;
-  mc_kernel(U, S, true)<<<grid_for(c, t1 - t0, smem, S, true, U), c->threads, smem, st>>>(
-      a, c->fc);
+  a.split = shape.split;
+  a.chunk = shape.chunk;
+  a.fold = shape.fold;
+  launch_kernel(shape, true)<<<grid_for(c, t1 - t0, shape, true), launch_threads(shape),
+                               smem_bytes(shape), st>>>(a, c->fc);
 }
 
 /* the graph of n_steps steps (collect: plain steps that store samples), one chain per stream */
 int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGraphExec_t *out) {
   DaState *d = c->da;
-  const int U = da_unroll(c, S);
-  const long long key = ((long long)U << 44) | ((long long)n_steps << 7) | ((long long)S << 2) |
+  const LaunchShape shape = da_shape(c, S);
+  const long long key = ((long long)shape.unroll << 44) | ((long long)n_steps << 7) | ((long long)S << 2) |
                         (exchange ? 2 : 0) | (collect ? 1 : 0);
   auto it = d->graphs.find(key);
   if (it != d->graphs.end()) {
@@ -343,8 +379,7 @@ int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGrap
   }
   if ((rc = da_upload_epi(c))) return rc;
   CK(cudaStreamSynchronize(c->stream));
-  const size_t smem = smem_bytes(c);
-  if ((rc = set_kernel_attrs(c, smem, S, true, U))) return rc;
+  if ((rc = set_kernel_attrs(shape, true))) return rc;
   const gd::GdDaDev a = da_args(c);
   const int spe = c->mc.steps_per_exchange;
   const int ng = (int)d->groups.size();
@@ -361,7 +396,7 @@ int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGrap
     for (int j = 0; j < n_steps; ++j) {
       frc |= gd::da_front(a, collect ? GD_DA_COLLECT : GD_DA_STEP, j,
                           d->d_cnt + (size_t)(j & 1) * ng, ch.r0, ch.r1, st);
-      da_launch_exact(c, ch, k, n_steps, j, collect, smem, st, S, U);
+      da_launch_exact(c, ch, k, n_steps, j, collect, st, shape);
       if (exchange && (j + 1) % spe == 0) {
         const int i = (j + 1) / spe - 1;
         gd::gd_exchange_kernel<<<(ch.xg1 - ch.xg0 + 127) / 128, 128, 0, st>>>(

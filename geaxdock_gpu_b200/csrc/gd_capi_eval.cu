@@ -8,6 +8,30 @@
 
 using namespace gdc;
 
+namespace gdc {
+
+LaunchShape eval_shape(const gd_ctx *c, int ci, int n, int *k) {
+  const ComplexInfo &x = c->info[ci];
+  if (!c->tile_auto) {
+    *k = x.k;
+    return ctx_shape(c);
+  }
+  std::vector<int> ks;
+  const int S = auto_split(c, {{1, n, x.lna}}, &ks);
+  if (S > 1) {
+    *k = ks[0];
+    return split_shape(S, *k * x.lna, *k, x.pnp_pad);
+  }
+  /* one lane per atom: a CTA of 128..256 lanes with the least left over */
+  int best = 256;
+  for (int T = 128; T <= GD_MAX_TPB; T += 32)
+    if (T >= x.lna && (T / x.lna) * x.lna * best > (best / x.lna) * x.lna * T) best = T;
+  *k = std::min(GD_MAX_SLOTS, best / x.lna);
+  return {best, GD_CHUNK, GD_CHUNK, 1, 2, 1, *k};
+}
+
+}  // namespace gdc
+
 namespace {
 
 /* Energies of n poses of one (complex, protein conformer, ligand conformer): moved by
@@ -51,12 +75,14 @@ int eval_poses(gd_ctx *c, int ci, int prt_conf, int lig_conf, const float *mm, c
     c->eval_cap = n;
   }
   std::vector<GdTileDesc> tiles;
-  for (int i = 0; i < n; i += x.k) {
+  int k = 1;
+  const LaunchShape shape = eval_shape(c, ci, n, &k);
+  for (int i = 0; i < n; i += k) {
     GdTileDesc t;
     t.complex_index = ci;
     t.prt_conf = prt_conf;
     t.rep_begin = i;
-    t.count = std::min(x.k, n - i);
+    t.count = std::min(k, n - i);
     tiles.push_back(t);
   }
   if ((int)tiles.size() > c->eval_tiles_cap) {
@@ -87,7 +113,7 @@ int eval_poses(gd_ctx *c, int ci, int prt_conf, int lig_conf, const float *mm, c
   a.e_out = c->d_e_out;
   a.rec = nullptr;
   a.trace_e = nullptr;
-  int rc = launch_mc(c, a, c->d_eval_tiles, (int)tiles.size(), c->d_counters);
+  int rc = launch_mc(c, a, c->d_eval_tiles, (int)tiles.size(), c->d_counters, shape);
   if (rc) return rc;
   if ((rc = gd_sync(c))) return rc;
   CK(cudaMemcpy(out, c->d_e_out, sizeof(gd_energy) * n, cudaMemcpyDeviceToHost));

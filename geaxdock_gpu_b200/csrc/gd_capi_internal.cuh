@@ -89,6 +89,13 @@ struct ComplexInfo {
                         thread share their atom's pair parameters) */
 };
 
+/* The shape of one launch of the Monte Carlo kernel: lanes per CTA (pack lanes per thread), points
+ * per ring buffer and per FP32 sum (fold), splits per atom, point pairs in flight, the largest
+ * replica count of a tile. */
+struct LaunchShape {
+  int lanes, chunk, fold, split, unroll, pack, kmax;
+};
+
 /* One chain of the fused loops: a contiguous range of (complex, protein conformer) blocks,
  * their replicas, exchange groups and tiles. Chains share nothing, so the graph runs them on
  * separate streams and one chain's kernels fill the other's tail. */
@@ -110,10 +117,11 @@ struct gd_ctx {
   cudaStream_t stream = nullptr;
   gd_mc_params mc{};
   int n_complex = 0, n_rep = 0, n_groups = 0;
-  int threads = 256, chunk = 512, unroll = 2, split = 1, num_sms = 148;
+  int threads = 256, chunk = GD_CHUNK, fold = GD_CHUNK, unroll = 2, split = 1, num_sms = 148;
   int pack = 1; /* replicas per thread of the plain launches: the tile's lanes (threads) run on
                    threads / pack threads */
   int fill_threads = 0, fill_cap = 0; /* the last gd_set_tile in fill mode (threads > 0) */
+  bool tile_auto = true; /* no gd_set_tile yet: launches of few lanes are split over more warps */
   std::vector<gdc::ComplexInfo> info;
   std::vector<void *> allocs;      /* cudaMalloc'd buffers */
   std::vector<void *> pool_allocs; /* buffers from the device's context pool (ctx_pool) */
@@ -222,21 +230,31 @@ int upload(gd_ctx *c, T **p, const std::vector<T> &v) {
 int check_complex(const gd_complex_desc &d, int idx);
 int pick_threads(const std::vector<ComplexInfo> &info);
 void build_tiles(const gd_ctx *c, int r0, int r1, std::vector<GdTileDesc> &out);
-size_t smem_bytes(const gd_ctx *c);
+size_t smem_bytes(const LaunchShape &s);
+/* the shape of the context's tile */
+LaunchShape ctx_shape(const gd_ctx *c);
+/* One work list of a launch: n_blocks runs of `block` replicas (a protein conformer's) of an
+ * lna-atom ligand, none sharing a tile with another. */
+struct WorkList {
+  long long n_blocks;
+  int block, lna;
+};
+/* the splits of a launch of these lists (1: none), and the replicas a tile then takes of each */
+int auto_split(const gd_ctx *c, const std::vector<WorkList> &w, std::vector<int> *k);
+/* a split launch: lanes for k replicas of lna atoms, the ring holding the whole protein */
+LaunchShape split_shape(int split, int k_lna, int kmax, int pnp_pad);
 int ensure_counters(gd_ctx *c, int n);
 /* the pinned host cursor of the graph launches (made on first use) */
 int ensure_cursor(gd_ctx *c);
 typedef void (*McKernel)(GdMcArgs, GdForceConst);
 McKernel mc_kernel(int unroll, int split, bool da = false, int pack = 1);
-int launch_pack(const gd_ctx *c, int split, bool da);
-int launch_threads(const gd_ctx *c, int split = 0, bool da = false);
-/* unroll 0: the tile's */
-McKernel launch_kernel(const gd_ctx *c, int split = 0, bool da = false, int unroll = 0);
-int grid_for(gd_ctx *c, int n_tiles, size_t smem, int split = 0, bool da = false, int unroll = 0);
+McKernel launch_kernel(const LaunchShape &s, bool da = false);
+int launch_threads(const LaunchShape &s);
+int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da = false);
 GdMcArgs base_args(gd_ctx *c);
-int set_kernel_attrs(const gd_ctx *c, size_t smem, int split = 0, bool da = false,
-                     int unroll = 0);
-int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter);
+int set_kernel_attrs(const LaunchShape &s, bool da = false);
+int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter,
+              const LaunchShape &s);
 int upload_tiles(gd_ctx *c, int r0, int r1, int *n_out);
 int check_range(const gd_ctx *c, int r0, int r1);
 void build_chains(gd_ctx *c, int want, std::vector<Chain> &ch, std::vector<GdTileDesc> *tiles);
@@ -246,6 +264,10 @@ cudaStream_t chain_stream(gd_ctx *c, int k);
 void chains_fork(gd_ctx *c, int n);
 void chains_join(gd_ctx *c, int n);
 void drop_graphs(gd_ctx *c);
+
+/* ---- pose evaluation (gd_capi_eval.cu) ---- */
+/* the launch shape and replicas per CTA of an evaluation of n poses of complex ci */
+LaunchShape eval_shape(const gd_ctx *c, int ci, int n, int *k);
 
 /* ---- the record stream (gd_capi_stream.cu) ---- */
 int rs_enqueue(gd_ctx *c, int rows_per_rep);

@@ -113,7 +113,9 @@ extern "C" int gd_eval_energy_noalloc(gd_ctx *c, int ci, int prt_conf, int lig_c
   NoallocScratch *s = nullptr;
   int rc = noalloc_scratch(c->device, &s);
   if (rc) return rc;
-  const int k = x.k, n_tiles = (n + k - 1) / k;
+  int k = 1;
+  const LaunchShape shape = eval_shape(c, ci, n, &k);
+  const int n_tiles = (n + k - 1) / k;
   gd_noalloc_fill<<<(n + 255) / 256, 256, 0, c->stream>>>(ci, prt_conf, lig_conf, n, k);
   CK(cudaGetLastError());
   GdMcArgs a = base_args(c);
@@ -127,10 +129,12 @@ extern "C" int gd_eval_energy_noalloc(gd_ctx *c, int ci, int prt_conf, int lig_c
   a.tiles = s->tiles;
   a.n_tiles = n_tiles;
   a.tile_counter = &s->counter;
-  const size_t smem = smem_bytes(c);
-  if ((rc = set_kernel_attrs(c, smem))) return rc;
-  const int grid = grid_for(c, n_tiles, smem);
-  launch_kernel(c)<<<grid, launch_threads(c), smem, c->stream>>>(a, c->fc);
+  a.chunk = shape.chunk;
+  a.fold = shape.fold;
+  a.split = shape.split;
+  if ((rc = set_kernel_attrs(shape))) return rc;
+  const int grid = grid_for(c, n_tiles, shape);
+  launch_kernel(shape)<<<grid, launch_threads(shape), smem_bytes(shape), c->stream>>>(a, c->fc);
   CK(cudaGetLastError());
   return GD_OK;
 }

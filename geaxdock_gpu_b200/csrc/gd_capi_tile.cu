@@ -68,13 +68,22 @@ int gd_set_tile(gd_ctx *c, int k, const gd_tile *t) {
   }
   if (T > GD_MAX_TPB)
     return fail(GD_ERR_INVALID, "replicas_per_cta * split * lna exceeds %d lanes", GD_MAX_TPB);
+  if (S > 1) {
+    /* the splits of an atom run in different warps: whole warps per split (at most
+     * GD_MAX_TPB_SPLIT lanes, since k S lna fits GD_MAX_TPB) */
+    int wa = 1;
+    for (auto &x : info) wa = std::max(wa, (x.k * x.lna + 31) / 32);
+    T = S * wa * 32;
+    if (T > GD_MAX_TPB_SPLIT) return fail(GD_ERR_INVALID, "too many warps per split");
+  }
   c->info = info;
   c->threads = T;
-  c->chunk = t->chunk_points;
+  c->chunk = c->fold = t->chunk_points;
   c->split = S;
   c->fill_threads = t->threads;
   c->fill_cap = t->threads > 0 ? t->replicas_per_cta : 0;
   c->pack = P;
+  c->tile_auto = false;
   if (t->unroll) c->unroll = t->unroll;
   c->tile_gen += 1;
   build_tiles(c, 0, c->n_rep - 1, c->full_tiles);
@@ -118,6 +127,8 @@ int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile
   cudaEventCreate(&e1);
   const gd_tile keep_tile = {c->info[0].k, c->chunk, c->unroll, c->split, c->threads, c->pack};
   const int keep_fill_threads = c->fill_threads, keep_fill_cap = c->fill_cap;
+  const bool keep_auto = c->tile_auto;
+  const int keep_fold = c->fold;
   std::vector<int> keep_k;
   for (auto &x : c->info) keep_k.push_back(x.k);
   const int keep_threads = c->threads;
@@ -149,9 +160,9 @@ int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile
     a.trace_acc = nullptr;
     if (probe_steps == 0) {
       a.n_steps = 1;
-      if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters))) break; /* loads the kernel */
+      if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters, ctx_shape(c)))) break; /* loads the kernel */
       cudaEventRecord(e0, c->stream);
-      if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters))) break;
+      if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters, ctx_shape(c)))) break;
       cudaEventRecord(e1, c->stream);
       if (cudaEventSynchronize(e1) != cudaSuccess) {
         rc = fail(GD_ERR_CUDA, "gd_autotune: probe failed");
@@ -162,10 +173,10 @@ int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile
       probe_steps = std::max(1, std::min(c->mc.steps_per_exchange, (int)(20.0f / std::max(t1, 1e-3f))));
     }
     a.n_steps = probe_steps;
-    if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters))) break; /* warm-up */
+    if ((rc = launch_mc(c, a, c->d_tiles, n, c->d_counters, ctx_shape(c)))) break; /* warm-up */
     cudaEventRecord(e0, c->stream);
     for (int r = 0; r < repeats && rc == GD_OK; ++r)
-      rc = launch_mc(c, a, c->d_tiles, n, c->d_counters);
+      rc = launch_mc(c, a, c->d_tiles, n, c->d_counters, ctx_shape(c));
     cudaEventRecord(e1, c->stream);
     if (cudaEventSynchronize(e1) != cudaSuccess) {
       rc = fail(GD_ERR_CUDA, "gd_autotune: probe failed");
@@ -201,11 +212,13 @@ int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile
     for (int i = 0; i < c->n_complex; ++i) c->info[i].k = keep_k[i];
     c->threads = keep_threads;
     c->chunk = keep_tile.chunk_points;
+    c->fold = keep_fold;
     c->unroll = keep_tile.unroll;
     c->split = keep_tile.split;
     c->pack = keep_tile.replicas_per_lane;
     c->fill_threads = keep_fill_threads;
     c->fill_cap = keep_fill_cap;
+    c->tile_auto = keep_auto;
     c->tile_gen += 1;
     build_tiles(c, 0, c->n_rep - 1, c->full_tiles);
     if (rc == GD_OK) rc = fail(GD_ERR_INVALID, "gd_autotune: no candidate fits this batch");

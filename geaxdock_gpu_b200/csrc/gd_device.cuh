@@ -51,6 +51,15 @@
 #define GD_MAX_CELLS (1 << 22) /* cells per conformer grid; a larger box widens the cells */
 #define GD_MAX_CELLS_ALL (1 << 25) /* cells of all conformers of a complex together */
 #define GD_MAX_TPB 256         /* threads per CTA: 3 CTAs of 256 fit the register file */
+#define GD_CHUNK 512           /* slots per ring buffer and FP32 sum of the default tile */
+#define GD_MAX_TPB_SPLIT 512   /* threads per CTA of the split launches */
+/* work of the per-atom terms that a split's segments are balanced against, in units of one point
+ * pair: a segment's own set-up, the contact list, the kind list, the restraints, the tail */
+#define GD_COST_SEG 8
+#define GD_COST_CON 70
+#define GD_COST_KIND 90
+#define GD_COST_MCS 40
+#define GD_COST_TAIL 40
 #define GD_SLOT_BYTES 192      /* shared-memory bytes per replica slot (sizeof gd::Slot) */
 /* resident 256-thread CTAs per SM the register budget is set for, per unroll depth: 80
  * registers at four point pairs in flight, 64 below (no spills); the delayed-acceptance
@@ -217,6 +226,7 @@ struct GdMcArgs {
   int step0;                  /* step number of the first step (s1 + s2), added to *step_base */
   const int *step_base;       /* device cursor for graph replays (null: 0) */
   int chunk;                  /* protein points per shared-memory buffer (multiple of 4) */
+  int fold;                   /* slots after which a segment's FP32 sums go to FP64 (divides chunk) */
   int split;                  /* lanes per ligand atom (protein split), >= 1 */
   int move_kind;
   uint64_t seed;

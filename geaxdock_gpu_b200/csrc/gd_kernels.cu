@@ -212,30 +212,49 @@ __device__ __forceinline__ void pair_range(const float4 *__restrict__ PA,
   if (i1 & 1) pair_body<HDB, false, FAR>(PA[m1], PB[m1], ax2, ay2, az2, q, f, a);
 }
 
-/* Pair loop of one of the S lanes of an atom (split sp) over slots [i0, i1) of a segment:
- * every S-th point pair from pair i0 / 2 + sp, the pairs before slot im (even, or i1) in the
- * full form and the rest in the far form; the odd tail point goes to the lane whose turn it
- * is. Each lane's pairs and their order do not depend on im, and the two forms give the same
- * result on far pairs, so neither does its sum. */
-template <bool HDB, int UNROLL>
-__device__ __forceinline__ void pair_range_split(const float4 *__restrict__ PA,
-                                                 const float4 *__restrict__ PB, int i0, int im,
-                                                 int i1, int sp, int S, float ax, float ay,
-                                                 float az, const Pair2 &q,
-                                                 const GdForceConst &f, Acc &a) {
-  const float2 ax2 = f2(ax), ay2 = f2(ay), az2 = f2(az);
-  const int mm = im >> 1, m1 = i1 >> 1;
-  int m = (i0 >> 1) + sp;
-#pragma unroll UNROLL
-  for (; m < mm; m += S) pair_body<HDB, true, false>(PA[m], PB[m], ax2, ay2, az2, q, f, a);
-#pragma unroll UNROLL
-  for (; m < m1; m += S) pair_body<HDB, true, true>(PA[m], PB[m], ax2, ay2, az2, q, f, a);
-  if ((i1 & 1) && m == m1) {
-    if (2 * m1 >= im)
-      pair_body<HDB, false, true>(PA[m1], PB[m1], ax2, ay2, az2, q, f, a);
-    else
-      pair_body<HDB, false, false>(PA[m1], PB[m1], ax2, ay2, az2, q, f, a);
+/* One pair of slots of which the first n (0, 1, 2) are points of the range: the values of
+ * pair_body, kept for those. */
+template <bool HDB, bool FAR>
+__device__ __forceinline__ void pair_body_n(const float4 A, const float4 B, float2 ax, float2 ay,
+                                            float2 az, const Pair2 &q, const GdForceConst &f,
+                                            Acc &a, int n) {
+  Acc t = a;
+  pair_body<HDB, true, FAR>(A, B, ax, ay, az, q, f, t);
+  if (n > 0) {
+    a.vdw.x = t.vdw.x;
+    a.ele.x = t.ele.x;
+    a.pmf.x = t.pmf.x;
+    if (HDB) a.hdb.x = t.hdb.x;
   }
+  if (n > 1) {
+    a.vdw.y = t.vdw.y;
+    a.ele.y = t.ele.y;
+    a.pmf.y = t.pmf.y;
+    if (HDB) a.hdb.y = t.hdb.y;
+  }
+}
+
+/* pair_range for the split launches, where a warp has few others beside it and the latency of a
+ * body counts: the points left after the whole groups of four pairs run as one more group, its
+ * pairs in flight together, instead of one after the other (segments of a small pocket are some
+ * seven pairs long). The slots read past the range lie in the CTA's shared memory. */
+template <bool HDB, int UNROLL, bool FAR>
+__device__ __forceinline__ void pair_range_lat(const float4 *__restrict__ PA,
+                                               const float4 *__restrict__ PB, int i0, int i1,
+                                               float ax, float ay, float az, const Pair2 &q,
+                                               const GdForceConst &f, Acc &a) {
+  const float2 ax2 = f2(ax), ay2 = f2(ay), az2 = f2(az);
+  int m = i0 >> 1;
+#pragma unroll 1
+  for (; 2 * (m + UNROLL) <= i1; m += UNROLL)
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      pair_body<HDB, true, FAR>(PA[m + u], PB[m + u], ax2, ay2, az2, q, f, a);
+  const int r = i1 - 2 * m;
+  if (r > 0)
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u)
+      pair_body_n<HDB, FAR>(PA[m + u], PB[m + u], ax2, ay2, az2, q, f, a, r - 2 * u);
 }
 
 /* The same range for the same atom of two replicas (the lane's two slots): one load of each
@@ -281,11 +300,7 @@ __device__ __forceinline__ void short_range(const GdDevComplex &cx, int pc,
                                             const float *__restrict__ thr,
                                             const float *__restrict__ psprow,
                                             const GdForceConst &f, float ax, float ay, float az,
-                                            int part, int parts, ShortSums &s) {
-  s.hsum = 0.0;
-  s.psp = 0.0f;
-  s.ele = 0.0f;
-  s.ncon = 0;
+                                            ShortSums &s) {
   const int nx = cx.sr_n[0], ny = cx.sr_n[1], nz = cx.sr_n[2];
   const float R = cx.sr_r, R2 = cx.sr_r * cx.sr_r, ic = cx.sr_inv_cell, e = cx.sr_cell;
   const float r2max = cx.sr_r2;
@@ -314,20 +329,13 @@ __device__ __forceinline__ void short_range(const GdDevComplex &cx, int pc,
     b0 = __ldg(st + row + x0);
     b1 = __ldg(st + row + x1 + 1);
   };
-  /* rows part, part + parts, ... of the (iy, iz) order: the lanes of a split atom share them */
-  const int ny_span = y1 - y0 + 1;
-  int iy = y0 + part, iz = z0, n0 = 0, n1 = 0;
-  while (iy > y1) {
-    iy -= ny_span;
-    ++iz;
-  }
-  bool more = iz <= z1;
-  if (more) bounds(iy, iz, n0, n1);
+  int iy = y0, iz = z0, n0 = 0, n1 = 0;
+  bool more = true;
+  bounds(iy, iz, n0, n1);
   while (more) {
     const int c0 = n0, c1 = n1;
-    iy += parts;
-    while (iy > y1) {
-      iy -= ny_span;
+    if (++iy > y1) {
+      iy = y0;
       ++iz;
     }
     more = iz <= z1;
@@ -364,27 +372,23 @@ __device__ __forceinline__ void short_range(const GdDevComplex &cx, int pc,
 }
 
 /* The same terms for an atom inside the pocket grid, from its cell's two point lists
- * (gd_pocket.cu): the same points' terms added in the same order as short_range with parts = 1.
- * With parts > 1 (the S lanes of a split atom) lane `part` takes every parts-th quad. Bound by the
- * latency of a load per point: four points are in flight, and a point past the end of a list
- * is the sentinel. A warp's pass went from 87-135 k cycles (the row walk) to 20-34 k: 6,820
- * replicas of 40 atoms on 3,000 points, 11 steps, 11.75 -> 9.64 ms with the epilogue's changes. */
+ * (gd_pocket.cu), the contact list (con), the kind list (kind) or both: the same points' terms
+ * added in the same order as short_range. Bound by the latency of a load per point: four points
+ * are in flight, and a point past the end of a list is the sentinel. A warp's pass went from
+ * 87-135 k cycles (the row walk) to 20-34 k: 6,820 replicas of 40 atoms on 3,000 points, 11 steps,
+ * 11.75 -> 9.64 ms with the epilogue's changes. */
 __device__ __forceinline__ void short_range_lists(const GdDevComplex &cx, int pc, int cell,
                                                   const float *__restrict__ thr,
                                                   const float *__restrict__ psprow,
                                                   const GdForceConst &f, float ax, float ay,
-                                                  float az, int part, int parts, ShortSums &s) {
-  s.hsum = 0.0;
-  s.psp = 0.0f;
-  s.ele = 0.0f;
-  s.ncon = 0;
+                                                  float az, bool con, bool kind, ShortSums &s) {
   const int *__restrict__ st = cx.pg_start + (size_t)pc * (2 * GD_PG_CELLS + 1) + 2 * cell;
   const int s0 = __ldg(st), s1 = __ldg(st + 1), s2 = __ldg(st + 2);
   const ushort4 *__restrict__ ix =
       reinterpret_cast<const ushort4 *>(cx.pg_idx + __ldg(cx.pg_base + pc));
   const float4 *__restrict__ PA = cx.sr_a + (size_t)pc * (cx.pnp + 1);
   const float4 *__restrict__ PB = cx.sr_b + (size_t)pc * (cx.pnp + 1);
-  for (int i = (s0 >> 2) + part; i < (s1 >> 2); i += parts) {
+  for (int i = s0 >> 2; con && i < (s1 >> 2); ++i) {
     const ushort4 id = __ldg(ix + i);
     const int k[4] = {id.x, id.y, id.z, id.w};
     float4 p[4];
@@ -404,7 +408,7 @@ __device__ __forceinline__ void short_range_lists(const GdDevComplex &cx, int pc
       }
     }
   }
-  for (int i = (s1 >> 2) + part; i < (s2 >> 2); i += parts) {
+  for (int i = s1 >> 2; kind && i < (s2 >> 2); ++i) {
     const ushort4 id = __ldg(ix + i);
     const int k[4] = {id.x, id.y, id.z, id.w};
     float4 p[4];
@@ -525,19 +529,114 @@ struct Slot {
 };
 static_assert(sizeof(Slot) == GD_SLOT_BYTES, "slot layout");
 
-/* deterministic warp sum of a double */
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-
 #define NQ 10 /* vdw ele pmf psp hdb hsum->hpc kde rmsd ncon tp */
 #define MCS_U 4 /* restraint positions in flight in the epilogue */
 
+/* MCS position restraints of one replica's atoms, sum over positions of tcc rmsd (every lane of the
+ * warp returns it): MCS_U positions at a time, so that their loads and shuffles overlap, and the
+ * square roots of up to 32 positions at once, one per lane (one position after the other they took
+ * 20-29 k cycles a step at 8-11 positions, with lane 0's square roots 8-10 k). */
+__device__ __forceinline__ double restraints(const GdDevComplex &cx, int lig_conf, int L,
+                                             const float4 *atoms, int lane) {
+  double elhm = 0.0;
+  const int *meta_y = &cx.lig_meta[lig_conf * L].y;
+#pragma unroll 1
+  for (int mb = 0; mb < cx.pos; mb += 32) {
+    const int me = min(cx.pos, mb + 32);
+    double mine = 0.0; /* lane's position mb + lane: squared distances, atoms */
+    unsigned mine_n = 0;
+#pragma unroll 1
+    for (int m0 = mb; m0 < me; m0 += MCS_U) {
+      double sm[MCS_U];
+      unsigned cnt = 0; /* the positions' atom counts (<= GD_MAXLIG), 8 bits each */
+#pragma unroll
+      for (int u = 0; u < MCS_U; ++u) sm[u] = 0.0;
+      for (int i = lane; i < L; i += 32) {
+        const int idx = __ldg(meta_y + 2 * i);
+        const float4 at = atoms[i];
+#pragma unroll
+        for (int u = 0; u < MCS_U; ++u) {
+          const int m = min(m0 + u, cx.pos - 1);
+          const float4 r = __ldg(cx.mcs + (size_t)m * cx.mcs_ld + idx);
+          if (r.x != GD_MCS_INVALID_COORD) {
+            const float dx = at.x - r.x, dy = at.y - r.y, dz = at.z - r.z;
+            sm[u] += (double)(dx * dx + dy * dy + dz * dz);
+            cnt += 1u << (8 * u);
+          }
+        }
+      }
+      cnt = __reduce_add_sync(0xffffffffu, cnt);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int u = 0; u < MCS_U; ++u) sm[u] += __shfl_down_sync(0xffffffffu, sm[u], o);
+#pragma unroll
+      for (int u = 0; u < MCS_U; ++u) {
+        const double v = __shfl_sync(0xffffffffu, sm[u], 0);
+        if (mb + lane == m0 + u) {
+          mine = v;
+          mine_n = (cnt >> (8 * u)) & 255u;
+        }
+      }
+    }
+    double tcc = 0.0, root = 0.0;
+    if (mb + lane < me && mine_n) {
+      tcc = (double)cx.mcs_tcc[mb + lane];
+      root = sqrt(mine / (double)mine_n);
+    }
+    /* added in position order */
+    for (int m = mb; m < me; ++m)
+      elhm += __shfl_sync(0xffffffffu, tcc, m - mb) * __shfl_sync(0xffffffffu, root, m - mb);
+  }
+  return elhm;
+}
+
+/* The segments that split sp of S runs, as a bit mask (computed by a whole warp): the segments in
+ * the order of their number modulo S (so that every split has segments in every chunk) are cut
+ * into S ranges of about equal work, work in units of one point pair; the splits that also have a
+ * short-range list, the restraints or the per-atom tail get less of it. */
+__device__ __forceinline__ unsigned split_segments(const int4 *__restrict__ segs, int nseg, int sp,
+                                                   int S, int con_sp, int kind_sp, int mcs_sp,
+                                                   int lane) {
+  const int q = nseg / S, r = nseg - q * S;
+  int sg = 0, cost = 0;
+  if (lane < nseg) {
+    const int head = r * (q + 1);
+    const int c = lane < head ? lane / (q + 1) : r + (lane - head) / max(q, 1);
+    const int j = lane < head ? lane - c * (q + 1) : (lane - head) - (c - r) * max(q, 1);
+    sg = j * S + c;
+    const int4 g = __ldg(segs + sg);
+    const int n = (g.y - g.x + 1) >> 1;
+    cost = GD_COST_SEG + n + ((g.w & 4) ? n >> 2 : 0);
+  }
+  int sum = cost;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= o) sum += v;
+  }
+  const int total = __shfl_sync(0xffffffffu, sum, 31);
+  const int target = (total + GD_COST_CON + GD_COST_KIND + GD_COST_MCS + GD_COST_TAIL) / S;
+  auto room = [&](int p) {
+    return (float)max(1, target - (p == con_sp ? GD_COST_CON : 0) -
+                             (p == kind_sp ? GD_COST_KIND : 0) - (p == mcs_sp ? GD_COST_MCS : 0) -
+                             (p == 0 ? GD_COST_TAIL : 0));
+  };
+  float all = 0.0f;
+  for (int p = 0; p < S; ++p) all += room(p);
+  const float at = ((float)sum - 0.5f * (float)cost) * all / (float)max(total, 1);
+  int owner = 0;
+  float end = 0.0f;
+  for (int p = 0; p < S - 1; ++p) {
+    end += room(p);
+    owner += at >= end ? 1 : 0;
+  }
+  return __reduce_or_sync(0xffffffffu, lane < nseg && owner == sp ? 1u << sg : 0u);
+}
+
 /* One segment range of the pair loop, dispatched on the segment's flags (bit 2: live
  * hydrogen-bond term). */
-template <int UNROLL, int PACK, bool FAR>
+template <int UNROLL, int PACK, bool FAR, bool LAT = false>
 __device__ __forceinline__ void pair_dispatch(int flags, const float4 *PA, const float4 *PB,
                                               int i0, int i1, const float *ax, const float *ay,
                                               const float *az, const Pair2 &pq,
@@ -545,6 +644,8 @@ __device__ __forceinline__ void pair_dispatch(int flags, const float4 *PA, const
 #define GD_PR(H)                                                                             \
   if constexpr (PACK == 2)                                                                   \
     pair_range2<H, UNROLL, FAR>(PA, PB, i0, i1, ax, ay, az, pq, f, acc);                     \
+  else if constexpr (LAT)                                                                    \
+    pair_range_lat<H, UNROLL, FAR>(PA, PB, i0, i1, ax[0], ay[0], az[0], pq, f, acc[0]);      \
   else                                                                                       \
     pair_range<H, UNROLL, FAR>(PA, PB, i0, i1, ax[0], ay[0], az[0], pq, f, acc[0])
   if (flags & 4) {
@@ -655,7 +756,8 @@ __device__ __forceinline__ void da_decide(const GdMcArgs &a, const GdDevComplex 
  * word, the CTA leaves at the next step barrier after letting its copies in flight land.
  */
 template <int UNROLL, bool SPLIT, bool DA, int PACK>
-__global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, PACK, DA))
+__global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
+                                  SPLIT ? 1 : GD_MIN_BLOCKS_PACK(UNROLL, PACK, DA))
     gd_mc_kernel(GdMcArgs a, GdForceConst f) {
   static_assert(PACK == 1 || (PACK == 2 && !SPLIT && !DA),
                 "two replicas per lane: plain modes with one lane per atom");
@@ -674,6 +776,8 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
   __shared__ int s_tile, s_abort;
   __shared__ int s_done[2];
   __shared__ unsigned s_issued[2];
+  __shared__ double s_lhm[SPLIT ? GD_MAX_SLOTS : 1]; /* the slots' restraint sums */
+  __shared__ double s_norm[3][GD_MAXWEI];            /* a_para, b_para, w */
 
   if (tid == 0) {
     mbar_init(&bar[0], 1);
@@ -684,6 +788,13 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
     s_issued[0] = s_issued[1] = 0;
   }
   for (int i = tid; i < GD_MAXTP2 * GD_MAXTP1; i += NT) thr_s[i] = a.pp[i].thr;
+#pragma unroll
+  for (int i = 0; i < GD_MAXWEI; ++i)
+    if (tid == i) {
+      s_norm[0][i] = (double)f.a_para[i];
+      s_norm[1][i] = (double)f.b_para[i];
+      s_norm[2][i] = (double)f.w[i];
+    }
   __syncthreads();
   uint32_t consumed0 = 0, consumed1 = 0; /* completed phases waited for, per buffer */
   const int step_first = a.step0 + (a.step_base ? *a.step_base : 0);
@@ -710,14 +821,19 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       continue;
     }
     const GdDevComplex &cx = a.cx[tile.complex_index];
-    /* lane = (slot j, protein split sp, ligand atom l): the S copies of an atom each take
-     * every S-th point pair of every protein segment; S = 1 is one lane per atom */
-    const int L = cx.lna, S = SPLIT ? a.split : 1, SL = S * L;
+    /* lane = (split sp, slot j, ligand atom l): the S copies of an atom, in different warps (A
+     * lanes, whole warps, per split), each run some of the protein's segments and some of the
+     * other per-atom terms; S = 1 is one lane per atom */
+    const int L = cx.lna, S = SPLIT ? a.split : 1;
+    const int A = SPLIT ? NT / S : T;
     const int kp = (k + PACK - 1) / PACK; /* lane groups */
-    const bool active = tid < kp * SL;
-    const int jj = active ? tid / SL : 0;
-    const int sp = active ? (tid - jj * SL) / L : 0;
-    const int l = active ? tid - jj * SL - sp * L : 0;
+    const int sp = SPLIT ? tid / A : 0, ai = SPLIT ? tid - sp * A : tid;
+    const bool active = ai < kp * L;
+    const int jj = active ? ai / L : 0;
+    const int l = active ? ai - jj * L : 0;
+    /* the splits that run the short-range lists and the restraints (split 0: the far field, the
+     * per-atom tail) */
+    const int con_sp = S - 1, kind_sp = max(S - 2, 0), mcs_sp = S >= 4 ? S - 3 : S == 2 ? 1 : 0;
     /* the thread's lanes: slot jj (PACK 1), or slots 2 jj and 2 jj + 1, the same atom of two
      * replicas (PACK 2); a missing second slot (odd k) repeats the first one's atom and stores
      * nothing. sl_of: each lane's slot; vl: its index in the placed-atom and partial arrays */
@@ -728,7 +844,7 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       const int jh = jj * PACK + h;
       ok[h] = active && jh < k;
       sl_of[h] = ok[h] ? jh : jj * PACK;
-      vl[h] = sl_of[h] * SL + sp * L + l;
+      vl[h] = sp * A + sl_of[h] * L + l;
     }
 
     /* ---- slot set-up (one thread per replica) ---- */
@@ -789,43 +905,57 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
     const GdPairParam *pprow = a.pp + tl * GD_MAXTP1;
     const int4 *segs = cx.seg + pc * GD_MAX_SEG;
     const int nseg = cx.seg_count[pc];
+    const unsigned own =
+        SPLIT ? split_segments(segs, nseg, sp, S, con_sp, kind_sp, mcs_sp, lane) : 0u;
     bool aborted = false;
 
     for (int s = 0; s < nsteps; ++s) {
-      /* ---- Move_d: one thread per replica draws the move and builds the rotation ---- */
-      if (tid < k) {
-        Slot &sl = slots[tid];
-        float mmn[6], u = 0.0f;
-        if (a.mode == 0) {
-          float delta[6];
-          gd_draw_step(a.seed, (uint32_t)cx.stream, (uint32_t)(sl.rep - cx.rep_offset),
-                       (uint32_t)(step_first + s), a.move_kind, a.move_scale, delta, &u);
-#pragma unroll
-          for (int i = 0; i < 6; ++i) mmn[i] = GD_ADD(sl.mm_old[i], delta[i]);
-        } else if (a.mode == 2 || a.mode == 3) {
-#pragma unroll
-          for (int i = 0; i < 6; ++i) mmn[i] = a.mm_in[(size_t)sl.rep * 6 + i];
-        } else {
-#pragma unroll
-          for (int i = 0; i < 6; ++i) mmn[i] = 0.0f;
+      /* ---- Move_d: four lanes per replica draw the move (a Box-Muller pair each) and build the
+       * rotation (an angle each); one lane took 2.3-4 k cycles with every warp waiting ---- */
+      for (int jb = 0; jb < k; jb += NT >> 2) {
+        const int j = jb + (tid >> 2), q = tid & 3;
+        const bool mine = j < k && q < 3;
+        Slot &sl = slots[j < k ? j : 0];
+        float m0 = 0.0f, m1 = 0.0f, u = 0.0f; /* movematrix[2 q], [2 q + 1] */
+        if (mine) {
+          if (a.mode == 0) {
+            float d0, d1;
+            gd_draw_pair(a.seed, (uint32_t)cx.stream, (uint32_t)(sl.rep - cx.rep_offset),
+                         (uint32_t)(step_first + s), a.move_kind, q, &d0, &d1, &u);
+            m0 = GD_ADD(sl.mm_old[2 * q], GD_MUL(a.move_scale[2 * q], d0));
+            m1 = GD_ADD(sl.mm_old[2 * q + 1], GD_MUL(a.move_scale[2 * q + 1], d1));
+          } else if (a.mode == 2 || a.mode == 3) {
+            m0 = a.mm_in[(size_t)sl.rep * 6 + 2 * q];
+            m1 = a.mm_in[(size_t)sl.rep * 6 + 2 * q + 1];
+          }
+          sl.mm_new[2 * q] = m0;
+          sl.mm_new[2 * q + 1] = m1;
+          if (q == 2) sl.u = u;
         }
-        float rot[9];
-        gd_rotation(mmn, rot);
-#pragma unroll
-        for (int i = 0; i < 9; ++i) sl.rot[i] = rot[i];
-#pragma unroll
-        for (int i = 0; i < 6; ++i) sl.mm_new[i] = mmn[i];
-        const float *lc = cx.lig_center + sl.lig_conf * 3;
-        sl.tx = GD_ADD(mmn[0], lc[0]);
-        sl.ty = GD_ADD(mmn[1], lc[1]);
-        sl.tz = GD_ADD(mmn[2], lc[2]);
-        if (a.mode == 4) {
-          /* given coordinates: the ligand centre comes with them (Ligand.coord_new.center) */
-          sl.tx = a.center_in[(size_t)sl.rep * 3];
-          sl.ty = a.center_in[(size_t)sl.rep * 3 + 1];
-          sl.tz = a.center_in[(size_t)sl.rep * 3 + 2];
+        __syncwarp();
+        float sn = 0.0f, cn = 0.0f;
+        if (mine) gd_sincosf(sl.mm_new[3 + q], &sn, &cn);
+        const int l0 = lane & ~3;
+        const float s1 = __shfl_sync(0xffffffffu, sn, l0), c1 = __shfl_sync(0xffffffffu, cn, l0),
+                    s2 = __shfl_sync(0xffffffffu, sn, l0 + 1),
+                    c2 = __shfl_sync(0xffffffffu, cn, l0 + 1),
+                    s3 = __shfl_sync(0xffffffffu, sn, l0 + 2),
+                    c3 = __shfl_sync(0xffffffffu, cn, l0 + 2);
+        if (mine) {
+          if (q == 0) gd_rotation_sc(s1, c1, s2, c2, s3, c3, sl.rot);
+          if (q == 1) {
+            const float *lc = cx.lig_center + sl.lig_conf * 3;
+            sl.tx = GD_ADD(sl.mm_new[0], lc[0]);
+            sl.ty = GD_ADD(sl.mm_new[1], lc[1]);
+            sl.tz = GD_ADD(sl.mm_new[2], lc[2]);
+            if (a.mode == 4) {
+              /* given coordinates: the ligand centre comes with them (Ligand.coord_new.center) */
+              sl.tx = a.center_in[(size_t)sl.rep * 3];
+              sl.ty = a.center_in[(size_t)sl.rep * 3 + 1];
+              sl.tz = a.center_in[(size_t)sl.rep * 3 + 2];
+            }
+          }
         }
-        sl.u = u;
       }
       __syncthreads();
       float ax[PACK], ay[PACK], az[PACK];
@@ -843,7 +973,7 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
             gd_place_atom(sl.rot, sl.tx, sl.ty, sl.tz, orig[h].x, orig[h].y, orig[h].z, &ax[h],
                           &ay[h], &az[h]);
           }
-          if (ok[h]) atoms[vl[h]] = make_float4(ax[h], ay[h], az[h], 0.0f);
+          if (ok[h] && sp == 0) atoms[vl[h]] = make_float4(ax[h], ay[h], az[h], 0.0f);
         }
       }
       /* each lane clears its own partials (the only ones the epilogue reads) */
@@ -853,9 +983,19 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
 #pragma unroll
           for (int qi = 0; qi < NQ; ++qi) part[qi * T + vl[h]] = 0.0;
 
-      /* ---- short-range terms from the cell list (the S lanes of an atom take every S-th row
-       * of its walk), before the pair loop: warps whose walk is short start the loop while
-       * the others still walk ---- */
+      if constexpr (SPLIT) {
+        /* the restraints beside the pair loop, by the warps of one split */
+        __syncthreads();
+        const int wa = A >> 5, w0 = mcs_sp * wa;
+        if (warp >= w0 && warp < w0 + wa)
+          for (int js = warp - w0; js < k; js += wa) {
+            const double v = restraints(cx, slots[js].lig_conf, L, atoms + js * L, lane);
+            if (lane == 0) s_lhm[js] = v;
+          }
+      }
+
+      /* ---- short-range terms from the pocket grid's lists (or the cell list), before the pair
+       * loop: warps whose lists are short start the loop while the others still read ---- */
       /* lbin: the radius bin past which each lane's points come from the far fields
        * (GD_FAR_BINS - 1: every point runs in the loop) */
       int lbin[PACK];
@@ -863,18 +1003,25 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
       for (int h = 0; h < PACK; ++h) {
         lbin[h] = GD_FAR_BINS - 1;
         if (!ok[h]) continue;
-        ShortSums sr;
-        const int cell = pocket_cell(cx, ax[h], ay[h], az[h]);
-        if (cell >= 0)
-          short_range_lists(cx, pc, cell, thr_s + tl * GD_MAXTP1, psprow, f, ax[h], ay[h], az[h],
-                            sp, S, sr);
-        else
-          short_range(cx, pc, thr_s + tl * GD_MAXTP1, psprow, f, ax[h], ay[h], az[h], sp, S, sr);
         const int v = vl[h];
-        part[1 * T + v] = (double)sr.ele;
-        part[3 * T + v] = (double)sr.psp;
-        part[5 * T + v] = sr.hsum;
-        part[8 * T + v] = (double)sr.ncon;
+        const int cell = pocket_cell(cx, ax[h], ay[h], az[h]);
+        /* outside the grid the contact split walks the rows for both lists */
+        const bool con = sp == con_sp, kind = sp == (cell >= 0 ? kind_sp : con_sp);
+        if (con || kind) {
+          ShortSums sr = {0.0, 0.0f, 0.0f, 0};
+          const float *thr = thr_s + tl * GD_MAXTP1;
+          if (cell >= 0)
+            short_range_lists(cx, pc, cell, thr, psprow, f, ax[h], ay[h], az[h], con, kind, sr);
+          else
+            short_range(cx, pc, thr, psprow, f, ax[h], ay[h], az[h], sr);
+          part[1 * T + v] = (double)sr.ele;
+          part[3 * T + v] = (double)sr.psp;
+          part[8 * T + v] = (double)sr.ncon;
+          if (kind) {
+            const double hpc2 = (sr.hsum - (double)f.hpl0[tl]) / (double)f.hpl1[tl];
+            part[5 * T + v] = 0.5 * hpc2 * hpc2 - (double)f.hpl2[tl];
+          }
+        }
         const int fcell = cx.ff_tab != nullptr ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
         if (fcell >= 0) {
           const int id = __ldg(cx.ff_id + fcell);
@@ -928,50 +1075,46 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
           const float4 *PA = bpa + b * (D >> 1); /* local slot = slot - c0 */
           const float4 *PB = bpb + b * (D >> 1);
           const int c0 = ci * D, c1 = min(pnp_pad, c0 + D);
-          for (int sg = sg0; sg < nseg; ++sg) {
-            const int4 g = segs[sg];
-            if (g.x >= c1) break;
-            if (g.y <= c1) sg0 = sg + 1;
-            const int i0 = max(g.x, c0) - c0;
-            /* each lane's end of the segment: where its far field takes over */
-            int il[PACK], i1 = 0;
+          /* blocks of `fold` slots, at whose ends a segment's sums go to FP64: the whole chunk, or
+           * the default tile's chunks where the ring's are larger */
+          for (int b0 = c0; b0 < c1; b0 += a.fold) {
+            const int b1 = min(c1, b0 + a.fold);
+            for (int sg = sg0; sg < nseg; ++sg) {
+              const int4 g = segs[sg];
+              if (g.x >= b1) break;
+              if (g.y <= b1) sg0 = sg + 1;
+              if (SPLIT && !((own >> sg) & 1u)) continue;
+              const int i0 = max(g.x, b0) - c0;
+              /* each lane's end of the segment: where its far field takes over */
+              int il[PACK], i1 = 0;
 #pragma unroll
-            for (int h = 0; h < PACK; ++h) {
-              const int e = PACK > 1 && !ok[h] ? g.x
-                            : lbin[h] == GD_FAR_BINS - 1 ? g.y
-                                                         : gd_ff_near(cx, pc, sg, g, lbin[h]);
-              il[h] = min(e, c1) - c0;
-              i1 = max(i1, il[h]);
-            }
-            if (i0 >= i1) continue;
-            const float4 *pr = reinterpret_cast<const float4 *>(pprow + g.z);
-            const float4 q0 = __ldg(pr), q1 = __ldg(pr + 1), q2 = __ldg(pr + 2);
-            Pair2 pq;
-            pq.p1a = f2(q0.x); pq.mp2a = f2(-q0.y); pq.p1l = f2(q0.z);
-            pq.p1ll = f2(q0.z * f.lj1); pq.hc1 = f2(q1.z); pq.hc0 = f2(q1.w);
-            pq.hs = f2(q2.x); pq.b2 = f2(q2.z); pq.c2 = f2(q2.w);
-            const float2 z2 = f2(0.0f);
-            Acc acc[PACK];
+              for (int h = 0; h < PACK; ++h) {
+                const int e = PACK > 1 && !ok[h] ? g.x
+                              : lbin[h] == GD_FAR_BINS - 1 ? g.y
+                                                           : gd_ff_near(cx, pc, sg, g, lbin[h]);
+                il[h] = min(e, b1) - c0;
+                i1 = max(i1, il[h]);
+              }
+              if (i0 >= i1) continue;
+              const float4 *pr = reinterpret_cast<const float4 *>(pprow + g.z);
+              const float4 q0 = __ldg(pr), q1 = __ldg(pr + 1), q2 = __ldg(pr + 2);
+              Pair2 pq;
+              pq.p1a = f2(q0.x); pq.mp2a = f2(-q0.y); pq.p1l = f2(q0.z);
+              pq.p1ll = f2(q0.z * f.lj1); pq.hc1 = f2(q1.z); pq.hc0 = f2(q1.w);
+              pq.hs = f2(q2.x); pq.b2 = f2(q2.z); pq.c2 = f2(q2.w);
+              const float2 z2 = f2(0.0f);
+              Acc acc[PACK];
 #pragma unroll
-            for (int h = 0; h < PACK; ++h) acc[h] = {z2, z2, z2, z2};
-            /* the segment's near points [i0, im) and far points [im, i1); the split slot is
-             * even (the segment starts on one), so the near part keeps whole slot pairs */
-            const int fs = g.x + ((__ldg(fcnt + sg * GD_FAR_BINS) + 1) & ~1) - c0;
-            const int im = min(i1, max(i0, fs));
-            if constexpr (SPLIT) {
-              /* the S lanes of an atom take every S-th point pair of the range */
-              if (g.w & 4)
-                pair_range_split<true, UNROLL>(PA, PB, i0, im, i1, sp, S, ax[0], ay[0], az[0],
-                                               pq, f, acc[0]);
-              else
-                pair_range_split<false, UNROLL>(PA, PB, i0, im, i1, sp, S, ax[0], ay[0], az[0],
-                                                pq, f, acc[0]);
-            } else {
+              for (int h = 0; h < PACK; ++h) acc[h] = {z2, z2, z2, z2};
+              /* the segment's near points [i0, im) and far points [im, i1); the split slot is
+               * even (the segment starts on one), so the near part keeps whole slot pairs */
+              const int fs = g.x + ((__ldg(fcnt + sg * GD_FAR_BINS) + 1) & ~1) - c0;
+              const int im = min(i1, max(i0, fs));
               if constexpr (PACK == 1) {
                 if (i0 < im)
-                  pair_dispatch<UNROLL, 1, false>(g.w, PA, PB, i0, im, ax, ay, az, pq, f, acc);
+                  pair_dispatch<UNROLL, 1, false, SPLIT>(g.w, PA, PB, i0, im, ax, ay, az, pq, f, acc);
                 if (im < i1)
-                  pair_dispatch<UNROLL, 1, true>(g.w, PA, PB, im, i1, ax, ay, az, pq, f, acc);
+                  pair_dispatch<UNROLL, 1, true, SPLIT>(g.w, PA, PB, im, i1, ax, ay, az, pq, f, acc);
               } else {
                 /* both lanes' points together, then the rest of the lane that has more */
                 const int ib = max(i0, min(il[0], il[1])), imb = min(im, ib);
@@ -990,15 +1133,15 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
                                                    pq, f, acc + h);
                 }
               }
-            }
 #pragma unroll
-            for (int h = 0; h < PACK; ++h) {
-              if (!ok[h]) continue;
-              const int v = vl[h];
-              part[0 * T + v] += (double)acc[h].vdw.x + (double)acc[h].vdw.y;
-              part[1 * T + v] += (double)acc[h].ele.x + (double)acc[h].ele.y;
-              part[2 * T + v] += (double)q1.y * ((double)acc[h].pmf.x + (double)acc[h].pmf.y);
-              part[4 * T + v] += (double)acc[h].hdb.x + (double)acc[h].hdb.y;
+              for (int h = 0; h < PACK; ++h) {
+                if (!ok[h]) continue;
+                const int v = vl[h];
+                part[0 * T + v] += (double)acc[h].vdw.x + (double)acc[h].vdw.y;
+                part[1 * T + v] += (double)acc[h].ele.x + (double)acc[h].ele.y;
+                part[2 * T + v] += (double)q1.y * ((double)acc[h].pmf.x + (double)acc[h].pmf.y);
+                part[4 * T + v] += (double)acc[h].hdb.x + (double)acc[h].hdb.y;
+              }
             }
           }
         }
@@ -1023,24 +1166,13 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
         }
       }
 
-      /* ---- per-atom tail (split 0 of each atom): hpc, kde, rmsd, reference contacts ---- */
-      if (S > 1) {
-        /* hpc is nonlinear in the atom's hydrophobic sum: gather the splits' parts first */
-        __syncthreads();
-        if (ok[0] && sp == 0)
-          for (int q = 1; q < S; ++q) {
-            part[5 * T + vl[0]] += part[5 * T + vl[0] + q * L];
-            part[5 * T + vl[0] + q * L] = 0.0;
-          }
-      }
+      /* ---- per-atom tail (split 0 of each atom): kde, rmsd, reference contacts ---- */
 #pragma unroll
       for (int h = 0; h < PACK; ++h) {
         if (!ok[h] || aborted) continue;
         const int v = vl[h];
         part[1 * T + v] *= (double)orig[h].w;
         if (sp != 0) continue;
-        const double hpc2 = (part[5 * T + v] - (double)f.hpl0[tl]) / (double)f.hpl1[tl];
-        part[5 * T + v] = 0.5 * hpc2 * hpc2 - (double)f.hpl2[tl];
         float ks = 0.0f;
         /* the KDE points lie sorted by type, in their given order within a type: the atom sums
          * its own type's points only. Latency-bound (a chain of additions per atom): four loads
@@ -1072,20 +1204,32 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
         break;
       }
 
+      if constexpr (SPLIT) {
+        /* each atom's partials of its splits, added in split order by all threads */
+        for (int i = tid; i < NQ * k * L; i += NT) {
+          const int q = i / (k * L);
+          double *p = part + q * T + (i - q * k * L);
+          double t = p[0];
+          for (int z = 1; z < S; ++z) t += p[z * A];
+          p[0] = t;
+        }
+        __syncthreads();
+      }
+
       /* ---- per-replica epilogue: one warp per slot ---- */
       for (int js = warp; js < k; js += nwarps) {
         Slot &sl = slots[js];
         /* slot totals are written back over the slot's first partial; five quantities at a time,
          * so that their shuffles overlap (one at a time the chain took 7-9 k cycles a step) */
-        double *tot = part + js * SL;
+        double *tot = part + js * L;
 #pragma unroll 1
         for (int q0 = 0; q0 < NQ; q0 += 5) {
           double v[5];
 #pragma unroll
           for (int u = 0; u < 5; ++u) v[u] = 0.0;
-          for (int i = lane; i < SL; i += 32)
+          for (int i = lane; i < L; i += 32)
 #pragma unroll
-            for (int u = 0; u < 5; ++u) v[u] += part[(q0 + u) * T + js * SL + i];
+            for (int u = 0; u < 5; ++u) v[u] += part[(q0 + u) * T + js * L + i];
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
@@ -1094,77 +1238,47 @@ __global__ void __launch_bounds__(GD_MAX_TPB / PACK, GD_MIN_BLOCKS_PACK(UNROLL, 
 #pragma unroll
             for (int u = 0; u < 5; ++u) tot[(q0 + u) * T] = v[u];
         }
-        /* MCS position restraints, MCS_U positions at a time: their loads and shuffles overlap
-         * (one at a time, each waited for its own: 20-29 k cycles a step at 8-11 positions) */
-        double elhm = 0.0;
-        const int *meta_y = &cx.lig_meta[sl.lig_conf * L].y;
-#pragma unroll 1
-        for (int m0 = 0; m0 < cx.pos; m0 += MCS_U) {
-          double sm[MCS_U];
-          unsigned cnt = 0; /* the positions' atom counts (<= GD_MAXLIG), 8 bits each */
-#pragma unroll
-          for (int u = 0; u < MCS_U; ++u) sm[u] = 0.0;
-          for (int i = lane; i < L; i += 32) {
-            const int idx = __ldg(meta_y + 2 * i);
-            const float4 at = atoms[js * SL + i];
-#pragma unroll
-            for (int u = 0; u < MCS_U; ++u) {
-              const int m = min(m0 + u, cx.pos - 1);
-              const float4 r = __ldg(cx.mcs + (size_t)m * cx.mcs_ld + idx);
-              if (r.x != GD_MCS_INVALID_COORD) {
-                const float dx = at.x - r.x, dy = at.y - r.y, dz = at.z - r.z;
-                sm[u] += (double)(dx * dx + dy * dy + dz * dz);
-                cnt += 1u << (8 * u);
-              }
-            }
-          }
-          cnt = __reduce_add_sync(0xffffffffu, cnt);
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int u = 0; u < MCS_U; ++u) sm[u] += __shfl_down_sync(0xffffffffu, sm[u], o);
-          if (lane == 0)
-#pragma unroll
-            for (int u = 0; u < MCS_U; ++u) {
-              const unsigned n = (cnt >> (8 * u)) & 255u;
-              if (m0 + u < cx.pos && n)
-                elhm += (double)cx.mcs_tcc[m0 + u] * sqrt(sm[u] / (double)n);
-            }
+        const double elhm = SPLIT ? s_lhm[js] : restraints(cx, sl.lig_conf, L, atoms + js * L, lane);
+        /* the nine normalised terms, MCC and RMSD, a lane each; the total in term order (all by
+         * lane 0 they took 3-5 k cycles) */
+        __syncwarp();
+        const double Ld = (double)L;
+        /* every lane's division, square root and logarithm at the same time as the others' */
+        const double tp = tot[9 * T];
+        const double fp = tot[8 * T] - tp, fn = (double)cx.nref_total - tp;
+        const double tn = Ld * (double)P - tp - fp - fn;
+        double e = lane < 6 ? tot[lane * T] : lane == 6 ? tot[6 * T] : lane == 7 ? elhm : tot[7 * T];
+        e /= lane == 6 ? (double)f.kde3 : lane == 7 ? (double)cx.pos : Ld;
+        if (lane >= 8) {
+          const double dx = (double)sl.tx - (double)cx.pocket[0];
+          const double dy = (double)sl.ty - (double)cx.pocket[1];
+          const double dz = (double)sl.tz - (double)cx.pocket[2];
+          e = sqrt(lane == 8 ? dx * dx + dy * dy + dz * dz
+                   : lane == 9 ? (tp + fp) * (tp + fn) * (tn + fp) * (tn + fn) : e);
+        } else if (lane == 7) {
+          e = log(e);
         }
-        if (lane == 0) {
-          const double Ld = (double)L;
-          double e[GD_MAXWEI];
-          e[0] = tot[0 * T] / Ld;
-          e[1] = tot[1 * T] / Ld;
-          e[2] = tot[2 * T] / Ld;
-          e[3] = tot[3 * T] / Ld;
-          e[4] = tot[4 * T] / Ld;
-          e[5] = tot[5 * T] / Ld;
-          e[6] = tot[6 * T] / (double)f.kde3 / Ld;
-          e[7] = log(elhm / (double)cx.pos);
-          {
-            const double dx = (double)sl.tx - (double)cx.pocket[0];
-            const double dy = (double)sl.ty - (double)cx.pocket[1];
-            const double dz = (double)sl.tz - (double)cx.pocket[2];
-            e[8] = sqrt(dx * dx + dy * dy + dz * dz);
-          }
-          double etot = 0.0;
-          gd_energy en;
+        float side = 0.0f; /* lane 9: MCC, lane 10: RMSD */
+        if (lane == 6 || lane == 9) {
+          const double q = (lane == 6 ? e : tp * tn - fp * fn) / (lane == 6 ? Ld : e);
+          side = e != 0.0 ? (float)q : 0.0f;
+          if (lane == 6) e = q;
+        } else if (lane == 10) {
+          side = (float)e;
+        }
+        if (lane < GD_MAXWEI - 1) e = s_norm[0][lane] * e + s_norm[1][lane];
+        gd_energy en;
+        double etot = 0.0;
 #pragma unroll
-          for (int i = 0; i < GD_MAXWEI - 1; ++i) {
-            const double v = (double)f.a_para[i] * e[i] + (double)f.b_para[i];
-            en.e[i] = (float)v;
-            etot += v * (double)f.w[i];
-          }
-          en.e[GD_MAXWEI - 1] = (float)etot;
-          {
-            const double tp = tot[9 * T], ncn = tot[8 * T];
-            const double fp = ncn - tp, fn = (double)cx.nref_total - tp;
-            const double tn = Ld * (double)P - tp - fp - fn;
-            const double dv2 = sqrt((tp + fp) * (tp + fn) * (tn + fp) * (tn + fn));
-            en.cms = dv2 != 0.0 ? (float)((tp * tn - fp * fn) / dv2) : 0.0f;
-          }
-          en.rmsd = (float)sqrt(tot[7 * T] / Ld);
+        for (int i = 0; i < GD_MAXWEI - 1; ++i) {
+          const double v = __shfl_sync(0xffffffffu, e, i);
+          en.e[i] = (float)v;
+          etot += v * s_norm[2][i];
+        }
+        en.e[GD_MAXWEI - 1] = (float)etot;
+        en.cms = __shfl_sync(0xffffffffu, side, 9);
+        en.rmsd = __shfl_sync(0xffffffffu, side, 10);
+        if (lane == 0) {
           const int rid = sl.rep;
           if (a.mode == 2 || a.mode == 4) {
             a.e_out[rid] = en;

@@ -168,25 +168,34 @@ GD_HD void gd_box_muller(uint32_t a, uint32_t b, float *z0, float *z1) {
 }
 
 /* ---------------- proposal for one replica and one step ---------------- */
-/* Draws the six move deltas and the accept uniform for (stream, replica, step).
- * stream identifies the complex (so a complex run alone or inside a batch draws the same
- * numbers); replica is the complex-local flat index n_tmp*n_lig*p + n_lig*t + l. */
+/* Components 2 q and 2 q + 1 (q = 0..2) of the unscaled move of (stream, replica, step), and the
+ * accept uniform when q is 2. stream identifies the complex (so a complex run alone or inside a
+ * batch draws the same numbers); replica is the complex-local flat index
+ * n_tmp*n_lig*p + n_lig*t + l. */
+GD_HD void gd_draw_pair(uint64_t seed, uint32_t stream, uint32_t replica, uint32_t step,
+                        int move_kind, int q, float *d0, float *d1, float *u_accept) {
+  const gd_u32x4 a = gd_philox4x32_10(replica, step, stream, q < 2 ? GD_RNG_MOVE : GD_RNG_MOVE2,
+                                      (uint32_t)seed, (uint32_t)(seed >> 32));
+  const uint32_t w0 = q == 1 ? a.v[2] : a.v[0], w1 = q == 1 ? a.v[3] : a.v[1];
+  if (move_kind == 1) {
+    gd_box_muller(w0, w1, d0, d1);
+  } else {
+    *d0 = gd_sym11(w0);
+    *d1 = gd_sym11(w1);
+  }
+  if (q == 2) *u_accept = gd_u01(a.v[2]);
+}
+
+/* The six scaled move deltas and the accept uniform of (stream, replica, step). */
 GD_HD void gd_draw_step(uint64_t seed, uint32_t stream, uint32_t replica, uint32_t step,
                         int move_kind, const float scale[6], float delta[6], float *u_accept) {
-  const uint32_t k0 = (uint32_t)seed, k1 = (uint32_t)(seed >> 32);
-  const gd_u32x4 a = gd_philox4x32_10(replica, step, stream, GD_RNG_MOVE, k0, k1);
-  const gd_u32x4 b = gd_philox4x32_10(replica, step, stream, GD_RNG_MOVE2, k0, k1);
-  if (move_kind == 1) {
-    float z[6];
-    gd_box_muller(a.v[0], a.v[1], &z[0], &z[1]);
-    gd_box_muller(a.v[2], a.v[3], &z[2], &z[3]);
-    gd_box_muller(b.v[0], b.v[1], &z[4], &z[5]);
-    for (int i = 0; i < 6; ++i) delta[i] = GD_MUL(scale[i], z[i]);
-  } else {
-    const uint32_t w[6] = {a.v[0], a.v[1], a.v[2], a.v[3], b.v[0], b.v[1]};
-    for (int i = 0; i < 6; ++i) delta[i] = GD_MUL(scale[i], gd_sym11(w[i]));
+GD_UNROLL
+  for (int q = 0; q < 3; ++q) {
+    float d0, d1;
+    gd_draw_pair(seed, stream, replica, step, move_kind, q, &d0, &d1, u_accept);
+    delta[2 * q] = GD_MUL(scale[2 * q], d0);
+    delta[2 * q + 1] = GD_MUL(scale[2 * q + 1], d1);
   }
-  *u_accept = gd_u01(b.v[2]);
 }
 
 /* Uniform of the surrogate (first) stage of a delayed-acceptance step: the spare word of the
@@ -208,12 +217,9 @@ GD_HD float gd_draw_exchange(uint64_t seed, uint32_t stream, uint32_t group,
 }
 
 /* ---------------- rigid-body transform (reference Move_d, src/kernel_cuda_l2_move.cu:21-80) ---------------- */
-/* Z-Y-X Euler rotation from movematrix[3..5]. */
-GD_HD void gd_rotation(const float mm[6], float rot[9]) {
-  float s1, c1, s2, c2, s3, c3;
-  gd_sincosf(mm[3], &s1, &c1);
-  gd_sincosf(mm[4], &s2, &c2);
-  gd_sincosf(mm[5], &s3, &c3);
+/* Z-Y-X Euler rotation from the sines and cosines of movematrix[3..5]. */
+GD_HD void gd_rotation_sc(float s1, float c1, float s2, float c2, float s3, float c3,
+                          float rot[9]) {
   rot[0] = GD_MUL(c1, c2);
   rot[1] = GD_SUB(GD_MUL(GD_MUL(c1, s2), s3), GD_MUL(c3, s1));
   rot[2] = GD_ADD(GD_MUL(s1, s3), GD_MUL(GD_MUL(c1, c3), s2));
@@ -223,6 +229,14 @@ GD_HD void gd_rotation(const float mm[6], float rot[9]) {
   rot[6] = -s2;
   rot[7] = GD_MUL(c2, s3);
   rot[8] = GD_MUL(c2, c3);
+}
+
+GD_HD void gd_rotation(const float mm[6], float rot[9]) {
+  float s1, c1, s2, c2, s3, c3;
+  gd_sincosf(mm[3], &s1, &c1);
+  gd_sincosf(mm[4], &s2, &c2);
+  gd_sincosf(mm[5], &s3, &c3);
+  gd_rotation_sc(s1, c1, s2, c2, s3, c3, rot);
 }
 
 /* x_lab = R x_orig + t + c_orig, with the translation folded first. */

@@ -165,10 +165,11 @@ typedef struct {
   int replicas_per_cta;     /* replicas sharing one protein tile in one CTA */
   int chunk_points;         /* protein points staged per shared-memory buffer */
   int unroll;               /* protein point pairs in flight per lane: 1, 2 or 4 (0: keep) */
-  int split;                /* lanes per ligand atom, each walking 1/split of every protein
-                               segment (0 or 1: one lane per atom); replicas_per_cta * split *
-                               atoms must fit one CTA. The energies' FP32 summation order depends
-                               on it (results within the parity tolerance of each other). */
+  int split;                /* lanes per ligand atom, in different warps, each running some of
+                               the protein's type segments (0 or 1: one lane per atom);
+                               replicas_per_cta * split * atoms must fit 256 lanes. Only the order
+                               of FP64 additions depends on it. A context without gd_set_tile
+                               splits launches of few replicas by itself. */
   int threads;              /* CTA size (multiple of 32, <= 256); 0: the smallest that holds
                                replicas_per_cta replicas of every complex. With threads > 0 each
                                complex gets as many replicas as fill the CTA (at most
@@ -372,7 +373,7 @@ typedef struct {
                                below this reverts to plain MC (0: never) */
   long long fallback_window;/* surviving proposals per complex between decisions */
   uint64_t seed;            /* weight init and batch draws */
-  int split;                /* protein split of the exact stage (gd_tile.split); 0: chosen per
+  int split;                /* split of the exact stage (gd_tile.split); 0: chosen per
                                gd_da_run from the surrogate stage's pass rate (1 when every
                                proposal survives, up to the CTA's limit when few do) */
   int pad;
