@@ -41,9 +41,9 @@
 #define GD_PG_CELLS (GD_PG_N * GD_PG_N * GD_PG_N)
 #define GD_PG_EDGE 4.0f
 /* the far fields: cells of GD_FF_EDGE A, a cube of GD_FF_N^3 centred on the pocket centre, of
- * which those reaching no further than half its edge from the centre are tabulated; Chebyshev
- * series of total degree GD_FF_DEG, GD_FF_NC coefficients (padded to whole float4) */
-#define GD_FF_N 18
+ * which those of a ball are tabulated; Chebyshev series of total degree GD_FF_DEG, GD_FF_NC
+ * coefficients (padded to whole float4) */
+#define GD_FF_N 22
 #define GD_FF_CELLS (GD_FF_N * GD_FF_N * GD_FF_N)
 #define GD_FF_EDGE 2.0f
 #define GD_FF_DEG 4
@@ -60,7 +60,10 @@
 #define GD_COST_KIND 90
 #define GD_COST_MCS 40
 #define GD_COST_TAIL 40
-#define GD_SLOT_BYTES 192      /* shared-memory bytes per replica slot (sizeof gd::Slot) */
+#define GD_SLOT_BYTES 248      /* shared-memory bytes per replica slot (sizeof gd::Slot) */
+/* a decision on a field-based energy stands when it is the same at this share of the sum of its
+ * weighted terms' magnitudes above and below (the fields' error is some 1e-7 of it) */
+#define GD_CERT 1e-5f
 /* resident 256-thread CTAs per SM the register budget is set for, per unroll depth: 80
  * registers at four point pairs in flight, 64 below (no spills); the delayed-acceptance
  * variants keep one CTA fewer (80 at two pairs, 128 at four), where 64 and 80 would spill */

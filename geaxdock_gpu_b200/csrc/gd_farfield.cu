@@ -293,18 +293,7 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
     for (int i = 0; i < d.n_lig * d.lna; ++i) g->used[d.lig_t[i]] = true;
   }
   if (groups.empty()) return GD_OK;
-  /* the tabulated cells: boxes within half the cube's edge of the centre */
-  std::vector<int> cells;
-  std::vector<short> id(GD_FF_CELLS, -1);
-  for (int k = 0; k < GD_FF_CELLS; ++k)
-    if (4 * cell_reach2(k) <= GD_FF_N * GD_FF_N) {
-      id[k] = (short)cells.size();
-      cells.push_back(k);
-    }
-  int *d_cells = nullptr;
-  short *d_id = nullptr;
   int rc;
-  if ((rc = upload(c, &d_cells, cells)) || (rc = upload(c, &d_id, id))) return rc;
   CK(cudaFuncSetAttribute(gd::farfield_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)((1 + GD_MAXTP2) * gd::NODES * sizeof(double))));
   std::vector<gd::FfArgs> jobs;
@@ -312,9 +301,25 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
   for (auto &gp : groups) {
     gd::FfArgs a{};
     a.pp = c->d_pp;
+    a.rep = gp->members[0];
+    /* the tabulated cells: those whose far radius leaves a tenth of a ball of points beyond it,
+     * at most the cube's inscribed ball (22 A; an atom outside runs all points in its loop) */
+    const double rad_max = (GD_FAR_BINS - 1) / (double)dcx[a.rep].far_inv_w;
+    const double reach =
+        std::min(0.5 * GD_FF_N, std::max(4.0, (0.965 * rad_max - r_f) / GD_FF_EDGE));
+    std::vector<int> cells;
+    std::vector<short> id(GD_FF_CELLS, -1);
+    for (int k = 0; k < GD_FF_CELLS; ++k)
+      if (cell_reach2(k) <= reach * reach) {
+        id[k] = (short)cells.size();
+        cells.push_back(k);
+      }
+    int *d_cells = nullptr;
+    short *d_id = nullptr;
+    if ((rc = upload(c, &d_cells, cells)) || (rc = upload(c, &d_id, id))) return rc;
+    CK(cudaStreamSynchronize(c->stream)); /* the host vectors end here */
     a.cells = d_cells;
     a.n_cells = (int)cells.size();
-    a.rep = gp->members[0];
     a.lj1 = ff->lj1;
     unsigned char slot[GD_MAXTP2] = {};
     for (int t = 0; t < GD_MAXTP2; ++t)

@@ -526,6 +526,11 @@ struct Slot {
   float tx, ty, tz;
   gd_energy e_old;
   gd_replica replica;
+  /* a decision too close to take from the fields' energies: the proposal's energies, and its total
+   * by the pair loop over every point */
+  gd_energy e_prop;
+  float e_full;
+  int open;
 };
 static_assert(sizeof(Slot) == GD_SLOT_BYTES, "slot layout");
 
@@ -773,7 +778,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
   float4 *atoms = bpb + D;
   double *part = reinterpret_cast<double *>(atoms + T);
   Slot *slots = reinterpret_cast<Slot *>(part + NQ * T);
-  __shared__ int s_tile, s_abort;
+  __shared__ int s_tile, s_abort, s_open;
   __shared__ int s_done[2];
   __shared__ unsigned s_issued[2];
   __shared__ double s_lhm[SPLIT ? GD_MAX_SLOTS : 1]; /* the slots' restraint sums */
@@ -784,6 +789,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     mbar_init(&bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_abort = 0;
+    s_open = 0;
     s_done[0] = s_done[1] = 0;
     s_issued[0] = s_issued[1] = 0;
   }
@@ -853,6 +859,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
       const int id = tile.rep_begin + tid;
       s.rep = id;
       s.accept = 0;
+      s.open = 0;
       if (a.mode >= 2) {
         s.lig_conf = a.lig_conf_in[id];
       } else {
@@ -909,7 +916,14 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         SPLIT ? split_segments(segs, nseg, sp, S, con_sp, kind_sp, mcs_sp, lane) : 0u;
     bool aborted = false;
 
-    for (int s = 0; s < nsteps; ++s) {
+    /* A step may take three passes. Energies from the far fields differ from those of the pair
+     * loop over every point in the last FP32 digits; a Metropolis decision that could hang on
+     * that (about one in 10^4, GD_CERT) is left open in the first pass (phase 0), the CTA then
+     * evaluates the proposal (phase 1) and the current pose (phase 2) without the fields, and the
+     * slots left open decide on those: every decision is the one the plain loop takes. */
+    const bool certify = a.mode == 0 && cx.ff_tab != nullptr;
+    int phase = 0, q_run = 0;
+    for (int s = 0; s < nsteps;) {
       /* ---- Move_d: four lanes per replica draw the move (a Box-Muller pair each) and build the
        * rotation (an angle each); one lane took 2.3-4 k cycles with every warp waiting ---- */
       for (int jb = 0; jb < k; jb += NT >> 2) {
@@ -917,7 +931,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         const bool mine = j < k && q < 3;
         Slot &sl = slots[j < k ? j : 0];
         float m0 = 0.0f, m1 = 0.0f, u = 0.0f; /* movematrix[2 q], [2 q + 1] */
-        if (mine) {
+        const float *mm = phase == 2 ? sl.mm_old : sl.mm_new;
+        if (mine && phase == 0) {
           if (a.mode == 0) {
             float d0, d1;
             gd_draw_pair(a.seed, (uint32_t)cx.stream, (uint32_t)(sl.rep - cx.rep_offset),
@@ -934,7 +949,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         }
         __syncwarp();
         float sn = 0.0f, cn = 0.0f;
-        if (mine) gd_sincosf(sl.mm_new[3 + q], &sn, &cn);
+        if (mine) gd_sincosf(mm[3 + q], &sn, &cn);
         const int l0 = lane & ~3;
         const float s1 = __shfl_sync(0xffffffffu, sn, l0), c1 = __shfl_sync(0xffffffffu, cn, l0),
                     s2 = __shfl_sync(0xffffffffu, sn, l0 + 1),
@@ -945,9 +960,9 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
           if (q == 0) gd_rotation_sc(s1, c1, s2, c2, s3, c3, sl.rot);
           if (q == 1) {
             const float *lc = cx.lig_center + sl.lig_conf * 3;
-            sl.tx = GD_ADD(sl.mm_new[0], lc[0]);
-            sl.ty = GD_ADD(sl.mm_new[1], lc[1]);
-            sl.tz = GD_ADD(sl.mm_new[2], lc[2]);
+            sl.tx = GD_ADD(mm[0], lc[0]);
+            sl.ty = GD_ADD(mm[1], lc[1]);
+            sl.tz = GD_ADD(mm[2], lc[2]);
             if (a.mode == 4) {
               /* given coordinates: the ligand centre comes with them (Ligand.coord_new.center) */
               sl.tx = a.center_in[(size_t)sl.rep * 3];
@@ -1022,7 +1037,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
             part[5 * T + v] = 0.5 * hpc2 * hpc2 - (double)f.hpl2[tl];
           }
         }
-        const int fcell = cx.ff_tab != nullptr ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
+        const int fcell = cx.ff_tab != nullptr && phase == 0 ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
         if (fcell >= 0) {
           const int id = __ldg(cx.ff_id + fcell);
           const int bin = gd_ff_bin(cx, fcell);
@@ -1058,9 +1073,9 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
        * past the chunks done) ---- */
       int sg0 = 0;
       for (int ci = 0; ci < nch; ++ci) {
-        const int q = resident ? ci : s * nch + ci;
+        const int q = resident ? ci : q_run + ci;
         const int b = q & 1;
-        if (!resident || s == 0) {
+        if (!resident || q_run == 0) {
           bool ok = !*(volatile int *)&s_abort;
           if (ok) ok = mbar_wait_bounded(&bar[b], b ? (consumed1 & 1u) : (consumed0 & 1u),
                                          a.timeout_ns);
@@ -1153,7 +1168,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
             const int prev = atomicAdd(&s_done[b], 1);
             if (prev == nwarps - 1) {
               s_done[b] = 0;
-              if (q + 2 < total_q) {
+              if (certify || q + 2 < total_q) {
                 const int c0 = ((q + 2) % nch) * D, n = min(D, pnp_pad - c0);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 s_issued[b] += 1;
@@ -1269,11 +1284,13 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         if (lane < GD_MAXWEI - 1) e = s_norm[0][lane] * e + s_norm[1][lane];
         gd_energy en;
         double etot = 0.0;
+        float mag = 0.0f;
 #pragma unroll
         for (int i = 0; i < GD_MAXWEI - 1; ++i) {
           const double v = __shfl_sync(0xffffffffu, e, i);
           en.e[i] = (float)v;
           etot += v * s_norm[2][i];
+          mag += fabsf((float)(v * s_norm[2][i]));
         }
         en.e[GD_MAXWEI - 1] = (float)etot;
         en.cms = __shfl_sync(0xffffffffu, side, 9);
@@ -1286,8 +1303,33 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
             da_decide(a, cx, tile.complex_index, rid, en, sl.mm_new, step_first + s);
           } else {
             int acc = 1;
-            if (a.mode == 0)
-              acc = gd_metropolis(en.e[GD_MAXWEI - 1], sl.e_old.e[GD_MAXWEI - 1], sl.mb, sl.u);
+            bool decide = phase == 0;
+            if (a.mode == 0) {
+              const float etn = en.e[GD_MAXWEI - 1], eto = sl.e_old.e[GD_MAXWEI - 1];
+              if (phase == 0) {
+                acc = gd_metropolis(etn, eto, sl.mb, sl.u);
+                if (certify) {
+                  const float tol = GD_CERT * mag;
+                  if (gd_metropolis(etn + tol, eto, sl.mb, sl.u) !=
+                      gd_metropolis(etn - tol, eto, sl.mb, sl.u)) {
+                    sl.e_prop = en;
+                    sl.open = 1;
+                    s_open = 1;
+                    decide = false;
+                  }
+                }
+              } else if (sl.open) {
+                if (phase == 1) {
+                  sl.e_full = etn;
+                } else {
+                  acc = gd_metropolis(sl.e_full, etn, sl.mb, sl.u);
+                  en = sl.e_prop;
+                  sl.open = 0;
+                  decide = true;
+                }
+              }
+            }
+            if (decide) {
             sl.accept = acc;
             if (acc) {
               sl.e_old = en;
@@ -1316,10 +1358,34 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
                 a.trace_acc[(size_t)rid * a.trace_cap + ti] = acc;
               }
             }
+            }
           }
         }
       }
       __syncthreads();
+      q_run += nch;
+      if (phase == 0 && !(certify && s_open)) {
+        ++s;
+      } else if (phase < 2) {
+        ++phase;
+      } else {
+        phase = 0;
+        ++s;
+        if (tid == 0) s_open = 0; /* read again only after the next step's barriers */
+      }
+    }
+    if (certify && !resident && !aborted) {
+      /* the ring was refilled for a pass that did not come: let its two chunks land */
+      for (int i = 0; i < 2; ++i) {
+        const int b = (q_run + i) & 1;
+        if (!mbar_wait_bounded(&bar[b], b ? (consumed1 & 1u) : (consumed0 & 1u), a.timeout_ns)) {
+          aborted = true;
+          if (lane == 0) { s_abort = 1; atomicOr(a.err, GD_DEV_ERR_TIMEOUT); }
+          break;
+        }
+        if (b) ++consumed1; else ++consumed0;
+      }
+      aborted = __syncthreads_or(aborted);
     }
 
     if (aborted) {
