@@ -29,6 +29,16 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
     lig_meta[i] = make_int2(d.lig_t[i], d.lig_n[i] + 1);
   }
   std::vector<float> lig_center(d.lig_center, d.lig_center + 3 * d.n_lig);
+  std::vector<unsigned char> lig_rank((size_t)d.n_lig * L);
+  for (int lc = 0; lc < d.n_lig; ++lc) {
+    const float4 *p = lig_pos.data() + (size_t)lc * L;
+    unsigned char *r = lig_rank.data() + (size_t)lc * L;
+    for (int i = 0; i < L; ++i) r[i] = (unsigned char)i;
+    std::stable_sort(r, r + L, [&](int a, int b) {
+      return p[a].x * p[a].x + p[a].y * p[a].y + p[a].z * p[a].z <
+             p[b].x * p[b].x + p[b].y * p[b].y + p[b].z * p[b].z;
+    });
+  }
   std::vector<float4> sr_a, sr_b;
   std::vector<int> sr_start;
 
@@ -264,12 +274,14 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
   std::vector<float> mb(d.n_tmp);
   for (int t = 0; t < d.n_tmp; ++t) mb[t] = d.temp[t].minus_beta;
 
+  unsigned char *p_lig_rank;
   float4 *p_lig_pos; int2 *p_lig_meta; float *p_lig_center; float4 *p_pt_a, *p_pt_b;
   float4 *p_sr_a, *p_sr_b; int *p_sr_start;
   int4 *p_seg; int *p_seg_count; unsigned short *p_far_cnt; float4 *p_kde, *p_mcs; int *p_kde_start;
   float *p_mt, *p_psp, *p_mb;
   int *p_ref_start; float4 *p_ref_pts;
   if ((rc = upload(c, &p_lig_pos, lig_pos)) || (rc = upload(c, &p_lig_meta, lig_meta)) ||
+      (rc = upload(c, &p_lig_rank, lig_rank)) ||
       (rc = upload(c, &p_lig_center, lig_center)) || (rc = upload(c, &p_pt_a, pt_a)) ||
       (rc = upload(c, &p_pt_b, pt_b)) || (rc = upload(c, &p_sr_a, sr_a)) ||
       (rc = upload(c, &p_sr_b, sr_b)) || (rc = upload(c, &p_sr_start, sr_start)) ||
@@ -283,6 +295,7 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
   /* the host vectors die at the end of this iteration: finish the copies first */
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
     return fail(GD_ERR_CUDA, "upload failed: %s", cudaGetErrorString(cudaGetLastError()));
+  g.lig_rank = p_lig_rank;
   g.lig_pos = p_lig_pos; g.lig_meta = p_lig_meta; g.lig_center = p_lig_center;
   g.pt_a = p_pt_a; g.pt_b = p_pt_b; g.seg = p_seg; g.seg_count = p_seg_count;
   g.far_cnt = p_far_cnt;

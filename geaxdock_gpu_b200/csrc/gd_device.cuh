@@ -51,6 +51,7 @@
 #define GD_MAX_CELLS (1 << 22) /* cells per conformer grid; a larger box widens the cells */
 #define GD_MAX_CELLS_ALL (1 << 25) /* cells of all conformers of a complex together */
 #define GD_MAX_TPB 256         /* threads per CTA: 3 CTAs of 256 fit the register file */
+#define GD_NUM_SMS 148         /* B200 (only a placement hint: any value gives the same results) */
 #define GD_CHUNK 512           /* slots per ring buffer and FP32 sum of the default tile */
 #define GD_MAX_TPB_SPLIT 512   /* threads per CTA of the split launches */
 /* work of the per-atom terms that a split's segments are balanced against, in units of one point
@@ -103,6 +104,7 @@ struct GdDevComplex {
   int sr_n[4];                /* nx, ny, nz, cells */
   const float4 *lig_pos;      /* [n_lig*lna] */
   const int2 *lig_meta;       /* [n_lig*lna] type, MCS index (n + 1) */
+  const unsigned char *lig_rank; /* [n_lig*lna] the conformer's atoms by distance from its centre */
   const float *lig_center;    /* [n_lig*3] */
   /* protein points in pairs (slots 2m, 2m+1), [n_prt*pnp_pad/2] each:
    *   pt_a = (-x0, -x1, -y0, -y1), pt_b = (-z0, -z1, ele0 / el1, ele1 / el1) */
