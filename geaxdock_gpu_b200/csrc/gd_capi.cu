@@ -508,8 +508,8 @@ int upload_tiles(gd_ctx *c, int r0, int r1, int *n_out) {
   if ((int)src->size() > c->tiles_cap) return fail(GD_ERR_INVALID, "tile list overflow");
   CK(cudaStreamSynchronize(c->stream));
   if (!src->empty())
-    CK(cudaMemcpy(c->d_tiles, src->data(), src->size() * sizeof(GdTileDesc),
-                  cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(c->d_tiles, src->data(), src->size() * sizeof(GdTileDesc),
+                  cudaMemcpyHostToDevice, c->stream));
   c->tiles_r0 = r0;
   c->tiles_r1 = r1;
   c->tiles_gen = c->tile_gen;
@@ -607,8 +607,8 @@ int ensure_chains(gd_ctx *c) {
     CK(cudaMalloc(&c->d_chain_tiles, sizeof(GdTileDesc) * tiles.size()));
     c->chain_tiles_cap = (int)tiles.size();
   }
-  CK(cudaMemcpy(c->d_chain_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
-                cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->d_chain_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
+                cudaMemcpyHostToDevice, c->stream));
   int rc = ensure_chain_streams(c, (int)ch.size());
   if (rc) return rc;
   c->chain = ch;
@@ -1269,12 +1269,17 @@ int gd_set_state(gd_ctx *c, const gd_replica_state *st, int r0, int r1) {
     ac[i] = st[i].n_exchange;
   }
   CK(cudaStreamSynchronize(c->stream));
-  CK(cudaMemcpy(c->d_mm + (size_t)r0 * 6, mm.data(), sizeof(float) * 6 * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_eold + r0, e.data(), sizeof(gd_energy) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_etotal + r0, et.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_replica + r0, rp.data(), sizeof(gd_replica) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_nacc + r0, na.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_acs + r0, ac.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->d_mm + (size_t)r0 * 6, mm.data(), sizeof(float) * 6 * n,
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_eold + r0, e.data(), sizeof(gd_energy) * n,
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_etotal + r0, et.data(), sizeof(float) * n,
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_replica + r0, rp.data(), sizeof(gd_replica) * n,
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_nacc + r0, na.data(), sizeof(int) * n,
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_acs + r0, ac.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
   c->initialized = true;
   return GD_OK;
 }

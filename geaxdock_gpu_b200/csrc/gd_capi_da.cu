@@ -133,7 +133,7 @@ int da_upload_epi(gd_ctx *c) {
   e.tr_cap = d->tr_cap;
   e.tr_step0 = d->tr_step0;
   CK(cudaStreamSynchronize(c->stream));
-  CK(cudaMemcpy(d->d_epi, &e, sizeof(e), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(d->d_epi, &e, sizeof(e), cudaMemcpyHostToDevice, c->stream));
   return GD_OK;
 }
 
@@ -224,10 +224,11 @@ int da_build_groups(gd_ctx *c, int S) {
     if ((rc = da_alloc(d, &d->d_group_b0, g.size()))) return rc;
     if ((rc = da_alloc(d, &d->d_rep_group, (size_t)c->n_rep))) return rc;
     if ((rc = da_alloc(d, &d->d_cnt, 2 * g.size()))) return rc;
-    CK(cudaMemcpy(d->d_group_b0, b0s.data(), sizeof(int) * b0s.size(), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(d->d_rep_group, rep_group.data(), sizeof(int) * c->n_rep,
-                  cudaMemcpyHostToDevice));
-    CK(cudaMemset(d->d_cnt, 0, sizeof(int) * 2 * g.size()));
+    CK(cudaMemcpyAsync(d->d_group_b0, b0s.data(), sizeof(int) * b0s.size(),
+                       cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(d->d_rep_group, rep_group.data(), sizeof(int) * c->n_rep,
+                  cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemsetAsync(d->d_cnt, 0, sizeof(int) * 2 * g.size(), c->stream));
   }
   if ((int)tiles.size() > d->n_tiles) {
     if (d->d_tiles) {
@@ -239,8 +240,8 @@ int da_build_groups(gd_ctx *c, int S) {
     int rc = da_alloc(d, &d->d_tiles, tiles.size());
     if (rc) return rc;
   }
-  CK(cudaMemcpy(d->d_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
-                cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(d->d_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
+                cudaMemcpyHostToDevice, c->stream));
   d->groups = g;
   d->n_tiles = (int)tiles.size();
   d->built_gen = c->tile_gen;
@@ -469,8 +470,8 @@ int da_read_stats(gd_ctx *c, std::vector<unsigned long long> &st, std::vector<do
 int da_upload_active(gd_ctx *c) {
   DaState *d = c->da;
   CK(cudaStreamSynchronize(c->stream));
-  CK(cudaMemcpy(d->d_active, d->active.data(), sizeof(int) * c->n_complex,
-                cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(d->d_active, d->active.data(), sizeof(int) * c->n_complex,
+                cudaMemcpyHostToDevice, c->stream));
   return GD_OK;
 }
 
@@ -670,12 +671,14 @@ int gd_sur_create(gd_ctx *c, const gd_sur_params *p) {
   }
 #undef DA_TRY
   d->active.assign(c->n_complex, 0); /* off until trained */
-  CK(cudaMemcpy(d->d_rep_cx, rep_cx.data(), sizeof(int) * R, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(d->d_emb_base, emb_base.data(), sizeof(int) * c->n_complex,
-                cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(d->d_pocket, pf.data(), sizeof(float) * pf.size(), cudaMemcpyHostToDevice));
-  CK(cudaMemset(d->d_s_cur, 0, sizeof(float) * R));
-  CK(cudaMemset(d->d_s_new, 0, sizeof(float) * R));
+  CK(cudaMemcpyAsync(d->d_rep_cx, rep_cx.data(), sizeof(int) * R,
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(d->d_emb_base, emb_base.data(), sizeof(int) * c->n_complex,
+                cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(d->d_pocket, pf.data(), sizeof(float) * pf.size(),
+                     cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemsetAsync(d->d_s_cur, 0, sizeof(float) * R, c->stream));
+  CK(cudaMemsetAsync(d->d_s_new, 0, sizeof(float) * R, c->stream));
   rc = da_upload_active(c);
   if (!rc) rc = da_reset_counters(c);
   if (!rc) rc = da_build_groups(c, c->split);
@@ -882,7 +885,7 @@ int gd_sur_predict(gd_ctx *c, int ci, int prt_conf, int lig_conf, const float *m
   }
   /* the work buffers may have moved: graphs that point at them are stale */
   da_drop_graphs(c);
-  CK(cudaMemcpy(d->d_pred_mm, mm, sizeof(float) * 6 * n, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(d->d_pred_mm, mm, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, c->stream));
   gd::GdDaDev a = da_args(c);
   gd::da_pose_features(a, ci, prt_conf, lig_conf, d->d_pred_mm, n, c->stream);
   if (gd::mlp_forward(d->net, n, c->stream))
@@ -922,7 +925,7 @@ int gd_da_trace_enable(gd_ctx *c, int step0, int max_steps) {
   CK(cudaMalloc(&d->tr_s, sizeof(float) * n));
   CK(cudaMalloc(&d->tr_e, sizeof(float) * n));
   CK(cudaMalloc(&d->tr_flag, sizeof(int) * n));
-  CK(cudaMemset(d->tr_flag, 0xff, sizeof(int) * n));
+  CK(cudaMemsetAsync(d->tr_flag, 0xff, sizeof(int) * n, c->stream));
   d->tr_cap = max_steps;
   return da_upload_epi(c);
 }
@@ -998,7 +1001,7 @@ int gd_mlp_set_params(gd_mlp *m, const float *theta, long long n) {
   if (n != (long long)m->net.L.total) return fail(GD_ERR_INVALID, "parameter count mismatch");
   CK(cudaSetDevice(m->device));
   CK(cudaStreamSynchronize(m->stream));
-  CK(cudaMemcpy(m->net.theta, theta, sizeof(float) * n, cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(m->net.theta, theta, sizeof(float) * n, cudaMemcpyHostToDevice, m->stream));
   if (gd::mlp_refresh_bf16(m->net, m->stream)) return fail(GD_ERR_CUDA, "bf16 refresh failed");
   CK(cudaStreamSynchronize(m->stream));
   return GD_OK;

@@ -94,15 +94,16 @@ int eval_poses(gd_ctx *c, int ci, int prt_conf, int lig_conf, const float *mm, c
   std::vector<int> lc(n, lig_conf);
   CK(cudaStreamSynchronize(c->stream));
   if (given) {
-    CK(cudaMemcpy(c->d_xyz_in, xyz, sizeof(float) * (size_t)n * x.lna * 3,
-                  cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(c->d_ctr_in, center, sizeof(float) * 3 * n, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(c->d_xyz_in, xyz, sizeof(float) * (size_t)n * x.lna * 3,
+                  cudaMemcpyHostToDevice, c->stream));
+    CK(cudaMemcpyAsync(c->d_ctr_in, center, sizeof(float) * 3 * n,
+                       cudaMemcpyHostToDevice, c->stream));
   } else {
-    CK(cudaMemcpy(c->d_mm_in, mm, sizeof(float) * 6 * n, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(c->d_mm_in, mm, sizeof(float) * 6 * n, cudaMemcpyHostToDevice, c->stream));
   }
-  CK(cudaMemcpy(c->d_lc_in, lc.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-  CK(cudaMemcpy(c->d_eval_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
-                cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->d_lc_in, lc.data(), sizeof(int) * n, cudaMemcpyHostToDevice, c->stream));
+  CK(cudaMemcpyAsync(c->d_eval_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
+                cudaMemcpyHostToDevice, c->stream));
   GdMcArgs a = base_args(c);
   a.mode = given ? 4 : 2;
   a.n_steps = 1;
@@ -168,8 +169,8 @@ int gd_place_ligand(gd_ctx *c, int ci, int lig_conf, const float *mm, int n, flo
   CK(cudaStreamSynchronize(c->stream));
   cudaError_t e = cudaMalloc(&d_mm, sizeof(float) * 6 * (size_t)n);
   if (e == cudaSuccess) e = cudaMalloc(&d_xyz, out_bytes);
-  if (e == cudaSuccess) e = cudaMemcpy(d_mm, mm, sizeof(float) * 6 * (size_t)n,
-                                       cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(d_mm, mm, sizeof(float) * 6 * (size_t)n,
+                                       cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
     const long long total = (long long)n * x.lna;
     gd_place_kernel<<<(unsigned)((total + 255) / 256), 256, 0, c->stream>>>(c->d_cx, ci, lig_conf,
@@ -196,7 +197,7 @@ int gd_trace_enable(gd_ctx *c, int max_steps) {
   if (max_steps == 0) return GD_OK;
   CK(cudaMalloc(&c->d_trace_e, sizeof(float) * (size_t)c->n_rep * max_steps));
   CK(cudaMalloc(&c->d_trace_acc, sizeof(int) * (size_t)c->n_rep * max_steps));
-  CK(cudaMemset(c->d_trace_acc, 0xff, sizeof(int) * (size_t)c->n_rep * max_steps));
+  CK(cudaMemsetAsync(c->d_trace_acc, 0xff, sizeof(int) * (size_t)c->n_rep * max_steps, c->stream));
   c->trace_cap = max_steps;
   c->trace_step0 = 0;
   return GD_OK;

@@ -250,8 +250,8 @@ int gd_set_rng_stream(gd_ctx *c, int k, int stream) {
     return fail(GD_ERR_INVALID, "bad complex index or stream");
   CK(cudaSetDevice(c->device));
   CK(cudaStreamSynchronize(c->stream));
-  CK(cudaMemcpy(reinterpret_cast<char *>(c->d_cx + k) + offsetof(GdDevComplex, stream), &stream,
-                sizeof(int), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(reinterpret_cast<char *>(c->d_cx + k) + offsetof(GdDevComplex, stream), &stream,
+                sizeof(int), cudaMemcpyHostToDevice, c->stream));
   c->info[k].stream = stream;
   return GD_OK;
 }
@@ -261,7 +261,7 @@ int gd_set_wait_timeout(gd_ctx *c, long long ns) {
   c->timeout_ns = ns;
   drop_graphs(c);
   CK(cudaStreamSynchronize(c->stream));
-  CK(cudaMemset(c->d_err, 0, sizeof(unsigned)));
+  CK(cudaMemsetAsync(c->d_err, 0, sizeof(unsigned), c->stream));
   return GD_OK;
 }
 

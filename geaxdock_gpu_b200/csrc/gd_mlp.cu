@@ -330,6 +330,8 @@ int mlp_reserve(Mlp &n, int rows) {
     return -3;
   cudaMemset(n.X, 0, R * GD_MLP_IN * 2);
   cudaMemset(n.conf, 0xff, R * 4);
+  /* the network's stream does not wait for the default stream */
+  if (cudaStreamSynchronize(cudaStreamLegacy) != cudaSuccess) return -2;
   n.cap = (int)R;
   return 0;
 }
