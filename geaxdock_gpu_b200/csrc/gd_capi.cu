@@ -400,15 +400,6 @@ McKernel launch_kernel(const LaunchShape &s, bool da) {
   return mc_kernel(s.unroll, s.split, da, s.pack);
 }
 
-int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da) {
-  int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, launch_kernel(s, da), launch_threads(s),
-                                                    smem_bytes(s)) != cudaSuccess ||
-      nb < 1)
-    nb = 1;
-  return std::max(1, std::min(n_tiles, nb * c->num_sms));
-}
-
 GdMcArgs base_args(gd_ctx *c) {
   GdMcArgs a;
   memset(&a, 0, sizeof(a));
@@ -437,20 +428,45 @@ GdMcArgs base_args(gd_ctx *c) {
   return a;
 }
 
-int set_kernel_attrs(const LaunchShape &s, bool da) {
+namespace {
+/* What the process last set a kernel variant's attributes for, per device, and the CTAs an SM then
+ * holds: the dozen driver calls of a launch's set-up are made when another shape comes. */
+struct KernelSetting {
+  int threads = 0, blocks = 0;
+  size_t smem = 0;
+};
+std::mutex g_attr_mu;
+std::map<std::pair<McKernel, int>, KernelSetting> g_attr;
+
+int kernel_setting(const LaunchShape &s, bool da, int *blocks) {
   const McKernel k = launch_kernel(s, da);
   const size_t smem = smem_bytes(s);
-  CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int threads = launch_threads(s);
+  int dev = 0;
+  CK(cudaGetDevice(&dev));
+  std::lock_guard<std::mutex> lock(g_attr_mu);
+  KernelSetting &have = g_attr[{k, dev}];
+  if (have.blocks > 0 && have.smem == smem && have.threads == threads) {
+    if (blocks) *blocks = have.blocks;
+    return GD_OK;
+  }
+  have.blocks = 0;
+  int nb = 0, per_sm = 0, reserved = 0;
+  CK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
+  CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
+  int optin = 0;
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  /* the device's limit less the variant's own static shared memory, once and for all shapes: a
+   * launch of another context never finds it lowered */
+  cudaFuncAttributes fa;
+  CK(cudaFuncGetAttributes(&fa, k));
+  CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                          optin - (int)fa.sharedSizeBytes));
   /* shared memory for the CTAs an SM can hold and the rest as L1, which caches the cell
    * lists of the short-range pass: the carveout is the share of the SM's maximum shared
    * memory those CTAs take (the driver rounds it up to a supported split) */
   CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                           cudaSharedmemCarveoutMaxShared));
-  int nb = 0, dev = 0, per_sm = 0, reserved = 0;
-  CK(cudaGetDevice(&dev));
-  CK(cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
-  CK(cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, dev));
-  const int threads = launch_threads(s);
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, threads, smem));
   if (nb >= 1 && per_sm > 0) {
     /* the driver rounds the carveout up to one of the SM's shared-memory sizes; aim at the
@@ -472,7 +488,27 @@ int set_kernel_attrs(const LaunchShape &s, bool da) {
       CK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout,
                               cudaSharedmemCarveoutMaxShared));
   }
+  if (nb < 1) return fail(GD_ERR_INVALID, "the tile's %zu bytes of shared memory do not fit", smem);
+  have.threads = threads;
+  have.smem = smem;
+  have.blocks = nb;
+  if (blocks) *blocks = nb;
   return GD_OK;
+}
+}  // namespace
+
+void forget_kernel_attrs(int device) {
+  std::lock_guard<std::mutex> lock(g_attr_mu);
+  for (auto &x : g_attr)
+    if (x.first.second == device) x.second.blocks = 0;
+}
+
+int set_kernel_attrs(const LaunchShape &s, bool da) { return kernel_setting(s, da, nullptr); }
+
+int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da) {
+  int nb = 1;
+  if (kernel_setting(s, da, &nb) != GD_OK) nb = 1;
+  return std::max(1, std::min(n_tiles, nb * c->num_sms));
 }
 
 int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter,
@@ -515,6 +551,14 @@ int upload_tiles(gd_ctx *c, int r0, int r1, int *n_out) {
   c->tiles_gen = c->tile_gen;
   c->tiles_n = (int)src->size();
   *n_out = c->tiles_n;
+  return GD_OK;
+}
+
+int device_status(unsigned err) {
+  if (err & GD_DEV_ERR_TIMEOUT)
+    return fail(GD_ERR_TIMEOUT, "a bounded device wait gave up (protein tile copy)");
+  if (err & GD_DEV_ERR_RECORD_FULL)
+    return fail(GD_ERR_RECORD_FULL, "a replica's record buffer overflowed; reset records per dump");
   return GD_OK;
 }
 
@@ -736,12 +780,9 @@ int gd_destroy(gd_ctx *c) {
   if (c->d_counters && !c->counters_pooled) cudaFree(c->d_counters);
   if (c->d_trace_e) cudaFree(c->d_trace_e);
   if (c->d_trace_acc) cudaFree(c->d_trace_acc);
-  if (c->d_mm_in) cudaFree(c->d_mm_in);
-  if (c->d_lc_in) cudaFree(c->d_lc_in);
+  if (c->d_eval_in) cudaFree(c->d_eval_in);
   if (c->d_e_out) cudaFree(c->d_e_out);
-  if (c->d_xyz_in) cudaFree(c->d_xyz_in);
-  if (c->d_ctr_in) cudaFree(c->d_ctr_in);
-  if (c->d_eval_tiles) cudaFree(c->d_eval_tiles);
+  if (c->h_eval) cudaFreeHost(c->h_eval);
   if (c->h_cursor) cudaFreeHost(c->h_cursor);
   if (c->d_chain_tiles) cudaFree(c->d_chain_tiles);
   for (cudaStream_t st : c->aux) cudaStreamDestroy(st);
@@ -796,6 +837,7 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
     return fail(GD_ERR_NODEVICE, "device %d is sm_%d%d; this library is built for sm_100a",
                 device, cc_major, cc_minor);
   CK(cudaSetDevice(device));
+  forget_kernel_attrs(device); /* the device may have been reset since */
 
   {
     const int rc0 = noalloc_prepare(device);
@@ -1132,11 +1174,7 @@ int gd_sync(gd_ctx *c) {
   CK(cudaStreamSynchronize(c->stream));
   unsigned err = 0;
   CK(cudaMemcpy(&err, c->d_err, sizeof(err), cudaMemcpyDeviceToHost));
-  if (err & GD_DEV_ERR_TIMEOUT)
-    return fail(GD_ERR_TIMEOUT, "a bounded device wait gave up (protein tile copy)");
-  if (err & GD_DEV_ERR_RECORD_FULL)
-    return fail(GD_ERR_RECORD_FULL, "a replica's record buffer overflowed; reset records per dump");
-  return GD_OK;
+  return device_status(err);
 }
 
 int gd_get_stream(gd_ctx *c, void **stream) {

@@ -525,41 +525,62 @@ struct gd_mlp {
   cudaStream_t stream = nullptr;
   gd::Mlp net;
   float *d_x = nullptr, *d_t = nullptr;
-  int *d_conf = nullptr;
   int cap = 0;
+  std::vector<int> conf; /* the call's embedding rows, read by a copy that it waits for */
 };
 
 namespace {
 
+/* queues the rows' upload and conversion; the caller waits for the stream before it returns */
 int mlp_stage_rows(gd_mlp *m, const float *x, const int *conf, int rows) {
   if (rows > m->cap) {
     if (m->d_x) cudaFree(m->d_x);
     if (m->d_t) cudaFree(m->d_t);
-    if (m->d_conf) cudaFree(m->d_conf);
     m->d_x = m->d_t = nullptr;
-    m->d_conf = nullptr;
     m->cap = 0;
     CK(cudaMalloc(&m->d_x, sizeof(float) * GD_MLP_IN * rows));
     CK(cudaMalloc(&m->d_t, sizeof(float) * rows));
-    CK(cudaMalloc(&m->d_conf, sizeof(int) * rows));
     m->cap = rows;
   }
   if (gd::mlp_reserve(m->net, rows)) return fail(GD_ERR_NOMEM, "network buffers");
-  std::vector<int> cf(rows, -1);
+  m->conf.assign(rows, -1);
   if (conf) {
     for (int i = 0; i < rows; ++i) {
       if (conf[i] >= m->net.L.n_emb) return fail(GD_ERR_INVALID, "conf %d out of range", conf[i]);
-      cf[i] = m->net.L.n_emb ? conf[i] : -1;
+      if (m->net.L.n_emb) m->conf[i] = conf[i];
     }
   }
   CK(cudaMemcpyAsync(m->d_x, x, sizeof(float) * GD_MLP_IN * rows, cudaMemcpyHostToDevice,
                      m->stream));
-  CK(cudaMemcpyAsync(m->d_conf, cf.data(), sizeof(int) * rows, cudaMemcpyHostToDevice,
+  CK(cudaMemcpyAsync(m->net.conf, m->conf.data(), sizeof(int) * rows, cudaMemcpyHostToDevice,
                      m->stream));
-  if (gd::mlp_set_rows(m->net, m->d_x, m->d_conf, rows, m->stream))
-    return fail(GD_ERR_CUDA, "row upload failed");
-  if (gd::mlp_embed(m->net, rows, m->stream)) return fail(GD_ERR_CUDA, "embedding failed");
-  CK(cudaStreamSynchronize(m->stream)); /* cf leaves scope */
+  if (gd::mlp_set_rows(m->net, m->d_x, rows, m->stream) ||
+      gd::mlp_embed(m->net, rows, m->stream))
+    return fail(GD_ERR_CUDA, "row conversion failed");
+  return GD_OK;
+}
+
+int mlp_queue_forward(gd_mlp *m, const float *x, const int *conf, int rows, float *y) {
+  const int rc = mlp_stage_rows(m, x, conf, rows);
+  if (rc) return rc;
+  if (gd::mlp_forward(m->net, rows, m->stream)) return fail(GD_ERR_CUDA, "forward failed");
+  CK(cudaMemcpyAsync(y, m->net.y, sizeof(float) * rows, cudaMemcpyDeviceToHost, m->stream));
+  return GD_OK;
+}
+
+int mlp_queue_backward(gd_mlp *m, const float *x, const int *conf, const float *t, int rows,
+                       float *loss, float *grad, int *wait_err) {
+  const int rc = mlp_stage_rows(m, x, conf, rows);
+  if (rc) return rc;
+  CK(cudaMemcpyAsync(m->d_t, t, sizeof(float) * rows, cudaMemcpyHostToDevice, m->stream));
+  if (gd::mlp_loss_backward(m->net, rows, m->d_t, m->stream))
+    return fail(GD_ERR_CUDA, "backward failed");
+  if (grad)
+    CK(cudaMemcpyAsync(grad, m->net.grad, sizeof(float) * m->net.L.total, cudaMemcpyDeviceToHost,
+                       m->stream));
+  if (loss)
+    CK(cudaMemcpyAsync(loss, m->net.loss, sizeof(float), cudaMemcpyDeviceToHost, m->stream));
+  CK(cudaMemcpyAsync(wait_err, m->net.err, sizeof(int), cudaMemcpyDeviceToHost, m->stream));
   return GD_OK;
 }
 
@@ -975,7 +996,6 @@ int gd_mlp_destroy(gd_mlp *m) {
   gd::mlp_destroy(m->net);
   if (m->d_x) cudaFree(m->d_x);
   if (m->d_t) cudaFree(m->d_t);
-  if (m->d_conf) cudaFree(m->d_conf);
   cudaStreamDestroy(m->stream);
   delete m;
   return GD_OK;
@@ -1011,11 +1031,11 @@ int gd_mlp_forward(gd_mlp *m, const float *x, const int *conf, int rows, float *
   if (!m || !x || !y || rows < 0) return fail(GD_ERR_INVALID, "bad argument");
   if (rows == 0) return GD_OK;
   CK(cudaSetDevice(m->device));
-  int rc = mlp_stage_rows(m, x, conf, rows);
+  const int rc = mlp_queue_forward(m, x, conf, rows, y);
+  /* also after an error: the caller's arrays are no longer read or written */
+  const cudaError_t e = cudaStreamSynchronize(m->stream);
   if (rc) return rc;
-  if (gd::mlp_forward(m->net, rows, m->stream)) return fail(GD_ERR_CUDA, "forward failed");
-  CK(cudaStreamSynchronize(m->stream));
-  CK(cudaMemcpy(y, m->net.y, sizeof(float) * rows, cudaMemcpyDeviceToHost));
+  CK(e);
   return GD_OK;
 }
 
@@ -1023,16 +1043,15 @@ int gd_mlp_backward(gd_mlp *m, const float *x, const int *conf, const float *t, 
                     float *loss, float *grad) {
   if (!m || !x || !t || rows < 1) return fail(GD_ERR_INVALID, "bad argument");
   CK(cudaSetDevice(m->device));
-  int rc = mlp_stage_rows(m, x, conf, rows);
+  int wait_err = 0;
+  const int rc = mlp_queue_backward(m, x, conf, t, rows, loss, grad, &wait_err);
+  const cudaError_t e = cudaStreamSynchronize(m->stream);
   if (rc) return rc;
-  CK(cudaMemcpyAsync(m->d_t, t, sizeof(float) * rows, cudaMemcpyHostToDevice, m->stream));
-  if (gd::mlp_loss_backward(m->net, rows, m->d_t, m->stream))
-    return fail(GD_ERR_CUDA, "backward failed");
-  CK(cudaStreamSynchronize(m->stream));
-  if (gd::mlp_status(m->net)) return fail(GD_ERR_CUDA, "tensor-core GEMM wait timed out");
-  if (loss) CK(cudaMemcpy(loss, m->net.loss, sizeof(float), cudaMemcpyDeviceToHost));
-  if (grad)
-    CK(cudaMemcpy(grad, m->net.grad, sizeof(float) * m->net.L.total, cudaMemcpyDeviceToHost));
+  CK(e);
+  if (wait_err) { /* a GEMM's bounded wait ran out */
+    CK(cudaMemsetAsync(m->net.err, 0, sizeof(int), m->stream));
+    return fail(GD_ERR_CUDA, "tensor-core GEMM wait timed out");
+  }
   return GD_OK;
 }
 
@@ -1064,6 +1083,7 @@ int gd_kmeans(int device, const float *objects, int n, int dim, const int *seg_o
   job.seed = seed;
   job.threshold = threshold;
   job.max_iter = max_iter;
+  job.pool = ctx_pool(device);
   gd::KmeansResult res;
   std::string err;
   if (gd::kmeans_device(job, res, err)) return fail(GD_ERR_CUDA, "gd_kmeans: %s", err.c_str());

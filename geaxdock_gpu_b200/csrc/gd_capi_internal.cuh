@@ -158,15 +158,11 @@ struct gd_ctx {
   /* graph cache */
   std::map<long long, cudaGraphExec_t> graphs;
   /* pose evaluation scratch */
-  float *d_mm_in = nullptr;
-  int *d_lc_in = nullptr;
+  void *d_eval_in = nullptr; /* poses, or given coordinates and centres */
+  size_t eval_in_cap = 0;    /* bytes */
   gd_energy *d_e_out = nullptr;
   int eval_cap = 0;
-  float *d_xyz_in = nullptr, *d_ctr_in = nullptr; /* given coordinates and centres (mode 4) */
-  size_t xyz_cap = 0;                             /* floats of d_xyz_in */
-  int ctr_cap = 0;                                /* poses of d_ctr_in */
-  GdTileDesc *d_eval_tiles = nullptr;
-  int eval_tiles_cap = 0;
+  char *h_eval = nullptr;    /* page-locked, GD_EVAL_STAGE bytes, made on first use */
   long long timeout_ns = 2000000000LL;
   /* surrogate and delayed acceptance (gd_sur_create) */
   struct DaState *da = nullptr;
@@ -186,6 +182,7 @@ struct gd_ctx {
 };
 
 #define GD_MAX_DEVICES 64
+#define GD_EVAL_STAGE ((size_t)256 << 10) /* bytes of a context's staging buffer */
 
 namespace gdc {
 
@@ -253,10 +250,14 @@ int launch_threads(const LaunchShape &s);
 int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da = false);
 GdMcArgs base_args(gd_ctx *c);
 int set_kernel_attrs(const LaunchShape &s, bool da = false);
+/* the next launch on the device sets its kernel's attributes again */
+void forget_kernel_attrs(int device);
 int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter,
               const LaunchShape &s);
 int upload_tiles(gd_ctx *c, int r0, int r1, int *n_out);
 int check_range(const gd_ctx *c, int r0, int r1);
+/* the status that the device error word stands for */
+int device_status(unsigned err);
 void build_chains(gd_ctx *c, int want, std::vector<Chain> &ch, std::vector<GdTileDesc> *tiles);
 int ensure_chain_streams(gd_ctx *c, int n);
 int ensure_chains(gd_ctx *c);

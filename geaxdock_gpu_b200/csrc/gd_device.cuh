@@ -221,7 +221,9 @@ struct GdDaEpi {
 struct GdMcArgs {
   const GdDevComplex *cx;     /* [n_complex] */
   const GdPairParam *pp;      /* [GD_MAXTP2*GD_MAXTP1] */
-  const GdTileDesc *tiles;    /* [n_tiles] */
+  const GdTileDesc *tiles;    /* [n_tiles], or null: tile i is poses [i u.count, ..) of u, up to u_n */
+  GdTileDesc u;               /* (complex, protein conformer, ligand conformer in rep_begin, count) */
+  int u_n;
   int n_tiles;
   int *tile_counter;          /* persistent-CTA work queue head */
   int mode;                   /* 0: MC steps, 1: init (energy at movematrix 0), 2: eval poses,

@@ -813,7 +813,14 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     __syncthreads();
     const int t = s_tile;
     if (t >= a.n_tiles || s_abort) break;
-    const GdTileDesc tile = a.tiles[t];
+    GdTileDesc tile;
+    if (a.tiles) {
+      tile = a.tiles[t];
+    } else {
+      tile = a.u;
+      tile.rep_begin = t * a.u.count;
+      tile.count = min(a.u.count, a.u_n - tile.rep_begin);
+    }
     int k = tile.count;
     if (DA && a.mode == 3) {
       /* slot (group, capacity): the survivors of the group past this tile's first slot */
@@ -857,7 +864,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
       s.accept = 0;
       s.open = 0;
       if (a.mode >= 2) {
-        s.lig_conf = a.lig_conf_in[id];
+        s.lig_conf = a.tiles ? a.lig_conf_in[id] : a.u.rep_begin;
       } else {
         s.replica = a.replica[id];
         s.lig_conf = s.replica.idx_lig;

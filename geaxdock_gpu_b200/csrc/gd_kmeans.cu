@@ -404,10 +404,47 @@ void pin_give(int *p) {
   cudaFreeHost(p);
 }
 
-template <class T>
-cudaError_t dmalloc(T **p, size_t n) {
-  return cudaMalloc(reinterpret_cast<void **>(p), (n ? n : 1) * sizeof(T));
+/* segment of every object and of every cluster, one CTA per segment */
+__global__ void seg_of_kernel(const Seg *__restrict__ seg, int *__restrict__ seg_of,
+                              int *__restrict__ cseg) {
+  const int s = blockIdx.x;
+  const Seg g = seg[s];
+  for (int i = threadIdx.x; i < g.n; i += blockDim.x) seg_of[g.off + i] = s;
+  for (int i = threadIdx.x; i < g.k; i += blockDim.x) cseg[g.cbase + i] = s;
 }
+
+/* One block of device memory for all of a call's arrays, each at a 256-byte boundary: sized in a
+ * first round of take() calls, which return offsets, and made by alloc(). (Some twenty
+ * cudaMalloc and cudaFree a call took 8-10 ms of host time, now and then 100 ms and more.) */
+struct Arena {
+  char *base = nullptr;
+  size_t used = 0;
+  bool pooled = false;
+  template <class T>
+  size_t take(size_t n) {
+    const size_t at = used;
+    used += ((n ? n : 1) * sizeof(T) + 255) & ~(size_t)255;
+    return at;
+  }
+  template <class T>
+  T *at(size_t off) const {
+    return reinterpret_cast<T *>(base + off);
+  }
+  cudaError_t alloc(void *pool, cudaStream_t st) {
+    pooled = pool != nullptr;
+    return pooled ? cudaMallocFromPoolAsync(reinterpret_cast<void **>(&base), used,
+                                            (cudaMemPool_t)pool, st)
+                  : cudaMalloc(reinterpret_cast<void **>(&base), used);
+  }
+  void release(cudaStream_t st) {
+    if (!base) return;
+    if (pooled)
+      cudaFreeAsync(base, st); /* after the stream's work; cudaFree waits for it by itself */
+    else
+      cudaFree(base);
+    base = nullptr;
+  }
+};
 
 }  // namespace
 
@@ -425,9 +462,7 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
   }
   const int n_seg = (int)job.seg_off.size() - 1;
   std::vector<Seg> seg(n_seg);
-  std::vector<int> seg_of, cseg;
   int n_obj = job.seg_off.back(), n_cl = 0;
-  seg_of.resize(n_obj);
   for (int s = 0; s < n_seg; ++s) {
     Seg &g = seg[s];
     g.off = job.seg_off[s];
@@ -437,8 +472,6 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
     g.k = job.k[s] <= g.n ? job.k[s] : g.n;
     g.cbase = n_cl;
     n_cl += g.k;
-    for (int p = g.off; p < g.off + g.n; ++p) seg_of[p] = s;
-    for (int c = 0; c < g.k; ++c) cseg.push_back(s);
   }
   res.membership.assign(n_obj, -1);
   res.medoid.assign(n_cl, -1);
@@ -448,11 +481,6 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
   res.passes.assign(n_seg, 0);
   if (n_obj == 0 || n_cl == 0) return 0;
 
-  float *obj = nullptr, *sh = nullptr, *cen = nullptr;
-  Seg *dseg = nullptr;
-  int *dseg_of = nullptr, *dcseg = nullptr, *perm = nullptr, *mem = nullptr, *changed = nullptr,
-      *loops = nullptr, *n_act = nullptr, *medoid = nullptr, *size = nullptr, *orig = nullptr;
-  unsigned char *act = nullptr;
   int *h_act = nullptr; /* pinned: active segments after the even and the odd passes */
   cudaEvent_t ev[2] = {nullptr, nullptr};
   cudaStream_t st = (cudaStream_t)job.stream;
@@ -463,49 +491,43 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
   };
   ok(pin_take(&h_act));
   for (cudaEvent_t &v : ev) ok(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
-  ok(dmalloc(&obj, (size_t)n_obj * D));
-  ok(dmalloc(&sh, (size_t)n_obj * D));
-  ok(dmalloc(&cen, (size_t)n_cl * D));
-  ok(dmalloc(&dseg, n_seg));
-  ok(dmalloc(&dseg_of, n_obj));
-  ok(dmalloc(&dcseg, n_cl));
-  ok(dmalloc(&perm, n_obj));
-  ok(dmalloc(&mem, n_obj));
-  ok(dmalloc(&orig, n_obj));
-  ok(dmalloc(&changed, n_seg));
-  ok(dmalloc(&loops, n_seg));
-  ok(dmalloc(&act, n_seg));
-  ok(dmalloc(&n_act, 2));
-  ok(dmalloc(&medoid, n_cl));
-  ok(dmalloc(&size, n_cl));
   int max_n = 0;
   for (const Seg &g : seg) max_n = g.n > max_n ? g.n : max_n;
   const bool sorted = max_n > 8192;
   int key_bits = 1; /* keys 0 .. n_cl */
   while (key_bits < 31 && (n_cl >> key_bits)) ++key_bits;
-  int *key = nullptr, *key2 = nullptr, *pos = nullptr, *pos2 = nullptr, *cb = nullptr,
-      *ce = nullptr;
-  void *tmp = nullptr;
+  const size_t no = n_obj, nc = n_cl, ns = n_seg, srt = sorted ? no : 0;
   size_t tmp_bytes = 0;
-  if (sorted) {
-    ok(dmalloc(&key, n_obj));
-    ok(dmalloc(&key2, n_obj));
-    ok(dmalloc(&pos, n_obj));
-    ok(dmalloc(&pos2, n_obj));
-    ok(dmalloc(&cb, n_cl));
-    ok(dmalloc(&ce, n_cl));
-    ok(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, key, key2, pos, pos2, n_obj, 0, key_bits,
-                                       st));
-    ok(cudaMalloc(&tmp, tmp_bytes ? tmp_bytes : 1));
-  }
+  if (sorted)
+    ok(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, (int *)nullptr, (int *)nullptr,
+                                       (int *)nullptr, (int *)nullptr, n_obj, 0, key_bits, st));
+  Arena m;
+  const size_t o_obj = m.take<float>(no * D), o_sh = m.take<float>(no * D),
+               o_cen = m.take<float>(nc * D), o_seg = m.take<Seg>(ns), o_so = m.take<int>(no),
+               o_cs = m.take<int>(nc), o_perm = m.take<int>(no), o_mem = m.take<int>(no),
+               o_orig = m.take<int>(no), o_chg = m.take<int>(ns), o_loop = m.take<int>(ns),
+               o_act = m.take<unsigned char>(ns), o_na = m.take<int>(2), o_med = m.take<int>(nc),
+               o_size = m.take<int>(nc), o_key = m.take<int>(srt), o_key2 = m.take<int>(srt),
+               o_pos = m.take<int>(srt), o_pos2 = m.take<int>(srt), o_cb = m.take<int>(nc),
+               o_ce = m.take<int>(nc), o_tmp = m.take<char>(tmp_bytes);
+  ok(m.alloc(job.pool, st));
+  float *obj = m.at<float>(o_obj), *sh = m.at<float>(o_sh), *cen = m.at<float>(o_cen);
+  Seg *dseg = m.at<Seg>(o_seg);
+  int *dseg_of = m.at<int>(o_so), *dcseg = m.at<int>(o_cs), *perm = m.at<int>(o_perm),
+      *mem = m.at<int>(o_mem), *orig = m.at<int>(o_orig), *changed = m.at<int>(o_chg),
+      *loops = m.at<int>(o_loop), *n_act = m.at<int>(o_na), *medoid = m.at<int>(o_med),
+      *size = m.at<int>(o_size), *key = m.at<int>(o_key), *key2 = m.at<int>(o_key2),
+      *pos = m.at<int>(o_pos), *pos2 = m.at<int>(o_pos2), *cb = m.at<int>(o_cb),
+      *ce = m.at<int>(o_ce);
+  unsigned char *act = m.at<unsigned char>(o_act);
+  void *tmp = m.at<char>(o_tmp);
   if (e == cudaSuccess) {
     std::vector<unsigned char> a0(n_seg);
     for (int s = 0; s < n_seg; ++s) a0[s] = seg[s].k > 0 && job.k[s] <= seg[s].n;
     ok(cudaMemcpyAsync(obj, job.objects, sizeof(float) * (size_t)n_obj * D,
                        cudaMemcpyHostToDevice, st));
     ok(cudaMemcpyAsync(dseg, seg.data(), sizeof(Seg) * n_seg, cudaMemcpyHostToDevice, st));
-    ok(cudaMemcpyAsync(dseg_of, seg_of.data(), sizeof(int) * n_obj, cudaMemcpyHostToDevice, st));
-    ok(cudaMemcpyAsync(dcseg, cseg.data(), sizeof(int) * n_cl, cudaMemcpyHostToDevice, st));
+    seg_of_kernel<<<n_seg, 128, 0, st>>>(dseg, dseg_of, dcseg);
     ok(cudaMemcpyAsync(act, a0.data(), n_seg, cudaMemcpyHostToDevice, st));
     ok(cudaMemsetAsync(mem, 0xff, sizeof(int) * n_obj, st));
     ok(cudaMemsetAsync(changed, 0, sizeof(int) * n_seg, st));
@@ -562,11 +584,8 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
                        st));
     ok(cudaStreamSynchronize(st));
   }
-  void *ps[] = {obj, sh, cen, dseg, dseg_of, dcseg, perm, mem, orig, changed, loops, act, n_act,
-                medoid, size, key, key2, pos, pos2, cb, ce, tmp};
-  cudaStreamSynchronize(st); /* nothing still reads or writes what is freed */
-  for (void *p : ps)
-    if (p) cudaFree(p);
+  m.release(st);
+  cudaStreamSynchronize(st); /* the pool can give the block back (gd_release_memory) */
   pin_give(h_act);
   for (cudaEvent_t v : ev)
     if (v) cudaEventDestroy(v);

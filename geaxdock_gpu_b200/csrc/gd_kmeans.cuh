@@ -19,6 +19,7 @@ struct KmeansJob {
   float threshold = 0.001f;
   int max_iter = 500;
   void *stream = nullptr;
+  void *pool = nullptr;           /* cudaMemPool_t of the device's work memory (null: cudaMalloc) */
 };
 
 struct KmeansResult {

@@ -306,8 +306,7 @@ int mlp_create(Mlp &n, int hidden, int n_emb, uint64_t seed, cudaStream_t s) {
 }
 
 void mlp_destroy(Mlp &n) {
-  void *ps[] = {n.theta, n.grad, n.m, n.v, n.wh, n.wf, n.loss, n.err, n.adam_dev, n.X, n.A1, n.A2, n.A3, n.D, n.D2, n.Pb,
-                n.Z1, n.Z2, n.Z3, n.C, n.y, n.dy, n.conf, n.P};
+  void *ps[] = {n.theta, n.grad, n.m, n.v, n.wh, n.wf, n.loss, n.err, n.adam_dev, n.work, n.P};
   for (void *p : ps)
     if (p) cudaFree(p);
   n = Mlp();
@@ -316,18 +315,28 @@ void mlp_destroy(Mlp &n) {
 int mlp_reserve(Mlp &n, int rows) {
   rows = (rows + 15) & ~15;
   if (rows <= n.cap) return 0;
-  void *ps[] = {n.X, n.A1, n.A2, n.A3, n.D, n.D2, n.Z1, n.Z2, n.Z3, n.C, n.y, n.dy, n.conf, n.Pb};
-  for (void *p : ps)
-    if (p) cudaFree(p);
-  const size_t H = n.L.hidden, R = rows;
-  if (cudaMalloc(&n.X, R * GD_MLP_IN * 2) || cudaMalloc(&n.A1, R * H * 2) ||
-      cudaMalloc(&n.A2, R * H * 2) || cudaMalloc(&n.A3, R * H * 2) ||
-      cudaMalloc(&n.D, R * H * 2) || cudaMalloc(&n.D2, R * H * 2) || cudaMalloc(&n.Z1, R * H * 4) ||
-      cudaMalloc(&n.Z2, R * H * 4) || cudaMalloc(&n.Z3, R * H * 4) ||
-      cudaMalloc(&n.C, R * (H > GD_MLP_IN ? H : GD_MLP_IN) * 4) || cudaMalloc(&n.y, R * 4) ||
-      cudaMalloc(&n.dy, R * 4) || cudaMalloc(&n.conf, R * 4) ||
-      cudaMalloc(&n.Pb, ((R + 127) / 128) * H * 4))
-    return -3;
+  const size_t H = n.L.hidden, R = rows, C = H > GD_MLP_IN ? H : GD_MLP_IN;
+  /* one block, each array at a 256-byte boundary (TMA wants 16) */
+  size_t used = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = used;
+    used += (bytes + 255) & ~(size_t)255;
+    return at;
+  };
+  const size_t oX = take(R * GD_MLP_IN * 2), oA1 = take(R * H * 2), oA2 = take(R * H * 2),
+               oA3 = take(R * H * 2), oD = take(R * H * 2), oD2 = take(R * H * 2),
+               oZ1 = take(R * H * 4), oZ2 = take(R * H * 4), oZ3 = take(R * H * 4),
+               oC = take(R * C * 4), oy = take(R * 4), ody = take(R * 4), oconf = take(R * 4),
+               oPb = take(((R + 127) / 128) * H * 4);
+  if (n.work) cudaFree(n.work);
+  n.work = nullptr;
+  n.cap = 0;
+  if (cudaMalloc(&n.work, used) != cudaSuccess) return -3;
+  auto h = [&](size_t at) { return reinterpret_cast<bf16 *>(n.work + at); };
+  auto f = [&](size_t at) { return reinterpret_cast<float *>(n.work + at); };
+  n.X = h(oX), n.A1 = h(oA1), n.A2 = h(oA2), n.A3 = h(oA3), n.D = h(oD), n.D2 = h(oD2);
+  n.Z1 = f(oZ1), n.Z2 = f(oZ2), n.Z3 = f(oZ3), n.C = f(oC), n.y = f(oy), n.dy = f(ody);
+  n.conf = reinterpret_cast<int *>(n.work + oconf), n.Pb = f(oPb);
   cudaMemset(n.X, 0, R * GD_MLP_IN * 2);
   cudaMemset(n.conf, 0xff, R * 4);
   /* the network's stream does not wait for the default stream */
@@ -336,10 +345,9 @@ int mlp_reserve(Mlp &n, int rows) {
   return 0;
 }
 
-int mlp_set_rows(Mlp &n, const float *x, const int *conf, int rows, cudaStream_t s) {
+int mlp_set_rows(Mlp &n, const float *x, int rows, cudaStream_t s) {
   if (rows > n.cap) return -4;
   to_bf16<<<blocks((size_t)rows * GD_MLP_IN), 256, 0, s>>>(x, n.X, (size_t)rows * GD_MLP_IN);
-  cudaMemcpyAsync(n.conf, conf, sizeof(int) * rows, cudaMemcpyDeviceToDevice, s);
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 

@@ -68,6 +68,7 @@ struct Mlp {
   int *adam_dev = nullptr;            /* [1] Adam step count and [2] its bias corrections (as
                                          floats) on the device, for graph-replayed steps */
   int cap = 0;                        /* rows of the work buffers */
+  char *work = nullptr;               /* the block that holds them, X to Pb below */
   __nv_bfloat16 *X = nullptr, *A1 = nullptr, *A2 = nullptr, *A3 = nullptr, *D = nullptr;
   __nv_bfloat16 *D2 = nullptr;        /* second buffer of the back-propagated dZ (ping-pong) */
   int *err = nullptr;                 /* [1] nonzero when a tensor-core GEMM's wait ran out */
@@ -85,8 +86,8 @@ int mlp_reserve(Mlp &n, int rows);
 /* rows of X (bf16, 64 wide) -> y; the embedding columns of rows with conf >= 0 are taken from
  * the table (one fused kernel for H = 128 and 256, layer by layer otherwise) */
 int mlp_forward(Mlp &n, int rows, cudaStream_t s);
-/* rows of X from device FP32 rows (rounded to BF16) and their conformer ids */
-int mlp_set_rows(Mlp &n, const float *x, const int *conf, int rows, cudaStream_t s);
+/* rows of X from device FP32 rows (rounded to BF16); their conformer ids go to n.conf */
+int mlp_set_rows(Mlp &n, const float *x, int rows, cudaStream_t s);
 /* fills the embedding columns of X from theta for the rows' conformer ids (n.conf >= 0) */
 int mlp_embed(Mlp &n, int rows, cudaStream_t s);
 /* forward + MSE loss against t (normalised targets) + backward into n.grad (zeroed first) */
