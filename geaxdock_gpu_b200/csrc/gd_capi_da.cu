@@ -554,8 +554,7 @@ int mlp_stage_rows(gd_mlp *m, const float *x, const int *conf, int rows) {
                      m->stream));
   CK(cudaMemcpyAsync(m->net.conf, m->conf.data(), sizeof(int) * rows, cudaMemcpyHostToDevice,
                      m->stream));
-  if (gd::mlp_set_rows(m->net, m->d_x, rows, m->stream) ||
-      gd::mlp_embed(m->net, rows, m->stream))
+  if (gd::mlp_set_rows(m->net, m->d_x, rows, m->stream))
     return fail(GD_ERR_CUDA, "row conversion failed");
   return GD_OK;
 }
@@ -748,7 +747,7 @@ int gd_sur_train(gd_ctx *c, int iterations, float *losses) {
   gd::GdDaDev a = da_args(c);
   const int B = d->prm.batch;
   if (!d->d_train_ctr && (rc = da_alloc(d, &d->d_train_ctr, 2))) return rc;
-  /* One Adam step: batch draw, forward, loss, backward, Adam, the BF16 weight copies (about 30
+  /* One Adam step: batch draw, forward, loss, backward, Adam, the BF16 weight copies (about 20
    * launches). Its per-step values live on the device (the draw's iteration count and the
    * loss slot in d_train_ctr, Adam's step count in the network), so the step is run once
    * eagerly -- which sets up every allocation and kernel attribute it needs -- then captured in

@@ -7,9 +7,9 @@
  *   forward        Z = X W + b, A = bf16(SiLU(Z))         (X K-major, W MN-major)
  *   input grad     dZ' = bf16((dZ W^T) SiLU'(Z'))         (dZ K-major, W K-major)
  *   weight grad    dW = A^T dZ over chunks of 256 rows    (both MN-major, split-K partials)
- * The 256 -> 1 output layer, the loss, column sums for the bias gradients, the embedding
- * gradient (atomic scatter) and Adam are elementwise kernels. Batch reductions add per-chunk
- * partials in a fixed order. Master parameters, gradients and Adam moments are FP32; W1..W3
+ * The 256 -> 1 output layer with the loss and its gradient (out_loss), the column sums it needs,
+ * the embedding gradient (atomic scatter) and Adam are kernels of their own. Batch reductions
+ * add per-chunk partials in a fixed order, all in one launch at the end (reduce_batch). Master parameters, gradients and Adam moments are FP32; W1..W3
  * are mirrored in BF16 (row-major, and in MMA-fragment order for the one-kernel forward) after
  * every update.
  */
@@ -42,58 +42,75 @@ __global__ void out_layer(const bf16 *__restrict__ A3, const float *__restrict__
   if (lane == 0) y[r] = s + b4[0];
 }
 
-/* dy = 2 (y - t) / rows; squared errors to e2 */
-__global__ void mse_grad(const float *__restrict__ y, const float *__restrict__ t,
-                         float *__restrict__ dy, float *__restrict__ e2, int rows) {
-  const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= rows) return;
-  const float d = y[r] - t[r];
-  dy[r] = 2.0f * d / (float)rows;
-  e2[r] = d * d;
-}
-
-/* deterministic mean of e2 into out[0] (one block) */
-__global__ void mean_reduce(const float *__restrict__ e2, int rows, float *out) {
-  __shared__ double sh[256];
-  double s = 0.0;
-  for (int i = threadIdx.x; i < rows; i += 256) s += e2[i];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 128; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
+/* The output layer, the loss and what they send back, one warp per row of M:
+ *   y = A3 . w4 + b4, dy = 2 (y - t) / rows, e2 = (y - t)^2, D = bf16((dy w4^T) SiLU'(Z3)).
+ * Rows past `rows` (padding) get dy = 0 and D = 0. Four kernels and two clears did this, at
+ * 8,192 rows of 256 about 30 us; the row's A3 and Z3 are read once either way, so what goes is
+ * the launches and the passes over y and dy. */
+__global__ void __launch_bounds__(256) out_loss(const bf16 *__restrict__ A3,
+                                                const float *__restrict__ Z3,
+                                                const float *__restrict__ w4,
+                                                const float *__restrict__ b4,
+                                                const float *__restrict__ t, int rows, int M, int h,
+                                                float *__restrict__ y, float *__restrict__ dy,
+                                                float *__restrict__ e2, bf16 *__restrict__ D) {
+  const int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (r >= M) return;
+  const size_t r0 = (size_t)r * h;
+  if (r >= rows) {
+    if (lane == 0) dy[r] = 0.0f;
+    for (int j = lane; j < h; j += 32) D[r0 + j] = __float2bfloat16_rn(0.0f);
+    return;
   }
-  if (threadIdx.x == 0) out[0] = (float)(sh[0] / (double)rows);
-}
-
-/* dZ3 = (dy w4^T) * SiLU'(Z3) -> bf16 */
-__global__ void out_backward(const float *__restrict__ dy, const float *__restrict__ w4,
-                             const float *__restrict__ Z3, bf16 *__restrict__ D, int rows, int h) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (size_t)rows * h) return;
-  const int r = (int)(i / h), j = (int)(i % h);
-  D[i] = __float2bfloat16_rn(dy[r] * w4[j] * silu_grad(Z3[i]));
+  float s = 0.0f;
+#pragma unroll 8
+  for (int j = lane; j < h; j += 32) s += __bfloat162float(A3[r0 + j]) * w4[j];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  const float yr = __shfl_sync(0xffffffffu, s + b4[0], 0);
+  const float d = yr - t[r], g = 2.0f * d / (float)rows;
+  if (lane == 0) {
+    y[r] = yr;
+    dy[r] = g;
+    e2[r] = d * d;
+  }
+#pragma unroll 8
+  for (int j = lane; j < h; j += 32)
+    D[r0 + j] = __float2bfloat16_rn(g * w4[j] * silu_grad(Z3[r0 + j]));
 }
 
 /* Reductions over the batch are split into chunks of SPLIT_ROWS rows: each chunk writes a
  * partial result, reduce_partials adds the chunks in a fixed order (deterministic). */
 constexpr int SPLIT_ROWS = 256;
 
-/* partial column sums of a [rows][n] BF16 matrix, optionally weighted per row by w; with
- * w != null an extra column n holds sum_r w[r]. Block: 32 columns x 8 row lanes; grid
- * (columns / 32, chunks). part[chunk][ncol], ncol = n + (w != null). */
-__global__ void __launch_bounds__(256) colsum_split(const bf16 *__restrict__ A, const float *__restrict__ w,
-                                                    int rows, int n, float *__restrict__ part) {
+/* Partial column sums of the output layer's two [rows][n] BF16 matrices, one per grid z:
+ *   z = 0  A3 weighted per row by dy, with an extra column n that holds sum_r dy[r]
+ *   z = 1  dZ3
+ * Block: 32 columns x 8 row lanes; grid (columns / 32, chunks, 2). part_z[chunk][ncol]. A chain of
+ * dependent additions over 32 rows a lane: the loads are issued eight at a time ahead of it (one
+ * at a time, in two launches: 14.5 and 17.7 us at 8,192 rows of 256). */
+__global__ void __launch_bounds__(256) colsum_split(const bf16 *__restrict__ A3,
+                                                    const float *__restrict__ dy,
+                                                    const bf16 *__restrict__ D, int rows, int n,
+                                                    float *__restrict__ part0,
+                                                    float *__restrict__ part1) {
   __shared__ float sh[8][33];
   const int cx = threadIdx.x & 31, ry = threadIdx.x >> 5;
   const int col = blockIdx.x * 32 + cx, chunk = blockIdx.y;
-  const int ncol = n + (w ? 1 : 0);
+  const bool weighted = blockIdx.z == 0;
+  const int ncol = n + (weighted ? 1 : 0);
   const int r0 = chunk * SPLIT_ROWS, r1 = min(rows, r0 + SPLIT_ROWS);
   float s = 0.0f;
   if (col < ncol) {
-    for (int r = r0 + ry; r < r1; r += 8) {
-      const float a = col < n ? __bfloat162float(A[(size_t)r * n + col]) : 1.0f;
-      s += w ? a * w[r] : a;
+    if (weighted) {
+#pragma unroll 8
+      for (int r = r0 + ry; r < r1; r += 8) {
+        const float a = col < n ? __bfloat162float(A3[(size_t)r * n + col]) : 1.0f;
+        s += a * dy[r];
+      }
+    } else {
+#pragma unroll 8
+      for (int r = r0 + ry; r < r1; r += 8) s += __bfloat162float(D[(size_t)r * n + col]);
     }
   }
   sh[ry][cx] = s;
@@ -102,18 +119,51 @@ __global__ void __launch_bounds__(256) colsum_split(const bf16 *__restrict__ A, 
     float t = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) t += sh[k][cx];
-    part[(size_t)chunk * ncol + col] = t;
+    (weighted ? part0 : part1)[(size_t)chunk * ncol + col] = t;
   }
 }
 
-/* out[i] += sum_c part[c * count + i] */
-__global__ void reduce_partials(const float *__restrict__ part, int chunks, size_t count,
-                                float *__restrict__ out) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+/* One job per parameter tensor: out[i] = sum_c part[c * count + i] in the order of the chunks, by
+ * blocks [first, next job's first); the last block is the loss, the mean of e2. One launch at the
+ * end for the seven sums and the loss (launches of their own between the GEMMs: 6 us each). */
+struct ReduceJobs {
+  static constexpr int N = 7;
+  struct {
+    const float *part;
+    float *out;
+    int chunks, count, first;
+  } job[N];
+};
+
+__global__ void __launch_bounds__(256) reduce_batch(const ReduceJobs jobs,
+                                                    const float *__restrict__ e2, int rows,
+                                                    float *__restrict__ loss) {
+  if (blockIdx.x == gridDim.x - 1) {
+    __shared__ double sh[256];
+    double s = 0.0;
+#pragma unroll 8
+    for (int i = threadIdx.x; i < rows; i += 256) s += e2[i];
+    sh[threadIdx.x] = s;
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
+      __syncthreads();
+    }
+    if (threadIdx.x == 0) loss[0] = (float)(sh[0] / (double)rows);
+    return;
+  }
+  int k = 0;
+#pragma unroll
+  for (int q = 1; q < ReduceJobs::N; ++q)
+    if ((int)blockIdx.x >= jobs.job[q].first) k = q;
+  const int i = ((int)blockIdx.x - jobs.job[k].first) * 256 + threadIdx.x;
+  const int count = jobs.job[k].count, chunks = jobs.job[k].chunks;
   if (i >= count) return;
+  const float *__restrict__ p = jobs.job[k].part + i;
   float s = 0.0f;
-  for (int c = 0; c < chunks; ++c) s += part[(size_t)c * count + i];
-  out[i] += s;
+#pragma unroll 8
+  for (int c = 0; c < chunks; ++c) s += p[(size_t)c * count];
+  jobs.job[k].out[i] = 0.0f + s;
 }
 
 /* embedding gradient: columns [7, 39) of dX1 scattered to the rows' conformer entries */
@@ -208,6 +258,31 @@ __global__ void to_frag(const float *__restrict__ theta, MlpLayout L, bf16 *__re
   const size_t k = 16 * ks + 2 * (lane & 3) + (q & 1) + 8 * (q >> 1);
   const size_t n = 8 * ((size_t)nt8 * w + j) + (lane >> 2);
   wf[i] = __float2bfloat16_rn(W[k * H + n]);
+}
+
+/* FP32 rows to BF16 rows of X, eight columns a thread, with the embedding columns of rows with
+ * conf >= 0 from the table in place of the row's own */
+__global__ void __launch_bounds__(256) rows_to_x(const float4 *__restrict__ x,
+                                                 const int *__restrict__ conf,
+                                                 const float *__restrict__ emb, int rows,
+                                                 uint4 *__restrict__ X) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  const int r = i / (GD_MLP_IN / 8), c0 = (i - r * (GD_MLP_IN / 8)) * 8;
+  if (r >= rows) return;
+  const float4 a = x[2 * (size_t)i], b = x[2 * (size_t)i + 1];
+  float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  const int e = emb ? conf[r] : -1;
+  if (e >= 0) {
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int c = c0 + k - GD_MLP_EMB_OFF;
+      if (c >= 0 && c < GD_MLP_EMB) v[k] = emb[(size_t)e * GD_MLP_EMB + c];
+    }
+  }
+  __align__(16) __nv_bfloat162 o[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) o[k] = __floats2bfloat162_rn(v[2 * k], v[2 * k + 1]);
+  X[i] = *reinterpret_cast<const uint4 *>(o);
 }
 
 /* uniform(-scale, scale) from Philox, keyed by (seed, tensor id) */
@@ -326,8 +401,7 @@ int mlp_reserve(Mlp &n, int rows) {
   const size_t oX = take(R * GD_MLP_IN * 2), oA1 = take(R * H * 2), oA2 = take(R * H * 2),
                oA3 = take(R * H * 2), oD = take(R * H * 2), oD2 = take(R * H * 2),
                oZ1 = take(R * H * 4), oZ2 = take(R * H * 4), oZ3 = take(R * H * 4),
-               oC = take(R * C * 4), oy = take(R * 4), ody = take(R * 4), oconf = take(R * 4),
-               oPb = take(((R + 127) / 128) * H * 4);
+               oC = take(R * C * 4), oy = take(R * 4), ody = take(R * 4), oconf = take(R * 4);
   if (n.work) cudaFree(n.work);
   n.work = nullptr;
   n.cap = 0;
@@ -336,7 +410,7 @@ int mlp_reserve(Mlp &n, int rows) {
   auto f = [&](size_t at) { return reinterpret_cast<float *>(n.work + at); };
   n.X = h(oX), n.A1 = h(oA1), n.A2 = h(oA2), n.A3 = h(oA3), n.D = h(oD), n.D2 = h(oD2);
   n.Z1 = f(oZ1), n.Z2 = f(oZ2), n.Z3 = f(oZ3), n.C = f(oC), n.y = f(oy), n.dy = f(ody);
-  n.conf = reinterpret_cast<int *>(n.work + oconf), n.Pb = f(oPb);
+  n.conf = reinterpret_cast<int *>(n.work + oconf);
   cudaMemset(n.X, 0, R * GD_MLP_IN * 2);
   cudaMemset(n.conf, 0xff, R * 4);
   /* the network's stream does not wait for the default stream */
@@ -347,7 +421,9 @@ int mlp_reserve(Mlp &n, int rows) {
 
 int mlp_set_rows(Mlp &n, const float *x, int rows, cudaStream_t s) {
   if (rows > n.cap) return -4;
-  to_bf16<<<blocks((size_t)rows * GD_MLP_IN), 256, 0, s>>>(x, n.X, (size_t)rows * GD_MLP_IN);
+  rows_to_x<<<blocks((size_t)rows * (GD_MLP_IN / 8)), 256, 0, s>>>(
+      reinterpret_cast<const float4 *>(x), n.conf, n.L.n_emb ? n.theta + n.L.emb : nullptr, rows,
+      reinterpret_cast<uint4 *>(n.X));
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
@@ -357,8 +433,8 @@ int mlp_embed(Mlp &n, int rows, cudaStream_t s) {
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
-/* forward over `rows` rows of n.X; keeps Z1..Z3 when `keep` for the backward pass */
-static int forward_impl(Mlp &n, int rows, bool keep, cudaStream_t s) {
+/* the hidden layers over `rows` rows of n.X; keeps Z1..Z3 when `keep` for the backward pass */
+static int hidden_forward(Mlp &n, int rows, bool keep, cudaStream_t s) {
   const int M = (rows + 15) & ~15, H = n.L.hidden;
   if (M > n.cap) return -4;
   /* Z_l = A_{l-1} W_l + b_l, A_l = bf16(SiLU(Z_l)) in one tensor-core kernel per layer */
@@ -377,9 +453,7 @@ static int forward_impl(Mlp &n, int rows, bool keep, cudaStream_t s) {
       (rc = layer(n.A1, H, n.L.w2, n.L.b2, n.Z2, n.A2)) ||
       (rc = layer(n.A2, H, n.L.w3, n.L.b3, n.Z3, n.A3)))
     return rc;
-  out_layer<<<blocks((size_t)rows * 32), 256, 0, s>>>(n.A3, n.theta + n.L.w4, n.theta + n.L.b4,
-                                                      n.y, rows, H);
-  return cudaGetLastError() == cudaSuccess ? 0 : -2;
+  return 0;
 }
 
 int mlp_forward(Mlp &n, int rows, cudaStream_t s) {
@@ -394,24 +468,29 @@ int mlp_forward(Mlp &n, int rows, cudaStream_t s) {
         n.X, n.conf, n.theta, n.wf, n.L, rows, n.y);
   } else {
     int rc = mlp_embed(n, rows, s);
-    if (rc) return rc;
-    return forward_impl(n, rows, false, s);
+    if (rc || (rc = hidden_forward(n, rows, false, s))) return rc;
+    out_layer<<<blocks((size_t)rows * 32), 256, 0, s>>>(n.A3, n.theta + n.L.w4, n.theta + n.L.b4,
+                                                        n.y, rows, H);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -2;
 }
 
 int mlp_loss_backward(Mlp &n, int rows, const float *t, cudaStream_t s) {
   const int M = (rows + 15) & ~15, H = n.L.hidden;
-  int rc = forward_impl(n, rows, true, s);
+  int rc = hidden_forward(n, rows, true, s);
   if (rc) return rc;
-  cudaMemsetAsync(n.grad, 0, n.L.total * 4, s);
-  /* padded rows (rows..M) carry zero gradient */
-  cudaMemsetAsync(n.dy, 0, (size_t)M * 4, s);
-  mse_grad<<<blocks(rows), 256, 0, s>>>(n.y, t, n.dy, n.C, rows);
-  mean_reduce<<<1, 256, 0, s>>>(n.C, rows, n.loss);
-  /* batch reductions in chunks of SPLIT_ROWS rows, partials added in a fixed order */
-  const int S = (M + SPLIT_ROWS - 1) / SPLIT_ROWS;
-  const size_t need = (size_t)S * (size_t)H * (size_t)(H > GD_MLP_IN ? H : GD_MLP_IN) + S;
+  /* batch reductions in chunks of SPLIT_ROWS rows and tiles of 128, whose partials are added in a
+   * fixed order at the end: a part of P for each */
+  const int S = (M + SPLIT_ROWS - 1) / SPLIT_ROWS, T = (M + 127) / 128;
+  size_t need = 0;
+  auto part = [&](size_t count) {
+    const size_t at = need;
+    need += (count + 63) & ~(size_t)63;
+    return at;
+  };
+  const size_t p_w1 = part((size_t)S * GD_MLP_IN * H), p_w2 = part((size_t)S * H * H),
+               p_w3 = part((size_t)S * H * H), p_w4 = part((size_t)S * (H + 1)),
+               p_b3 = part((size_t)S * H), p_b2 = part((size_t)T * H), p_b1 = part((size_t)T * H);
   if (need > n.p_cap) {
     if (n.P) cudaFree(n.P);
     n.P = nullptr;
@@ -419,64 +498,67 @@ int mlp_loss_backward(Mlp &n, int rows, const float *t, cudaStream_t s) {
     if (cudaMalloc(&n.P, need * sizeof(float)) != cudaSuccess) return -3;
     n.p_cap = need;
   }
-  auto colsum = [&](const bf16 *A, const float *w, float *g) {
-    const int ncol = H + (w ? 1 : 0);
-    colsum_split<<<dim3((ncol + 31) / 32, S), 256, 0, s>>>(A, w, M, H, n.P);
-    reduce_partials<<<blocks(ncol), 256, 0, s>>>(n.P, S, (size_t)ncol, g);
+  ReduceJobs jobs;
+  int n_jobs = 0, red_blocks = 0;
+  auto reduce = [&](size_t at, int chunks, int count, float *out) {
+    jobs.job[n_jobs++] = {n.P + at, out, chunks, count, red_blocks};
+    red_blocks += blocks(count);
   };
+  /* the embedding's gradient is scattered, b4 is padded to four; the rest is written whole */
+  cudaMemsetAsync(n.grad + n.L.b4, 0, (n.L.total - n.L.b4) * 4, s);
   /* dW[i][j] = sum_r Aprev[r][i] dZ[r][j] in chunks of SPLIT_ROWS rows (both operands
    * MN-major, the rows are the reduction); W1 (64 rows) is computed as dW1^T = dZ1^T X so that
    * the 128-row MMA tile runs along the hidden dimension, and stored transposed */
-  auto weight_grad = [&](const bf16 *Aprev, int K, const bf16 *D, float *g) {
+  auto weight_grad = [&](const bf16 *Aprev, int K, const bf16 *D, size_t at, float *g) {
     UmmaEpilogue e{};
     e.kind = UMMA_F32;
-    e.Of = n.P;
+    e.Of = n.P + at;
     e.ldo = H;
     e.split_stride = (size_t)K * H;
-    int rc;
-    if (K == H) {
-      rc = umma_gemm(UmmaOperand{Aprev, M, K, 1}, UmmaOperand{D, M, H, 1}, K, H, SPLIT_ROWS, S,
-                     e, n.err, s);
-    } else {
-      e.trans = 1;
-      rc = umma_gemm(UmmaOperand{D, M, H, 1}, UmmaOperand{Aprev, M, K, 1}, H, K, SPLIT_ROWS, S,
-                     e, n.err, s);
-    }
-    if (rc) return rc;
-    reduce_partials<<<blocks((size_t)K * H), 256, 0, s>>>(n.P, S, (size_t)K * H, g);
-    return 0;
+    reduce(at, S, K * H, g);
+    if (K == H)
+      return umma_gemm(UmmaOperand{Aprev, M, K, 1}, UmmaOperand{D, M, H, 1}, K, H, SPLIT_ROWS, S,
+                       e, n.err, s);
+    e.trans = 1;
+    return umma_gemm(UmmaOperand{D, M, H, 1}, UmmaOperand{Aprev, M, K, 1}, H, K, SPLIT_ROWS, S, e,
+                     n.err, s);
   };
   /* dZ_{l-1} = bf16((dZ_l W_l^T) SiLU'(Z_{l-1})), and its column sums (db_{l-1}) per 128-row
    * tile, added in tile order */
-  auto input_grad = [&](const bf16 *D, size_t w, const float *Zprev, bf16 *Dout, float *gb) {
+  auto input_grad = [&](const bf16 *D, size_t w, const float *Zprev, bf16 *Dout, size_t at,
+                        float *gb) {
     UmmaEpilogue e{};
     e.kind = UMMA_DGRAD;
     e.Zin = Zprev;
     e.Ob = Dout;
-    e.colsum = n.Pb;
+    e.colsum = n.P + at;
     e.ldo = H;
-    const int rc = umma_gemm(UmmaOperand{D, M, H, 0}, UmmaOperand{n.wh + w, H, H, 0}, M, H, H, 1,
-                             e, n.err, s);
-    if (rc) return rc;
-    reduce_partials<<<blocks(H), 256, 0, s>>>(n.Pb, (M + 127) / 128, (size_t)H, gb);
-    return 0;
+    reduce(at, T, H, gb);
+    return umma_gemm(UmmaOperand{D, M, H, 0}, UmmaOperand{n.wh + w, H, H, 0}, M, H, H, 1, e, n.err,
+                     s);
   };
   bf16 *Dc = n.D, *Dn = n.D2;
-  /* output layer: dw4 = A3^T dy and db4 = sum dy (b4 follows w4 in theta) */
-  colsum(n.A3, n.dy, n.grad + n.L.w4);
-  out_backward<<<blocks((size_t)M * H), 256, 0, s>>>(n.dy, n.theta + n.L.w4, n.Z3, Dc, M, H);
-  /* layer 3: dW3 = A2^T dZ3, db3, dZ2 */
-  if ((rc = weight_grad(n.A2, H, Dc, n.grad + n.L.w3))) return rc;
-  colsum(Dc, nullptr, n.grad + n.L.b3);
-  if ((rc = input_grad(Dc, n.L.w3, n.Z2, Dn, n.grad + n.L.b2))) return rc;
+  /* output layer and loss: dZ3, dw4 = A3^T dy, db4 = sum dy (b4 follows w4 in theta), db3 */
+  float *e2 = n.C;
+  out_loss<<<blocks((size_t)M * 32), 256, 0, s>>>(n.A3, n.Z3, n.theta + n.L.w4, n.theta + n.L.b4, t,
+                                                  rows, M, H, n.y, n.dy, e2, Dc);
+  colsum_split<<<dim3((H + 32) / 32, S, 2), 256, 0, s>>>(n.A3, n.dy, Dc, M, H, n.P + p_w4,
+                                                         n.P + p_b3);
+  reduce(p_w4, S, H + 1, n.grad + n.L.w4);
+  reduce(p_b3, S, H, n.grad + n.L.b3);
+  /* layer 3: dW3 = A2^T dZ3, dZ2 with db2 */
+  if ((rc = weight_grad(n.A2, H, Dc, p_w3, n.grad + n.L.w3)) ||
+      (rc = input_grad(Dc, n.L.w3, n.Z2, Dn, p_b2, n.grad + n.L.b2)))
+    return rc;
   std::swap(Dc, Dn);
-  /* layer 2 (db2 came with dZ2) */
-  if ((rc = weight_grad(n.A1, H, Dc, n.grad + n.L.w2))) return rc;
-  if ((rc = input_grad(Dc, n.L.w2, n.Z1, Dn, n.grad + n.L.b1))) return rc;
+  /* layer 2: dW2, dZ1 with db1 */
+  if ((rc = weight_grad(n.A1, H, Dc, p_w2, n.grad + n.L.w2)) ||
+      (rc = input_grad(Dc, n.L.w2, n.Z1, Dn, p_b1, n.grad + n.L.b1)))
+    return rc;
   std::swap(Dc, Dn);
-  /* layer 1: dW1 = X^T dZ1 (64 x H) (db1 came with dZ1); dX = dZ1 W1^T (FP32) for the
-   * embedding */
-  if ((rc = weight_grad(n.X, GD_MLP_IN, Dc, n.grad + n.L.w1))) return rc;
+  /* layer 1: dW1 = X^T dZ1 (64 x H); dX = dZ1 W1^T (FP32) for the embedding */
+  if ((rc = weight_grad(n.X, GD_MLP_IN, Dc, p_w1, n.grad + n.L.w1))) return rc;
+  reduce_batch<<<red_blocks + 1, 256, 0, s>>>(jobs, e2, rows, n.loss);
   if (n.L.n_emb) {
     UmmaEpilogue e{};
     e.kind = UMMA_F32;

@@ -68,15 +68,14 @@ struct Mlp {
   int *adam_dev = nullptr;            /* [1] Adam step count and [2] its bias corrections (as
                                          floats) on the device, for graph-replayed steps */
   int cap = 0;                        /* rows of the work buffers */
-  char *work = nullptr;               /* the block that holds them, X to Pb below */
+  char *work = nullptr;               /* the block that holds them, X to conf below */
   __nv_bfloat16 *X = nullptr, *A1 = nullptr, *A2 = nullptr, *A3 = nullptr, *D = nullptr;
   __nv_bfloat16 *D2 = nullptr;        /* second buffer of the back-propagated dZ (ping-pong) */
   int *err = nullptr;                 /* [1] nonzero when a tensor-core GEMM's wait ran out */
   float *Z1 = nullptr, *Z2 = nullptr, *Z3 = nullptr, *C = nullptr, *y = nullptr, *dy = nullptr;
   float *loss = nullptr;              /* [1] */
   int *conf = nullptr;                /* [cap] embedding row per input row */
-  float *P = nullptr;                 /* per-chunk partials of the batch reductions */
-  float *Pb = nullptr;                /* [cap / 128][hidden] per-tile bias-gradient partials */
+  float *P = nullptr;                 /* partials of the batch reductions */
   size_t p_cap = 0;
 };
 
@@ -86,7 +85,8 @@ int mlp_reserve(Mlp &n, int rows);
 /* rows of X (bf16, 64 wide) -> y; the embedding columns of rows with conf >= 0 are taken from
  * the table (one fused kernel for H = 128 and 256, layer by layer otherwise) */
 int mlp_forward(Mlp &n, int rows, cudaStream_t s);
-/* rows of X from device FP32 rows (rounded to BF16); their conformer ids go to n.conf */
+/* rows of X from device FP32 rows (rounded to BF16), their embedding columns from theta for the
+ * conformer ids in n.conf */
 int mlp_set_rows(Mlp &n, const float *x, int rows, cudaStream_t s);
 /* fills the embedding columns of X from theta for the rows' conformer ids (n.conf >= 0) */
 int mlp_embed(Mlp &n, int rows, cudaStream_t s);
