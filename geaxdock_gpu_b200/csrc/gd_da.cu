@@ -98,8 +98,8 @@ __device__ void write_features(const GdDaDev &d, int ci, int lc, const float mm[
 }
 
 template <int NT>
-__global__ void __launch_bounds__(256) front_kernel(GdDaDev d, int mode, int step0, int *cnt,
-                                                    int r_begin, int r_end) {
+__global__ void __launch_bounds__(fwd::Dims<NT>::THREADS) front_kernel(
+    GdDaDev d, int mode, int step0, int *cnt, int r_begin, int r_end) {
   using D = fwd::Dims<NT>;
   constexpr int FR = fwd::FR;
   extern __shared__ __align__(128) unsigned char fsm[];
@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(256) front_kernel(GdDaDev d, int mode, int ste
     rowi[tid][1] = lc;
   }
   /* the first weight fragments are in flight while warp 0 finishes the proposals */
-  fwd::Ring<NT> ring;
+  fwd::Ring ring;
   if (mode != GD_DA_COLLECT) fwd::prefetch_first<NT>(ring, d.wf, tid);
   __syncthreads();
   if (mode != GD_DA_COLLECT) {
@@ -332,9 +332,11 @@ int da_front(const GdDaDev &d, int mode, int step0, int *cnt, int r_begin, int r
   if (r_end <= r_begin) return 0;
   const int grid = nblk(r_end - r_begin, fwd::FR);
   if (d.L.hidden == 128)
-    front_kernel<1><<<grid, 256, fwd::Dims<1>::smem, s>>>(d, mode, step0, cnt, r_begin, r_end);
+    front_kernel<1><<<grid, fwd::Dims<1>::THREADS, fwd::Dims<1>::smem, s>>>(
+        d, mode, step0, cnt, r_begin, r_end);
   else if (d.L.hidden == 256)
-    front_kernel<2><<<grid, 256, fwd::Dims<2>::smem, s>>>(d, mode, step0, cnt, r_begin, r_end);
+    front_kernel<2><<<grid, fwd::Dims<2>::THREADS, fwd::Dims<2>::smem, s>>>(
+        d, mode, step0, cnt, r_begin, r_end);
   else
     return -1; /* the fused step needs H = 128 or 256 */
   return cudaGetLastError() == cudaSuccess ? 0 : -2;

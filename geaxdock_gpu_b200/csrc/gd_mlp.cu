@@ -9,9 +9,9 @@
  *   weight grad    dW = A^T dZ over chunks of 256 rows    (both MN-major, split-K partials)
  * The 256 -> 1 output layer with the loss and its gradient (out_loss), the column sums it needs,
  * the embedding gradient (atomic scatter) and Adam are kernels of their own. Batch reductions
- * add per-chunk partials in a fixed order, all in one launch at the end (reduce_batch). Master parameters, gradients and Adam moments are FP32; W1..W3
- * are mirrored in BF16 (row-major, and in MMA-fragment order for the one-kernel forward) after
- * every update.
+ * add per-chunk partials in a fixed order, all in one launch at the end (reduce_batch). Master
+ * parameters, gradients and Adam moments are FP32; W1..W3 are mirrored in BF16 (row-major, and
+ * in MMA-fragment order for the one-kernel forward) after every update.
  */
 #include <algorithm>
 #include <cmath>
@@ -229,11 +229,11 @@ __global__ void to_bf16(const float *__restrict__ a, bf16 *__restrict__ b, size_
   if (i < n) b[i] = __float2bfloat16_rn(a[i]);
 }
 
-/* Fragment-ordered BF16 copy of W1, W2, W3 for the fused forward (H = 64 NT8, NT8 = 2 or 4):
- * in each layer block, element (((ks 8 + w) 32 + lane) NT8 + j) 4 + q holds W[k][n] with
- * k = 16 ks + 2 (lane % 4) + (q % 2) + 8 (q / 2) and n = 8 (NT8 w + j) + lane / 4, the
+/* Fragment-ordered BF16 copy of W1, W2, W3 for the fused forward (H = 128 or 256, W = H / 16
+ * warps): in each layer block, element (((ks W + w) 32 + lane) 2 + j) 4 + q holds W[k][n] with
+ * k = 16 ks + 2 (lane % 4) + (q % 2) + 8 (q / 2) and n = 8 (2 w + j) + lane / 4, the
  * m16n8k16 B-operand fragment {b0, b1, b2, b3} of lane `lane` for 8-column tile j of warp w at
- * k-step ks, so that a lane's fragments of one k-step are NT8 x 8 contiguous bytes. */
+ * k-step ks, so that a lane's fragments of one k-step are 16 contiguous bytes. */
 __global__ void to_frag(const float *__restrict__ theta, MlpLayout L, bf16 *__restrict__ wf) {
   const size_t H = L.hidden, n1 = (size_t)GD_MLP_IN * H, i = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (i >= n1 + 2 * H * H) return;
@@ -246,17 +246,12 @@ __global__ void to_frag(const float *__restrict__ theta, MlpLayout L, bf16 *__re
     e -= n1;
     W = theta + L.w2;
   }
-  const int nt8 = (int)(H / 64);
-  const int q = (int)(e & 3);
-  size_t t = e >> 2;
-  const int j = (int)(t % nt8);
-  t /= nt8;
-  const int lane = (int)(t & 31);
-  t >>= 5;
-  const int w = (int)(t & 7);
-  const size_t ks = t >> 3;
+  const int warps = (int)(H / 16);
+  const int q = (int)(e & 3), j = (int)((e >> 2) & 1), lane = (int)((e >> 3) & 31);
+  const size_t t = e >> 8, ks = t / warps;
+  const int w = (int)(t - ks * warps);
   const size_t k = 16 * ks + 2 * (lane & 3) + (q & 1) + 8 * (q >> 1);
-  const size_t n = 8 * ((size_t)nt8 * w + j) + (lane >> 2);
+  const size_t n = 8 * (2 * w + j) + (lane >> 2);
   wf[i] = __float2bfloat16_rn(W[k * H + n]);
 }
 
@@ -294,9 +289,9 @@ __global__ void init_uniform(float *p, size_t n, float scale, uint32_t tensor, u
   p[i] = scale * gd_sym11(r.v[0]);
 }
 
-/* The whole forward pass of fwd::FR rows in one CTA of 8 warps (gd_mlp_fwd.cuh). */
+/* The whole forward pass of fwd::FR rows in one CTA (gd_mlp_fwd.cuh). */
 template <int NT>
-__global__ void __launch_bounds__(256) fused_forward(const bf16 *__restrict__ X,
+__global__ void __launch_bounds__(fwd::Dims<NT>::THREADS) fused_forward(const bf16 *__restrict__ X,
                                                      const int *__restrict__ conf,
                                                      const float *__restrict__ theta,
                                                      const bf16 *__restrict__ wf, MlpLayout L,
@@ -310,10 +305,10 @@ __global__ void __launch_bounds__(256) fused_forward(const bf16 *__restrict__ X,
   bf16 *xs = sm.xs;
   const int tid = threadIdx.x;
   const int row0 = blockIdx.x * FR;
-  fwd::Ring<NT> ring;
+  fwd::Ring ring;
   fwd::prefetch_first<NT>(ring, wf, tid);
   fwd::stage_params<NT>(sm, theta, L, tid);
-  for (int i = tid; i < FR * 8; i += 256) {
+  for (int i = tid; i < FR * 8; i += D::THREADS) {
     const int r = i >> 3, c = i & 7;
     uint4 v = make_uint4(0u, 0u, 0u, 0u);
     if (row0 + r < rows) v = reinterpret_cast<const uint4 *>(X + (size_t)(row0 + r) * GD_MLP_IN)[c];
@@ -461,10 +456,10 @@ int mlp_forward(Mlp &n, int rows, cudaStream_t s) {
   if (rows > n.cap) return -4;
   if (rows < 1) return 0;
   if (H == 128) {
-    fused_forward<1><<<(rows + FR - 1) / FR, 256, FusedDims<1>::smem, s>>>(
+    fused_forward<1><<<(rows + FR - 1) / FR, FusedDims<1>::THREADS, FusedDims<1>::smem, s>>>(
         n.X, n.conf, n.theta, n.wf, n.L, rows, n.y);
   } else if (H == 256) {
-    fused_forward<2><<<(rows + FR - 1) / FR, 256, FusedDims<2>::smem, s>>>(
+    fused_forward<2><<<(rows + FR - 1) / FR, FusedDims<2>::THREADS, FusedDims<2>::smem, s>>>(
         n.X, n.conf, n.theta, n.wf, n.L, rows, n.y);
   } else {
     int rc = mlp_embed(n, rows, s);

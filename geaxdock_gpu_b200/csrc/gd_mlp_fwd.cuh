@@ -3,13 +3,17 @@
  * code shared by the stand-alone forward kernel (gd_mlp.cu) and the delayed-acceptance front
  * kernel (gd_da.cu).
  *
- * One CTA of 8 warps, FR = 32 rows (two 16-row MMA tiles); warp w owns output columns
- * [w H/8, (w+1) H/8) of every layer. Each layer is a chain of BF16 m16n8k16 tensor-core MMAs
- * (mma.sync, FP32 accumulate; PTX ISA "Matrix fragments for mma.m16n8k16"):
+ * One CTA of H / 16 warps, FR = 32 rows (two 16-row MMA tiles); warp w owns output columns
+ * [16 w, 16 (w + 1)) of every layer. What bounds it is one warp's chain: its weights from L2, its
+ * MMAs and, most of the instructions, its SiLUs (an expf and a division each), so the columns are
+ * spread over as many warps as have two n8 tiles each: at H = 256 with 8 warps of four tiles the
+ * front kernel took 26.4 us, with 16 warps 20.1; weights further ahead than RING change nothing.
+ * Each layer is a chain of BF16 m16n8k16 tensor-core MMAs (mma.sync, FP32 accumulate; PTX ISA
+ * "Matrix fragments for mma.m16n8k16"):
  *
  *   A  the layer's input rows, BF16 in shared memory, loaded with ldmatrix.x4;
  *   B  the weights, read straight into registers from a fragment-ordered BF16 copy in global
- *      memory (to_frag in gd_mlp.cu: one coalesced 16- or 32-byte load per lane and k-step,
+ *      memory (to_frag in gd_mlp.cu: one coalesced 16-byte load per lane and k-step,
  *      served by L2) through a ring of RING k-steps that runs across the three layers, so
  *      the next layer's first k-steps are in flight while this one finishes;
  *   C  bias + SiLU + BF16 rounding applied in registers to the accumulator fragments, written
@@ -35,12 +39,13 @@ constexpr int FR = 32; /* rows per CTA: short per-CTA chains, many CTAs */
 
 __device__ __forceinline__ float silu(float z) { return mlp_silu(z); }
 
-template <int NT> /* H = 128 * NT; a warp owns 2 NT 8-column MMA tiles */
+constexpr int NT8 = 2;  /* 8-column MMA tiles of a warp */
+constexpr int RING = 4; /* weight k-steps in flight per lane, 4 registers each */
+
+template <int NT> /* H = 128 * NT */
 struct Dims {
-  static constexpr int H = 128 * NT, NT8 = 2 * NT, LDX = GD_MLP_IN + 8, LDA = H + 8;
-  /* weight k-steps in flight per lane: 16 registers of fragments either way, which keeps the
-   * kernels at <= 96 registers a thread, so they fit beside two CTAs of the exact-energy kernel */
-  static constexpr int RING = 4 / NT;
+  static constexpr int H = 128 * NT, LDX = GD_MLP_IN + 8, LDA = H + 8;
+  static constexpr int WARPS = H / (8 * NT8), THREADS = 32 * WARPS;
   static constexpr size_t xs_bytes = (size_t)FR * LDX * 2;
   static constexpr size_t act_bytes = (size_t)FR * LDA * 2;
   static constexpr size_t par_bytes = (size_t)4 * H * 4; /* b1, b2, b3, w4 */
@@ -77,34 +82,24 @@ __device__ __forceinline__ void stage_params(const Smem<NT> &sm, const float *__
   if (tid == 0) sm.b4[0] = theta[L.b4];
 }
 
-/* this lane's weight fragments of one k-step: NT x 16 bytes = 2 NT n8 tiles x {b0b1, b2b3} */
-template <int NT>
+/* this lane's weight fragments of a k-step: 2 n8 tiles x {b0b1, b2b3} */
 struct Ring {
-  uint4 q[Dims<NT>::RING][NT];
+  uint4 q[RING];
 };
 
 /* lane `lane` of warp `warp`, k-step ks of a layer block of the fragment-ordered copy */
 template <int NT>
-__device__ __forceinline__ const uint4 *frag_ptr(const bf16 *__restrict__ wf, int ks, int warp,
-                                                 int lane) {
-  return reinterpret_cast<const uint4 *>(wf) + ((size_t)(ks * 8 + warp) * 32 + lane) * NT;
-}
-
-template <int NT>
-__device__ __forceinline__ void ring_load(uint4 (&dst)[NT], const bf16 *__restrict__ wf, int ks,
-                                          int warp, int lane) {
-  const uint4 *p = frag_ptr<NT>(wf, ks, warp, lane);
-#pragma unroll
-  for (int j = 0; j < NT; ++j) dst[j] = __ldg(p + j);
+__device__ __forceinline__ uint4 frag_load(const bf16 *__restrict__ wf, int ks, int warp,
+                                           int lane) {
+  return __ldg(reinterpret_cast<const uint4 *>(wf) + (ks * Dims<NT>::WARPS + warp) * 32 + lane);
 }
 
 /* the first RING k-steps of W1 (call before the barrier that precedes rows_forward, so
  * that the loads overlap the caller's own work) */
 template <int NT>
-__device__ __forceinline__ void prefetch_first(Ring<NT> &ring, const bf16 *__restrict__ wf,
-                                               int tid) {
+__device__ __forceinline__ void prefetch_first(Ring &ring, const bf16 *__restrict__ wf, int tid) {
 #pragma unroll
-  for (int s = 0; s < Dims<NT>::RING; ++s) ring_load<NT>(ring.q[s], wf, s, tid >> 5, tid & 31);
+  for (int s = 0; s < RING; ++s) ring.q[s] = frag_load<NT>(wf, s, tid >> 5, tid & 31);
 }
 
 __device__ __forceinline__ void ldmatrix_x4(uint32_t (&a)[4], unsigned addr) {
@@ -132,11 +127,10 @@ __device__ __forceinline__ uint32_t pack_silu(float z0, float z1) {
  * the ring's sequence (slot = (G0 + ks) % RING); on entry the ring holds this layer's k-steps
  * 0..RING-1, on exit the next layer's (wf_next, when given). */
 template <int NT, int KS, int G0>
-__device__ __forceinline__ void layer(Ring<NT> &ring, const bf16 *A, int lda,
+__device__ __forceinline__ void layer(Ring &ring, const bf16 *A, int lda,
                                       const bf16 *__restrict__ wf, const bf16 *__restrict__ wf_next,
                                       const float *bias, bf16 *out, int warp, int lane) {
   using D = Dims<NT>;
-  constexpr int NT8 = D::NT8, RING = D::RING;
   float acc[2][NT8][4];
 #pragma unroll
   for (int m = 0; m < 2; ++m)
@@ -149,23 +143,19 @@ __device__ __forceinline__ void layer(Ring<NT> &ring, const bf16 *A, int lda,
 #pragma unroll
   for (int ks = 0; ks < KS; ++ks) {
     const int slot = (G0 + ks) % RING;
-    uint4 b[NT];
-#pragma unroll
-    for (int j = 0; j < NT; ++j) b[j] = ring.q[slot][j];
+    const uint4 b = ring.q[slot];
     if (ks + RING < KS)
-      ring_load<NT>(ring.q[slot], wf, ks + RING, warp, lane);
+      ring.q[slot] = frag_load<NT>(wf, ks + RING, warp, lane);
     else if (wf_next)
-      ring_load<NT>(ring.q[slot], wf_next, ks + RING - KS, warp, lane);
+      ring.q[slot] = frag_load<NT>(wf_next, ks + RING - KS, warp, lane);
     uint32_t a[2][4];
 #pragma unroll
     for (int m = 0; m < 2; ++m) ldmatrix_x4(a[m], a0 + (unsigned)((m * 16 * lda + ks * 16) * 2));
 #pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        mma_bf16(acc[m][2 * j], a[m], b[j].x, b[j].y);
-        mma_bf16(acc[m][2 * j + 1], a[m], b[j].z, b[j].w);
-      }
+    for (int m = 0; m < 2; ++m) {
+      mma_bf16(acc[m][0], a[m], b.x, b.y);
+      mma_bf16(acc[m][1], a[m], b.z, b.w);
+    }
   }
   /* accumulator fragment: c0, c1 at (row g, columns 2t, 2t+1), c2, c3 at row g + 8 */
   const int g = lane >> 2, t = lane & 3;
@@ -204,7 +194,7 @@ __device__ __forceinline__ void fill_embedding(bf16 *xs, const int *conf_smem,
  * stage_params and prefetch_first must have been called before the last barrier; wf is the
  * fragment-ordered weight copy (W1, W2, W3 blocks; to_frag in gd_mlp.cu). */
 template <int NT>
-__device__ __forceinline__ void rows_forward(const Smem<NT> &sm, Ring<NT> &ring,
+__device__ __forceinline__ void rows_forward(const Smem<NT> &sm, Ring &ring,
                                              const bf16 *__restrict__ wf, float *y_smem,
                                              int tid) {
   using D = Dims<NT>;
@@ -222,6 +212,7 @@ __device__ __forceinline__ void rows_forward(const Smem<NT> &sm, Ring<NT> &ring,
   const float *w4 = sm.par + 3 * D::H;
   for (int r = warp; r < FR; r += (blockDim.x >> 5)) {
     float s = 0.0f;
+#pragma unroll
     for (int j = lane; j < D::H; j += 32) s += __bfloat162float(sm.act0[r * D::LDA + j]) * w4[j];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);

@@ -34,3 +34,22 @@ def test_gradients_at_the_edges(hidden, rows):
         off, size = orc.L[name]
         a, b = g[off:off + size], go[off:off + size]
         assert np.linalg.norm(a - b) <= 0.02 * np.linalg.norm(b) + 1e-6, name
+
+
+@pytest.mark.parametrize("hidden", [128, 256])
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 31, 32, 33, 64, 65])
+def test_one_kernel_forward_at_the_edges(hidden, rows):
+    """Rows around the CTA's 32 and its two 16-row tiles. Each hidden unit's rounding may fall the
+    other way (2^-9 of it, random signs); the output sums them with the last layer's weights, so
+    1 % of the outputs' spread bounds it with room. One row alone is compared with itself among
+    others: a row's sums do not depend on its neighbours."""
+    rng = np.random.default_rng(hidden + rows)
+    net = engine.Mlp(hidden=hidden, n_embedding=7, seed=6)
+    x = rng.normal(0, 1.5, (rows + 40, 64)).astype(np.float32)
+    conf = rng.integers(-1, 7, rows + 40).astype(np.int32)
+    big = net.forward(x, conf)
+    y = net.forward(x[:rows], conf[:rows])
+    yo = mo.MlpOracle(net.params(), hidden, 7, bf16_mode=True).forward(x, conf)
+    net.close()
+    assert np.array_equal(y.view(np.uint32), big[:rows].view(np.uint32))
+    assert np.abs(big - yo).max() <= 0.01 * yo.std() + 1e-4
