@@ -354,8 +354,8 @@ void da_launch_exact(gd_ctx *c, const Chain &ch, int k, int n_steps, int j, bool
 int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGraphExec_t *out) {
   DaState *d = c->da;
   const LaunchShape shape = da_shape(c, S);
-  const long long key = ((long long)shape.unroll << 44) | ((long long)n_steps << 7) | ((long long)S << 2) |
-                        (exchange ? 2 : 0) | (collect ? 1 : 0);
+  const long long key = ((long long)shape.unroll << 44) | ((long long)n_steps << 7) |
+                        ((long long)S << 2) | (exchange ? 2 : 0) | (collect ? 1 : 0);
   auto it = d->graphs.find(key);
   if (it != d->graphs.end()) {
     *out = it->second;

@@ -110,8 +110,8 @@ struct GdDevComplex {
    *   pt_a = (-x0, -x1, -y0, -y1), pt_b = (-z0, -z1, ele0 / el1, ele1 / el1) */
   const float4 *pt_a;
   const float4 *pt_b;
-  /* the cell list, [n_prt*(pnp + 1)] points (the last of a conformer a sentinel far away) and [n_prt*(sr_n[3] + 1)] cell starts (conformer-local
-   * point indices): sr_a = (x, y, z, bits of type | 256 if hydrophobic | 512 if class 2),
+  /* the cell list, [n_prt*(pnp + 1)] points (the last of a conformer a sentinel far away) and
+   * [n_prt*(sr_n[3] + 1)] cell starts (conformer-local point indices): sr_a = (x, y, z, bits of type | 256 if hydrophobic | 512 if class 2),
    * sr_b = (hpp, PSP column bits, ele / el1, 0) */
   const float4 *sr_a;
   const float4 *sr_b;
@@ -141,7 +141,7 @@ struct GdDevComplex {
    * the atom, where every type pair's pmf exponent is below -25.5 in base 2. */
   const unsigned short *far_cnt;
   float far_r, far_inv_w;
-  /* the far fields (gd_farfield.cu; ff_tab null: none). Far-field cell c's table is number ff_id[c] (-1:
+  /* the far fields (gd_farfield.cu; ff_tab null: none). Cell c's table is number ff_id[c] (-1:
    * not tabulated) of its conformer's ff_cells, ff_fields series of GD_FF_NC coefficients: ele,
    * then vdw of ligand type t at 1 + ff_slot[t]. ff_pmf[(pc * GD_FAR_BINS + bin) * GD_MAXTP2 + t]:
    * the far points' pmf sum. A cell's far points: in each segment those past the count of bin

@@ -5,17 +5,21 @@
  * evaluation (reference src/kernel_cuda_l1_montecarlo.cu:12-127). Each CTA pulls tiles from
  * a work queue; a tile is `count` replicas of one protein conformer. Lane (slot j, atom l)
  * owns one ligand atom of one replica for all steps of the launch (a thread holds one lane,
- * or with PACK = 2 the lanes of the same atom in two slots, which share every load):
+ * or with PACK = 2 the lanes of the same atom in two slots, which share every load; with SPLIT the
+ * lanes of an atom in several warps run some of the protein's segments each):
  *   Move_d        (src/kernel_cuda_l2_move.cu:21-80)       placed in registers from a
  *                                                         Philox draw, no HBM traffic;
  *   CalcEnergy_d  (src/kernel_cuda_l2_calcenergy.cu:19-360) the terms every pair has (vdw,
  *                 ele in its far form, pmf, hdb) in a loop over all protein points staged by
  *                 cp.async.bulk into a shared-memory double buffer, points sorted by type so
  *                 each lane keeps its pair parameters in registers per segment, MUFU rsqrt /
- *                 rcp / ex2, FP32 range sums folded into FP64; the short-range terms
- *                 (contacts, psp, hpc, the ele soft core) from a walk of the conformer's cell
- *                 list over the points within 9 A;
- *   CalcMcc_d     (src/kernel_cuda_l2_calcmcc.cu:148-206) contact count in the cell walk,
+ *                 rcp / ex2, FP32 range sums folded into FP64; the far points of a large
+ *                 protein as tabulated fields (gd_farfield.cu), with the decisions that could
+ *                 hang on their rounding taken on the pair loop's energies; the short-range
+ *                 terms (contacts, psp, hpc, the ele soft core) from the point lists of the
+ *                 atom's pocket-grid cell (gd_pocket.cu), outside the grid from a walk of the
+ *                 conformer's cell list;
+ *   CalcMcc_d     (src/kernel_cuda_l2_calcmcc.cu:148-206) contact count in the same pass,
  *                 true positives from the sparse reference-contact list;
  *   CalcRmsd_d, KDE, MCS, dst, CombineEnergy_d (src/kernel_cuda_l3_combineenergy.cu:23-37),
  *                 of moved poses (modes 0-3) or of given placed coordinates (mode 4),
@@ -1059,7 +1063,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
             part[5 * T + v] = 0.5 * hpc2 * hpc2 - (double)f.hpl2[tl];
           }
         }
-        const int fcell = cx.ff_tab != nullptr && phase == 0 ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
+        const int fcell =
+            cx.ff_tab != nullptr && phase == 0 ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
         if (fcell >= 0) {
           const int id = __ldg(cx.ff_id + fcell);
           const int bin = gd_ff_bin(cx, fcell);
@@ -1070,7 +1075,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
               far_field(cx, pc, fcell, id, tl, ax[h], ay[h], az[h], fe, fv);
               part[0 * T + v] = (double)fv;
               part[1 * T + v] += (double)fe;
-              part[2 * T + v] = __ldg(cx.ff_pmf + ((size_t)pc * GD_FAR_BINS + bin) * GD_MAXTP2 + tl);
+              part[2 * T + v] =
+                  __ldg(cx.ff_pmf + ((size_t)pc * GD_FAR_BINS + bin) * GD_MAXTP2 + tl);
             }
           }
         }
@@ -1149,9 +1155,11 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
               const int im = min(i1, max(i0, fs));
               if constexpr (PACK == 1) {
                 if (i0 < im)
-                  pair_dispatch<UNROLL, 1, false, SPLIT>(g.w, PA, PB, i0, im, ax, ay, az, pq, f, acc);
+                  pair_dispatch<UNROLL, 1, false, SPLIT>(g.w, PA, PB, i0, im, ax, ay, az, pq, f,
+                                                         acc);
                 if (im < i1)
-                  pair_dispatch<UNROLL, 1, true, SPLIT>(g.w, PA, PB, im, i1, ax, ay, az, pq, f, acc);
+                  pair_dispatch<UNROLL, 1, true, SPLIT>(g.w, PA, PB, im, i1, ax, ay, az, pq, f,
+                                                        acc);
               } else {
                 /* both lanes' points together, then the rest of the lane that has more */
                 const int ib = max(i0, min(il[0], il[1])), imb = min(im, ib);
@@ -1275,7 +1283,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
 #pragma unroll
             for (int u = 0; u < 5; ++u) tot[(q0 + u) * T] = v[u];
         }
-        const double elhm = SPLIT ? s_lhm[js] : restraints(cx, sl.lig_conf, L, atoms + js * L, lane);
+        const double elhm =
+            SPLIT ? s_lhm[js] : restraints(cx, sl.lig_conf, L, atoms + js * L, lane);
         /* the nine normalised terms, MCC and RMSD, a lane each; the total in term order (all by
          * lane 0 they took 3-5 k cycles) */
         __syncwarp();
@@ -1284,7 +1293,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         const double tp = tot[9 * T];
         const double fp = tot[8 * T] - tp, fn = (double)cx.nref_total - tp;
         const double tn = Ld * (double)P - tp - fp - fn;
-        double e = lane < 6 ? tot[lane * T] : lane == 6 ? tot[6 * T] : lane == 7 ? elhm : tot[7 * T];
+        double e =
+            lane < 6 ? tot[lane * T] : lane == 6 ? tot[6 * T] : lane == 7 ? elhm : tot[7 * T];
         e /= lane == 6 ? (double)f.kde3 : lane == 7 ? (double)cx.pos : Ld;
         if (lane >= 8) {
           const double dx = (double)sl.tx - (double)cx.pocket[0];

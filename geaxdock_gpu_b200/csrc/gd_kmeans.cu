@@ -257,11 +257,11 @@ __global__ void __launch_bounds__(ASSIGN_T) assign_kernel(
  * move from l, and only objects with u not clearly below l are scanned again, with the distances
  * and the comparisons of assign_kernel. Rounding: a computed squared distance is within 8e-7 of
  * the exact one of the same FP32 operands (nine differences, products and sums) but for an
- * underflow of at most 9 x 2^-126, so u < l with KM_REL and KM_ABS to spare means that the scan would
- * find the same centre, strictly nearest; a NaN or an infinite move fails the comparison and is
+ * underflow of at most 9 x 2^-126, so u < l with KM_REL and KM_ABS to spare means that the scan
+ * would find the same centre, strictly nearest; a NaN or an infinite move fails the comparison and is
  * scanned. 170,484 objects without structure (independent normal terms, the bounds' worst case:
- * 63 % scanned in the 6th pass, 50 % in the 30th, 25 % from the 46th on) and 500 clusters: a call of
- * 147 passes 26.0 -> 22.3 ms; of wandering energies, 22 passes, 4.7 -> 4.2 ms. */
+ * 63 % scanned in the 6th pass, 50 % in the 30th, 25 % from the 46th on) and 500 clusters: a call
+ * of 147 passes 26.0 -> 22.3 ms; of wandering energies, 22 passes, 4.7 -> 4.2 ms. */
 constexpr float KM_REL = 4e-6f, KM_ABS = 4e-18f;
 
 __global__ void __launch_bounds__(256)
@@ -347,8 +347,8 @@ __global__ void update_kernel(const float *__restrict__ sh, const Seg *__restric
 }
 
 __global__ void cluster_key_kernel(const Seg *__restrict__ seg, const int *__restrict__ seg_of,
-                                   const int *__restrict__ mem, int n_obj, int n_cl, int *__restrict__ key,
-                                   int *__restrict__ pos) {
+                                   const int *__restrict__ mem, int n_obj, int n_cl,
+                                   int *__restrict__ key, int *__restrict__ pos) {
   const int p = blockIdx.x * blockDim.x + threadIdx.x;
   if (p >= n_obj) return;
   const int m = mem[p];
@@ -695,7 +695,8 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
     if (sorted) {
       /* member lists of the final memberships */
       cluster_key_kernel<<<bo, T, 0, st>>>(dseg, dseg_of, mem, n_obj, n_cl, key, pos);
-      ok(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key2, pos, pos2, n_obj, 0, key_bits, st));
+      ok(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key2, pos, pos2, n_obj, 0, key_bits,
+                                         st));
       ok(cudaMemsetAsync(cb, 0, sizeof(int) * 2 * n_cl, st));
       bounds_kernel<<<bo, T, 0, st>>>(key2, n_obj, n_cl, cb, ce);
       medoid_sorted_kernel<<<bc, T, 0, st>>>(n_cl, cb, ce, pos2, perm, medoid, size);
