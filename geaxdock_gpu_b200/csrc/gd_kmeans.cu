@@ -157,8 +157,9 @@ struct Nearest {
 };
 
 template <int D, bool SECOND>
-__device__ __forceinline__ void scan_pairs(const float *sc, int k, const float *__restrict__ sh,
-                                           int pa, int pb, Nearest &a, Nearest &b) {
+__device__ __forceinline__ void scan_pairs(const float *sc, int c0, int c1,
+                                           const float *__restrict__ sh, int pa, int pb, Nearest &a,
+                                           Nearest &b) {
   float2 oa[D], ob[D];
 #pragma unroll
   for (int j = 0; j < D; ++j) {
@@ -167,9 +168,8 @@ __device__ __forceinline__ void scan_pairs(const float *sc, int k, const float *
     oa[j] = make_float2(va, va);
     ob[j] = make_float2(vb, vb);
   }
-  const int kp = (k + 1) >> 1;
 #pragma unroll 2
-  for (int c = 0; c < kp; ++c) {
+  for (int c = c0; c < c1; ++c) { /* centre pairs */
     const float2 *q = reinterpret_cast<const float2 *>(sc) + c * D;
     float2 sa = make_float2(0.0f, 0.0f), sb = sa;
 #pragma unroll
@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(ASSIGN_T) assign_kernel(
     const int ia = p0 + threadIdx.x, ib = ia + ASSIGN_T;
     const int pa = ia < n_obj ? ia : -1, pb = ib < n_obj ? ib : -1;
     Nearest a, b;
-    scan_pairs<D, false>(sc, gl.k, sh, pa, pb, a, b);
+    scan_pairs<D, false>(sc, 0, (gl.k + 1) >> 1, sh, pa, pb, a, b);
     int n = 0;
     if (pa >= 0) {
       n += mem[pa] != a.best ? 1 : 0;
@@ -258,10 +258,10 @@ __global__ void __launch_bounds__(ASSIGN_T) assign_kernel(
  * and the comparisons of assign_kernel. Rounding: a computed squared distance is within 8e-7 of
  * the exact one of the same FP32 operands (nine differences, products and sums) but for an
  * underflow of at most 9 x 2^-126, so u < l with KM_REL and KM_ABS to spare means that the scan
- * would find the same centre, strictly nearest; a NaN or an infinite move fails the comparison and is
- * scanned. 170,484 objects without structure (independent normal terms, the bounds' worst case:
+ * would find the same centre, strictly nearest; a NaN or an infinite move fails the comparison
+ * and is scanned. 170,484 objects without structure (independent normal terms, the bounds' worst case:
  * 63 % scanned in the 6th pass, 50 % in the 30th, 25 % from the 46th on) and 500 clusters: a call
- * of 147 passes 26.0 -> 22.3 ms; of wandering energies, 22 passes, 4.7 -> 4.2 ms. */
+ * of 147 passes 26.4 -> 21.2 ms; of wandering energies, 22 passes, 5.0 -> 4.2 ms. */
 constexpr float KM_REL = 4e-6f, KM_ABS = 4e-18f;
 
 __global__ void __launch_bounds__(256)
@@ -290,32 +290,73 @@ __global__ void __launch_bounds__(256)
   if (scan) list[at] = p;
 }
 
+/* stage_pairs' layout in global memory (update_sorted_kernel keeps it up) */
+template <int D>
+__device__ __forceinline__ void put_pair(float *__restrict__ pairs, int c, int k, int j, float v) {
+  float *p = pairs + (size_t)(c >> 1) * (2 * D) + 2 * j + (c & 1);
+  p[0] = -v;
+  if (c == k - 1 && !(c & 1)) p[1] = -v;
+}
+
+template <int D>
+__global__ void pairs_kernel(const float *__restrict__ cen, int k, float *__restrict__ pairs) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < k * D) put_pair<D>(pairs, i / D, k, i % D, cen[i]);
+}
+
+/* The listed objects, LIST_N a CTA: half of its threads scan the first half of the centres, half
+ * the second, two objects a thread. Lists are shorter than the object array, and CTAs of 256
+ * objects left two to three an SM: 22.3 -> 21.5 ms for the 147 passes; with the centres copied
+ * from the paired layout that update_sorted_kernel keeps (float4 loads, no divisions) 21.2 ms.
+ * The second half starts from no centre (infinity), so that a comparison between the halves is
+ * the scan's own: only a strictly nearer centre replaces one of lower index, and a first centre
+ * that is not a number is never replaced. */
+constexpr int LIST_N = ASSIGN_T;
+
 template <int D>
 __global__ void __launch_bounds__(ASSIGN_T) assign_list_kernel(
     const float *__restrict__ sh, int k, const int *__restrict__ list,
-    const int *__restrict__ n_list, const float *__restrict__ cen, int *__restrict__ mem,
+    const int *__restrict__ n_list, const float4 *__restrict__ pairs, int *__restrict__ mem,
     float2 *__restrict__ ul, int *__restrict__ changed) {
   __shared__ __align__(16) float sc[SMEM_CL * D];
-  const int n = *n_list, i0 = blockIdx.x * (2 * ASSIGN_T);
+  __shared__ float4 other[LIST_N]; /* the second half's (best, d, lo1, lo2) */
+  const int n = *n_list, i0 = blockIdx.x * LIST_N;
   if (i0 >= n) return;
-  stage_pairs<D>(cen, 0, k, sc);
+  const int quads = (((k + 1) >> 1) * 2 * D + 3) >> 2;
+#pragma unroll 8
+  for (int i = threadIdx.x; i < quads; i += ASSIGN_T)
+    reinterpret_cast<float4 *>(sc)[i] = pairs[i];
   __syncthreads();
-  const int ia = i0 + threadIdx.x, ib = ia + ASSIGN_T;
+  constexpr int G = ASSIGN_T / 2;
+  const int half = threadIdx.x / G, t = threadIdx.x - half * G;
+  const int ia = i0 + t, ib = ia + G;
   const int pa = ia < n ? list[ia] : -1, pb = ib < n ? list[ib] : -1;
+  const int kp = (k + 1) >> 1, km = (kp + 1) >> 1;
   Nearest a, b;
-  scan_pairs<D, true>(sc, k, sh, pa, pb, a, b);
+  if (half) a.d = b.d = INFINITY;
+  scan_pairs<D, true>(sc, half ? km : 0, half ? kp : km, sh, pa, pb, a, b);
+  if (half) {
+    other[t] = make_float4(__int_as_float(a.best), a.d, a.lo1, a.lo2);
+    other[t + G] = make_float4(__int_as_float(b.best), b.d, b.lo1, b.lo2);
+  }
+  __syncthreads();
+  if (half) return;
   int ch = 0;
-  auto put = [&](int p, const Nearest &q) {
+  auto put = [&](int p, const Nearest &q, float4 o) {
     if (p < 0) return;
-    ch += mem[p] != q.best ? 1 : 0;
-    mem[p] = q.best;
+    const bool second = o.y < q.d;
+    const int best = second ? __float_as_int(o.x) : q.best;
+    const float d = second ? o.y : q.d;
+    const float lo2 = fminf(fmaxf(q.lo1, o.z), fminf(q.lo2, o.w));
+    ch += mem[p] != best ? 1 : 0;
+    mem[p] = best;
     /* u from the scan's own distance, NaN if the first centre's is: then never skipped; l of a
      * square that overflowed is what is known of it */
-    ul[p] = make_float2(sqrtf(q.d) * (1.0f + 1e-6f) + KM_ABS,
-                        sqrtf(fminf(q.lo2, 3.4028235e38f)) * (1.0f - 1e-6f) - KM_ABS);
+    ul[p] = make_float2(sqrtf(d) * (1.0f + 1e-6f) + KM_ABS,
+                        sqrtf(fminf(lo2, 3.4028235e38f)) * (1.0f - 1e-6f) - KM_ABS);
   };
-  put(pa, a);
-  put(pb, b);
+  put(pa, a, other[t]);
+  put(pb, b, other[t + G]);
   ch = __reduce_add_sync(0xffffffffu, ch);
   if ((threadIdx.x & 31) == 0 && ch) atomicAdd(changed, ch);
 }
@@ -380,7 +421,7 @@ __global__ void __launch_bounds__(UPD_T)
                          const unsigned char *__restrict__ act, const int *__restrict__ begin,
                          const int *__restrict__ end, const int *__restrict__ pos,
                          float *__restrict__ cen, float *__restrict__ move,
-                         unsigned *__restrict__ most) {
+                         unsigned *__restrict__ most, float *__restrict__ pairs) {
   __shared__ float tile[2][UPD_T * D];
   const int c = blockIdx.x, t = threadIdx.x;
   if (!act[cseg[c]]) return;
@@ -421,6 +462,7 @@ __global__ void __launch_bounds__(UPD_T)
     const float v = __fdiv_rn(s, (float)(e - b));
     step = v - cen[(size_t)c * D + t];
     cen[(size_t)c * D + t] = v;
+    if (move) put_pair<D>(pairs, c, (int)gridDim.x, t, v);
   }
   if (!move || t >= 32) return;
   /* how far the centre went, rounded up (prune_kernel); infinite when it is not a number */
@@ -607,7 +649,7 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
   for (const Seg &g : seg) max_n = g.n > max_n ? g.n : max_n;
   const bool sorted = max_n > 8192;
   /* a single large segment whose centres fit in shared memory (the pooled stage): bounds decide
-   * which objects a pass scans (26.0 -> 22.3 ms, above). Small segments are bound by their sums,
+   * which objects a pass scans (26.4 -> 21.2 ms, above). Small segments are bound by their sums,
    * and several large ones at once do not occur in the clustering this serves */
   const bool pruned = sorted && n_seg == 1 && n_cl <= SMEM_CL;
   int key_bits = 1; /* keys 0 .. n_cl */
@@ -627,7 +669,7 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
                o_pos = m.take<int>(srt), o_pos2 = m.take<int>(srt), o_cb = m.take<int>(2 * nc),
                o_tmp = m.take<char>(tmp_bytes), o_ul = m.take<float2>(pruned ? no : 0),
                o_list = m.take<int>(pruned ? no : 0), o_move = m.take<float>(nc),
-               o_cnt = m.take<int>(2);
+               o_cnt = m.take<int>(2), o_pairs = m.take<float>(pruned ? (nc + 1) * D + 3 : 0);
   ok(m.alloc(job.pool, st));
   float *obj = m.at<float>(o_obj), *sh = m.at<float>(o_sh), *cen = m.at<float>(o_cen);
   Seg *dseg = m.at<Seg>(o_seg);
@@ -638,7 +680,7 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
       *pos = m.at<int>(o_pos), *pos2 = m.at<int>(o_pos2), *cb = m.at<int>(o_cb),
       *ce = cb + n_cl, *list = m.at<int>(o_list), *n_list = m.at<int>(o_cnt);
   float2 *ul = m.at<float2>(o_ul);
-  float *move = m.at<float>(o_move);
+  float *move = m.at<float>(o_move), *pairs = m.at<float>(o_pairs);
   unsigned *most = reinterpret_cast<unsigned *>(n_list + 1);
   unsigned char *act = m.at<unsigned char>(o_act);
   void *tmp = m.at<char>(o_tmp);
@@ -657,13 +699,14 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
     const int ba = (n_obj + 2 * ASSIGN_T - 1) / (2 * ASSIGN_T);
     gather_kernel<<<bo, T, 0, st>>>(obj, D, dseg, dseg_of, n_obj, job.seed, sh, perm);
     init_centres<<<bc, T, 0, st>>>(sh, D, dseg, dcseg, n_cl, cen);
+    if (pruned) pairs_kernel<9><<<(n_cl * 9 + T - 1) / T, T, 0, st>>>(cen, n_cl, pairs);
     ok(cudaGetLastError());
     for (int pass = 0; e == cudaSuccess; ++pass) {
       if (pruned) {
         ok(cudaMemsetAsync(n_list, 0, sizeof(int), st));
         prune_kernel<<<bo, T, 0, st>>>(act, n_obj, pass == 0, mem, move, most, ul, list, n_list);
-        assign_list_kernel<9><<<ba, ASSIGN_T, 0, st>>>(sh, n_cl, list, n_list, cen, mem, ul,
-                                                       changed);
+        assign_list_kernel<9><<<(n_obj + LIST_N - 1) / LIST_N, ASSIGN_T, 0, st>>>(
+            sh, n_cl, list, n_list, reinterpret_cast<const float4 *>(pairs), mem, ul, changed);
         ok(cudaMemsetAsync(most, 0, sizeof(unsigned), st));
       } else {
         assign_kernel<9><<<ba, ASSIGN_T, 0, st>>>(sh, dseg, dseg_of, act, n_obj, cen, mem, changed);
@@ -676,7 +719,7 @@ int kmeans_device(const KmeansJob &job, KmeansResult &res, std::string &err) {
         ok(cudaMemsetAsync(cb, 0, sizeof(int) * 2 * n_cl, st));
         bounds_kernel<<<bo, T, 0, st>>>(key2, n_obj, n_cl, cb, ce);
         update_sorted_kernel<9><<<n_cl, UPD_T, 0, st>>>(sh, dcseg, act, cb, ce, pos2, cen,
-                                                        pruned ? move : nullptr, most);
+                                                        pruned ? move : nullptr, most, pairs);
       } else {
         update_kernel<9><<<bc, T, 0, st>>>(sh, dseg, dcseg, act, n_cl, mem, cen);
       }
