@@ -26,6 +26,7 @@
 #include <cmath>
 #include <condition_variable>
 #include <deque>
+#include <limits>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>

@@ -190,7 +190,10 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
     g.sr_n[1] = (int)n[1];
     g.sr_n[2] = (int)n[2];
     g.sr_n[3] = ncell;
-    sr_a.assign((size_t)d.n_prt * (P + 1), make_float4(1e6f, 1e6f, 1e6f, 0.0f));
+    /* the point behind a conformer's own, which pads the pocket grid's lists: infinitely far, so
+     * that every comparison of its distance fails wherever the complex lies */
+    const float inf = std::numeric_limits<float>::infinity();
+    sr_a.assign((size_t)d.n_prt * (P + 1), make_float4(inf, inf, inf, 0.0f));
     sr_b.assign((size_t)d.n_prt * (P + 1), make_float4(0, 0, 0, 0));
     sr_start.assign((size_t)d.n_prt * (ncell + 1), 0);
     std::vector<int> cid(P);

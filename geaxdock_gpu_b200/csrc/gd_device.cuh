@@ -110,7 +110,7 @@ struct GdDevComplex {
    *   pt_a = (-x0, -x1, -y0, -y1), pt_b = (-z0, -z1, ele0 / el1, ele1 / el1) */
   const float4 *pt_a;
   const float4 *pt_b;
-  /* the cell list, [n_prt*(pnp + 1)] points (the last of a conformer a sentinel far away) and
+  /* the cell list, [n_prt*(pnp + 1)] points (the last of a conformer a sentinel at infinity) and
    * [n_prt*(sr_n[3] + 1)] cell starts (conformer-local point indices): sr_a = (x, y, z, bits of type | 256 if hydrophobic | 512 if class 2),
    * sr_b = (hpp, PSP column bits, ele / el1, 0) */
   const float4 *sr_a;

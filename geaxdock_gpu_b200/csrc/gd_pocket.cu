@@ -14,7 +14,7 @@
  * Entries are 16-bit point indices of the conformer's cell list, in its order (rows of cells by
  * z, y, then x), so that the sums add the same terms in the same order as the row walk, which
  * atoms outside the cube still take; every list is padded to whole quads with the sentinel
- * point behind the conformer's points (1e6 A away: no term). Memory: about 0.2 MB a conformer.
+ * point behind the conformer's points (infinitely far: no term). Memory: about 0.2 MB a conformer.
  * One warp builds one cell's two lists, in two passes (count, fill).
  */
 #include "gd_capi_internal.cuh"
