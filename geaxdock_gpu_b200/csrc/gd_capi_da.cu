@@ -144,13 +144,16 @@ int da_fill(int S, int lna, int lna_max) {
 }
 
 /* The exact stage's replicas per CTA for complex ci at split S: what fills the warps of a split,
- * at most the tile's count where one was set. */
+ * at most the tile's count where one was set. Unsplit, a tile whose own launches are split (the
+ * automatic one of few replicas) holds what fills an unsplit CTA. */
 int da_tile_k(const gd_ctx *c, int ci, int S) {
   const ComplexInfo &x = c->info[ci];
-  if (S <= 1) return x.k;
+  if (S <= 1 && c->split <= 1) return x.k;
+  const int most = c->tile_auto ? x.n_tmp * x.n_lig : x.k;
+  if (S <= 1) return std::min(most, std::min(GD_MAX_SLOTS, GD_MAX_TPB / x.lna));
   int lna = 1;
   for (const auto &y : c->info) lna = std::max(lna, y.lna);
-  return std::min(c->tile_auto ? x.n_tmp * x.n_lig : x.k, da_fill(S, x.lna, lna));
+  return std::min(most, da_fill(S, x.lna, lna));
 }
 
 /* point pairs in flight of the exact stage at split S: with one lane per atom (most proposals
@@ -161,7 +164,7 @@ int da_tile_k(const gd_ctx *c, int ci, int S) {
 LaunchShape da_shape(const gd_ctx *c, int S) {
   LaunchShape s = ctx_shape(c);
   s.pack = 1;
-  if (S <= 1) {
+  if (S <= 1 && c->split <= 1) {
     s.unroll = std::min(s.unroll, 2);
     return s;
   }
@@ -172,6 +175,13 @@ LaunchShape da_shape(const gd_ctx *c, int S) {
     k_lna = std::max(k_lna, k * c->info[ci].lna);
     s.kmax = std::max(s.kmax, k);
     pad = std::max(pad, c->info[ci].pnp_pad);
+  }
+  if (S <= 1) {
+    s.lanes = (k_lna + 31) / 32 * 32;
+    s.split = 1;
+    s.unroll = std::min(s.unroll, 2);
+    if (c->tile_auto) s.chunk = s.fold = GD_CHUNK;
+    return s;
   }
   const LaunchShape q = split_shape(S, k_lna, s.kmax, pad);
   if (c->tile_auto) return q;
@@ -249,7 +259,7 @@ int da_build_groups(gd_ctx *c, int S) {
   return GD_OK;
 }
 
-/* largest split every complex of the batch fits into the context's CTA */
+/* largest split that every complex of the batch fits into a split launch's CTA */
 int da_max_split(const gd_ctx *c) {
   int m = 16;
   for (const auto &x : c->info) m = std::min(m, GD_MAX_TPB_SPLIT / 32 / ((x.lna + 31) / 32));
