@@ -6,7 +6,9 @@ pairs in flight per lane, protein split, CTA lanes in fill mode, replicas per th
 each candidate from the same copy of the chain state, which is put back afterwards), re-times
 the fastest few with more launches, applies the fastest and stores it in a JSON cache keyed by
 (ligand atoms, protein points, replicas, device name); later engines with the same key reuse
-the entry without timing.
+the entry without timing. The candidates have one lane per atom (split 1). A context of few
+replicas runs faster in its automatic tile, which splits an atom's work over several warps:
+`t = engine.tile()` before and `engine.set_tile(*t)` after tuning go back to it.
 """
 from __future__ import annotations
 

@@ -343,6 +343,40 @@ LaunchShape split_shape(int split, int k_lna, int kmax, int pnp_pad) {
   return {split * ((k_lna + 31) / 32) * 32, chunk, GD_CHUNK, split, 4, 1, kmax};
 }
 
+void make_auto_tile(gd_ctx *c) {
+  LaunchShape &s = c->auto_shape;
+  s = {pick_threads(c->info), GD_CHUNK, GD_CHUNK, 1, 2, 1, 1};
+  int k_lna = 1, pad = 4;
+  std::vector<WorkList> work;
+  std::vector<int> k;
+  for (const auto &x : c->info) {
+    c->auto_k.push_back(
+        std::max(1, std::min(s.lanes / x.lna, std::min(GD_MAX_SLOTS, x.n_tmp * x.n_lig))));
+    work.push_back({x.n_prt, x.n_tmp * x.n_lig, x.lna});
+    pad = std::max(pad, x.pnp_pad);
+  }
+  const int S = auto_split(c, work, &k);
+  if (S > 1) c->auto_k = k;
+  for (int ci = 0; ci < c->n_complex; ++ci) {
+    k_lna = std::max(k_lna, c->auto_k[ci] * c->info[ci].lna);
+    s.kmax = std::max(s.kmax, c->auto_k[ci]);
+  }
+  if (S > 1) s = split_shape(S, k_lna, s.kmax, pad);
+}
+
+void use_auto_tile(gd_ctx *c) {
+  const LaunchShape &s = c->auto_shape;
+  for (int ci = 0; ci < c->n_complex; ++ci) c->info[ci].k = c->auto_k[ci];
+  c->threads = s.lanes;
+  c->chunk = s.chunk;
+  c->fold = s.fold;
+  c->split = s.split;
+  c->unroll = s.unroll;
+  c->pack = 1;
+  c->fill_threads = c->fill_cap = 0;
+  c->tile_auto = true;
+}
+
 int ensure_counters(gd_ctx *c, int n) {
   if (n <= c->counters_cap) return GD_OK;
   if (c->d_counters) {
@@ -980,34 +1014,8 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   }
 
   /* ---- tiles ---- */
-  c->threads = pick_threads(c->info);
-  for (auto &x : c->info)
-    x.k = std::max(1, std::min(c->threads / x.lna, std::min(GD_MAX_SLOTS, x.n_tmp * x.n_lig)));
-  {
-    int lna = 1, pad = 4, k_lna = 1, kmax = 1;
-    for (const auto &x : c->info) {
-      lna = std::max(lna, x.lna);
-      pad = std::max(pad, x.pnp_pad);
-    }
-    std::vector<WorkList> work;
-    std::vector<int> k;
-    for (const auto &x : c->info) work.push_back({x.n_prt, x.n_tmp * x.n_lig, x.lna});
-    const int S = auto_split(c, work, &k);
-    if (S > 1) {
-      for (int ci = 0; ci < n_complexes; ++ci) {
-        ComplexInfo &x = c->info[ci];
-        x.k = k[ci];
-        k_lna = std::max(k_lna, x.k * x.lna);
-        kmax = std::max(kmax, x.k);
-      }
-      const LaunchShape s = split_shape(S, k_lna, kmax, pad);
-      c->threads = s.lanes;
-      c->chunk = s.chunk;
-      c->fold = s.fold;
-      c->split = s.split;
-      c->unroll = s.unroll;
-    }
-  }
+  make_auto_tile(c);
+  use_auto_tile(c);
   build_tiles(c, 0, R - 1, c->full_tiles);
   c->tiles_cap = (int)c->full_tiles.size() + 16 * n_complexes;
   {

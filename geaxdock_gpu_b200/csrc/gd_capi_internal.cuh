@@ -122,7 +122,9 @@ struct gd_ctx {
   int pack = 1; /* replicas per thread of the plain launches: the tile's lanes (threads) run on
                    threads / pack threads */
   int fill_threads = 0, fill_cap = 0; /* the last gd_set_tile in fill mode (threads > 0) */
-  bool tile_auto = true; /* no gd_set_tile yet: launches of few lanes are split over more warps */
+  bool tile_auto = true; /* the automatic tile: launches of few lanes are split over more warps */
+  gdc::LaunchShape auto_shape{}; /* the automatic tile, and its replicas per CTA by complex */
+  std::vector<int> auto_k;
   std::vector<gdc::ComplexInfo> info;
   std::vector<void *> allocs;      /* cudaMalloc'd buffers */
   std::vector<void *> pool_allocs; /* buffers from the device's context pool (ctx_pool) */
@@ -231,6 +233,9 @@ void build_tiles(const gd_ctx *c, int r0, int r1, std::vector<GdTileDesc> &out);
 size_t smem_bytes(const LaunchShape &s);
 /* the shape of the context's tile */
 LaunchShape ctx_shape(const gd_ctx *c);
+/* chooses the automatic tile (gd_create) / makes it the context's tile */
+void make_auto_tile(gd_ctx *c);
+void use_auto_tile(gd_ctx *c);
 /* One work list of a launch: n_blocks runs of `block` replicas (a protein conformer's) of an
  * lna-atom ligand, none sharing a tile with another. */
 struct WorkList {

@@ -7,6 +7,48 @@
 
 using namespace gdc;
 
+namespace {
+
+/* whether t is what gd_get_tile reports of complex ci under the automatic tile */
+bool is_auto_tile(const gd_ctx *c, int ci, const gd_tile *t) {
+  const LaunchShape &s = c->auto_shape;
+  return t->replicas_per_cta == c->auto_k[ci] && t->chunk_points == s.chunk &&
+         t->unroll == s.unroll && std::max(t->split, 1) == s.split && t->threads == 0 &&
+         t->replicas_per_lane != 2;
+}
+
+/* whether gd_set_tile(c, k, t) puts the automatic tile back. For every complex of a ragged batch
+ * an unsplit tile of these numbers is a caller's own: the same replica count everywhere. */
+bool restores_auto(const gd_ctx *c, int k, const gd_tile *t) {
+  if (!is_auto_tile(c, std::max(k, 0), t)) return false;
+  if (k >= 0) return c->n_complex == 1 || c->tile_auto;
+  if (c->auto_shape.split > 1) return true;
+  for (int i = 0; i < c->n_complex; ++i)
+    if (c->auto_k[i] != std::min(t->replicas_per_cta, c->info[i].n_tmp * c->info[i].n_lig))
+      return false;
+  return true;
+}
+
+/* a changed tile's work list, and room for it on the device */
+int tile_changed(gd_ctx *c) {
+  c->tile_gen += 1;
+  build_tiles(c, 0, c->n_rep - 1, c->full_tiles);
+  int blocks = 0;
+  for (auto &x : c->info) blocks += x.n_prt;
+  const int need = (int)c->full_tiles.size() + 2 * blocks + 16;
+  if (need > c->tiles_cap) {
+    GdTileDesc *p = nullptr;
+    CK(cudaMalloc(&p, need * sizeof(GdTileDesc)));
+    c->allocs.push_back(p);
+    c->d_tiles = p;
+    c->tiles_cap = need;
+  }
+  drop_graphs(c);
+  return GD_OK;
+}
+
+}  // namespace
+
 extern "C" {
 
 int gd_set_tile(gd_ctx *c, int k, const gd_tile *t) {
@@ -25,6 +67,12 @@ int gd_set_tile(gd_ctx *c, int k, const gd_tile *t) {
   if (k < -1 || k >= c->n_complex) return fail(GD_ERR_INVALID, "bad complex index");
   if (t->replicas_per_lane < 0 || t->replicas_per_lane > 2)
     return fail(GD_ERR_INVALID, "replicas_per_lane must be 0, 1 or 2");
+  /* the automatic tile as gd_get_tile reports it: put back whole, since its lanes and the length of
+   * its FP32 sums are not those of a caller's tile of the same numbers */
+  if (restores_auto(c, k, t)) {
+    use_auto_tile(c);
+    return tile_changed(c);
+  }
   const int S = t->split ? t->split : 1;
   const int P = t->replicas_per_lane == 2 ? 2 : 1;
   if ((t->chunk_points / 2) < S)
@@ -85,20 +133,7 @@ int gd_set_tile(gd_ctx *c, int k, const gd_tile *t) {
   c->pack = P;
   c->tile_auto = false;
   if (t->unroll) c->unroll = t->unroll;
-  c->tile_gen += 1;
-  build_tiles(c, 0, c->n_rep - 1, c->full_tiles);
-  int blocks = 0;
-  for (auto &x : c->info) blocks += x.n_prt;
-  const int need = (int)c->full_tiles.size() + 2 * blocks + 16;
-  if (need > c->tiles_cap) {
-    GdTileDesc *p = nullptr;
-    CK(cudaMalloc(&p, need * sizeof(GdTileDesc)));
-    c->allocs.push_back(p);
-    c->d_tiles = p;
-    c->tiles_cap = need;
-  }
-  drop_graphs(c);
-  return GD_OK;
+  return tile_changed(c);
 }
 
 int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile *best,
@@ -268,7 +303,8 @@ int gd_set_wait_timeout(gd_ctx *c, long long ns) {
 int gd_get_tile(const gd_ctx *c, int k, gd_tile *t) {
   if (!c || !t || k < 0 || k >= c->n_complex) return fail(GD_ERR_INVALID, "bad argument");
   /* the tile as set: in fill mode the cap (0: none) and the CTA size, so that gd_set_tile of
-   * the result restores it; gd_get_replicas_per_cta gives each complex's count */
+   * the result restores it, the automatic tile too; gd_get_replicas_per_cta gives each complex's
+   * count */
   t->replicas_per_cta = c->fill_threads > 0 ? c->fill_cap : c->info[k].k;
   t->chunk_points = c->chunk;
   t->unroll = c->unroll;

@@ -169,7 +169,8 @@ typedef struct {
                                the protein's type segments (0 or 1: one lane per atom);
                                replicas_per_cta * split * atoms must fit 256 lanes. Only the order
                                of FP64 additions depends on it. A context without gd_set_tile
-                               splits launches of few replicas by itself. */
+                               splits launches of few replicas by itself; gd_set_tile of the tile
+                               that gd_get_tile reported then puts that back. */
   int threads;              /* CTA size (multiple of 32, <= 256); 0: the smallest that holds
                                replicas_per_cta replicas of every complex. With threads > 0 each
                                complex gets as many replicas as fill the CTA (at most
