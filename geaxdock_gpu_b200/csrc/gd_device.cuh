@@ -53,6 +53,7 @@
 #define GD_MAX_TPB 256         /* threads per CTA: 3 CTAs of 256 fit the register file */
 #define GD_NUM_SMS 148         /* B200 (only a placement hint: any value gives the same results) */
 #define GD_CHUNK 512           /* slots per ring buffer and FP32 sum of the default tile */
+#define GD_ROAM 5.0f           /* A from the pocket: where a tile's lanes go by slot, not by rank */
 #define GD_MAX_TPB_SPLIT 512   /* threads per CTA of the split launches */
 /* work of the per-atom terms that a split's segments are balanced against, in units of one point
  * pair: a segment's own set-up, the contact list, the kind list, the restraints, the tail */

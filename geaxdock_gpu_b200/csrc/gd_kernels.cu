@@ -538,6 +538,22 @@ struct Slot {
 };
 static_assert(sizeof(Slot) == GD_SLOT_BYTES, "slot layout");
 
+/* Whether the slot's replica, or a proposal one root-mean-square move from it, lies GD_ROAM or more
+ * from the pocket centre. */
+__device__ __forceinline__ bool slot_roams(const GdMcArgs &a, const GdDevComplex &cx,
+                                           const Slot &s, int id) {
+  float v[3], step2 = 0.0f, d2 = 0.0f;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    v[i] = a.mode == 4 ? a.center_in[(size_t)id * 3 + i]
+                       : cx.lig_center[s.lig_conf * 3 + i] +
+                             (a.mode >= 2 ? a.mm_in[(size_t)id * 6 + i] : s.mm_old[i]);
+    d2 += (v[i] - cx.pocket[i]) * (v[i] - cx.pocket[i]);
+    step2 += a.mode == 0 ? a.move_scale[i] * a.move_scale[i] : 0.0f;
+  }
+  return sqrtf(d2) + sqrtf(step2) > GD_ROAM;
+}
+
 #define NQ 10 /* vdw ele pmf psp hdb hsum->hpc kde rmsd ncon tp */
 #define MCS_U 4 /* restraint positions in flight in the epilogue */
 
@@ -845,22 +861,11 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     const int A = SPLIT ? NT / S : T;
     const int kp = (k + PACK - 1) / PACK; /* lane groups */
     const int sp = SPLIT ? tid / A : 0;
-    /* Unsplit lanes run over the atoms' ranks by distance from the ligand's centre, the tile's
-     * slots within a rank: a warp's atoms lie about as far out, so that its inner warps end their
-     * segments early (a warp runs to the largest near radius among its atoms): 6,820 replicas of
-     * 40 atoms on 3,000 points, 11 steps, 7.24 -> 6.79 ms. The outer warps' place in the CTA goes
-     * round with the tile, so that the tiles an SM holds (about GD_NUM_SMS apart) load its four
-     * schedulers alike. Split lanes keep the chain's order, whose neighbours share list entries
-     * (2 % faster there). */
-    const int wr = SPLIT ? warp - sp * (A >> 5) : (warp + t + t / GD_NUM_SMS) % nwarps;
-    const int ai = wr * 32 + lane;
-    const bool active = ai < kp * L;
-    const int hi = active ? ai / (SPLIT ? L : kp) : 0, lo = active ? ai - hi * (SPLIT ? L : kp) : 0;
-    const int jj = SPLIT ? hi : lo, rank = SPLIT ? lo : hi;
     /* the splits that run the short-range lists and the restraints (split 0: the far field, the
      * per-atom tail) */
     const int con_sp = S - 1, kind_sp = max(S - 2, 0), mcs_sp = S >= 4 ? S - 3 : S == 2 ? 1 : 0;
     /* ---- slot set-up (one thread per replica) ---- */
+    bool roams = false;
     if (tid < k) {
       Slot &s = slots[tid];
       const int id = tile.rep_begin + tid;
@@ -886,6 +891,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
           for (int i = 0; i < 6; ++i) s.mm_old[i] = 0.0f;
         }
       }
+      if constexpr (!SPLIT) roams = slot_roams(a, cx, s, id);
     }
 
     /* ---- protein tile pipeline ---- */
@@ -907,9 +913,32 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         bulk_g2s(bpb + b * (D >> 1), gb + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
       }
     }
-    __syncthreads();
+    if constexpr (SPLIT)
+      __syncthreads();
+    else
+      roams = __syncthreads_or(roams);
 
     /* ---- per-lane constants ---- */
+    /* Unsplit lanes of a tile whose replicas are all at the pocket run over the atoms' ranks by
+     * distance from the ligand's centre, the tile's slots within a rank: a warp's atoms lie about
+     * as far out, so that its inner warps end their segments early (a warp runs to the largest near
+     * radius among its atoms): 6,820 replicas of 40 atoms on 3,000 points, 11 steps from the
+     * pocket, 7.24 -> 6.79 ms; of 60 atoms on 1,500 points, 20 steps, 15.8 -> 15.3 ms. One replica
+     * further away (GD_ROAM) would make every warp of the CTA run about as far as its atoms need:
+     * then each slot's atoms lie together, in the chain's order, whose neighbours share list
+     * entries. The 6,820 replicas after 1,000 steps, by rank / by slot / as chosen, ms per 10
+     * steps: moves of 0.1 A 6.60 / 6.76 / 6.56, of 2 A 9.33 / 8.36 / 8.38, of 6 A 10.66 / 9.97 /
+     * 9.93 (six replicas a CTA and four pairs in flight 9.86 / 9.24 / 9.22); lines at 8 and 11 A
+     * and at the ligand's radius are up to 3 % slower at 2 A. The warps' place in the CTA goes
+     * round with the tile, so that the tiles an SM holds (about GD_NUM_SMS apart) load its four
+     * schedulers alike. Split lanes keep the slots' order (2 % faster there). */
+    const bool by_slot = SPLIT || roams;
+    const int wr = SPLIT ? warp - sp * (A >> 5) : (warp + t + t / GD_NUM_SMS) % nwarps;
+    const int ai = wr * 32 + lane;
+    const bool active = ai < kp * L;
+    const int hi = active ? ai / (by_slot ? L : kp) : 0,
+              lo = active ? ai - hi * (by_slot ? L : kp) : 0;
+    const int jj = by_slot ? hi : lo, rank = by_slot ? lo : hi;
     /* the thread's lanes: slot jj (PACK 1), or slots 2 jj and 2 jj + 1, the same atom of two
      * replicas (PACK 2); a missing second slot (odd k) repeats the first one's atom and stores
      * nothing. sl_of: each lane's slot; vl: its index in the placed-atom and partial arrays */
@@ -928,7 +957,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     for (int h = 0; h < PACK; ++h) {
       /* (a thread's two lanes hold the same atom of two slots, so PACK 2 keeps the atoms' order) */
       const int lc = slots[sl_of[h]].lig_conf;
-      l_of[h] = PACK == 1 && !SPLIT ? cx.lig_rank[lc * L + rank] : rank;
+      l_of[h] = PACK == 1 && !by_slot ? cx.lig_rank[lc * L + rank] : rank;
       orig[h] = cx.lig_pos[lc * L + l_of[h]];
       vl[h] = sp * A + sl_of[h] * L + l_of[h];
     }
