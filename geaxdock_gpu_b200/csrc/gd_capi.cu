@@ -388,10 +388,18 @@ int ensure_counters(gd_ctx *c, int n) {
   int *p = nullptr;
   cudaMemPool_t pool = ctx_pool(c->device);
   if (pool) {
-    CK(cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), sizeof(int) * n, pool,
-                               c->stream));
+    auto take = [&] {
+      return cudaMallocFromPoolAsync(reinterpret_cast<void **>(&p), sizeof(int) * n, pool,
+                                     c->stream);
+    };
+    cudaError_t e = take();
+    if (e == cudaErrorMemoryAllocation && release_fields(c)) {
+      cudaGetLastError();
+      e = take();
+    }
+    CK(e);
   } else {
-    CK(cudaMalloc(&p, sizeof(int) * n));
+    CK(cmalloc(c, &p, sizeof(int) * n));
   }
   if (c->d_counters) {
     if (c->counters_pooled)
@@ -682,7 +690,7 @@ int ensure_chains(gd_ctx *c) {
     if (c->d_chain_tiles) cudaFree(c->d_chain_tiles);
     c->d_chain_tiles = nullptr;
     c->chain_tiles_cap = 0;
-    CK(cudaMalloc(&c->d_chain_tiles, sizeof(GdTileDesc) * tiles.size()));
+    CK(cmalloc(c, &c->d_chain_tiles, sizeof(GdTileDesc) * tiles.size()));
     c->chain_tiles_cap = (int)tiles.size();
   }
   CK(cudaMemcpyAsync(c->d_chain_tiles, tiles.data(), sizeof(GdTileDesc) * tiles.size(),
@@ -984,10 +992,6 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   c->n_groups = goff;
   if ((rc = upload(c, &c->d_cx, dcx)) || (rc = upload(c, &c->d_group_base, group_base)))
     return bail(rc);
-  if ((rc = build_pocket_lists(c, dcx)) || (rc = build_far_fields(c, ff, cxs, dcx)))
-    return bail(rc);
-  CK(cudaMemcpyAsync(c->d_cx, dcx.data(), sizeof(GdDevComplex) * dcx.size(),
-                     cudaMemcpyHostToDevice, c->stream));
 
   /* ---- replica state ---- */
   const int R = c->n_rep;
@@ -1027,8 +1031,27 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   if ((rc = dalloc(c, &c->d_tiles, c->tiles_cap))) return bail(rc);
   if ((rc = ensure_counters(c, 64))) return bail(rc);
   if ((rc = dalloc(c, &c->d_cursor, 2))) return bail(rc);
+  /* ---- what makes steps faster, in the memory that is left ---- */
+  if ((rc = build_pocket_lists(c, dcx)) || (rc = build_far_fields(c, ff, cxs, dcx)))
+    return bail(rc);
+  CK(cudaMemcpyAsync(c->d_cx, dcx.data(), sizeof(GdDevComplex) * dcx.size(),
+                     cudaMemcpyHostToDevice, c->stream));
   CK(cudaStreamSynchronize(c->stream));
   *out = c;
+  return GD_OK;
+}
+
+int gd_release_far_fields(gd_ctx *c) {
+  if (!c) return fail(GD_ERR_INVALID, "null context");
+  CK(cudaSetDevice(c->device));
+  CK(cudaStreamSynchronize(c->stream));
+  release_fields(c);
+  return GD_OK;
+}
+
+int gd_far_field_bytes(const gd_ctx *c, long long *n) {
+  if (!c || !n) return fail(GD_ERR_INVALID, "null argument");
+  *n = (long long)c->field_bytes;
   return GD_OK;
 }
 

@@ -19,6 +19,7 @@ struct DaState {
   int split = 1;                                 /* protein split of the exact stage */
   double last_pass = 1.0;                        /* surrogate-stage pass rate, last window */
   unsigned long long prev_prop = 0, prev_pass = 0;
+  gd_ctx *ctx = nullptr;                         /* the context it belongs to */
   std::vector<void *> allocs;
   int *d_rep_cx = nullptr, *d_rep_group = nullptr, *d_group_b0 = nullptr;
   int *d_emb_base = nullptr, *d_active = nullptr;
@@ -64,12 +65,22 @@ template <class T>
 int da_alloc(DaState *d, T **p, size_t n) {
   *p = nullptr;
   void *q = nullptr;
-  cudaError_t e = cudaMalloc(&q, std::max<size_t>(1, n) * sizeof(T));
+  cudaError_t e = cmalloc(d->ctx, &q, std::max<size_t>(1, n) * sizeof(T));
   if (e != cudaSuccess)
     return fail(GD_ERR_NOMEM, "cudaMalloc(%zu) failed: %s", n * sizeof(T), cudaGetErrorString(e));
   d->allocs.push_back(q);
   *p = (T *)q;
   return GD_OK;
+}
+
+/* the network's work buffers for `rows` rows */
+int da_reserve(gd_ctx *c, int rows) {
+  int rc = gd::mlp_reserve(c->da->net, rows);
+  if (rc == -3 && release_fields(c)) {
+    cudaGetLastError();
+    rc = gd::mlp_reserve(c->da->net, rows);
+  }
+  return rc;
 }
 
 void da_free_trace(DaState *d) {
@@ -385,7 +396,7 @@ int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGrap
     }
     d->d_counters = nullptr;
     d->counters_cap = 0;
-    CK(cudaMalloc(&d->d_counters, sizeof(int) * n_steps * nch));
+    CK(cmalloc(c, &d->d_counters, sizeof(int) * n_steps * nch));
     d->counters_cap = n_steps * nch;
   }
   if ((rc = da_upload_epi(c))) return rc;
@@ -624,6 +635,7 @@ int gd_sur_create(gd_ctx *c, const gd_sur_params *p) {
   CK(cudaStreamSynchronize(c->stream));
   da_free(c);
   DaState *d = new DaState();
+  d->ctx = c;
   c->da = d;
   d->prm = *p;
   int n_emb = 0;
@@ -640,12 +652,18 @@ int gd_sur_create(gd_ctx *c, const gd_sur_params *p) {
     da_free(c);          \
     return rc;           \
   }
-  if (gd::mlp_create(d->net, p->hidden, p->embedding ? n_emb : 0, p->seed, c->stream)) {
-    da_free(c);
-    return fail(GD_ERR_NOMEM, "network allocation failed");
+  auto net_create = [&] {
+    return gd::mlp_create(d->net, p->hidden, p->embedding ? n_emb : 0, p->seed, c->stream);
+  };
+  if (net_create()) {
+    gd::mlp_destroy(d->net);
+    if (!release_fields(c) || (cudaGetLastError(), net_create())) {
+      da_free(c);
+      return fail(GD_ERR_NOMEM, "network allocation failed");
+    }
   }
   const int rows = p->batch; /* DA steps keep their rows in shared memory */
-  if (gd::mlp_reserve(d->net, rows)) {
+  if (da_reserve(c, rows)) {
     da_free(c);
     return fail(GD_ERR_NOMEM, "network work buffers (%d rows)", rows);
   }
@@ -751,7 +769,7 @@ int gd_sur_train(gd_ctx *c, int iterations, float *losses) {
     if (d->d_loss_hist) cudaFree(d->d_loss_hist);
     d->d_loss_hist = nullptr;
     d->loss_cap = 0;
-    CK(cudaMalloc(&d->d_loss_hist, sizeof(float) * iterations));
+    CK(cmalloc(c, &d->d_loss_hist, sizeof(float) * iterations));
     d->loss_cap = iterations;
   }
   gd::GdDaDev a = da_args(c);
@@ -905,12 +923,12 @@ int gd_sur_predict(gd_ctx *c, int ci, int prt_conf, int lig_conf, const float *m
   DaState *d = c->da;
   CK(cudaSetDevice(c->device));
   CK(cudaStreamSynchronize(c->stream));
-  if (gd::mlp_reserve(d->net, n)) return fail(GD_ERR_NOMEM, "network work buffers");
+  if (da_reserve(c, n)) return fail(GD_ERR_NOMEM, "network work buffers");
   if (n > d->pred_cap) {
     if (d->d_pred_mm) cudaFree(d->d_pred_mm);
     d->d_pred_mm = nullptr;
     d->pred_cap = 0;
-    CK(cudaMalloc(&d->d_pred_mm, sizeof(float) * 6 * n));
+    CK(cmalloc(c, &d->d_pred_mm, sizeof(float) * 6 * n));
     d->pred_cap = n;
   }
   /* the work buffers may have moved: graphs that point at them are stale */
@@ -952,9 +970,9 @@ int gd_da_trace_enable(gd_ctx *c, int step0, int max_steps) {
   d->tr_step0 = step0;
   if (max_steps == 0) return da_upload_epi(c);
   const size_t n = (size_t)c->n_rep * max_steps;
-  CK(cudaMalloc(&d->tr_s, sizeof(float) * n));
-  CK(cudaMalloc(&d->tr_e, sizeof(float) * n));
-  CK(cudaMalloc(&d->tr_flag, sizeof(int) * n));
+  CK(cmalloc(c, &d->tr_s, sizeof(float) * n));
+  CK(cmalloc(c, &d->tr_e, sizeof(float) * n));
+  CK(cmalloc(c, &d->tr_flag, sizeof(int) * n));
   CK(cudaMemsetAsync(d->tr_flag, 0xff, sizeof(int) * n, c->stream));
   d->tr_cap = max_steps;
   return da_upload_epi(c);

@@ -52,14 +52,14 @@ int eval_poses(gd_ctx *c, int ci, int prt_conf, int lig_conf, const float *mm, c
     if (c->d_eval_in) cudaFree(c->d_eval_in);
     c->d_eval_in = nullptr;
     c->eval_in_cap = 0;
-    CK(cudaMalloc(&c->d_eval_in, row * n));
+    CK(cmalloc(c, &c->d_eval_in, row * n));
     c->eval_in_cap = row * n;
   }
   if (n > c->eval_cap) {
     if (c->d_e_out) cudaFree(c->d_e_out);
     c->d_e_out = nullptr;
     c->eval_cap = 0;
-    CK(cudaMalloc(&c->d_e_out, sizeof(gd_energy) * n));
+    CK(cmalloc(c, &c->d_e_out, sizeof(gd_energy) * n));
     c->eval_cap = n;
   }
   /* small calls go through a page-locked buffer of the context, so that the copies and the kernel
@@ -161,8 +161,8 @@ int gd_place_ligand(gd_ctx *c, int ci, int lig_conf, const float *mm, int n, flo
   const size_t out_bytes = sizeof(float) * 3 * (size_t)x.lna * n;
   float *d_mm = nullptr, *d_xyz = nullptr;
   CK(cudaStreamSynchronize(c->stream));
-  cudaError_t e = cudaMalloc(&d_mm, sizeof(float) * 6 * (size_t)n);
-  if (e == cudaSuccess) e = cudaMalloc(&d_xyz, out_bytes);
+  cudaError_t e = cmalloc(c, &d_mm, sizeof(float) * 6 * (size_t)n);
+  if (e == cudaSuccess) e = cmalloc(c, &d_xyz, out_bytes);
   if (e == cudaSuccess) e = cudaMemcpyAsync(d_mm, mm, sizeof(float) * 6 * (size_t)n,
                                        cudaMemcpyHostToDevice, c->stream);
   if (e == cudaSuccess) {
@@ -189,8 +189,8 @@ int gd_trace_enable(gd_ctx *c, int max_steps) {
   c->trace_cap = 0;
   drop_graphs(c);
   if (max_steps == 0) return GD_OK;
-  CK(cudaMalloc(&c->d_trace_e, sizeof(float) * (size_t)c->n_rep * max_steps));
-  CK(cudaMalloc(&c->d_trace_acc, sizeof(int) * (size_t)c->n_rep * max_steps));
+  CK(cmalloc(c, &c->d_trace_e, sizeof(float) * (size_t)c->n_rep * max_steps));
+  CK(cmalloc(c, &c->d_trace_acc, sizeof(int) * (size_t)c->n_rep * max_steps));
   CK(cudaMemsetAsync(c->d_trace_acc, 0xff, sizeof(int) * (size_t)c->n_rep * max_steps, c->stream));
   c->trace_cap = max_steps;
   c->trace_step0 = 0;

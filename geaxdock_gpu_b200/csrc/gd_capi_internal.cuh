@@ -128,6 +128,8 @@ struct gd_ctx {
   std::vector<gdc::ComplexInfo> info;
   std::vector<void *> allocs;      /* cudaMalloc'd buffers */
   std::vector<void *> pool_allocs; /* buffers from the device's context pool (ctx_pool) */
+  std::vector<void *> field_allocs; /* those of them that hold the far fields' tables */
+  size_t field_bytes = 0;
   GdForceConst fc{};
   GdDevComplex *d_cx = nullptr;
   GdPairParam *d_pp = nullptr;
@@ -208,9 +210,11 @@ int dalloc(gd_ctx *c, T **p, size_t n) {
   cudaMemPool_t pool = ctx_pool(c->device);
   cudaError_t e = pool ? cudaMallocFromPoolAsync(&q, n * sizeof(T), pool, c->stream)
                        : cudaMalloc(&q, n * sizeof(T));
-  if (e != cudaSuccess)
+  if (e != cudaSuccess) {
+    cudaGetLastError();
     return fail(GD_ERR_NOMEM, "allocation of %zu bytes failed: %s", n * sizeof(T),
                 cudaGetErrorString(e));
+  }
   (pool ? c->pool_allocs : c->allocs).push_back(q);
   *p = (T *)q;
   return GD_OK;
@@ -218,6 +222,22 @@ int dalloc(gd_ctx *c, T **p, size_t n) {
 
 /* frees a buffer of dalloc before the context ends (stream-ordered) */
 void dfree(gd_ctx *c, void *p);
+
+/* Gives the far fields' tables back to the driver: every pair runs in the loop from then on (the
+ * same decisions; energies in which no far point is a series). False if there are none. */
+bool release_fields(gd_ctx *c);
+/* cudaMalloc for a buffer the context needs: the optional tables make room for it */
+template <class T>
+cudaError_t cmalloc(gd_ctx *c, T **p, size_t bytes) {
+  void *q = nullptr;
+  cudaError_t e = cudaMalloc(&q, bytes);
+  if (e == cudaErrorMemoryAllocation && release_fields(c)) {
+    cudaGetLastError();
+    e = cudaMalloc(&q, bytes);
+  }
+  *p = e == cudaSuccess ? static_cast<T *>(q) : nullptr;
+  return e;
+}
 
 template <class T>
 int upload(gd_ctx *c, T **p, const std::vector<T> &v) {
@@ -294,10 +314,11 @@ void da_drop_graphs(gd_ctx *c);
 int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1],
                    const gd_complex_desc &d, int ci, GdDevComplex &g);
 
-/* ---- the pocket grid's point lists (gd_pocket.cu) ---- */
+/* ---- the pocket grid's point lists (gd_pocket.cu): optional, left out without memory ---- */
 int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx);
 
-/* ---- the far fields of large proteins (gd_farfield.cu) ---- */
+/* ---- the far fields of large proteins (gd_farfield.cu): optional, in a quarter of the memory
+ * that is free when the context has all it needs ---- */
 int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs,
                      std::vector<GdDevComplex> &dcx);
 

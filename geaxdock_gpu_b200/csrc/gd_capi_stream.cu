@@ -200,7 +200,7 @@ int rs_enqueue(gd_ctx *c, int rows_per_rep) {
     if (r->d_pack[k]) cudaFree(r->d_pack[k]);
     r->d_pack[k] = nullptr;
     r->pack_rows[k] = 0;
-    e = cudaMalloc(&r->d_pack[k], (size_t)need * sizeof(gd_record_step));
+    e = cmalloc(c, &r->d_pack[k], (size_t)need * sizeof(gd_record_step));
     if (e == cudaSuccess) r->pack_rows[k] = need;
   }
   int *plan = r->d_plan[k], n = r->n_rep;
@@ -327,11 +327,11 @@ int gd_records_stream(gd_ctx *c, gd_record_step *steps, int cap) {
   r->d_rec = c->d_rec;
   r->snap.assign(c->n_rep, 0);
   cudaError_t e = cudaStreamCreateWithFlags(&r->cs, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&r->d_prev, sizeof(int) * (size_t)c->n_rep);
+  if (e == cudaSuccess) e = cmalloc(c, &r->d_prev, sizeof(int) * (size_t)c->n_rep);
   if (e == cudaSuccess) e = cudaMemsetAsync(r->d_prev, 0, sizeof(int) * (size_t)c->n_rep, c->stream);
   if (e == cudaSuccess) e = cudaHostAlloc(&r->h_plan, sizeof(int) * r->plan_ints(), 0);
   for (int i = 0; i < RecStream::NSNAP && e == cudaSuccess; ++i) {
-    e = cudaMalloc(&r->d_plan[i], sizeof(int) * r->plan_ints());
+    e = cmalloc(c, &r->d_plan[i], sizeof(int) * r->plan_ints());
     if (e == cudaSuccess)
       e = cudaEventCreateWithFlags(&r->ev[i], cudaEventDisableTiming | cudaEventBlockingSync);
   }

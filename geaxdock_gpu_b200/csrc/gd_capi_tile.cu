@@ -38,7 +38,7 @@ int tile_changed(gd_ctx *c) {
   const int need = (int)c->full_tiles.size() + 2 * blocks + 16;
   if (need > c->tiles_cap) {
     GdTileDesc *p = nullptr;
-    CK(cudaMalloc(&p, need * sizeof(GdTileDesc)));
+    CK(cmalloc(c, &p, need * sizeof(GdTileDesc)));
     c->allocs.push_back(p);
     c->d_tiles = p;
     c->tiles_cap = need;
@@ -147,7 +147,7 @@ int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile
   const size_t R = (size_t)c->n_rep;
   const size_t bytes = R * (6 * sizeof(float) + sizeof(gd_energy) + sizeof(float) + sizeof(int));
   char *keep = nullptr;
-  if (cudaMalloc(&keep, bytes) != cudaSuccess)
+  if (cmalloc(c, &keep, bytes) != cudaSuccess)
     return fail(GD_ERR_NOMEM, "gd_autotune: no memory for the copy of the chain state");
   float *k_mm = reinterpret_cast<float *>(keep);
   gd_energy *k_e = reinterpret_cast<gd_energy *>(k_mm + R * 6);

@@ -258,6 +258,40 @@ static bool ff_radii(const gd_enepara *ff, double *r_f, double *r_hdb) {
   return true;
 }
 
+/* Bytes the tables may take: a quarter of what the device has free once the context holds all it
+ * must (the pool's idle memory is free too), so that records, samples and poses asked for later
+ * and other users of the device find room; release_fields gives even that back. */
+static size_t field_budget(gd_ctx *c) {
+  size_t free_b = 0, total_b = 0;
+  if (cudaStreamSynchronize(c->stream) != cudaSuccess ||
+      cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  uint64_t held = 0, used = 0;
+  cudaMemPool_t pool = ctx_pool(c->device);
+  if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) ==
+                  cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess &&
+      held > used)
+    free_b += held - used;
+  return free_b / 4;
+}
+
+bool release_fields(gd_ctx *c) {
+  if (c->field_allocs.empty()) return false;
+  cudaStreamSynchronize(c->stream); /* no kernel reads the tables */
+  for (int ci = 0; ci < c->n_complex; ++ci)
+    cudaMemsetAsync(reinterpret_cast<char *>(c->d_cx + ci) + offsetof(GdDevComplex, ff_tab), 0,
+                    sizeof(float *), c->stream);
+  for (void *p : c->field_allocs) dfree(c, p);
+  c->field_allocs.clear();
+  c->field_bytes = 0;
+  cudaStreamSynchronize(c->stream);
+  if (cudaMemPool_t pool = ctx_pool(c->device)) cudaMemPoolTrimTo(pool, 0);
+  return true;
+}
+
 int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs,
                      std::vector<GdDevComplex> &dcx) {
   double r_f, r_hdb[GD_MAXTP1];
@@ -298,6 +332,7 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
                           (int)((1 + GD_MAXTP2) * gd::NODES * sizeof(double))));
   std::vector<gd::FfArgs> jobs;
   std::vector<double *> pmf;
+  const size_t budget = field_budget(c);
   for (auto &gp : groups) {
     gd::FfArgs a{};
     a.pp = c->d_pp;
@@ -314,11 +349,6 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
         id[k] = (short)cells.size();
         cells.push_back(k);
       }
-    int *d_cells = nullptr;
-    short *d_id = nullptr;
-    if ((rc = upload(c, &d_cells, cells)) || (rc = upload(c, &d_id, id))) return rc;
-    CK(cudaStreamSynchronize(c->stream)); /* the host vectors end here */
-    a.cells = d_cells;
     a.n_cells = (int)cells.size();
     a.lj1 = ff->lj1;
     unsigned char slot[GD_MAXTP2] = {};
@@ -329,13 +359,27 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
       }
     const int n_prt = c->info[a.rep].n_prt;
     const size_t per = (size_t)cells.size() * (1 + a.n_types) * GD_FF_NC;
+    const size_t n_pmf = (size_t)n_prt * GD_FAR_BINS * GD_MAXTP2;
+    const size_t bytes = sizeof(float) * per * n_prt + sizeof(double) * n_pmf +
+                         sizeof(int) * cells.size() + sizeof(short) * id.size();
+    /* a protein whose tables do not fit runs without them */
+    if (c->field_bytes + bytes > budget) continue;
+    int *d_cells = nullptr;
+    short *d_id = nullptr;
     double *p = nullptr;
-    /* a device too full for the tables runs without them */
-    if (dalloc(c, &a.tab, per * n_prt) || dalloc(c, &p, (size_t)n_prt * GD_FAR_BINS * GD_MAXTP2)) {
-      cudaGetLastError();
-      if (a.tab) dfree(c, a.tab);
-      continue;
+    const bool made = !upload(c, &d_cells, cells) && !upload(c, &d_id, id) &&
+                      !dalloc(c, &a.tab, per * n_prt) && !dalloc(c, &p, n_pmf);
+    CK(cudaStreamSynchronize(c->stream)); /* the host vectors end here */
+    for (void *q : {(void *)d_cells, (void *)d_id, (void *)a.tab, (void *)p}) {
+      if (!q) continue;
+      if (made)
+        c->field_allocs.push_back(q);
+      else
+        dfree(c, q);
     }
+    if (!made) continue;
+    c->field_bytes += bytes;
+    a.cells = d_cells;
     for (int ci : gp->members) {
       GdDevComplex &g = dcx[ci];
       g.ff_id = d_id;

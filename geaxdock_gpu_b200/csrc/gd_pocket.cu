@@ -102,10 +102,11 @@ __global__ void __launch_bounds__(32 * WARPS)
 
 namespace gdc {
 
+namespace {
+
 /* The lists of every conformer of the batch: counts on the device, starts on the host, the
- * lists in one buffer; fills in the complexes' pg_start / pg_idx (c->d_cx holds the complexes
- * without them; the caller uploads dcx again). */
-int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx) {
+ * lists in one buffer; fills in the complexes' pg_start / pg_idx. got: the buffers made */
+int pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx, std::vector<void *> &got) {
   std::vector<int2> conf;
   for (int ci = 0; ci < c->n_complex; ++ci)
     for (int p = 0; p < c->info[ci].n_prt; ++p) conf.push_back(make_int2(ci, p));
@@ -115,7 +116,10 @@ int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx) {
   int2 *d_conf = nullptr;
   int *d_cnt = nullptr;
   int rc;
-  if ((rc = upload(c, &d_conf, conf)) || (rc = dalloc(c, &d_cnt, (size_t)n_cells * 2))) return rc;
+  if ((rc = upload(c, &d_conf, conf))) return rc;
+  got.push_back(d_conf);
+  if ((rc = dalloc(c, &d_cnt, (size_t)n_cells * 2))) return rc;
+  got.push_back(d_cnt);
   const unsigned grid = (unsigned)((n_cells + gd::WARPS - 1) / gd::WARPS);
   gd::pocket_kernel<false><<<grid, 32 * gd::WARPS, 0, c->stream>>>(c->d_cx, d_conf, n_cells,
                                                                    d_cnt, nullptr, nullptr);
@@ -144,9 +148,12 @@ int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx) {
   unsigned short *d_idx = nullptr;
   int *d_start = nullptr;
   long long *d_base = nullptr;
-  if ((rc = upload(c, &d_start, start)) || (rc = upload(c, &d_base, base)) ||
-      (rc = dalloc(c, &d_idx, (size_t)total)))
-    return rc;
+  if ((rc = upload(c, &d_start, start))) return rc;
+  got.push_back(d_start);
+  if ((rc = upload(c, &d_base, base))) return rc;
+  got.push_back(d_base);
+  if ((rc = dalloc(c, &d_idx, (size_t)total))) return rc;
+  got.push_back(d_idx);
   CK(cudaMemcpyAsync(d_cnt, cnt.data(), sizeof(int) * cnt.size(), cudaMemcpyHostToDevice,
                      c->stream));
   gd::pocket_kernel<true><<<grid, 32 * gd::WARPS, 0, c->stream>>>(c->d_cx, d_conf, n_cells, d_cnt,
@@ -162,6 +169,21 @@ int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx) {
   }
   dfree(c, d_conf);
   dfree(c, d_cnt);
+  return GD_OK;
+}
+
+}  // namespace
+
+/* (c->d_cx holds the complexes without the lists; the caller uploads dcx again.) Without the
+ * memory for them no atom finds itself in the grid, and each walks the rows of the cell list. */
+int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx) {
+  std::vector<void *> got;
+  const int rc = pocket_lists(c, dcx, got);
+  if (rc != GD_ERR_NOMEM) return rc;
+  CK(cudaStreamSynchronize(c->stream)); /* the uploads' host arrays are gone */
+  for (void *p : got) dfree(c, p);
+  for (GdDevComplex &g : dcx)
+    for (float &o : g.pg_org) o = std::numeric_limits<float>::quiet_NaN();
   return GD_OK;
 }
 

@@ -50,6 +50,8 @@ def lib() -> C.CDLL:
         "gd_release_memory": [C.c_int],
         "gd_num_replicas": [vp, ip],
         "gd_replica_offset": [vp, C.c_int, ip],
+        "gd_far_field_bytes": [vp, C.POINTER(C.c_longlong)],
+        "gd_release_far_fields": [vp],
         "gd_set_tile": [vp, C.c_int, C.POINTER(abi.Tile)],
         "gd_get_tile": [vp, C.c_int, C.POINTER(abi.Tile)],
         "gd_mc_init": [vp],
@@ -207,6 +209,16 @@ class Engine:
 
     def sync(self):
         check(lib().gd_sync(self.h))
+
+    def far_field_bytes(self) -> int:
+        """Device bytes of the tables that let steps on large proteins skip far points (0: none)."""
+        n = C.c_longlong()
+        check(lib().gd_far_field_bytes(self.h, C.byref(n)))
+        return n.value
+
+    def release_far_fields(self):
+        """Gives that memory back; steps run every pair from then on."""
+        check(lib().gd_release_far_fields(self.h))
 
     def set_tile(self, replicas_per_cta: int, chunk_points: int, unroll: int = 0,
                  split: int = 0, threads: int = 0, replicas_per_lane: int = 1,

@@ -218,6 +218,12 @@ int gd_destroy(gd_ctx *ctx);
 /* Returns the memory the device's context pool holds without a live context to the driver
  * (no reference counterpart). */
 int gd_release_memory(int device);
+/* The tables that let steps on large proteins skip the far points: their bytes on the device (0:
+ * none), and their memory back to the driver. Without them steps are slower and energies differ
+ * in the last FP32 digits. They are made by gd_create in at most a quarter of the memory then
+ * free, and given back by themselves when the context needs the room. */
+int gd_far_field_bytes(const gd_ctx *ctx, long long *bytes);
+int gd_release_far_fields(gd_ctx *ctx);
 int gd_num_replicas(const gd_ctx *ctx, int *n_rep);
 int gd_replica_offset(const gd_ctx *ctx, int complex_index, int *offset);
 /* Tile of the fused kernel for one complex (-1: all); one CTA size per context. */
