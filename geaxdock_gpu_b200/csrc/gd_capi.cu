@@ -420,26 +420,30 @@ int ensure_cursor(gd_ctx *c) {
 
 
 /* the kernel variant for an unroll depth, a protein split and the mode-3 epilogue */
-template <bool S, bool D>
+template <bool S, int K>
 McKernel mc_variant(int unroll) {
-  if (unroll >= 4) return gd::gd_mc_kernel<4, S, D, 1>;
-  if (unroll >= 2) return gd::gd_mc_kernel<2, S, D, 1>;
-  return gd::gd_mc_kernel<1, S, D, 1>;
+  if (unroll >= 4) return gd::gd_mc_kernel<4, S, K, 1>;
+  if (unroll >= 2) return gd::gd_mc_kernel<2, S, K, 1>;
+  return gd::gd_mc_kernel<1, S, K, 1>;
 }
 
-McKernel mc_kernel(int unroll, int split, bool da, int pack) {
-  if (da) return split > 1 ? mc_variant<true, true>(unroll) : mc_variant<false, true>(unroll);
+McKernel mc_kernel(int unroll, int split, int kind, int pack) {
+  if (kind == GD_KIND_EXCHANGE) return gd::gd_mc_kernel<2, false, GD_KIND_EXCHANGE, 1>;
+  if (kind == GD_KIND_DA)
+    return split > 1 ? mc_variant<true, GD_KIND_DA>(unroll) : mc_variant<false, GD_KIND_DA>(unroll);
   if (pack == 2 && split <= 1)
-    return unroll >= 2 ? gd::gd_mc_kernel<2, false, false, 2> : gd::gd_mc_kernel<1, false, false, 2>;
-  return split > 1 ? mc_variant<true, false>(unroll) : mc_variant<false, false>(unroll);
+    return unroll >= 2 ? gd::gd_mc_kernel<2, false, GD_KIND_PLAIN, 2>
+                       : gd::gd_mc_kernel<1, false, GD_KIND_PLAIN, 2>;
+  return split > 1 ? mc_variant<true, GD_KIND_PLAIN>(unroll)
+                   : mc_variant<false, GD_KIND_PLAIN>(unroll);
 }
 
 /* threads per CTA of a launch: the tile's lanes over the replicas per thread (two only for the
  * plain modes without split) */
 int launch_threads(const LaunchShape &s) { return s.lanes / s.pack; }
 
-McKernel launch_kernel(const LaunchShape &s, bool da) {
-  return mc_kernel(s.unroll, s.split, da, s.pack);
+McKernel launch_kernel(const LaunchShape &s, int kind) {
+  return mc_kernel(s.unroll, s.split, kind, s.pack);
 }
 
 GdMcArgs base_args(gd_ctx *c) {
@@ -480,8 +484,8 @@ struct KernelSetting {
 std::mutex g_attr_mu;
 std::map<std::pair<McKernel, int>, KernelSetting> g_attr;
 
-int kernel_setting(const LaunchShape &s, bool da, int *blocks) {
-  const McKernel k = launch_kernel(s, da);
+int kernel_setting(const LaunchShape &s, int kind, int *blocks) {
+  const McKernel k = launch_kernel(s, kind);
   const size_t smem = smem_bytes(s);
   const int threads = launch_threads(s);
   int dev = 0;
@@ -545,12 +549,70 @@ void forget_kernel_attrs(int device) {
     if (x.first.second == device) x.second.blocks = 0;
 }
 
-int set_kernel_attrs(const LaunchShape &s, bool da) { return kernel_setting(s, da, nullptr); }
+int set_kernel_attrs(const LaunchShape &s, int kind) { return kernel_setting(s, kind, nullptr); }
 
-int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da) {
+int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, int kind) {
   int nb = 1;
-  if (kernel_setting(s, da, &nb) != GD_OK) nb = 1;
+  if (kernel_setting(s, kind, &nb) != GD_OK) nb = 1;
   return std::max(1, std::min(n_tiles, nb * c->num_sms));
+}
+
+void set_open_lists(gd_ctx *c, const Chain &ch, int k, GdMcArgs *a) {
+  a->x_open = c->d_xopen + 2 * k;
+  a->x_open_list = c->d_xopen + 2 * GD_MAX_CHAINS + ch.xg0;
+  a->x_open_cap = ch.xg1 - ch.xg0;
+  a->x_group_base = c->d_group_base;
+  a->x_acs = c->d_acs;
+}
+
+/* the pair loop's energies, their FP32 sums as long as the steps' */
+LaunchShape exchange_shape(const LaunchShape &s) {
+  return {GD_MAX_TPB, s.fold, s.fold, 1, 2, 1, 8};
+}
+
+int prepare_exchange(const gd_ctx *c, const LaunchShape &s) {
+  return c->field_bytes ? set_kernel_attrs(exchange_shape(s), GD_KIND_EXCHANGE) : GD_OK;
+}
+
+int launch_exchange(gd_ctx *c, const Chain &ch, int k, const LaunchShape &s, bool fused, int step0,
+                    const int *step_base, const int *call_base, int call_off, int mode_t,
+                    cudaStream_t st) {
+  GdMcArgs a = base_args(c);
+  set_open_lists(c, ch, k, &a);
+  const int n = ch.xg1 - ch.xg0;
+  if (!fused) {
+    const GdExchange ex = {a.replica, a.etotal, a.e_old, a.x_acs, a.seed};
+    gd::gd_exchange_kernel<<<(n + 127) / 128, 128, 0, st>>>(
+        c->d_cx, c->d_group_base, c->n_complex, ch.xg0, ch.xg1, ex, c->fc, call_base, call_off,
+        mode_t, a.x_open, a.x_open_list, c->d_err);
+    CK(cudaGetLastError());
+  }
+  if (!c->field_bytes || mode_t >= 2) return GD_OK;
+  const LaunchShape x = exchange_shape(s);
+  const int rc = set_kernel_attrs(x, GD_KIND_EXCHANGE);
+  if (rc) return rc;
+  a.mode = 2;
+  a.n_steps = 1;
+  a.step0 = step0;
+  a.step_base = step_base;
+  a.chunk = x.chunk;
+  a.fold = x.fold;
+  a.split = 1;
+  a.mm_in = c->d_mm;
+  a.u.count = x.kmax;
+  a.rec = nullptr;
+  a.trace_e = nullptr;
+  a.trace_acc = nullptr;
+  a.x_call_base = call_base;
+  a.x_call_off = call_off;
+  a.x_spd = c->mc.steps_per_dump;
+  a.x_spe = c->mc.steps_per_exchange;
+  a.x_mode_t = mode_t;
+  a.n_complex = c->n_complex;
+  launch_kernel(x, GD_KIND_EXCHANGE)<<<std::min(n, c->num_sms), launch_threads(x), smem_bytes(x),
+                                       st>>>(a, c->fc);
+  CK(cudaGetLastError());
+  return GD_OK;
 }
 
 int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter,
@@ -1003,8 +1065,10 @@ int gd_create(const gd_enepara *ff, const gd_complex_desc *cxs, int n_complexes,
   if ((rc = upload(c, &c->d_replica, rep)) || (rc = dalloc(c, &c->d_mm, (size_t)R * 6)) ||
       (rc = dalloc(c, &c->d_eold, R)) || (rc = dalloc(c, &c->d_etotal, R)) ||
       (rc = dalloc(c, &c->d_nacc, R)) || (rc = dalloc(c, &c->d_acs, R)) ||
-      (rc = dalloc(c, &c->d_rec_next, R)) || (rc = dalloc(c, &c->d_err, 1)))
+      (rc = dalloc(c, &c->d_rec_next, R)) || (rc = dalloc(c, &c->d_err, 1)) ||
+      (rc = dalloc(c, &c->d_xopen, (size_t)2 * GD_MAX_CHAINS + c->n_groups)))
     return bail(rc);
+  CK(cudaMemsetAsync(c->d_xopen, 0, sizeof(int) * 2 * GD_MAX_CHAINS, c->stream));
   CK(cudaMemsetAsync(c->d_mm, 0, sizeof(float) * 6 * R, c->stream));
   CK(cudaMemsetAsync(c->d_nacc, 0, sizeof(int) * R, c->stream));
   CK(cudaMemsetAsync(c->d_acs, 0, sizeof(int) * R, c->stream));
@@ -1120,10 +1184,11 @@ int gd_exchange(gd_ctx *c, int mode_l, int mode_t) {
   if (!c->initialized) return fail(GD_ERR_STATE, "gd_mc_init has not run");
   if (mode_t < 0) return fail(GD_ERR_INVALID, "mode_t must be >= 0");
   CK(cudaSetDevice(c->device));
-  gd::gd_exchange_kernel<<<(c->n_groups + 127) / 128, 128, 0, c->stream>>>(
-      c->d_cx, c->d_group_base, c->n_complex, 0, c->n_groups, c->d_replica, c->d_etotal,
-      c->d_acs, c->mc.seed, nullptr, c->exchange_calls, mode_t);
-  CK(cudaGetLastError());
+  Chain all{};
+  all.xg1 = c->n_groups;
+  const int rc = launch_exchange(c, all, 0, ctx_shape(c), false, 0, nullptr, nullptr,
+                                 c->exchange_calls, mode_t, c->stream);
+  if (rc) return rc;
   c->exchange_calls += 1;
   return GD_OK;
 }
@@ -1147,7 +1212,7 @@ int gd_mc_run_fused(gd_ctx *c, int s1, int n_steps, int exchange) {
   if (it == c->graphs.end()) {
     CK(cudaStreamSynchronize(c->stream));
     const LaunchShape shape = ctx_shape(c);
-    if ((rc = set_kernel_attrs(shape))) return rc;
+    if ((rc = set_kernel_attrs(shape)) || (rc = prepare_exchange(c, shape))) return rc;
     cudaGraph_t graph;
     CK(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemsetAsync(c->d_counters, 0, sizeof(int) * n_ctr, c->stream);
@@ -1168,18 +1233,24 @@ int gd_mc_run_fused(gd_ctx *c, int s1, int n_steps, int exchange) {
         if (exchange) {
           /* the chain's groups are whole (chains are made of protein-conformer blocks) */
           a.x_done = c->d_counters + chunks * nch + (size_t)i * c->n_groups;
-          a.x_group_base = c->d_group_base;
-          a.x_acs = c->d_acs;
+          set_open_lists(c, ch, k, &a);
           a.x_call_base = c->d_cursor + 1;
           a.x_call_off = i;
           a.x_spd = c->mc.steps_per_dump;
           a.x_spe = spe;
         }
         launch_kernel(shape)<<<grid, launch_threads(shape), smem_bytes(shape), st>>>(a, c->fc);
+        if (exchange && !rc)
+          rc = launch_exchange(c, ch, k, shape, true, a.step0, a.step_base, a.x_call_base, i, -1,
+                               st);
       }
     }
     chains_join(c, nch);
     cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
+    if (rc) {
+      if (ce == cudaSuccess) cudaGraphDestroy(graph);
+      return rc;
+    }
     if (ce != cudaSuccess) return fail(GD_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
     cudaGraphExec_t exec;
     ce = cudaGraphInstantiate(&exec, graph, 0);

@@ -367,7 +367,7 @@ void da_launch_exact(gd_ctx *c, const Chain &ch, int k, int n_steps, int j, bool
   a.split = shape.split;
   a.chunk = shape.chunk;
   a.fold = shape.fold;
-  launch_kernel(shape, true)<<<grid_for(c, t1 - t0, shape, true), launch_threads(shape),
+  launch_kernel(shape, GD_KIND_DA)<<<grid_for(c, t1 - t0, shape, GD_KIND_DA), launch_threads(shape),
                                smem_bytes(shape), st>>>(a, c->fc);
 }
 
@@ -401,7 +401,7 @@ int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGrap
   }
   if ((rc = da_upload_epi(c))) return rc;
   CK(cudaStreamSynchronize(c->stream));
-  if ((rc = set_kernel_attrs(shape, true))) return rc;
+  if ((rc = set_kernel_attrs(shape, GD_KIND_DA)) || (rc = prepare_exchange(c, shape))) return rc;
   const gd::GdDaDev a = da_args(c);
   const int spe = c->mc.steps_per_exchange;
   const int ng = (int)d->groups.size();
@@ -421,15 +421,19 @@ int da_graph(gd_ctx *c, int n_steps, int exchange, bool collect, int S, cudaGrap
       da_launch_exact(c, ch, k, n_steps, j, collect, st, shape);
       if (exchange && (j + 1) % spe == 0) {
         const int i = (j + 1) / spe - 1;
-        gd::gd_exchange_kernel<<<(ch.xg1 - ch.xg0 + 127) / 128, 128, 0, st>>>(
-            c->d_cx, c->d_group_base, c->n_complex, ch.xg0, ch.xg1, c->d_replica, c->d_etotal,
-            c->d_acs, c->mc.seed, c->d_cursor + 1, i, !(i % 2));
+        if (!rc)
+          rc = launch_exchange(c, ch, k, shape, false, 0, nullptr, c->d_cursor + 1, i, !(i % 2),
+                               st);
       }
     }
   }
   chains_join(c, nch);
   cudaError_t ce = cudaStreamEndCapture(c->stream, &graph);
   if (ce != cudaSuccess) return fail(GD_ERR_CUDA, "graph capture: %s", cudaGetErrorString(ce));
+  if (rc) {
+    cudaGraphDestroy(graph);
+    return rc;
+  }
   if (frc) {
     cudaGraphDestroy(graph);
     return fail(GD_ERR_INVALID, "delayed acceptance needs hidden = 128 or 256");

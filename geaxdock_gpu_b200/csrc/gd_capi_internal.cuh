@@ -42,20 +42,21 @@
 #include "gd_numerics.h"
 
 namespace gd {
-template <int UNROLL, bool SPLIT, bool DA, int PACK>
+template <int UNROLL, bool SPLIT, int KIND, int PACK>
 __global__ void gd_mc_kernel(GdMcArgs a, GdForceConst f);
-#define GD_EXT(U, S, D, P) \
-  extern template __global__ void gd_mc_kernel<U, S, D, P>(GdMcArgs, GdForceConst);
-GD_EXT(1, false, false, 1) GD_EXT(2, false, false, 1) GD_EXT(4, false, false, 1)
-GD_EXT(1, true, false, 1) GD_EXT(2, true, false, 1) GD_EXT(4, true, false, 1)
-GD_EXT(1, false, true, 1) GD_EXT(2, false, true, 1) GD_EXT(4, false, true, 1)
-GD_EXT(1, true, true, 1) GD_EXT(2, true, true, 1) GD_EXT(4, true, true, 1)
-GD_EXT(1, false, false, 2) GD_EXT(2, false, false, 2)
+#define GD_EXT(U, S, K, P) \
+  extern template __global__ void gd_mc_kernel<U, S, K, P>(GdMcArgs, GdForceConst);
+GD_EXT(1, false, 0, 1) GD_EXT(2, false, 0, 1) GD_EXT(4, false, 0, 1)
+GD_EXT(1, true, 0, 1) GD_EXT(2, true, 0, 1) GD_EXT(4, true, 0, 1)
+GD_EXT(1, false, 1, 1) GD_EXT(2, false, 1, 1) GD_EXT(4, false, 1, 1)
+GD_EXT(1, true, 1, 1) GD_EXT(2, true, 1, 1) GD_EXT(4, true, 1, 1)
+GD_EXT(1, false, 0, 2) GD_EXT(2, false, 0, 2)
+GD_EXT(2, false, 2, 1)
 #undef GD_EXT
 __global__ void gd_exchange_kernel(const GdDevComplex *cxs, const int *group_base, int n_complex,
-                                   int g_begin, int g_end, gd_replica *replica,
-                                   const float *etotal, int *acs, uint64_t seed,
-                                   const int *call_base, int call_off, int mode_t);
+                                   int g_begin, int g_end, GdExchange ex, GdForceConst f,
+                                   const int *call_base, int call_off, int mode_t, int *open,
+                                   int *open_list, unsigned *err);
 __global__ void gd_reset_records_kernel(int *rec_next, int r0, int r1);
 }  // namespace gd
 
@@ -151,6 +152,7 @@ struct gd_ctx {
   int *d_counters = nullptr; /* [counters_cap] persistent-CTA queue heads */
   int counters_cap = 0;
   bool counters_pooled = false; /* d_counters came from ctx_pool */
+  int *d_xopen = nullptr;    /* open exchange groups: [GD_MAX_CHAINS][2] counters, [n_groups] list */
   int *d_cursor = nullptr;   /* [2]: step base, exchange call base (graph replays) */
   int *h_cursor = nullptr;   /* pinned staging */
   unsigned *d_err = nullptr;
@@ -187,6 +189,7 @@ struct gd_ctx {
 };
 
 #define GD_MAX_DEVICES 64
+#define GD_MAX_CHAINS 16
 #define GD_EVAL_STAGE ((size_t)256 << 10) /* bytes of a context's staging buffer */
 
 namespace gdc {
@@ -223,8 +226,9 @@ int dalloc(gd_ctx *c, T **p, size_t n) {
 /* frees a buffer of dalloc before the context ends (stream-ordered) */
 void dfree(gd_ctx *c, void *p);
 
-/* Gives the far fields' tables back to the driver: every pair runs in the loop from then on (the
- * same decisions; energies in which no far point is a series). False if there are none. */
+/* Gives the far fields' tables back to the driver: every pair runs in the loop from then on. A
+ * replica's energy keeps the fields' last digits until its next accepted move. False if there are
+ * none. */
 bool release_fields(gd_ctx *c);
 /* cudaMalloc for a buffer the context needs: the optional tables make room for it */
 template <class T>
@@ -270,12 +274,22 @@ int ensure_counters(gd_ctx *c, int n);
 /* the pinned host cursor of the graph launches (made on first use) */
 int ensure_cursor(gd_ctx *c);
 typedef void (*McKernel)(GdMcArgs, GdForceConst);
-McKernel mc_kernel(int unroll, int split, bool da = false, int pack = 1);
-McKernel launch_kernel(const LaunchShape &s, bool da = false);
+/* kind: GD_KIND_* */
+McKernel mc_kernel(int unroll, int split, int kind = GD_KIND_PLAIN, int pack = 1);
+McKernel launch_kernel(const LaunchShape &s, int kind = GD_KIND_PLAIN);
 int launch_threads(const LaunchShape &s);
-int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, bool da = false);
+int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, int kind = GD_KIND_PLAIN);
 GdMcArgs base_args(gd_ctx *c);
-int set_kernel_attrs(const LaunchShape &s, bool da = false);
+int set_kernel_attrs(const LaunchShape &s, int kind = GD_KIND_PLAIN);
+/* The exchange of groups [ch.xg0, ch.xg1) of chain k after launches of shape s (unless `fused`:
+ * those launches did it), and the launch that decides the groups it left open on the pair loop's
+ * energies (contexts with far fields). mode_t -1: from the step, as the fused launches take it. */
+int launch_exchange(gd_ctx *c, const Chain &ch, int k, const LaunchShape &s, bool fused, int step0,
+                    const int *step_base, const int *call_base, int call_off, int mode_t,
+                    cudaStream_t st);
+/* sets up the second of them before a capture */
+int prepare_exchange(const gd_ctx *c, const LaunchShape &s);
+void set_open_lists(gd_ctx *c, const Chain &ch, int k, GdMcArgs *a);
 /* the next launch on the device sets its kernel's attributes again */
 void forget_kernel_attrs(int device);
 int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int *counter,

@@ -268,8 +268,9 @@ int gd_get_replicas_per_cta(const gd_ctx *c, int k, int *n) {
 }
 
 int gd_set_concurrency(gd_ctx *c, int plain_chains, int da_chains) {
-  if (!c || plain_chains < 1 || plain_chains > 16 || da_chains < 1 || da_chains > 16)
-    return fail(GD_ERR_INVALID, "chains must be in 1..16");
+  if (!c || plain_chains < 1 || plain_chains > GD_MAX_CHAINS || da_chains < 1 ||
+      da_chains > GD_MAX_CHAINS)
+    return fail(GD_ERR_INVALID, "chains must be in 1..%d", GD_MAX_CHAINS);
   CK(cudaSetDevice(c->device));
   CK(cudaStreamSynchronize(c->stream));
   c->chains = plain_chains;

@@ -62,10 +62,18 @@
 #define GD_COST_KIND 90
 #define GD_COST_MCS 40
 #define GD_COST_TAIL 40
-#define GD_SLOT_BYTES 248      /* shared-memory bytes per replica slot (sizeof gd::Slot) */
-/* a decision on a field-based energy stands when it is the same at this share of the sum of its
- * weighted terms' magnitudes above and below (the fields' error is some 1e-7 of it) */
-#define GD_CERT 1e-5f
+#define GD_SLOT_BYTES 252      /* shared-memory bytes per replica slot (sizeof gd::Slot) */
+/* A decision on field-based energies stands when it is the same above and below by what the fields
+ * may change both poses' energies: GD_CERT of a pose's weighted terms' magnitudes (the rounding of
+ * its FP32 results) and what the far points' sums can lose, GD_CERT_ELE of the electrostatic
+ * magnitude of all points at the far radius and GD_CERT_FAR of their vdw and pmf magnitudes
+ * (ff_cert). 600,000 poses of 5 to 100 atoms on 2,100 to 9,900 points, charges up to 90 times the
+ * usual, alternating too, contact weights of both signs 40 times, dispersion 50 times the usual:
+ * the largest change was 1.6e-7 of the magnitudes with usual charges (1.4e-5 with the largest),
+ * 8.2e-9 of the electrostatic bound, and 1/7 of a pose's sum of the three. */
+#define GD_CERT 1e-6f
+#define GD_CERT_ELE 5e-8
+#define GD_CERT_FAR 2.5e-7
 /* resident 256-thread CTAs per SM the register budget is set for, per unroll depth: 80
  * registers at four point pairs in flight, 64 below (no spills); the delayed-acceptance
  * variants keep one CTA fewer (80 at two pairs, 128 at four), where 64 and 80 would spill */
@@ -150,6 +158,7 @@ struct GdDevComplex {
   const float *ff_tab;
   const short *ff_id;
   const double *ff_pmf;
+  const float *ff_cert;       /* [n_prt*n_lig] what the far points' sums may differ by, per pose */
   int ff_fields, ff_cells;
   float ff_r;                 /* r_f: a cell's far points are at least this far from its atoms */
   unsigned char ff_slot[GD_MAXTP2], ff_extra[GD_MAXTP1 + 2];
@@ -218,6 +227,19 @@ struct GdDaEpi {
   int tr_cap, tr_step0;
 };
 
+/* What the Monte Carlo kernel is compiled for: plain steps and evaluations, delayed acceptance's
+ * exact stage, the exchange groups left open (gd_exchange_group). */
+enum { GD_KIND_PLAIN = 0, GD_KIND_DA = 1, GD_KIND_EXCHANGE = 2 };
+
+/* The replica state that exchanges read and write, and their draws' seed. */
+struct GdExchange {
+  gd_replica *replica;
+  const float *etotal;
+  const gd_energy *e_old;
+  int *acs;                   /* exchanges taken, per replica */
+  uint64_t seed;
+};
+
 /* Arguments of the fused Monte Carlo / energy kernel. */
 struct GdMcArgs {
   const GdDevComplex *cx;     /* [n_complex] */
@@ -280,6 +302,11 @@ struct GdMcArgs {
   int *x_acs;                 /* [n_rep] */
   const int *x_call_base;
   int x_call_off, x_spd, x_spe;
+  /* exchange groups (global numbers) whose decisions wait for the pair loop's energies: x_open[0]
+   * of them in x_open_list, taken by the GD_KIND_EXCHANGE launch that follows (its CTAs check out
+   * in x_open[1]); it takes mode_t from x_mode_t, or (-1) from the step as above */
+  int *x_open, *x_open_list;
+  int x_mode_t, x_open_cap, n_complex;
 };
 
 #endif

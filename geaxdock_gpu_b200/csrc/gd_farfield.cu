@@ -24,7 +24,8 @@
  * CTA per (conformer, cell). The vdw term (p1 - p2) / (1 + x), p1 = p1a r^-9, p2 = p2a r^-6, x =
  * p1l z, z = r^-9 + lj1 r^-7, is expanded in x, so that a segment (one point type) needs the sums of
  * r^-9 z^k and r^-6 z^k only, k = 0..3, for every ligand type at once; the tables are made only
- * when x <= 1/16 at r_f for every type pair (2^-16 of such a pair's term is left out).
+ * when x <= 1/32 at r_f for every type pair: less than 2^-20, a tenth of GD_CERT, of such a pair's
+ * term is left out (the reference's force field: x = 0.019).
  * Complexes of one batch on the same protein share one set of tables.
  */
 #include <memory>
@@ -254,8 +255,37 @@ static bool ff_radii(const gd_enepara *ff, double *r_f, double *r_hdb) {
   const double r3 = 1.0 / (*r_f * *r_f * *r_f), z = r3 * r3 * (r3 + std::fabs(ff->lj1) / *r_f);
   for (int tl = 0; tl < GD_MAXTP2; ++tl)
     for (int tp = 0; tp < GD_MAXTP1; ++tp)
-      if (!(std::fabs((double)ff->p1a[tl][tp] * ff->lj0) * z <= 1.0 / 16.0)) return false;
+      if (!(std::fabs((double)ff->p1a[tl][tp] * ff->lj0) * z <= 1.0 / 32.0)) return false;
   return true;
+}
+
+/* Appends ff_cert of a complex (GD_CERT_ELE, GD_CERT_FAR), by protein and ligand conformer. */
+static void certainty(const gd_ctx *c, const gd_enepara *ff, const gd_complex_desc &d, double r_f,
+                      std::vector<float> &out) {
+  double wa[3];
+  for (int k = 0; k < 3; ++k) wa[k] = std::fabs((double)c->fc.w[k] * c->fc.a_para[k]);
+  const double r3 = 1.0 / (r_f * r_f * r_f), r6 = r3 * r3, r9 = r6 * r3;
+  for (int p = 0; p < d.n_prt; ++p) {
+    double count[GD_MAXTP1] = {0.0}, by_type[GD_MAXTP2], ele = 0.0;
+    for (int i = p * d.pnp; i < (p + 1) * d.pnp; ++i) {
+      count[d.prt_t[i]] += 1.0;
+      ele += std::fabs((double)d.prt_ele[i]);
+    }
+    for (int t = 0; t < GD_MAXTP2; ++t) {
+      by_type[t] = 0.0;
+      for (int tp = 0; tp < GD_MAXTP1; ++tp)
+        by_type[t] += count[tp] * (wa[0] * (std::fabs((double)ff->p1a[t][tp]) * r9 +
+                                            std::fabs((double)ff->p2a[t][tp]) * r6) +
+                                   wa[2] * std::fabs((double)ff->pmf1[t][tp]));
+    }
+    ele *= wa[1] / ((double)ff->el1 * r_f);
+    for (int l = 0; l < d.n_lig; ++l) {
+      double s = 0.0;
+      for (int i = l * d.lna; i < (l + 1) * d.lna; ++i)
+        s += GD_CERT_ELE * ele * std::fabs((double)d.lig_c[i]) + GD_CERT_FAR * by_type[d.lig_t[i]];
+      out.push_back((float)(s / d.lna));
+    }
+  }
 }
 
 /* Bytes the tables may take: a quarter of what the device has free once the context holds all it
@@ -359,18 +389,22 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
       }
     const int n_prt = c->info[a.rep].n_prt;
     const size_t per = (size_t)cells.size() * (1 + a.n_types) * GD_FF_NC;
+    std::vector<float> cert;
+    for (int ci : gp->members) certainty(c, ff, cxs[ci], r_f, cert);
     const size_t n_pmf = (size_t)n_prt * GD_FAR_BINS * GD_MAXTP2;
     const size_t bytes = sizeof(float) * per * n_prt + sizeof(double) * n_pmf +
-                         sizeof(int) * cells.size() + sizeof(short) * id.size();
+                         sizeof(int) * cells.size() + sizeof(short) * id.size() +
+                         sizeof(float) * cert.size();
     /* a protein whose tables do not fit runs without them */
     if (c->field_bytes + bytes > budget) continue;
     int *d_cells = nullptr;
     short *d_id = nullptr;
     double *p = nullptr;
-    const bool made = !upload(c, &d_cells, cells) && !upload(c, &d_id, id) &&
+    float *d_cert = nullptr;
+    const bool made = !upload(c, &d_cert, cert) && !upload(c, &d_cells, cells) && !upload(c, &d_id, id) &&
                       !dalloc(c, &a.tab, per * n_prt) && !dalloc(c, &p, n_pmf);
     CK(cudaStreamSynchronize(c->stream)); /* the host vectors end here */
-    for (void *q : {(void *)d_cells, (void *)d_id, (void *)a.tab, (void *)p}) {
+    for (void *q : {(void *)d_cells, (void *)d_id, (void *)a.tab, (void *)p, (void *)d_cert}) {
       if (!q) continue;
       if (made)
         c->field_allocs.push_back(q);
@@ -385,6 +419,8 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
       g.ff_id = d_id;
       g.ff_tab = a.tab;
       g.ff_pmf = p;
+      g.ff_cert = d_cert;
+      d_cert += (size_t)cxs[ci].n_prt * cxs[ci].n_lig;
       g.ff_fields = 1 + a.n_types;
       g.ff_cells = (int)cells.size();
       g.ff_r = (float)(r_f + 0.05);

@@ -522,7 +522,8 @@ __device__ __forceinline__ void far_field(const GdDevComplex &cx, int pc, int ce
 /* Per-replica state of the CTA's slots, in shared memory. */
 struct Slot {
   int rep, lig_conf, accept, n_acc;
-  int rec_next, pad0;
+  int rec_next;
+  float mag; /* e_old's terms (cert_mag) */
   float mb, u;
   float mm_old[6];
   float mm_new[6];
@@ -534,6 +535,7 @@ struct Slot {
    * by the pair loop over every point */
   gd_energy e_prop;
   float e_full;
+  float cert; /* ff_cert of both poses */
   int open;
 };
 static_assert(sizeof(Slot) == GD_SLOT_BYTES, "slot layout");
@@ -681,56 +683,120 @@ __device__ __forceinline__ void pair_dispatch(int flags, const float4 *PA, const
 #undef GD_PR
 }
 
+/* The magnitudes of an energy's weighted terms, which its far fields' rounding is a share of. */
+__device__ __forceinline__ float cert_mag(const gd_energy &e, const GdForceConst &f) {
+  float m = 0.0f;
+#pragma unroll
+  for (int i = 0; i < GD_MAXWEI - 1; ++i) m += fabsf(e.e[i] * f.w[i]);
+  return m;
+}
+
 /* ExchangeReplicas_d (src/kernel_cuda_l1_exchangereplicas.cu:27-77) for one (protein
  * conformer, ligand conformer) group lg of complex cx: temperature pairs (2 j + mode_t, its
  * successor), accepted by the Metropolis test on their energies with one Philox draw per pair
  * of this exchange call. The group's replica states are read with L2 loads (.cg): inside the
- * Monte Carlo kernel other SMs wrote them in this launch. */
-__device__ __forceinline__ void gd_exchange_group(const GdDevComplex &cx, int lg,
-                                                  gd_replica *replica, const float *etotal,
-                                                  int *acs, uint64_t seed, int call, int mode_t) {
-  if (mode_t >= 2) return;
+ * Monte Carlo kernel other SMs wrote them in this launch.
+ * Where energies come from far fields, a group with a pair whose decision could hang on their
+ * rounding is left as it is: the result is nonzero, and list gets the temperature indexes of such
+ * pairs' replicas, two a pair. With their energies by the pair loop in full[] (by temperature index)
+ * those pairs decide on them. */
+__device__ __forceinline__ unsigned gd_exchange_group(const GdDevComplex &cx, int lg,
+                                                      const GdExchange &x, const GdForceConst &f,
+                                                      int call, int mode_t,
+                                                      const float *full = nullptr,
+                                                      int *list = nullptr) {
+  if (mode_t >= 2) return 0;
   const int nl = cx.n_lig, nt = cx.n_tmp;
-  const int p = lg / nl, l = lg - p * nl;
+  const int p = lg / nl, l = lg - p * nl, r0 = cx.rep_offset + nt * nl * p + l;
+  const bool certify = cx.ff_tab != nullptr;
+  const float cert = certify ? cx.ff_cert[lg] : 0.0f; /* lg = p n_lig + l */
   int temps[GD_MAXTMP], orders[GD_MAXTMP];
-  float en[GD_MAXTMP];
+  float en[GD_MAXTMP], tol[GD_MAXTMP];
   for (int t = 0; t < nt; ++t) {
-    const int f = cx.rep_offset + nt * nl * p + nl * t + l;
-    temps[t] = __ldcg(&replica[f].idx_tmp);
-    en[t] = __ldcg(etotal + f);
+    const int r = r0 + nl * t;
+    temps[t] = __ldcg(&x.replica[r].idx_tmp);
+    en[t] = __ldcg(x.etotal + r);
     orders[temps[t]] = t;
+    if (certify) {
+      gd_energy e;
+#pragma unroll
+      for (int i = 0; i < GD_MAXWEI - 1; ++i) e.e[i] = __ldcg(&x.e_old[r].e[i]);
+      tol[t] = GD_CERT * cert_mag(e, f) + cert;
+    }
   }
   const int maxpair = nt / 2 - (nt % 2 == 0) * (mode_t == 1);
+  unsigned taken = 0, open = 0;
+  int n = 0;
   for (int pair = 0; pair < maxpair; ++pair) {
     const int i1 = (pair << 1) + mode_t, i2 = i1 + 1;
     const int o1 = orders[i1], o2 = orders[i2];
-    const int tt = temps[o1];
     const float mb1 = cx.minus_beta[temps[o1]], mb2 = cx.minus_beta[temps[o2]];
-    const float u = gd_draw_exchange(seed, (uint32_t)cx.stream, (uint32_t)lg, (uint32_t)call,
+    const float u = gd_draw_exchange(x.seed, (uint32_t)cx.stream, (uint32_t)lg, (uint32_t)call,
                                      (uint32_t)pair);
-    if (gd_exchange_accept(en[o1], en[o2], mb1, mb2, u)) {
+    int acc = gd_exchange_accept(en[o1], en[o2], mb1, mb2, u);
+    if (certify) {
+      const float d = tol[o1] + tol[o2];
+      if (gd_exchange_accept(en[o1], en[o2] + d, mb1, mb2, u) !=
+          gd_exchange_accept(en[o1], en[o2] - d, mb1, mb2, u)) {
+        if (full) {
+          acc = gd_exchange_accept(full[o1], full[o2], mb1, mb2, u);
+        } else {
+          open |= 1u << pair;
+          if (list) {
+            list[n++] = o1;
+            list[n++] = o2;
+          }
+        }
+      }
+    }
+    if (acc) {
+      const int tt = temps[o1];
       temps[o1] = temps[o2];
       temps[o2] = tt;
-      acs[cx.rep_offset + nt * nl * p + nl * o1 + l] += 1;
-      acs[cx.rep_offset + nt * nl * p + nl * o2 + l] += 1;
+      taken |= 1u << pair;
     }
   }
-  for (int t = 0; t < nt; ++t) replica[cx.rep_offset + nt * nl * p + nl * t + l].idx_tmp = temps[t];
+  if (open) return open;
+  /* (counts without a result: a load and a store each, one after the other, kept the thread up to
+   * 3 us) */
+  for (int pair = 0; pair < maxpair; ++pair)
+    if ((taken >> pair) & 1u) {
+      atomicAdd(x.acs + r0 + nl * orders[(pair << 1) + mode_t], 1);
+      atomicAdd(x.acs + r0 + nl * orders[(pair << 1) + mode_t + 1], 1);
+    }
+  for (int t = 0; t < nt; ++t) x.replica[r0 + nl * t].idx_tmp = temps[t];
+  return 0;
+}
+
+/* Lists a group for the launch that decides it. The list holds every group once; it is full only
+ * when such a launch did not take place. */
+__device__ __forceinline__ void open_group(int *open, int *list, int cap, int g, unsigned *err) {
+  const int i = atomicAdd(open, 1);
+  if (i < cap)
+    list[i] = g;
+  else
+    atomicOr(err, GD_DEV_ERR_TIMEOUT);
 }
 
 /* Delayed acceptance, second stage, for the survivor in pose slot `pos` (mode 3): the
- * corrected Metropolis test u2 < exp(mb ((E_new - E_old) - (S_new - S_cur))) (gd_da_stage2),
- * surrogate-error sums, the collect step's training target, the trace, and on acceptance the
- * state update and the record, as the plain epilogue does them. */
-__device__ __forceinline__ void da_decide(const GdMcArgs &a, const GdDevComplex &cx, int ci, int pos,
-                                       const gd_energy &en, const float *mm_new, int step) {
+ * corrected Metropolis test u2 < exp(mb ((E_new - E_old) - (S_new - S_cur))) (gd_da_stage2)
+ * on the energies ea and eb, surrogate-error sums, the collect step's training target, the trace,
+ * and on acceptance the state update and the record, as the plain epilogue does them. tol > 0:
+ * nothing is done, and the result is false, when the decision is not the same that much above and
+ * below ea. */
+__device__ __forceinline__ bool da_decide(const GdMcArgs &a, const GdDevComplex &cx, int ci, int pos,
+                                          const gd_energy &en, float ea, float eb, float tol,
+                                          const float *mm_new, int step) {
   const GdDaEpi &da = *a.da;
   const int r = da.pose_rep[pos];
   const gd_replica rp = a.replica[r];
   const float mb = cx.minus_beta[rp.idx_tmp];
   const float enew = en.e[GD_MAXWEI - 1];
-  const float sn = da.s_new[r], so = da.s_cur[r];
-  const int acc = gd_da_stage2(enew, a.e_old[r].e[GD_MAXWEI - 1], sn, so, mb, da.u2[r]);
+  const float sn = da.s_new[r], so = da.s_cur[r], u2 = da.u2[r];
+  const int acc = gd_da_stage2(ea, eb, sn, so, mb, u2);
+  if (tol > 0.0f && gd_da_stage2(ea + tol, eb, sn, so, mb, u2) !=
+                        gd_da_stage2(ea - tol, eb, sn, so, mb, u2))
+    return false;
   const bool active = !a.da_collect && da.active[ci];
   if (active) {
     const double e = (double)sn - (double)enew;
@@ -748,7 +814,7 @@ __device__ __forceinline__ void da_decide(const GdMcArgs &a, const GdDevComplex 
       da.tr_flag[o] = 1 + acc;
     }
   }
-  if (!acc) return;
+  if (!acc) return true;
   a.e_old[r] = en;
   a.etotal[r] = enew;
 #pragma unroll
@@ -770,6 +836,7 @@ __device__ __forceinline__ void da_decide(const GdMcArgs &a, const GdDevComplex 
       atomicOr(a.err, GD_DEV_ERR_RECORD_FULL);
     }
   }
+  return true;
 }
 
 /*
@@ -780,11 +847,12 @@ __device__ __forceinline__ void da_decide(const GdMcArgs &a, const GdDevComplex 
  * chunk two ahead. Every wait is bounded (globaltimer); a wait that runs out sets the error
  * word, the CTA leaves at the next step barrier after letting its copies in flight land.
  */
-template <int UNROLL, bool SPLIT, bool DA, int PACK>
+template <int UNROLL, bool SPLIT, int KIND, int PACK>
 __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
-                                  SPLIT ? 1 : GD_MIN_BLOCKS_PACK(UNROLL, PACK, DA))
+                                  SPLIT ? 1 : GD_MIN_BLOCKS_PACK(UNROLL, PACK, KIND != GD_KIND_PLAIN))
     gd_mc_kernel(GdMcArgs a, GdForceConst f) {
-  static_assert(PACK == 1 || (PACK == 2 && !SPLIT && !DA),
+  constexpr bool DA = KIND == GD_KIND_DA, XCH = KIND == GD_KIND_EXCHANGE;
+  static_assert(PACK == 1 || (PACK == 2 && !SPLIT && KIND == GD_KIND_PLAIN),
                 "two replicas per lane: plain modes with one lane per atom");
   extern __shared__ __align__(16) unsigned char smem[];
   /* T: lanes of the tile (PACK per thread), the stride of the placed atoms and partials */
@@ -828,18 +896,61 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
   if (DA && a.mode == 3 && blockIdx.x == 0)
     for (int g = a.da_g0 + tid; g < a.da_g1; g += NT) a.da_cnt_next[g] = 0;
 
+  /* the open exchange groups (XCH): this CTA's xg-th, whose replicas x_list[xb .. xn) (temperature
+   * indexes) are still to be evaluated, their energies going to x_e */
+  __shared__ int x_list[XCH ? GD_MAXTMP : 1], x_n;
+  __shared__ float x_e[XCH ? GD_MAXTMP : 1];
+  int xg = (int)blockIdx.x - (int)gridDim.x, xb = 0, xn = 0, x_ci = 0, x_lg = 0;
+  bool x_has = false;
+  const int x_count = XCH ? min(__ldcg(a.x_open), a.x_open_cap) : 0;
+  const int x_mode = !XCH ? 0
+                     : a.x_mode_t >= 0 ? a.x_mode_t
+                                       : !(((step_first % a.x_spd) / a.x_spe) % 2);
+
   for (;;) {
-    if (tid == 0) s_tile = atomicAdd(a.tile_counter, 1);
-    __syncthreads();
-    const int t = s_tile;
-    if (t >= a.n_tiles || s_abort) break;
+    int t = 0;
     GdTileDesc tile;
-    if (a.tiles) {
-      tile = a.tiles[t];
+    if constexpr (XCH) {
+      if (xb >= xn) {
+        const GdExchange ex = {a.replica, a.etotal, a.e_old, a.x_acs, a.seed};
+        const int call = (a.x_call_base ? *a.x_call_base : 0) + a.x_call_off;
+        /* every replica of the group is evaluated: its pairs decide */
+        if (tid == 0 && x_has) gd_exchange_group(a.cx[x_ci], x_lg, ex, f, call, x_mode, x_e);
+        x_has = false;
+        xg += (int)gridDim.x;
+        if (xg >= x_count || s_abort) break;
+        const int g = a.x_open_list[xg];
+        int hi = a.n_complex - 1;
+        x_ci = 0;
+        while (x_ci < hi) {
+          const int mid = (x_ci + hi + 1) >> 1;
+          if (a.x_group_base[mid] <= g) x_ci = mid; else hi = mid - 1;
+        }
+        x_lg = g - a.x_group_base[x_ci];
+        if (tid == 0)
+          x_n = 2 * __popc(gd_exchange_group(a.cx[x_ci], x_lg, ex, f, call, x_mode, nullptr,
+                                             x_list));
+        __syncthreads();
+        x_has = x_n > 0;
+        xn = x_n;
+        xb = 0;
+        __syncthreads(); /* x_n is read before the next group's is written */
+        if (!x_has) continue;
+      }
+      t = xg;
+      tile = {x_ci, x_lg / a.cx[x_ci].n_lig, 0, min(min(a.u.count, T / a.cx[x_ci].lna), xn - xb)};
     } else {
-      tile = a.u;
-      tile.rep_begin = t * a.u.count;
-      tile.count = min(a.u.count, a.u_n - tile.rep_begin);
+      if (tid == 0) s_tile = atomicAdd(a.tile_counter, 1);
+      __syncthreads();
+      t = s_tile;
+      if (t >= a.n_tiles || s_abort) break;
+      if (a.tiles) {
+        tile = a.tiles[t];
+      } else {
+        tile = a.u;
+        tile.rep_begin = t * a.u.count;
+        tile.count = min(a.u.count, a.u_n - tile.rep_begin);
+      }
     }
     int k = tile.count;
     if (DA && a.mode == 3) {
@@ -861,6 +972,30 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     const int A = SPLIT ? NT / S : T;
     const int kp = (k + PACK - 1) / PACK; /* lane groups */
     const int sp = SPLIT ? tid / A : 0;
+    /* Unsplit lanes of a tile whose replicas are all at the pocket run over the atoms' ranks by
+     * distance from the ligand's centre, the tile's slots within a rank: a warp's atoms lie about
+     * as far out, so that its inner warps end their segments early (a warp runs to the largest near
+     * radius among its atoms): 6,820 replicas of 40 atoms on 3,000 points, 11 steps from the
+     * pocket, 7.24 -> 6.79 ms; of 60 atoms on 1,500 points, 20 steps, 15.8 -> 15.3 ms. One replica
+     * further away (GD_ROAM) would make every warp of the CTA run about as far as its atoms need:
+     * then each slot's atoms lie together, in the chain's order, whose neighbours share list
+     * entries. The 6,820 replicas after 1,000 steps, by rank / by slot / as chosen, ms per 10
+     * steps: moves of 0.1 A 6.60 / 6.76 / 6.56, of 2 A 9.33 / 8.36 / 8.38, of 6 A 10.66 / 9.97 /
+     * 9.93 (six replicas a CTA and four pairs in flight 9.86 / 9.24 / 9.22); lines at 8 and 11 A
+     * and at the ligand's radius are up to 3 % slower at 2 A. Delayed acceptance's tiles, of one
+     * step each, keep to the ranks (by slot 28.9 -> 30.2 ms for 50 steps at 0.1 A). The warps' place in the CTA goes
+     * round with the tile, so that the tiles an SM holds (about GD_NUM_SMS apart) load its four
+     * schedulers alike. Split lanes keep the slots' order (2 % faster there). */
+    const int wr = SPLIT ? warp - sp * (A >> 5) : (warp + t + t / GD_NUM_SMS) % nwarps;
+    const int ai = wr * 32 + lane;
+    const bool active = ai < kp * L;
+    int jj = 0, rank = 0;
+    auto take_lane = [&](bool by_slot) {
+      const int n = by_slot ? L : kp, hi = active ? ai / n : 0, lo = active ? ai - hi * n : 0;
+      jj = by_slot ? hi : lo;
+      rank = by_slot ? lo : hi;
+    };
+    take_lane(SPLIT);
     /* the splits that run the short-range lists and the restraints (split 0: the far field, the
      * per-atom tail) */
     const int con_sp = S - 1, kind_sp = max(S - 2, 0), mcs_sp = S >= 4 ? S - 3 : S == 2 ? 1 : 0;
@@ -868,18 +1003,27 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     bool roams = false;
     if (tid < k) {
       Slot &s = slots[tid];
-      const int id = tile.rep_begin + tid;
+      const int id = XCH ? cx.rep_offset + cx.n_lig * (cx.n_tmp * tile.prt_conf + x_list[xb + tid]) +
+                               x_lg % cx.n_lig
+                         : tile.rep_begin + tid;
       s.rep = id;
       s.accept = 0;
       s.open = 0;
-      if (a.mode >= 2) {
+      s.cert = 0.0f;
+      if (XCH) {
+        s.lig_conf = a.replica[id].idx_lig;
+      } else if (a.mode >= 2) {
         s.lig_conf = a.tiles ? a.lig_conf_in[id] : a.u.rep_begin;
+        if (DA)
+#pragma unroll
+          for (int i = 0; i < 6; ++i) s.mm_old[i] = 0.0f; /* a slot left open: its replica's pose */
       } else {
         s.replica = a.replica[id];
         s.lig_conf = s.replica.idx_lig;
         s.mb = cx.minus_beta[s.replica.idx_tmp];
         if (a.mode == 0) {
           s.e_old = a.e_old[id];
+          s.mag = cert_mag(s.e_old, f);
           s.n_acc = a.n_accept[id];
           s.rec_next = a.rec ? a.rec_next[id] : 0;
 #pragma unroll
@@ -891,7 +1035,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
           for (int i = 0; i < 6; ++i) s.mm_old[i] = 0.0f;
         }
       }
-      if constexpr (!SPLIT) roams = slot_roams(a, cx, s, id);
+      if (cx.ff_tab) s.cert = 2.0f * cx.ff_cert[tile.prt_conf * cx.n_lig + s.lig_conf];
+      if constexpr (!SPLIT && KIND == GD_KIND_PLAIN) roams = slot_roams(a, cx, s, id);
     }
 
     /* ---- protein tile pipeline ---- */
@@ -902,43 +1047,27 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     const int nch = (pnp_pad + D - 1) / D;
     const bool resident = nch <= 2;
     const int nsteps = a.mode == 0 ? a.n_steps : 1;
-    const int total_q = resident ? nch : nsteps * nch;
+    int total_q = resident ? nch : nsteps * nch;
+    /* chunk q of the passes into its buffer (one thread) */
+    auto issue = [&](int q) {
+      const int b = q & 1, c0 = (q % nch) * D, n = min(D, pnp_pad - c0);
+      s_issued[b] += 1;
+      mbar_expect_tx(&bar[b], (uint32_t)(n * 16));
+      bulk_g2s(bpa + b * (D >> 1), ga + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
+      bulk_g2s(bpb + b * (D >> 1), gb + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
+    };
     if (tid == 0) {
       s_done[0] = s_done[1] = 0;
-      for (int q = 0; q < min(2, total_q); ++q) {
-        const int b = q & 1, c0 = q * D, n = min(D, pnp_pad - c0);
-        s_issued[b] += 1;
-        mbar_expect_tx(&bar[b], (uint32_t)(n * 16));
-        bulk_g2s(bpa + b * (D >> 1), ga + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
-        bulk_g2s(bpb + b * (D >> 1), gb + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
-      }
+      for (int q = 0; q < min(2, total_q); ++q) issue(q);
     }
-    if constexpr (SPLIT)
-      __syncthreads();
-    else
+    if constexpr (!SPLIT && KIND == GD_KIND_PLAIN)
       roams = __syncthreads_or(roams);
+    else
+      __syncthreads();
 
     /* ---- per-lane constants ---- */
-    /* Unsplit lanes of a tile whose replicas are all at the pocket run over the atoms' ranks by
-     * distance from the ligand's centre, the tile's slots within a rank: a warp's atoms lie about
-     * as far out, so that its inner warps end their segments early (a warp runs to the largest near
-     * radius among its atoms): 6,820 replicas of 40 atoms on 3,000 points, 11 steps from the
-     * pocket, 7.24 -> 6.79 ms; of 60 atoms on 1,500 points, 20 steps, 15.8 -> 15.3 ms. One replica
-     * further away (GD_ROAM) would make every warp of the CTA run about as far as its atoms need:
-     * then each slot's atoms lie together, in the chain's order, whose neighbours share list
-     * entries. The 6,820 replicas after 1,000 steps, by rank / by slot / as chosen, ms per 10
-     * steps: moves of 0.1 A 6.60 / 6.76 / 6.56, of 2 A 9.33 / 8.36 / 8.38, of 6 A 10.66 / 9.97 /
-     * 9.93 (six replicas a CTA and four pairs in flight 9.86 / 9.24 / 9.22); lines at 8 and 11 A
-     * and at the ligand's radius are up to 3 % slower at 2 A. The warps' place in the CTA goes
-     * round with the tile, so that the tiles an SM holds (about GD_NUM_SMS apart) load its four
-     * schedulers alike. Split lanes keep the slots' order (2 % faster there). */
+    if (roams) take_lane(true);
     const bool by_slot = SPLIT || roams;
-    const int wr = SPLIT ? warp - sp * (A >> 5) : (warp + t + t / GD_NUM_SMS) % nwarps;
-    const int ai = wr * 32 + lane;
-    const bool active = ai < kp * L;
-    const int hi = active ? ai / (by_slot ? L : kp) : 0,
-              lo = active ? ai - hi * (by_slot ? L : kp) : 0;
-    const int jj = by_slot ? hi : lo, rank = by_slot ? lo : hi;
     /* the thread's lanes: slot jj (PACK 1), or slots 2 jj and 2 jj + 1, the same atom of two
      * replicas (PACK 2); a missing second slot (odd k) repeats the first one's atom and stores
      * nothing. sl_of: each lane's slot; vl: its index in the placed-atom and partial arrays */
@@ -973,10 +1102,15 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
 
     /* A step may take three passes. Energies from the far fields differ from those of the pair
      * loop over every point in the last FP32 digits; a Metropolis decision that could hang on
-     * that (about one in 10^4, GD_CERT) is left open in the first pass (phase 0), the CTA then
-     * evaluates the proposal (phase 1) and the current pose (phase 2) without the fields, and the
-     * slots left open decide on those: every decision is the one the plain loop takes. */
-    const bool certify = a.mode == 0 && cx.ff_tab != nullptr;
+     * that (about one in 10^4, GD_CERT), of a plain step or of delayed acceptance's second stage, is
+     * left open in the first pass (phase 0), the CTA then evaluates the proposal (phase 1) and the
+     * current pose (phase 2) without the fields, and the slots left open decide on those: every
+     * decision is the one the plain loop takes. Exchanges: gd_exchange_group. */
+    const bool certify = (a.mode == 0 || (DA && a.mode == 3)) && cx.ff_tab != nullptr;
+    /* a step's ring runs on into the next pass; delayed acceptance's single step issues the chunks
+     * of another pass when there is one (a third more copies otherwise: 29 -> 31 ms for 50 steps of
+     * 6,820 replicas on 3,000 points) */
+    const bool run_on = !DA && certify;
     int phase = 0, q_run = 0;
     for (int s = 0; s < nsteps;) {
       /* ---- Move_d: four lanes per replica draw the move (a Box-Muller pair each) and build the
@@ -1093,7 +1227,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
           }
         }
         const int fcell =
-            cx.ff_tab != nullptr && phase == 0 ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
+            !XCH && cx.ff_tab != nullptr && phase == 0 ? gd_ff_cell(cx, ax[h], ay[h], az[h]) : -1;
         if (fcell >= 0) {
           const int id = __ldg(cx.ff_id + fcell);
           const int bin = gd_ff_bin(cx, fcell);
@@ -1227,13 +1361,9 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
             const int prev = atomicAdd(&s_done[b], 1);
             if (prev == nwarps - 1) {
               s_done[b] = 0;
-              if (certify || q + 2 < total_q) {
-                const int c0 = ((q + 2) % nch) * D, n = min(D, pnp_pad - c0);
+              if (run_on || q + 2 < total_q) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-                s_issued[b] += 1;
-                mbar_expect_tx(&bar[b], (uint32_t)(n * 16));
-                bulk_g2s(bpa + b * (D >> 1), ga + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
-                bulk_g2s(bpb + b * (D >> 1), gb + (c0 >> 1), (uint32_t)(n * 8), &bar[b]);
+                issue(q + 2);
               }
             }
           }
@@ -1358,19 +1488,41 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         en.rmsd = __shfl_sync(0xffffffffu, side, 10);
         if (lane == 0) {
           const int rid = sl.rep;
-          if (a.mode == 2 || a.mode == 4) {
+          const float etn = en.e[GD_MAXWEI - 1];
+          if (XCH) {
+            x_e[x_list[xb + js]] = etn;
+          } else if (a.mode == 2 || a.mode == 4) {
             a.e_out[rid] = en;
           } else if (DA && a.mode == 3) {
-            da_decide(a, cx, tile.complex_index, rid, en, sl.mm_new, step_first + s);
+            const int ci = tile.complex_index, step = step_first + s;
+            if (phase == 0) {
+              const int r = a.da->pose_rep[rid];
+              const gd_energy &eo = a.e_old[r];
+              const float tol = certify ? GD_CERT * (mag + cert_mag(eo, f)) + sl.cert : 0.0f;
+              if (!da_decide(a, cx, ci, rid, en, etn, eo.e[GD_MAXWEI - 1], tol, sl.mm_new, step)) {
+#pragma unroll
+                for (int i = 0; i < 6; ++i) sl.mm_old[i] = a.mm_old[(size_t)r * 6 + i];
+                sl.e_prop = en;
+                sl.open = 1;
+                s_open = 1;
+              }
+            } else if (sl.open) {
+              if (phase == 1) {
+                sl.e_full = etn;
+              } else {
+                sl.open = 0;
+                da_decide(a, cx, ci, rid, sl.e_prop, sl.e_full, etn, 0.0f, sl.mm_new, step);
+              }
+            }
           } else {
             int acc = 1;
             bool decide = phase == 0;
             if (a.mode == 0) {
-              const float etn = en.e[GD_MAXWEI - 1], eto = sl.e_old.e[GD_MAXWEI - 1];
+              const float eto = sl.e_old.e[GD_MAXWEI - 1];
               if (phase == 0) {
                 acc = gd_metropolis(etn, eto, sl.mb, sl.u);
                 if (certify) {
-                  const float tol = GD_CERT * mag;
+                  const float tol = GD_CERT * (mag + sl.mag) + sl.cert;
                   if (gd_metropolis(etn + tol, eto, sl.mb, sl.u) !=
                       gd_metropolis(etn - tol, eto, sl.mb, sl.u)) {
                     sl.e_prop = en;
@@ -1385,40 +1537,42 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
                 } else {
                   acc = gd_metropolis(sl.e_full, etn, sl.mb, sl.u);
                   en = sl.e_prop;
+                  mag = cert_mag(en, f);
                   sl.open = 0;
                   decide = true;
                 }
               }
             }
             if (decide) {
-            sl.accept = acc;
-            if (acc) {
-              sl.e_old = en;
+              sl.accept = acc;
+              if (acc) {
+                sl.e_old = en;
+                sl.mag = mag;
 #pragma unroll
-              for (int i = 0; i < 6; ++i) sl.mm_old[i] = sl.mm_new[i];
-              if (a.mode == 0) sl.n_acc += 1;
-              if (a.rec) {
-                const int kslot = sl.rec_next;
-                if (kslot < a.rec_cap) {
-                  gd_record_step *r = a.rec + (size_t)rid * a.rec_cap + kslot;
-                  r->replica = sl.replica;
-                  r->energy = en;
+                for (int i = 0; i < 6; ++i) sl.mm_old[i] = sl.mm_new[i];
+                if (a.mode == 0) sl.n_acc += 1;
+                if (a.rec) {
+                  const int kslot = sl.rec_next;
+                  if (kslot < a.rec_cap) {
+                    gd_record_step *r = a.rec + (size_t)rid * a.rec_cap + kslot;
+                    r->replica = sl.replica;
+                    r->energy = en;
 #pragma unroll
-                  for (int i = 0; i < 6; ++i) r->movematrix[i] = sl.mm_new[i];
-                  r->step = a.mode == 0 ? step_first + s : 0;
-                  sl.rec_next = kslot + 1;
-                } else {
-                  atomicOr(a.err, GD_DEV_ERR_RECORD_FULL);
+                    for (int i = 0; i < 6; ++i) r->movematrix[i] = sl.mm_new[i];
+                    r->step = a.mode == 0 ? step_first + s : 0;
+                    sl.rec_next = kslot + 1;
+                  } else {
+                    atomicOr(a.err, GD_DEV_ERR_RECORD_FULL);
+                  }
                 }
               }
-            }
-            if (a.trace_e && a.mode == 0) {
-              const int ti = step_first + s - a.trace_step0;
-              if (ti >= 0 && ti < a.trace_cap) {
-                a.trace_e[(size_t)rid * a.trace_cap + ti] = en.e[GD_MAXWEI - 1];
-                a.trace_acc[(size_t)rid * a.trace_cap + ti] = acc;
+              if (a.trace_e && a.mode == 0) {
+                const int ti = step_first + s - a.trace_step0;
+                if (ti >= 0 && ti < a.trace_cap) {
+                  a.trace_e[(size_t)rid * a.trace_cap + ti] = en.e[GD_MAXWEI - 1];
+                  a.trace_acc[(size_t)rid * a.trace_cap + ti] = acc;
+                }
               }
-            }
             }
           }
         }
@@ -1429,13 +1583,21 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         ++s;
       } else if (phase < 2) {
         ++phase;
+        if (DA && !resident) {
+          total_q = q_run + nch;
+          if (tid == 0) {
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            issue(q_run);
+            issue(q_run + 1);
+          }
+        }
       } else {
         phase = 0;
         ++s;
         if (tid == 0) s_open = 0; /* read again only after the next step's barriers */
       }
     }
-    if (certify && !resident && !aborted) {
+    if (run_on && !resident && !aborted) {
       /* the ring was refilled for a pass that did not come: let its two chunks land */
       for (int i = 0; i < 2; ++i) {
         const int b = (q_run + i) & 1;
@@ -1480,33 +1642,43 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         if (atomicAdd(a.x_done + a.x_group_base[tile.complex_index] + lg, 1) == nt - 1) {
           __threadfence();
           const int mode_t = !(((step_first % a.x_spd) / a.x_spe) % 2);
-          gd_exchange_group(cx, lg, a.replica, a.etotal, a.x_acs, a.seed,
-                            (a.x_call_base ? *a.x_call_base : 0) + a.x_call_off, mode_t);
+          const GdExchange ex = {a.replica, a.etotal, a.e_old, a.x_acs, a.seed};
+          if (gd_exchange_group(cx, lg, ex, f, (a.x_call_base ? *a.x_call_base : 0) + a.x_call_off,
+                                mode_t))
+            open_group(a.x_open, a.x_open_list, a.x_open_cap,
+                       a.x_group_base[tile.complex_index] + lg, a.err);
         }
       }
     }
+    if (XCH) xb += k;
     __syncthreads();
+  }
+  if (XCH && tid == 0) {
+    /* every CTA has read the count: the last one clears it for the next exchange */
+    __threadfence();
+    if (atomicAdd(a.x_open + 1, 1) == (int)gridDim.x - 1) a.x_open[0] = a.x_open[1] = 0;
   }
 }
 
-/* the kernel variants the host can launch: point pairs in flight per lane; protein split
- * and the delayed-acceptance exact stage (mode 3) compiled out when false; replicas per
+/* the kernel variants the host can launch: point pairs in flight per lane; protein split; plain
+ * modes, the delayed-acceptance exact stage (mode 3) or the open exchange groups; replicas per
  * thread (two only for the plain modes without split) */
-#define GD_INST(U, S, D, P) \
-  template __global__ void gd_mc_kernel<U, S, D, P>(GdMcArgs, GdForceConst);
-GD_INST(1, false, false, 1) GD_INST(2, false, false, 1) GD_INST(4, false, false, 1)
-GD_INST(1, true, false, 1) GD_INST(2, true, false, 1) GD_INST(4, true, false, 1)
-GD_INST(1, false, true, 1) GD_INST(2, false, true, 1) GD_INST(4, false, true, 1)
-GD_INST(1, true, true, 1) GD_INST(2, true, true, 1) GD_INST(4, true, true, 1)
-GD_INST(1, false, false, 2) GD_INST(2, false, false, 2)
+#define GD_INST(U, S, K, P) \
+  template __global__ void gd_mc_kernel<U, S, K, P>(GdMcArgs, GdForceConst);
+GD_INST(1, false, 0, 1) GD_INST(2, false, 0, 1) GD_INST(4, false, 0, 1)
+GD_INST(1, true, 0, 1) GD_INST(2, true, 0, 1) GD_INST(4, true, 0, 1)
+GD_INST(1, false, 1, 1) GD_INST(2, false, 1, 1) GD_INST(4, false, 1, 1)
+GD_INST(1, true, 1, 1) GD_INST(2, true, 1, 1) GD_INST(4, true, 1, 1)
+GD_INST(1, false, 0, 2) GD_INST(2, false, 0, 2)
+GD_INST(2, false, 2, 1)
 #undef GD_INST
 
 /* ExchangeReplicas_d, one thread per (complex, protein conformer, ligand conformer) group of
  * the range [g_begin, g_end). */
 __global__ void gd_exchange_kernel(const GdDevComplex *cxs, const int *group_base, int n_complex,
-                                   int g_begin, int g_end, gd_replica *replica,
-                                   const float *etotal, int *acs, uint64_t seed,
-                                   const int *call_base, int call_off, int mode_t) {
+                                   int g_begin, int g_end, GdExchange ex, GdForceConst f,
+                                   const int *call_base, int call_off, int mode_t, int *open,
+                                   int *open_list, unsigned *err) {
   const int g = g_begin + blockIdx.x * blockDim.x + threadIdx.x;
   if (g >= g_end || mode_t >= 2) return;
   int lo = 0, hi = n_complex - 1;
@@ -1514,8 +1686,9 @@ __global__ void gd_exchange_kernel(const GdDevComplex *cxs, const int *group_bas
     const int mid = (lo + hi + 1) >> 1;
     if (group_base[mid] <= g) lo = mid; else hi = mid - 1;
   }
-  gd_exchange_group(cxs[lo], g - group_base[lo], replica, etotal, acs, seed,
-                    (call_base ? *call_base : 0) + call_off, mode_t);
+  if (gd_exchange_group(cxs[lo], g - group_base[lo], ex, f,
+                        (call_base ? *call_base : 0) + call_off, mode_t))
+    open_group(open, open_list, g_end - g_begin, g, err);
 }
 
 /* ResetCounter_d (src/kernel_cuda_l1_resetcounter.cu:12-22). */
