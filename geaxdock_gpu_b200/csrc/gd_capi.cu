@@ -287,12 +287,14 @@ void build_tiles(const gd_ctx *c, int r0, int r1, std::vector<GdTileDesc> &out) 
 }
 
 size_t smem_bytes(const LaunchShape &s) {
-  return 16 + GD_THR_BYTES + (size_t)2 * s.chunk * 16 + (size_t)s.lanes * 16 +
-         (size_t)10 * s.lanes * 8 + (size_t)s.kmax * GD_SLOT_BYTES;
+  const size_t T = s.pieces ? s.lanes / s.split : s.lanes;
+  return 16 + GD_THR_BYTES + (size_t)2 * s.chunk * 16 + T * 16 +
+         (10 + 3 * (size_t)s.pieces + s.hpieces) * T * 8 + (size_t)s.kmax * GD_SLOT_BYTES;
 }
 
 LaunchShape ctx_shape(const gd_ctx *c) {
-  LaunchShape s = {c->threads, c->chunk, c->fold, c->split, c->unroll, c->pack, 1};
+  LaunchShape s = {c->threads, c->chunk, c->fold, c->split, c->unroll, c->pack, 1, c->pieces,
+                   c->hpieces};
   for (const auto &x : c->info) s.kmax = std::max(s.kmax, x.k);
   return s;
 }
@@ -335,12 +337,22 @@ int auto_split(const gd_ctx *c, const std::vector<WorkList> &w, std::vector<int>
   return S;
 }
 
-LaunchShape split_shape(int split, int k_lna, int kmax, int pnp_pad) {
+bool split_shape(const gd_ctx *c, int ci, int split, int k_lna, int kmax, int pnp_pad,
+                 LaunchShape *s) {
   /* two buffers hold the protein; the sums fold where the default tile's do, so that the shape
    * does not change the energies */
   const int half = (pnp_pad + 1) / 2;
-  const int chunk = std::min(4096, std::max(1, (half + GD_CHUNK - 1) / GD_CHUNK) * GD_CHUNK);
-  return {split * ((k_lna + 31) / 32) * 32, chunk, GD_CHUNK, split, 4, 1, kmax};
+  const int chunk = std::max(1, (half + GD_CHUNK - 1) / GD_CHUNK) * GD_CHUNK;
+  *s = {split * ((k_lna + 31) / 32) * 32, chunk, GD_CHUNK, split, 4, 1, kmax, 1, 0};
+  for (int i = ci < 0 ? 0 : ci; i < (ci < 0 ? c->n_complex : ci + 1); ++i) {
+    s->pieces = std::max(s->pieces, c->info[i].pieces[split]);
+    s->hpieces = std::max(s->hpieces, c->info[i].hpieces[split]);
+  }
+  /* a block's opt-in limit less the kernel's static arrays */
+  if (smem_bytes(*s) <= (size_t)225 << 10) return true;
+  s->pieces = s->hpieces = 0;
+  s->chunk = std::min(4096, chunk);
+  return false;
 }
 
 void make_auto_tile(gd_ctx *c) {
@@ -355,13 +367,20 @@ void make_auto_tile(gd_ctx *c) {
     work.push_back({x.n_prt, x.n_tmp * x.n_lig, x.lna});
     pad = std::max(pad, x.pnp_pad);
   }
-  const int S = auto_split(c, work, &k);
-  if (S > 1) c->auto_k = k;
+  for (int kk : c->auto_k) s.kmax = std::max(s.kmax, kk);
+  int S = auto_split(c, work, &k);
+  if (S <= 1) return;
+  int kmax = 1;
   for (int ci = 0; ci < c->n_complex; ++ci) {
-    k_lna = std::max(k_lna, c->auto_k[ci] * c->info[ci].lna);
-    s.kmax = std::max(s.kmax, c->auto_k[ci]);
+    k_lna = std::max(k_lna, k[ci] * c->info[ci].lna);
+    kmax = std::max(kmax, k[ci]);
   }
-  if (S > 1) s = split_shape(S, k_lna, s.kmax, pad);
+  /* fewer splits store fewer pieces; only with room for them are the energies the unsplit ones' */
+  LaunchShape q;
+  while (S > 1 && !split_shape(c, -1, S, k_lna, kmax, pad, &q)) --S;
+  if (S <= 1) return;
+  s = q;
+  c->auto_k = k;
 }
 
 void use_auto_tile(gd_ctx *c) {
@@ -371,6 +390,8 @@ void use_auto_tile(gd_ctx *c) {
   c->chunk = s.chunk;
   c->fold = s.fold;
   c->split = s.split;
+  c->pieces = s.pieces;
+  c->hpieces = s.hpieces;
   c->unroll = s.unroll;
   c->pack = 1;
   c->fill_threads = c->fill_cap = 0;
@@ -419,32 +440,34 @@ int ensure_cursor(gd_ctx *c) {
 }
 
 
-/* the kernel variant for an unroll depth, a protein split and the mode-3 epilogue */
-template <bool S, int K>
+/* the kernel variant of a launch's shape */
+template <int S, int K>
 McKernel mc_variant(int unroll) {
   if (unroll >= 4) return gd::gd_mc_kernel<4, S, K, 1>;
   if (unroll >= 2) return gd::gd_mc_kernel<2, S, K, 1>;
   return gd::gd_mc_kernel<1, S, K, 1>;
 }
 
-McKernel mc_kernel(int unroll, int split, int kind, int pack) {
-  if (kind == GD_KIND_EXCHANGE) return gd::gd_mc_kernel<2, false, GD_KIND_EXCHANGE, 1>;
-  if (kind == GD_KIND_DA)
-    return split > 1 ? mc_variant<true, GD_KIND_DA>(unroll) : mc_variant<false, GD_KIND_DA>(unroll);
-  if (pack == 2 && split <= 1)
-    return unroll >= 2 ? gd::gd_mc_kernel<2, false, GD_KIND_PLAIN, 2>
-                       : gd::gd_mc_kernel<1, false, GD_KIND_PLAIN, 2>;
-  return split > 1 ? mc_variant<true, GD_KIND_PLAIN>(unroll)
-                   : mc_variant<false, GD_KIND_PLAIN>(unroll);
+template <int K>
+McKernel mc_kernel(const LaunchShape &s) {
+  if (s.split > 1)
+    return s.pieces ? gd::gd_mc_kernel<4, GD_SPLIT_ORDERED, K, 1>
+                    : mc_variant<GD_SPLIT_PARTIAL, K>(s.unroll);
+  return mc_variant<GD_UNSPLIT, K>(s.unroll);
+}
+
+McKernel launch_kernel(const LaunchShape &s, int kind) {
+  if (kind == GD_KIND_EXCHANGE) return gd::gd_mc_kernel<2, GD_UNSPLIT, GD_KIND_EXCHANGE, 1>;
+  if (kind == GD_KIND_DA) return mc_kernel<GD_KIND_DA>(s);
+  if (s.pack == 2 && s.split <= 1)
+    return s.unroll >= 2 ? gd::gd_mc_kernel<2, GD_UNSPLIT, GD_KIND_PLAIN, 2>
+                         : gd::gd_mc_kernel<1, GD_UNSPLIT, GD_KIND_PLAIN, 2>;
+  return mc_kernel<GD_KIND_PLAIN>(s);
 }
 
 /* threads per CTA of a launch: the tile's lanes over the replicas per thread (two only for the
  * plain modes without split) */
 int launch_threads(const LaunchShape &s) { return s.lanes / s.pack; }
-
-McKernel launch_kernel(const LaunchShape &s, int kind) {
-  return mc_kernel(s.unroll, s.split, kind, s.pack);
-}
 
 GdMcArgs base_args(gd_ctx *c) {
   GdMcArgs a;
@@ -454,6 +477,8 @@ GdMcArgs base_args(gd_ctx *c) {
   a.chunk = c->chunk;
   a.fold = c->fold;
   a.split = c->split;
+  a.pieces = c->pieces;
+  a.hpieces = c->hpieces;
   a.move_kind = c->mc.move_kind;
   a.seed = c->mc.seed;
   for (int i = 0; i < 6; ++i) a.move_scale[i] = c->mc.move_scale[i];
@@ -598,6 +623,7 @@ int launch_exchange(gd_ctx *c, const Chain &ch, int k, const LaunchShape &s, boo
   a.chunk = x.chunk;
   a.fold = x.fold;
   a.split = 1;
+  a.pieces = a.hpieces = 0;
   a.mm_in = c->d_mm;
   a.u.count = x.kmax;
   a.rec = nullptr;
@@ -623,6 +649,8 @@ int launch_mc(gd_ctx *c, GdMcArgs a, const GdTileDesc *d_tiles, int n_tiles, int
   a.chunk = s.chunk;
   a.fold = s.fold;
   a.split = s.split;
+  a.pieces = s.pieces;
+  a.hpieces = s.hpieces;
   a.tiles = d_tiles;
   a.n_tiles = n_tiles;
   a.tile_counter = counter;

@@ -190,14 +190,17 @@ LaunchShape da_shape(const gd_ctx *c, int S) {
   if (S <= 1) {
     s.lanes = (k_lna + 31) / 32 * 32;
     s.split = 1;
+    s.pieces = s.hpieces = 0;
     s.unroll = std::min(s.unroll, 2);
     if (c->tile_auto) s.chunk = s.fold = GD_CHUNK;
     return s;
   }
-  const LaunchShape q = split_shape(S, k_lna, s.kmax, pad);
+  LaunchShape q;
+  split_shape(c, -1, S, k_lna, s.kmax, pad, &q);
   if (c->tile_auto) return q;
   s.lanes = q.lanes;
   s.split = S;
+  s.pieces = s.hpieces = 0;
   return s;
 }
 
@@ -367,6 +370,8 @@ void da_launch_exact(gd_ctx *c, const Chain &ch, int k, int n_steps, int j, bool
   a.split = shape.split;
   a.chunk = shape.chunk;
   a.fold = shape.fold;
+  a.pieces = shape.pieces;
+  a.hpieces = shape.hpieces;
   launch_kernel(shape, GD_KIND_DA)<<<grid_for(c, t1 - t0, shape, GD_KIND_DA), launch_threads(shape),
                                smem_bytes(shape), st>>>(a, c->fc);
 }

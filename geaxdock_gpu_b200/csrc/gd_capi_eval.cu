@@ -17,10 +17,10 @@ LaunchShape eval_shape(const gd_ctx *c, int ci, int n, int *k) {
     return ctx_shape(c);
   }
   std::vector<int> ks;
-  const int S = auto_split(c, {{1, n, x.lna}}, &ks);
-  if (S > 1) {
+  LaunchShape s;
+  for (int S = auto_split(c, {{1, n, x.lna}}, &ks); S > 1; --S) {
     *k = ks[0];
-    return split_shape(S, *k * x.lna, *k, x.pnp_pad);
+    if (split_shape(c, ci, S, *k * x.lna, *k, x.pnp_pad, &s)) return s;
   }
   /* one lane per atom: a CTA of 128..256 lanes with the least left over */
   int best = 256;

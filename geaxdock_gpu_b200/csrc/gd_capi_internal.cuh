@@ -42,16 +42,17 @@
 #include "gd_numerics.h"
 
 namespace gd {
-template <int UNROLL, bool SPLIT, int KIND, int PACK>
+template <int UNROLL, int SPLITS, int KIND, int PACK>
 __global__ void gd_mc_kernel(GdMcArgs a, GdForceConst f);
 #define GD_EXT(U, S, K, P) \
   extern template __global__ void gd_mc_kernel<U, S, K, P>(GdMcArgs, GdForceConst);
-GD_EXT(1, false, 0, 1) GD_EXT(2, false, 0, 1) GD_EXT(4, false, 0, 1)
-GD_EXT(1, true, 0, 1) GD_EXT(2, true, 0, 1) GD_EXT(4, true, 0, 1)
-GD_EXT(1, false, 1, 1) GD_EXT(2, false, 1, 1) GD_EXT(4, false, 1, 1)
-GD_EXT(1, true, 1, 1) GD_EXT(2, true, 1, 1) GD_EXT(4, true, 1, 1)
-GD_EXT(1, false, 0, 2) GD_EXT(2, false, 0, 2)
-GD_EXT(2, false, 2, 1)
+GD_EXT(1, 0, 0, 1) GD_EXT(2, 0, 0, 1) GD_EXT(4, 0, 0, 1)
+GD_EXT(1, 1, 0, 1) GD_EXT(2, 1, 0, 1) GD_EXT(4, 1, 0, 1)
+GD_EXT(1, 0, 1, 1) GD_EXT(2, 0, 1, 1) GD_EXT(4, 0, 1, 1)
+GD_EXT(1, 1, 1, 1) GD_EXT(2, 1, 1, 1) GD_EXT(4, 1, 1, 1)
+GD_EXT(4, 2, 0, 1) GD_EXT(4, 2, 1, 1)
+GD_EXT(1, 0, 0, 2) GD_EXT(2, 0, 0, 2)
+GD_EXT(2, 0, 2, 1)
 #undef GD_EXT
 __global__ void gd_exchange_kernel(const GdDevComplex *cxs, const int *group_base, int n_complex,
                                    int g_begin, int g_end, GdExchange ex, GdForceConst f,
@@ -87,15 +88,18 @@ struct ComplexInfo {
   int n_lig, n_prt, n_tmp, lna, pnp, pnp_pad, pnk, pos;
   int rep_offset, n_rep, k;
   int stream;
+  /* stored pieces of a split launch whose sums run in the points' order, by split count */
+  int pieces[GD_MAX_SPLITS + 1], hpieces[GD_MAX_SPLITS + 1];
   int types_uniform; /* every ligand conformer has the same atom types (two replicas per
                         thread share their atom's pair parameters) */
 };
 
 /* The shape of one launch of the Monte Carlo kernel: lanes per CTA (pack lanes per thread), points
  * per ring buffer and per FP32 sum (fold), splits per atom, point pairs in flight, the largest
- * replica count of a tile. */
+ * replica count of a tile, and the pieces of sums in the points' order (0: sums per split). */
 struct LaunchShape {
   int lanes, chunk, fold, split, unroll, pack, kmax;
+  int pieces = 0, hpieces = 0; /* GdMcArgs */
 };
 
 /* One chain of the fused loops: a contiguous range of (complex, protein conformer) blocks,
@@ -120,6 +124,7 @@ struct gd_ctx {
   gd_mc_params mc{};
   int n_complex = 0, n_rep = 0, n_groups = 0;
   int threads = 256, chunk = GD_CHUNK, fold = GD_CHUNK, unroll = 2, split = 1, num_sms = 148;
+  int pieces = 0, hpieces = 0; /* LaunchShape */
   int pack = 1; /* replicas per thread of the plain launches: the tile's lanes (threads) run on
                    threads / pack threads */
   int fill_threads = 0, fill_cap = 0; /* the last gd_set_tile in fill mode (threads > 0) */
@@ -268,14 +273,16 @@ struct WorkList {
 };
 /* the splits of a launch of these lists (1: none), and the replicas a tile then takes of each */
 int auto_split(const gd_ctx *c, const std::vector<WorkList> &w, std::vector<int> *k);
-/* a split launch: lanes for k replicas of lna atoms, the ring holding the whole protein */
-LaunchShape split_shape(int split, int k_lna, int kmax, int pnp_pad);
+/* A split launch of complex ci (-1: of all): lanes for k replicas of lna atoms, the ring holding the
+ * whole protein, sums in the points' order. False where shared memory does not hold their pieces;
+ * the shape then has sums per split. */
+bool split_shape(const gd_ctx *c, int ci, int split, int k_lna, int kmax, int pnp_pad,
+                 LaunchShape *s);
 int ensure_counters(gd_ctx *c, int n);
 /* the pinned host cursor of the graph launches (made on first use) */
 int ensure_cursor(gd_ctx *c);
 typedef void (*McKernel)(GdMcArgs, GdForceConst);
 /* kind: GD_KIND_* */
-McKernel mc_kernel(int unroll, int split, int kind = GD_KIND_PLAIN, int pack = 1);
 McKernel launch_kernel(const LaunchShape &s, int kind = GD_KIND_PLAIN);
 int launch_threads(const LaunchShape &s);
 int grid_for(gd_ctx *c, int n_tiles, const LaunchShape &s, int kind = GD_KIND_PLAIN);

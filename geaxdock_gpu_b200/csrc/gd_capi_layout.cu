@@ -7,6 +7,77 @@
 
 namespace gdc {
 
+namespace {
+
+/* The segments (masks) that each of S splits runs: the segments in their order, or, for partial
+ * sums per split, in the order of their number modulo S (so that every split has segments in every
+ * chunk), cut into S ranges of about equal work, work in units of one point pair; the splits that
+ * also have a short-range list, the restraints or the per-atom tail get less of it. */
+void split_masks(const int4 *segs, int nseg, int S, bool ordered, unsigned *masks) {
+  const int con = ordered ? 0 : S - 1, tail = ordered ? S - 1 : 0;
+  const int kind = ordered && S < 3 ? S - 1 : std::max(S - 2, 0);
+  const int mcs = S >= 4 ? S - 3 : ordered ? S - 1 : S == 2 ? 1 : 0;
+  std::vector<int> order;
+  for (int r = 0; r < (ordered ? 1 : S); ++r)
+    for (int sg = r; sg < nseg; sg += ordered ? 1 : S) order.push_back(sg);
+  auto cost = [&](int sg) {
+    const int n = (segs[sg].y - segs[sg].x + 1) >> 1;
+    return GD_COST_SEG + n + ((segs[sg].w & 4) ? n >> 2 : 0);
+  };
+  int total = 0;
+  for (int sg = 0; sg < nseg; ++sg) total += cost(sg);
+  const int target = (total + GD_COST_CON + GD_COST_KIND + GD_COST_MCS + GD_COST_TAIL) / S;
+  double room[GD_MAX_SPLITS], all = 0.0;
+  for (int p = 0; p < S; ++p) {
+    room[p] = std::max(1, target - (p == con ? GD_COST_CON : 0) - (p == kind ? GD_COST_KIND : 0) -
+                              (p == mcs ? GD_COST_MCS : 0) - (p == tail ? GD_COST_TAIL : 0));
+    all += room[p];
+    masks[p] = 0;
+  }
+  double before = 0.0;
+  for (int sg : order) {
+    const double at = (before + 0.5 * cost(sg)) * all / total;
+    int p = 0;
+    for (double end = room[0]; p < S - 1 && at >= end; end += room[++p]) {
+    }
+    masks[p] |= 1u << sg;
+    before += cost(sg);
+  }
+}
+
+/* GdDevComplex.split_plan of one conformer; the stored pieces by split count into x */
+void split_plan(const int4 *segs, int nseg, ComplexInfo &x, unsigned *plan) {
+  unsigned hseg = 0;
+  for (int sg = 0; sg < nseg; ++sg) hseg |= (segs[sg].w & 4) ? 1u << sg : 0u;
+  plan[GD_SPLIT_WORDS - 1] = hseg;
+  for (int S = 1; S <= GD_MAX_SPLITS; ++S) {
+    split_masks(segs, nseg, S, false, plan + GD_SPLIT_AT(S, 0));
+    unsigned *own = plan + GD_SPLIT_MASKS + GD_SPLIT_AT(S, 0);
+    split_masks(segs, nseg, S, true, own);
+    /* piece (sg, block b of GD_CHUNK slots) has number sg + b, among the hydrogen-bond ones (sg's
+     * rank among such segments) + b; those of split 0 come first and are not stored */
+    int p0 = -1, p1 = -1, h0 = -1, h1 = -1, rank = 0;
+    for (int sg = 0; sg < nseg; ++sg) {
+      const int first = segs[sg].x / GD_CHUNK, last = (segs[sg].y - 1) / GD_CHUNK;
+      const bool hb = (hseg >> sg) & 1u;
+      if (!((own[0] >> sg) & 1u)) {
+        if (p0 < 0) p0 = sg + first;
+        p1 = sg + last;
+        if (hb) {
+          if (h0 < 0) h0 = rank + first;
+          h1 = rank + last;
+        }
+      }
+      rank += hb ? 1 : 0;
+    }
+    plan[2 * GD_SPLIT_MASKS + S - 1] = (unsigned)std::max(p0, 0) | (unsigned)std::max(h0, 0) << 16;
+    x.pieces[S] = std::max(x.pieces[S], p0 < 0 ? 1 : p1 - p0 + 1);
+    x.hpieces[S] = std::max(x.hpieces[S], h0 < 0 ? 0 : h1 - h0 + 1);
+  }
+}
+
+}  // namespace
+
 int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1],
                    const gd_complex_desc &d, int ci, GdDevComplex &g) {
   const ComplexInfo &x = c->info[ci];
@@ -121,6 +192,12 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
     g.far_r = (float)(rfar + 0.01);
     g.far_inv_w = (float)(1.0 / bin_w);
   }
+  std::vector<unsigned> plan((size_t)d.n_prt * GD_SPLIT_WORDS, 0u);
+  std::fill(std::begin(c->info[ci].pieces), std::end(c->info[ci].pieces), 0);
+  std::fill(std::begin(c->info[ci].hpieces), std::end(c->info[ci].hpieces), 0);
+  for (int pc = 0; pc < d.n_prt; ++pc)
+    split_plan(&seg[(size_t)pc * GD_MAX_SEG], seg_count[pc], c->info[ci],
+               &plan[(size_t)pc * GD_SPLIT_WORDS]);
   const int PP = (max_slots + 3) & ~3;
   c->info[ci].pnp_pad = PP;
   g.pnp_pad = PP;
@@ -278,13 +355,14 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
   for (int t = 0; t < d.n_tmp; ++t) mb[t] = d.temp[t].minus_beta;
 
   unsigned char *p_lig_rank;
+  unsigned *p_plan;
   float4 *p_lig_pos; int2 *p_lig_meta; float *p_lig_center; float4 *p_pt_a, *p_pt_b;
   float4 *p_sr_a, *p_sr_b; int *p_sr_start;
   int4 *p_seg; int *p_seg_count; unsigned short *p_far_cnt; float4 *p_kde, *p_mcs; int *p_kde_start;
   float *p_mt, *p_psp, *p_mb;
   int *p_ref_start; float4 *p_ref_pts;
   if ((rc = upload(c, &p_lig_pos, lig_pos)) || (rc = upload(c, &p_lig_meta, lig_meta)) ||
-      (rc = upload(c, &p_lig_rank, lig_rank)) ||
+      (rc = upload(c, &p_lig_rank, lig_rank)) || (rc = upload(c, &p_plan, plan)) ||
       (rc = upload(c, &p_lig_center, lig_center)) || (rc = upload(c, &p_pt_a, pt_a)) ||
       (rc = upload(c, &p_pt_b, pt_b)) || (rc = upload(c, &p_sr_a, sr_a)) ||
       (rc = upload(c, &p_sr_b, sr_b)) || (rc = upload(c, &p_sr_start, sr_start)) ||
@@ -299,6 +377,7 @@ int layout_complex(gd_ctx *c, const gd_enepara *ff, const float (*thr)[GD_MAXTP1
   if (cudaStreamSynchronize(c->stream) != cudaSuccess)
     return fail(GD_ERR_CUDA, "upload failed: %s", cudaGetErrorString(cudaGetLastError()));
   g.lig_rank = p_lig_rank;
+  g.split_plan = p_plan;
   g.lig_pos = p_lig_pos; g.lig_meta = p_lig_meta; g.lig_center = p_lig_center;
   g.pt_a = p_pt_a; g.pt_b = p_pt_b; g.seg = p_seg; g.seg_count = p_seg_count;
   g.far_cnt = p_far_cnt;

@@ -132,6 +132,8 @@ extern "C" int gd_eval_energy_noalloc(gd_ctx *c, int ci, int prt_conf, int lig_c
   a.chunk = shape.chunk;
   a.fold = shape.fold;
   a.split = shape.split;
+  a.pieces = shape.pieces;
+  a.hpieces = shape.hpieces;
   if ((rc = set_kernel_attrs(shape))) return rc;
   const int grid = grid_for(c, n_tiles, shape);
   launch_kernel(shape)<<<grid, launch_threads(shape), smem_bytes(shape), c->stream>>>(a, c->fc);

@@ -128,6 +128,7 @@ int gd_set_tile(gd_ctx *c, int k, const gd_tile *t) {
   c->threads = T;
   c->chunk = c->fold = t->chunk_points;
   c->split = S;
+  c->pieces = c->hpieces = 0;
   c->fill_threads = t->threads;
   c->fill_cap = t->threads > 0 ? t->replicas_per_cta : 0;
   c->pack = P;
@@ -254,6 +255,7 @@ int gd_autotune(gd_ctx *c, const gd_tile *cand, int n_cand, int repeats, gd_tile
     c->fill_threads = keep_fill_threads;
     c->fill_cap = keep_fill_cap;
     c->tile_auto = keep_auto;
+    if (keep_auto) use_auto_tile(c);
     c->tile_gen += 1;
     build_tiles(c, 0, c->n_rep - 1, c->full_tiles);
     if (rc == GD_OK) rc = fail(GD_ERR_INVALID, "gd_autotune: no candidate fits this batch");

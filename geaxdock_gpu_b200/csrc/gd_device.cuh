@@ -57,6 +57,10 @@
 #define GD_MAX_TPB_SPLIT 512   /* threads per CTA of the split launches */
 /* work of the per-atom terms that a split's segments are balanced against, in units of one point
  * pair: a segment's own set-up, the contact list, the kind list, the restraints, the tail */
+#define GD_MAX_SPLITS 16
+#define GD_SPLIT_AT(S, sp) ((S) * ((S) - 1) / 2 + (sp))
+#define GD_SPLIT_MASKS GD_SPLIT_AT(GD_MAX_SPLITS + 1, 0)
+#define GD_SPLIT_WORDS (2 * GD_SPLIT_MASKS + GD_MAX_SPLITS + 1)
 #define GD_COST_SEG 8
 #define GD_COST_CON 70
 #define GD_COST_KIND 90
@@ -133,6 +137,12 @@ struct GdDevComplex {
   const long long *pg_base;   /* [n_prt] */
   float pg_org[3];
   float pg_rc, pg_rh;         /* the lists' radii around a cell's box: contacts, hydrophobic */
+  /* who runs which segments of a split launch (layout_complex), GD_SPLIT_WORDS per conformer: the
+   * segment masks of split sp of S at GD_SPLIT_AT(S, sp), for partial sums per split and (from
+   * GD_SPLIT_MASKS on) for sums in the points' order; then for S = 1.. the first stored piece (low
+   * half) and the first stored hydrogen-bond piece of the latter; last, the segments with a live
+   * hydrogen-bond term */
+  const unsigned *split_plan;
   const int4 *seg;            /* [n_prt*GD_MAX_SEG] */
   const int *seg_count;       /* [n_prt] */
   const float4 *kde;          /* [pnk] x, y, z, 0: sorted by type, in their given order within one */
@@ -230,6 +240,9 @@ struct GdDaEpi {
 /* What the Monte Carlo kernel is compiled for: plain steps and evaluations, delayed acceptance's
  * exact stage, the exchange groups left open (gd_exchange_group). */
 enum { GD_KIND_PLAIN = 0, GD_KIND_DA = 1, GD_KIND_EXCHANGE = 2 };
+/* How it treats an atom's work: one lane; several, each with partial sums; several, whose sums run
+ * in the points' order. */
+enum { GD_UNSPLIT = 0, GD_SPLIT_PARTIAL = 1, GD_SPLIT_ORDERED = 2 };
 
 /* The replica state that exchanges read and write, and their draws' seed. */
 struct GdExchange {
@@ -258,6 +271,9 @@ struct GdMcArgs {
   int chunk;                  /* protein points per shared-memory buffer (multiple of 4) */
   int fold;                   /* slots after which a segment's FP32 sums go to FP64 (divides chunk) */
   int split;                  /* lanes per ligand atom (protein split), >= 1 */
+  int pieces, hpieces;        /* split launches whose sums run in the points' order: stored pieces
+                                 per atom and sum, of them hydrogen-bond pieces (0: partial sums
+                                 per split, added in split order) */
   int move_kind;
   uint64_t seed;
   float move_scale[6];

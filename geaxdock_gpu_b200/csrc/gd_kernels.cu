@@ -618,49 +618,6 @@ __device__ __forceinline__ double restraints(const GdDevComplex &cx, int lig_con
   return elhm;
 }
 
-/* The segments that split sp of S runs, as a bit mask (computed by a whole warp): the segments in
- * the order of their number modulo S (so that every split has segments in every chunk) are cut
- * into S ranges of about equal work, work in units of one point pair; the splits that also have a
- * short-range list, the restraints or the per-atom tail get less of it. */
-__device__ __forceinline__ unsigned split_segments(const int4 *__restrict__ segs, int nseg, int sp,
-                                                   int S, int con_sp, int kind_sp, int mcs_sp,
-                                                   int lane) {
-  const int q = nseg / S, r = nseg - q * S;
-  int sg = 0, cost = 0;
-  if (lane < nseg) {
-    const int head = r * (q + 1);
-    const int c = lane < head ? lane / (q + 1) : r + (lane - head) / max(q, 1);
-    const int j = lane < head ? lane - c * (q + 1) : (lane - head) - (c - r) * max(q, 1);
-    sg = j * S + c;
-    const int4 g = __ldg(segs + sg);
-    const int n = (g.y - g.x + 1) >> 1;
-    cost = GD_COST_SEG + n + ((g.w & 4) ? n >> 2 : 0);
-  }
-  int sum = cost;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, sum, o);
-    if (lane >= o) sum += v;
-  }
-  const int total = __shfl_sync(0xffffffffu, sum, 31);
-  const int target = (total + GD_COST_CON + GD_COST_KIND + GD_COST_MCS + GD_COST_TAIL) / S;
-  auto room = [&](int p) {
-    return (float)max(1, target - (p == con_sp ? GD_COST_CON : 0) -
-                             (p == kind_sp ? GD_COST_KIND : 0) - (p == mcs_sp ? GD_COST_MCS : 0) -
-                             (p == 0 ? GD_COST_TAIL : 0));
-  };
-  float all = 0.0f;
-  for (int p = 0; p < S; ++p) all += room(p);
-  const float at = ((float)sum - 0.5f * (float)cost) * all / (float)max(total, 1);
-  int owner = 0;
-  float end = 0.0f;
-  for (int p = 0; p < S - 1; ++p) {
-    end += room(p);
-    owner += at >= end ? 1 : 0;
-  }
-  return __reduce_or_sync(0xffffffffu, lane < nseg && owner == sp ? 1u << sg : 0u);
-}
-
 /* One segment range of the pair loop, dispatched on the segment's flags (bit 2: live
  * hydrogen-bond term). */
 template <int UNROLL, int PACK, bool FAR, bool LAT = false>
@@ -847,16 +804,22 @@ __device__ __forceinline__ bool da_decide(const GdMcArgs &a, const GdDevComplex 
  * chunk two ahead. Every wait is bounded (globaltimer); a wait that runs out sets the error
  * word, the CTA leaves at the next step barrier after letting its copies in flight land.
  */
-template <int UNROLL, bool SPLIT, int KIND, int PACK>
-__global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
-                                  SPLIT ? 1 : GD_MIN_BLOCKS_PACK(UNROLL, PACK, KIND != GD_KIND_PLAIN))
+template <int UNROLL, int SPLITS, int KIND, int PACK>
+__global__ void __launch_bounds__(SPLITS ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
+                                  SPLITS ? 1 : GD_MIN_BLOCKS_PACK(UNROLL, PACK, KIND != GD_KIND_PLAIN))
     gd_mc_kernel(GdMcArgs a, GdForceConst f) {
+  constexpr bool SPLIT = SPLITS != GD_UNSPLIT, ordered = SPLITS == GD_SPLIT_ORDERED;
   constexpr bool DA = KIND == GD_KIND_DA, XCH = KIND == GD_KIND_EXCHANGE;
   static_assert(PACK == 1 || (PACK == 2 && !SPLIT && KIND == GD_KIND_PLAIN),
                 "two replicas per lane: plain modes with one lane per atom");
   extern __shared__ __align__(16) unsigned char smem[];
-  /* T: lanes of the tile (PACK per thread), the stride of the placed atoms and partials */
-  const int NT = blockDim.x, T = NT * PACK, tid = threadIdx.x, D = a.chunk;
+  /* Sums in the points' order (ordered): the splits run contiguous ranges of segments; split 0 adds
+   * its own up as the unsplit lanes do, the others store theirs piece by piece, and the pieces are
+   * then added in order. The result is the unsplit launch's, bit for bit; otherwise each split has
+   * partial sums, added in split order. */
+  /* T: the stride of the placed atoms and partials: the tile's lanes (PACK per thread), of one split
+   * when ordered */
+  const int NT = blockDim.x, T = ordered ? NT / a.split : NT * PACK, tid = threadIdx.x, D = a.chunk;
   uint64_t *bar = reinterpret_cast<uint64_t *>(smem);
   /* contact thresholds [ligand type][point type], then the ring buffers: buffer b holds D
    * slots as D/2 pairs in two float4 streams */
@@ -865,7 +828,10 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
   float4 *bpb = bpa + D;
   float4 *atoms = bpb + D;
   double *part = reinterpret_cast<double *>(atoms + T);
-  Slot *slots = reinterpret_cast<Slot *>(part + NQ * T);
+  /* the stored pieces: three planes each (vdw, ele, pmf), then the hydrogen-bond pieces */
+  double *pcs = part + NQ * T;
+  const int n_planes = ordered ? 3 * a.pieces + a.hpieces : 0;
+  Slot *slots = reinterpret_cast<Slot *>(pcs + n_planes * T);
   __shared__ int s_tile, s_abort, s_open;
   __shared__ int s_done[2];
   __shared__ unsigned s_issued[2];
@@ -996,9 +962,11 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
       rank = by_slot ? lo : hi;
     };
     take_lane(SPLIT);
-    /* the splits that run the short-range lists and the restraints (split 0: the far field, the
-     * per-atom tail) */
-    const int con_sp = S - 1, kind_sp = max(S - 2, 0), mcs_sp = S >= 4 ? S - 3 : S == 2 ? 1 : 0;
+    /* the splits that run the short-range lists, the restraints and the per-atom tail (split 0: the
+     * far field; with it, where sums run in order, the contact list, whose ele term comes first) */
+    const int con_sp = ordered ? 0 : S - 1, tail_sp = ordered ? S - 1 : 0;
+    const int kind_sp = ordered && S < 3 ? S - 1 : max(S - 2, 0);
+    const int mcs_sp = S >= 4 ? S - 3 : ordered ? S - 1 : S == 2 ? 1 : 0;
     /* ---- slot set-up (one thread per replica) ---- */
     bool roams = false;
     if (tid < k) {
@@ -1088,7 +1056,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
       const int lc = slots[sl_of[h]].lig_conf;
       l_of[h] = PACK == 1 && !by_slot ? cx.lig_rank[lc * L + rank] : rank;
       orig[h] = cx.lig_pos[lc * L + l_of[h]];
-      vl[h] = sp * A + sl_of[h] * L + l_of[h];
+      vl[h] = (ordered ? 0 : sp * A) + sl_of[h] * L + l_of[h];
     }
     /* atom types are the same in every conformer of a ligand when PACK is 2 (host-checked) */
     const int tl = cx.lig_meta[slots[sl_of[0]].lig_conf * L + l_of[0]].x;
@@ -1096,9 +1064,32 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
     const GdPairParam *pprow = a.pp + tl * GD_MAXTP1;
     const int4 *segs = cx.seg + pc * GD_MAX_SEG;
     const int nseg = cx.seg_count[pc];
-    const unsigned own =
-        SPLIT ? split_segments(segs, nseg, sp, S, con_sp, kind_sp, mcs_sp, lane) : 0u;
+    unsigned own = 0, hseg = 0;
+    int p0 = 0, h0 = 0; /* the first stored piece, of all and of the hydrogen-bond ones */
+    if constexpr (SPLIT) {
+      const unsigned *plan = cx.split_plan + (size_t)pc * GD_SPLIT_WORDS;
+      own = __ldg(plan + (ordered ? GD_SPLIT_MASKS : 0) + GD_SPLIT_AT(S, sp));
+      if (ordered) {
+        const unsigned first = __ldg(plan + 2 * GD_SPLIT_MASKS + S - 1);
+        p0 = first & 0xffffu;
+        h0 = first >> 16;
+        hseg = __ldg(plan + GD_SPLIT_WORDS - 1);
+        /* pieces that no segment has (at a block's end) stay zero */
+        for (int i = tid; i < n_planes * T; i += NT) pcs[i] = 0.0;
+      }
+    }
     bool aborted = false;
+    /* the lane's piece (sg, block blk): vdw, ele, pmf, hydrogen bonds */
+    auto store_piece = [&](int sg, int blk, int flags, double e0, double e1, double e2,
+                           double e3) {
+      if (!ok[0]) return;
+      double *w = pcs + 3 * (sg + blk - p0) * T + vl[0];
+      w[0] = e0;
+      w[T] = e1;
+      w[2 * T] = e2;
+      if (flags & 4)
+        pcs[(3 * a.pieces + __popc(hseg & ((1u << sg) - 1u)) + blk - h0) * T + vl[0]] = e3;
+    };
 
     /* A step may take three passes. Energies from the far fields differ from those of the pair
      * loop over every point in the last FP32 digits; a Metropolis decision that could hang on
@@ -1183,7 +1174,7 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
       /* each lane clears its own partials (the only ones the epilogue reads) */
 #pragma unroll
       for (int h = 0; h < PACK; ++h)
-        if (ok[h])
+        if (ok[h] && (!ordered || sp == 0))
 #pragma unroll
           for (int qi = 0; qi < NQ; ++qi) part[qi * T + vl[h]] = 0.0;
 
@@ -1218,10 +1209,12 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
             short_range_lists(cx, pc, cell, thr, psprow, f, ax[h], ay[h], az[h], con, kind, sr);
           else
             short_range(cx, pc, thr, psprow, f, ax[h], ay[h], az[h], sr);
-          part[1 * T + v] = (double)sr.ele;
-          part[3 * T + v] = (double)sr.psp;
-          part[8 * T + v] = (double)sr.ncon;
+          if (con) {
+            part[1 * T + v] = (double)sr.ele;
+            part[8 * T + v] = (double)sr.ncon;
+          }
           if (kind) {
+            part[3 * T + v] = (double)sr.psp;
             const double hpc2 = (sr.hsum - (double)f.hpl0[tl]) / (double)f.hpl1[tl];
             part[5 * T + v] = 0.5 * hpc2 * hpc2 - (double)f.hpl2[tl];
           }
@@ -1283,7 +1276,8 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
           const int c0 = ci * D, c1 = min(pnp_pad, c0 + D);
           /* blocks of `fold` slots, at whose ends a segment's sums go to FP64: the whole chunk, or
            * the default tile's chunks where the ring's are larger */
-          for (int b0 = c0; b0 < c1; b0 += a.fold) {
+          int blk = SPLIT ? c0 / a.fold : 0;
+          for (int b0 = c0; b0 < c1; b0 += a.fold, ++blk) {
             const int b1 = min(c1, b0 + a.fold);
             for (int sg = sg0; sg < nseg; ++sg) {
               const int4 g = segs[sg];
@@ -1301,7 +1295,10 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
                 il[h] = min(e, b1) - c0;
                 i1 = max(i1, il[h]);
               }
-              if (i0 >= i1) continue;
+              if (i0 >= i1) {
+                if (ordered && sp > 0) store_piece(sg, blk, g.w, 0.0, 0.0, 0.0, 0.0);
+                continue;
+              }
               const float4 *pr = reinterpret_cast<const float4 *>(pprow + g.z);
               const float4 q0 = __ldg(pr), q1 = __ldg(pr + 1), q2 = __ldg(pr + 2);
               Pair2 pq;
@@ -1345,6 +1342,13 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
               for (int h = 0; h < PACK; ++h) {
                 if (!ok[h]) continue;
                 const int v = vl[h];
+                if (ordered && sp > 0) {
+                  store_piece(sg, blk, g.w, (double)acc[h].vdw.x + (double)acc[h].vdw.y,
+                              (double)acc[h].ele.x + (double)acc[h].ele.y,
+                              (double)q1.y * ((double)acc[h].pmf.x + (double)acc[h].pmf.y),
+                              (double)acc[h].hdb.x + (double)acc[h].hdb.y);
+                  continue;
+                }
                 part[0 * T + v] += (double)acc[h].vdw.x + (double)acc[h].vdw.y;
                 part[1 * T + v] += (double)acc[h].ele.x + (double)acc[h].ele.y;
                 part[2 * T + v] += (double)q1.y * ((double)acc[h].pmf.x + (double)acc[h].pmf.y);
@@ -1370,13 +1374,13 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
         }
       }
 
-      /* ---- per-atom tail (split 0 of each atom): kde, rmsd, reference contacts ---- */
+      /* ---- per-atom tail (one split of each atom): kde, rmsd, reference contacts ---- */
 #pragma unroll
       for (int h = 0; h < PACK; ++h) {
         if (!ok[h] || aborted) continue;
         const int v = vl[h];
-        part[1 * T + v] *= (double)orig[h].w;
-        if (sp != 0) continue;
+        if (!ordered) part[1 * T + v] *= (double)orig[h].w;
+        if (sp != tail_sp) continue;
         float ks = 0.0f;
         /* the KDE points lie sorted by type, in their given order within a type: the atom sums
          * its own type's points only. Latency-bound (a chain of additions per atom): four loads
@@ -1409,13 +1413,30 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
       }
 
       if constexpr (SPLIT) {
-        /* each atom's partials of its splits, added in split order by all threads */
-        for (int i = tid; i < NQ * k * L; i += NT) {
-          const int q = i / (k * L);
-          double *p = part + q * T + (i - q * k * L);
-          double t = p[0];
-          for (int z = 1; z < S; ++z) t += p[z * A];
-          p[0] = t;
+        if constexpr (ordered) {
+          /* each atom's pieces added to split 0's sums in the points' order, a sum per thread */
+          for (int i = tid; i < 4 * k * L; i += NT) {
+            const int q = i / (k * L), at = i - q * k * L, js = at / L;
+            const bool hb = q == 3;
+            double *p = part + (hb ? 4 : q) * T + at;
+            const double *w = pcs + (hb ? 3 * a.pieces : q) * T + at;
+            const int n = hb ? a.hpieces : a.pieces, st = hb ? T : 3 * T;
+            const float charge =
+                q == 1 ? __ldg(&cx.lig_pos[slots[js].lig_conf * L + at - js * L].w) : 1.0f;
+            double t = p[0];
+#pragma unroll 16
+            for (int j = 0; j < n; ++j) t += w[j * st];
+            p[0] = q == 1 ? t * (double)charge : t;
+          }
+        } else {
+          /* each atom's partials of its splits, added in split order by all threads */
+          for (int i = tid; i < NQ * k * L; i += NT) {
+            const int q = i / (k * L);
+            double *p = part + q * T + (i - q * k * L);
+            double t = p[0];
+            for (int z = 1; z < S; ++z) t += p[z * A];
+            p[0] = t;
+          }
         }
         __syncthreads();
       }
@@ -1660,17 +1681,18 @@ __global__ void __launch_bounds__(SPLIT ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
   }
 }
 
-/* the kernel variants the host can launch: point pairs in flight per lane; protein split; plain
- * modes, the delayed-acceptance exact stage (mode 3) or the open exchange groups; replicas per
+/* the kernel variants the host can launch: point pairs in flight per lane; no split, partial sums
+ * per split, or split with sums in the points' order (the automatic shapes, four pairs); plain modes, the delayed-acceptance exact stage (mode 3) or the open exchange groups; replicas per
  * thread (two only for the plain modes without split) */
 #define GD_INST(U, S, K, P) \
   template __global__ void gd_mc_kernel<U, S, K, P>(GdMcArgs, GdForceConst);
-GD_INST(1, false, 0, 1) GD_INST(2, false, 0, 1) GD_INST(4, false, 0, 1)
-GD_INST(1, true, 0, 1) GD_INST(2, true, 0, 1) GD_INST(4, true, 0, 1)
-GD_INST(1, false, 1, 1) GD_INST(2, false, 1, 1) GD_INST(4, false, 1, 1)
-GD_INST(1, true, 1, 1) GD_INST(2, true, 1, 1) GD_INST(4, true, 1, 1)
-GD_INST(1, false, 0, 2) GD_INST(2, false, 0, 2)
-GD_INST(2, false, 2, 1)
+GD_INST(1, 0, 0, 1) GD_INST(2, 0, 0, 1) GD_INST(4, 0, 0, 1)
+GD_INST(1, 1, 0, 1) GD_INST(2, 1, 0, 1) GD_INST(4, 1, 0, 1)
+GD_INST(1, 0, 1, 1) GD_INST(2, 0, 1, 1) GD_INST(4, 0, 1, 1)
+GD_INST(1, 1, 1, 1) GD_INST(2, 1, 1, 1) GD_INST(4, 1, 1, 1)
+GD_INST(4, 2, 0, 1) GD_INST(4, 2, 1, 1)
+GD_INST(1, 0, 0, 2) GD_INST(2, 0, 0, 2)
+GD_INST(2, 0, 2, 1)
 #undef GD_INST
 
 /* ExchangeReplicas_d, one thread per (complex, protein conformer, ligand conformer) group of
