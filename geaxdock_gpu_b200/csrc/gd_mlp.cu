@@ -14,6 +14,7 @@
  * in MMA-fragment order for the one-kernel forward) after every update.
  */
 #include <algorithm>
+#include <climits>
 #include <cmath>
 
 #include "gd_mlp.cuh"
@@ -82,6 +83,7 @@ __global__ void __launch_bounds__(256) out_loss(const bf16 *__restrict__ A3,
 /* Reductions over the batch are split into chunks of SPLIT_ROWS rows: each chunk writes a
  * partial result, reduce_partials adds the chunks in a fixed order (deterministic). */
 constexpr int SPLIT_ROWS = 256;
+constexpr size_t PARTS_MAX = (size_t)256 << 20; /* bytes */
 
 /* Partial column sums of the output layer's two [rows][n] BF16 matrices, one per grid z:
  *   z = 0  A3 weighted per row by dy, with an extra column n that holds sum_r dy[r]
@@ -124,8 +126,9 @@ __global__ void __launch_bounds__(256) colsum_split(const bf16 *__restrict__ A3,
 }
 
 /* One job per parameter tensor: out[i] = sum_c part[c * count + i] in the order of the chunks, by
- * blocks [first, next job's first); the last block is the loss, the mean of e2. One launch at the
- * end for the seven sums and the loss (launches of their own between the GEMMs: 6 us each). */
+ * blocks [first, next job's first); the last block is the loss, the mean of e2 (if given). One
+ * launch at the end for the seven sums and the loss (launches of their own between the GEMMs: 6 us
+ * each). */
 struct ReduceJobs {
   static constexpr int N = 7;
   struct {
@@ -138,7 +141,7 @@ struct ReduceJobs {
 __global__ void __launch_bounds__(256) reduce_batch(const ReduceJobs jobs,
                                                     const float *__restrict__ e2, int rows,
                                                     float *__restrict__ loss) {
-  if (blockIdx.x == gridDim.x - 1) {
+  if (e2 && blockIdx.x == gridDim.x - 1) {
     __shared__ double sh[256];
     double s = 0.0;
 #pragma unroll 8
@@ -475,17 +478,26 @@ int mlp_loss_backward(Mlp &n, int rows, const float *t, cudaStream_t s) {
   int rc = hidden_forward(n, rows, true, s);
   if (rc) return rc;
   /* batch reductions in chunks of SPLIT_ROWS rows and tiles of 128, whose partials are added in a
-   * fixed order at the end: a part of P for each */
+   * fixed order: a part of P for each, all added at the end, while they take at most PARTS_MAX
+   * together (112,000 rows at H = 256); past that one after the other in a buffer that holds the
+   * largest, so that the memory per row of a large batch is less than half. The six launches more
+   * are 1 % of such a pass. */
   const int S = (M + SPLIT_ROWS - 1) / SPLIT_ROWS, T = (M + 127) / 128;
-  size_t need = 0;
-  auto part = [&](size_t count) {
-    const size_t at = need;
-    need += (count + 63) & ~(size_t)63;
+  size_t need = 0, largest = 0;
+  auto part = [&](size_t count, bool beside = false) {
+    const size_t at = need, size = (count + 63) & ~(size_t)63;
+    need += size;
+    largest = beside ? largest + size : std::max(largest, size);
     return at;
   };
-  const size_t p_w1 = part((size_t)S * GD_MLP_IN * H), p_w2 = part((size_t)S * H * H),
-               p_w3 = part((size_t)S * H * H), p_w4 = part((size_t)S * (H + 1)),
-               p_b3 = part((size_t)S * H), p_b2 = part((size_t)T * H), p_b1 = part((size_t)T * H);
+  size_t p_w4 = part((size_t)S * (H + 1)), p_b3 = part((size_t)S * H, true),
+         p_w1 = part((size_t)S * GD_MLP_IN * H), p_w2 = part((size_t)S * H * H),
+         p_w3 = part((size_t)S * H * H), p_b2 = part((size_t)T * H), p_b1 = part((size_t)T * H);
+  const bool together = need * sizeof(float) <= PARTS_MAX;
+  if (!together) {
+    need = largest; /* w4 and b3 come from one launch, side by side */
+    p_w1 = p_w2 = p_w3 = p_b1 = p_b2 = 0;
+  }
   if (need > n.p_cap) {
     if (n.P) cudaFree(n.P);
     n.P = nullptr;
@@ -498,6 +510,17 @@ int mlp_loss_backward(Mlp &n, int rows, const float *t, cudaStream_t s) {
   auto reduce = [&](size_t at, int chunks, int count, float *out) {
     jobs.job[n_jobs++] = {n.P + at, out, chunks, count, red_blocks};
     red_blocks += blocks(count);
+  };
+  float *e2 = n.C;
+  /* adds up the jobs so far; the last time with the loss */
+  auto add_up = [&](bool last) {
+    for (int q = n_jobs; q < ReduceJobs::N; ++q) jobs.job[q].first = INT_MAX;
+    reduce_batch<<<red_blocks + (last ? 1 : 0), 256, 0, s>>>(jobs, last ? e2 : nullptr, rows,
+                                                             n.loss);
+    n_jobs = red_blocks = 0;
+  };
+  auto stage_done = [&] {
+    if (!together) add_up(false);
   };
   /* the embedding's gradient is scattered, b4 is padded to four; the rest is written whole */
   cudaMemsetAsync(n.grad + n.L.b4, 0, (n.L.total - n.L.b4) * 4, s);
@@ -534,26 +557,28 @@ int mlp_loss_backward(Mlp &n, int rows, const float *t, cudaStream_t s) {
   };
   bf16 *Dc = n.D, *Dn = n.D2;
   /* output layer and loss: dZ3, dw4 = A3^T dy, db4 = sum dy (b4 follows w4 in theta), db3 */
-  float *e2 = n.C;
   out_loss<<<blocks((size_t)M * 32), 256, 0, s>>>(n.A3, n.Z3, n.theta + n.L.w4, n.theta + n.L.b4, t,
                                                   rows, M, H, n.y, n.dy, e2, Dc);
   colsum_split<<<dim3((H + 32) / 32, S, 2), 256, 0, s>>>(n.A3, n.dy, Dc, M, H, n.P + p_w4,
                                                          n.P + p_b3);
   reduce(p_w4, S, H + 1, n.grad + n.L.w4);
   reduce(p_b3, S, H, n.grad + n.L.b3);
+  stage_done();
   /* layer 3: dW3 = A2^T dZ3, dZ2 with db2 */
-  if ((rc = weight_grad(n.A2, H, Dc, p_w3, n.grad + n.L.w3)) ||
-      (rc = input_grad(Dc, n.L.w3, n.Z2, Dn, p_b2, n.grad + n.L.b2)))
-    return rc;
+  if ((rc = weight_grad(n.A2, H, Dc, p_w3, n.grad + n.L.w3))) return rc;
+  stage_done();
+  if ((rc = input_grad(Dc, n.L.w3, n.Z2, Dn, p_b2, n.grad + n.L.b2))) return rc;
+  stage_done();
   std::swap(Dc, Dn);
   /* layer 2: dW2, dZ1 with db1 */
-  if ((rc = weight_grad(n.A1, H, Dc, p_w2, n.grad + n.L.w2)) ||
-      (rc = input_grad(Dc, n.L.w2, n.Z1, Dn, p_b1, n.grad + n.L.b1)))
-    return rc;
+  if ((rc = weight_grad(n.A1, H, Dc, p_w2, n.grad + n.L.w2))) return rc;
+  stage_done();
+  if ((rc = input_grad(Dc, n.L.w2, n.Z1, Dn, p_b1, n.grad + n.L.b1))) return rc;
+  stage_done();
   std::swap(Dc, Dn);
   /* layer 1: dW1 = X^T dZ1 (64 x H); dX = dZ1 W1^T (FP32) for the embedding */
   if ((rc = weight_grad(n.X, GD_MLP_IN, Dc, p_w1, n.grad + n.L.w1))) return rc;
-  reduce_batch<<<red_blocks + 1, 256, 0, s>>>(jobs, e2, rows, n.loss);
+  add_up(true);
   if (n.L.n_emb) {
     UmmaEpilogue e{};
     e.kind = UMMA_F32;
