@@ -569,7 +569,10 @@ __global__ void seg_of_kernel(const Seg *__restrict__ seg, int *__restrict__ seg
 
 /* One block of device memory for all of a call's arrays, each at a 256-byte boundary: sized in a
  * first round of take() calls, which return offsets, and made by alloc(). (Some twenty
- * cudaMalloc and cudaFree a call took 8-10 ms of host time, now and then 100 ms and more.) */
+ * cudaMalloc and cudaFree a call took 8-10 ms of host time, now and then 100 ms and more.) The pool
+ * keeps what it is given back, so a block past POOL_MAX comes from the driver and goes back to it:
+ * a call that large runs for tens of milliseconds, its cudaMalloc for about one. */
+constexpr size_t POOL_MAX = (size_t)64 << 20;
 struct Arena {
   char *base = nullptr;
   size_t used = 0;
@@ -585,7 +588,7 @@ struct Arena {
     return reinterpret_cast<T *>(base + off);
   }
   cudaError_t alloc(void *pool, cudaStream_t st) {
-    pooled = pool != nullptr;
+    pooled = pool != nullptr && used <= POOL_MAX;
     return pooled ? cudaMallocFromPoolAsync(reinterpret_cast<void **>(&base), used,
                                             (cudaMemPool_t)pool, st)
                   : cudaMalloc(reinterpret_cast<void **>(&base), used);
