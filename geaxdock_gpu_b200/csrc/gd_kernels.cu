@@ -667,13 +667,13 @@ __device__ __forceinline__ unsigned gd_exchange_group(const GdDevComplex &cx, in
   const int p = lg / nl, l = lg - p * nl, r0 = cx.rep_offset + nt * nl * p + l;
   const bool certify = cx.ff_tab != nullptr;
   const float cert = certify ? cx.ff_cert[lg] : 0.0f; /* lg = p n_lig + l */
-  int temps[GD_MAXTMP], orders[GD_MAXTMP];
+  short temps[GD_MAXTMP], orders[GD_MAXTMP];
   float en[GD_MAXTMP], tol[GD_MAXTMP];
   for (int t = 0; t < nt; ++t) {
     const int r = r0 + nl * t;
-    temps[t] = __ldcg(&x.replica[r].idx_tmp);
+    temps[t] = (short)__ldcg(&x.replica[r].idx_tmp);
     en[t] = __ldcg(x.etotal + r);
-    orders[temps[t]] = t;
+    orders[temps[t]] = (short)t;
     if (certify) {
       gd_energy e;
 #pragma unroll
@@ -707,7 +707,7 @@ __device__ __forceinline__ unsigned gd_exchange_group(const GdDevComplex &cx, in
       }
     }
     if (acc) {
-      const int tt = temps[o1];
+      const short tt = temps[o1];
       temps[o1] = temps[o2];
       temps[o2] = tt;
       taken |= 1u << pair;
