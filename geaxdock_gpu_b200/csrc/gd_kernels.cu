@@ -26,7 +26,9 @@
  *   Accept_d (src/kernel_cuda_l2_accept.cu:13-46), RecordLigand_d
  *   (src/kernel_cuda_l3_util.cu:74-106) in the per-replica epilogue run by one warp per slot.
  * gd_exchange_kernel: ExchangeReplicas_d (src/kernel_cuda_l1_exchangereplicas.cu:27-77), one
- * thread per (protein conformer, ligand conformer) group instead of one thread for all.
+ * thread per (protein conformer, ligand conformer) group instead of one thread for all; groups
+ * that it, or the exchange fused into gd_mc_kernel, leaves open for the far fields' rounding are
+ * exchanged by gd_mc_kernel's GD_KIND_EXCHANGE form.
  */
 #include <cuda_runtime.h>
 
@@ -949,9 +951,9 @@ __global__ void __launch_bounds__(SPLITS ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
      * steps: moves of 0.1 A 6.60 / 6.76 / 6.56, of 2 A 9.33 / 8.36 / 8.38, of 6 A 10.66 / 9.97 /
      * 9.93 (six replicas a CTA and four pairs in flight 9.86 / 9.24 / 9.22); lines at 8 and 11 A
      * and at the ligand's radius are up to 3 % slower at 2 A. Delayed acceptance's tiles, of one
-     * step each, keep to the ranks (by slot 28.9 -> 30.2 ms for 50 steps at 0.1 A). The warps' place in the CTA goes
-     * round with the tile, so that the tiles an SM holds (about GD_NUM_SMS apart) load its four
-     * schedulers alike. Split lanes keep the slots' order (2 % faster there). */
+     * step each, keep to the ranks (by slot 28.9 -> 30.2 ms for 50 steps at 0.1 A). The warps'
+     * place in the CTA goes round with the tile, so that the tiles an SM holds (about GD_NUM_SMS
+     * apart) load its four schedulers alike. Split lanes keep the slots' order (2 % faster there). */
     const int wr = SPLIT ? warp - sp * (A >> 5) : (warp + t + t / GD_NUM_SMS) % nwarps;
     const int ai = wr * 32 + lane;
     const bool active = ai < kp * L;
