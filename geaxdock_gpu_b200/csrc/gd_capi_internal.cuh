@@ -342,6 +342,9 @@ int build_pocket_lists(gd_ctx *c, std::vector<GdDevComplex> &dcx);
  * that is free when the context has all it needs ---- */
 int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs,
                      std::vector<GdDevComplex> &dcx);
+/* Distance from the pocket centre beyond which a complex's points are mostly fields, given memory
+ * for them (infinity: no tables for this force field and protein). */
+double field_reach(const gd_enepara *ff, const gd_complex_desc &d);
 
 /* ---- allocation-free pose evaluation (gd_capi_noalloc.cu) ---- */
 int noalloc_prepare(int device);

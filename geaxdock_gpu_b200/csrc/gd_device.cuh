@@ -66,6 +66,7 @@
 #define GD_COST_KIND 90
 #define GD_COST_MCS 40
 #define GD_COST_TAIL 40
+#define GD_COST_FAR 40
 #define GD_SLOT_BYTES 252      /* shared-memory bytes per replica slot (sizeof gd::Slot) */
 /* A decision on field-based energies stands when it is the same above and below by what the fields
  * may change both poses' energies: GD_CERT of a pose's weighted terms' magnitudes (the rounding of

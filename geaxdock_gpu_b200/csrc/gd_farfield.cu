@@ -259,6 +259,29 @@ static bool ff_radii(const gd_enepara *ff, double *r_f, double *r_hdb) {
   return true;
 }
 
+/* Complexes worth it: at least a quarter of the points lie beyond the far radius of a cell that
+ * reaches 10 A (with 19 % beyond, 1,500 points, a step got slower by the evaluation's latency; with
+ * 60 %, 3,000 points, faster). */
+static bool field_worth(const gd_complex_desc &d, double r_f) {
+  const size_t n = (size_t)d.n_prt * d.pnp;
+  size_t beyond = 0;
+  const double lim = (10.0 + r_f) * (10.0 + r_f);
+  for (size_t i = 0; i < n; ++i) {
+    const double x = (double)d.prt_x[i] - d.pocket_center[0],
+                 y = (double)d.prt_y[i] - d.pocket_center[1],
+                 z = (double)d.prt_z[i] - d.pocket_center[2];
+    beyond += x * x + y * y + z * z > lim ? 1 : 0;
+  }
+  return beyond * 4 >= n;
+}
+
+double field_reach(const gd_enepara *ff, const gd_complex_desc &d) {
+  double r_f, r_hdb[GD_MAXTP1];
+  if (!ff_radii(ff, &r_f, r_hdb) || !field_worth(d, r_f))
+    return std::numeric_limits<double>::infinity();
+  return 10.0 + r_f;
+}
+
 /* Appends ff_cert of a complex (GD_CERT_ELE, GD_CERT_FAR), by protein and ligand conformer. */
 static void certainty(const gd_ctx *c, const gd_enepara *ff, const gd_complex_desc &d, double r_f,
                       std::vector<float> &out) {
@@ -326,9 +349,7 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
                      std::vector<GdDevComplex> &dcx) {
   double r_f, r_hdb[GD_MAXTP1];
   if (!ff_radii(ff, &r_f, r_hdb)) return GD_OK;
-  /* complexes worth it: at least a quarter of the points lie beyond the far radius of a cell
-   * that reaches 10 A (with 19 % beyond, 1,500 points, a step got slower by the evaluation's
-   * latency; with 60 %, 3,000 points, faster); grouped by protein */
+  /* the complexes worth it, grouped by protein */
   struct Group { std::vector<int> members; bool used[GD_MAXTP2] = {}; };
   std::vector<std::unique_ptr<Group>> groups;
   std::map<uint64_t, std::vector<Group *>> by_hash;
@@ -339,16 +360,7 @@ int build_far_fields(gd_ctx *c, const gd_enepara *ff, const gd_complex_desc *cxs
     for (Group *q : by_hash[h])
       if (same_protein(cxs[q->members[0]], d)) g = q;
     if (!g) {
-      const size_t n = (size_t)d.n_prt * d.pnp;
-      size_t beyond = 0;
-      const double lim = (10.0 + r_f) * (10.0 + r_f);
-      for (size_t i = 0; i < n; ++i) {
-        const double x = (double)d.prt_x[i] - d.pocket_center[0],
-                     y = (double)d.prt_y[i] - d.pocket_center[1],
-                     z = (double)d.prt_z[i] - d.pocket_center[2];
-        beyond += x * x + y * y + z * z > lim ? 1 : 0;
-      }
-      if (beyond * 4 < n) continue;
+      if (!field_worth(d, r_f)) continue;
       groups.push_back(std::make_unique<Group>());
       g = groups.back().get();
       by_hash[h].push_back(g);

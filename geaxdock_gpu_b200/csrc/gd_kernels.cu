@@ -814,6 +814,7 @@ __global__ void __launch_bounds__(SPLITS ? GD_MAX_TPB_SPLIT : GD_MAX_TPB / PACK,
   constexpr bool DA = KIND == GD_KIND_DA, XCH = KIND == GD_KIND_EXCHANGE;
   static_assert(PACK == 1 || (PACK == 2 && !SPLIT && KIND == GD_KIND_PLAIN),
                 "two replicas per lane: plain modes with one lane per atom");
+  if (XCH && __ldcg(a.x_open) == 0) return; /* the usual case: no group is open */
   extern __shared__ __align__(16) unsigned char smem[];
   /* Sums in the points' order (ordered): the splits run contiguous ranges of segments; split 0 adds
    * its own up as the unsplit lanes do, the others store theirs piece by piece, and the pieces are
